@@ -453,11 +453,14 @@ struct HllArg {
   ModelArg m;
   Quad6D qd;
 };
+constexpr int kHllBlock = 64;
 // EL, ER: the caller's wave speeds of the left and right cell ([12][n] each, the
 // eigvals[1], eigvals[2] of NumFluxes.jl:90-91), or null for the cells' own.
 __global__ void k_hll(HllArg a, const double* Ql, const double* Qr, const double* EL, const double* ER, double* DMo,
                       double* DPo, int64_t n) {
-  IDX double ql[30], qr[30], fl[30], fr[30], dm[30], dp[30];
+  const int64_t i = (int64_t)blockIdx.x * kHllBlock + threadIdx.x;
+  if (i >= n) return;
+  double ql[30], qr[30], fl[30], fr[30], dm[30], dp[30];
   LD(ql, Ql, 30);
   LD(qr, Qr, 30);
   flux2(a.m.e, ql, fl);
@@ -497,7 +500,7 @@ extern "C" int hyp_eval_hll(const hyp_config* cfg, const double* Ql, const doubl
   HllArg a{model_arg(cfg), gauss_legendre6()};
   return run(n, {{Ql, nullptr, 30}, {Qr, nullptr, 30}, {nullptr, dm, 30}, {nullptr, dp, 30}},
              [](int64_t n, double** d, const void* p) {
-               k_hll<<<(unsigned)((n + 63) / 64), 64>>>(*(const HllArg*)p, d[0], d[1], nullptr, nullptr, d[2], d[3],
+               k_hll<<<(unsigned)((n + kHllBlock - 1) / kHllBlock), kHllBlock>>>(*(const HllArg*)p, d[0], d[1], nullptr, nullptr, d[2], d[3],
                                                         n);
              },
              &a);
@@ -510,7 +513,7 @@ extern "C" int hyp_eval_hll_eigvals(const hyp_config* cfg, const double* Ql, con
              {{Ql, nullptr, 30}, {Qr, nullptr, 30}, {eig_l, nullptr, 12}, {eig_r, nullptr, 12}, {nullptr, dm, 30},
               {nullptr, dp, 30}},
              [](int64_t n, double** d, const void* p) {
-               k_hll<<<(unsigned)((n + 63) / 64), 64>>>(*(const HllArg*)p, d[0], d[1], d[2], d[3], d[4], d[5], n);
+               k_hll<<<(unsigned)((n + kHllBlock - 1) / kHllBlock), kHllBlock>>>(*(const HllArg*)p, d[0], d[1], d[2], d[3], d[4], d[5], n);
              },
              &a);
 }
