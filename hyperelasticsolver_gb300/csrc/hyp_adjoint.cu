@@ -366,7 +366,6 @@ extern "C" int hyp_adjoint(hyp_ctx* c, const double* dL_dQ_final, double* dL_dQ0
   ACK(cudaMemsetAsync(t->seg_t, 0, (size_t)(t->K + 1) * sizeof(double), c->stream));
   const double dx = c->cfg.x_length / (double)n;
   const double inf = INFINITY;
-  const unsigned egrid = (unsigned)((n + kBlock - 1) / kBlock);
   int cur = 0;
   t->ms_recompute = t->ms_adjoint = 0.f;
   const int n_seg = (t->n_steps + t->K - 1) / t->K;
@@ -381,16 +380,10 @@ extern "C" int hyp_adjoint(hyp_ctx* c, const double* dL_dQ_final, double* dL_dQ0
       double* Qk = t->seg_Q + (size_t)k * 14 * n;
       double* Fk = t->seg_F + (size_t)k * kNFlux1 * n;
       double* lk = t->seg_lam + (size_t)k * n;
-      cell1_f64_kernel<<<egrid, kBlock, 0, c->stream>>>(Qk, n, c->eos[0], Fk, lk, &t->seg_lmax[k], &t->seg_t[k], inf,
-                                                        c->st);
-      ACK(cudaGetLastError());
-      if (k + 1 < L) {
-        update1_f64_kernel<<<egrid, kBlock, 0, c->stream>>>(Qk, Qk + 14 * n, n, Fk, lk, &t->seg_lmax[k],
-                                                            &t->seg_lmax[k + 1], &t->seg_t[k], &t->seg_t[k + 1],
-                                                            t->seg_steps, inf, c->cfg.cfl, dx, c->cfg.flux,
-                                                            c->cfg.bc);
-        ACK(cudaGetLastError());
-      }
+      ACK(launch_cell1(c->stream, Qk, n, c->eos[0], Fk, lk, &t->seg_lmax[k], &t->seg_t[k], inf, c->st));
+      if (k + 1 < L)
+        ACK(launch_update1(c->stream, Qk, Qk + 14 * n, n, Fk, lk, &t->seg_lmax[k], &t->seg_lmax[k + 1], &t->seg_t[k],
+                           &t->seg_t[k + 1], t->seg_steps, inf, c->cfg.cfl, dx, c->cfg.flux, c->cfg.bc));
     }
     ACK(cudaEventRecord(t->ev[1], c->stream));
     // adjoint steps a + L - 1 .. a

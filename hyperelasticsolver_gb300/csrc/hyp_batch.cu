@@ -25,6 +25,7 @@
 #include <vector>
 #include "hyp_internal.cuh"
 #include "hyp_mixed_tile.cuh"
+#include "hyp_step64.cuh"
 
 namespace hyp {
 
@@ -173,47 +174,26 @@ __global__ void __launch_bounds__(kBlock) batch_join_kernel(const float* __restr
 }
 
 // ---- FP64 ----------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) batch_f64_cell_kernel(const double* __restrict__ Q, int64_t n, EosC e,
-                                                                double* __restrict__ F, double* __restrict__ lam,
-                                                                const TileDesc* __restrict__ tiles, int ntiles,
-                                                                int tile_cells, BatchDev b, int par, double t_end,
-                                                                unsigned long long* slot_base, DevState* S) {
-  const int P = b.P;
-  for (int tix = blockIdx.x; tix < ntiles; tix += gridDim.x) {
-    const TileDesc d = tiles[tix];
-    if (!(b.t[par * P + d.problem] < t_end)) continue;
-    double l = 0.0;
-    for (int64_t i = d.first + threadIdx.x; i < d.first + tile_cells && i < d.hi; i += kBlock) {
-      double q[14];
-#pragma unroll
-      for (int v = 0; v < 14; ++v) q[v] = Q[v * n + i];
-      Prim Pm;
-      int st = cons_to_prim(e, 1.0, q + 1, q[4], q + 5, Pm);
-      StressC c = stress_coeffs(e, Pm.k, Pm.w, Pm.xm1);
-      double f[14], s0[3];
-      phase_flux(e, 1.0, Pm, c, f, s0);
-      const double li = fabs(Pm.u[0]) + phase_cmax(e, Pm, c);
-      if (!(li <= 1.79e308)) st |= HYP_CELL_NONFINITE;
-#pragma unroll
-      for (int v = 0; v < 14; ++v) {
-        const int sl = flux_slot1(v);
-        if (sl >= 0) F[sl * n + i] = f[v];
-      }
-      lam[i] = li;
-      if (st) mixed_record_err(S, st, i);
-      l = fmax(l, li);
-    }
-    __shared__ double red[kBlock / 32];
-    for (int o = 16; o > 0; o >>= 1) l = fmax(l, __shfl_xor_sync(0xffffffffu, l, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double m = red[0];
-      for (int w = 1; w < kBlock / 32; ++w) m = fmax(m, red[w]);
-      atomicMax(&slot_base[d.problem], (unsigned long long)__double_as_longlong(m));
-    }
-    __syncthreads();
+// One tile per block: the single problem's cell pass (cell1_pass) and the tile's
+// maximum into its problem's slot.
+template <int kDef>
+__global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* __restrict__ Q, int64_t n, EosC e,
+                                                                  Eos64 k, double* __restrict__ F,
+                                                                  double* __restrict__ lam,
+                                                                  const TileDesc* __restrict__ tiles, int tile_cells,
+                                                                  BatchDev b, int par, double t_end,
+                                                                  unsigned long long* slot_base, DevState* S) {
+  const TileDesc d = tiles[blockIdx.x];
+  if (!(b.t[par * b.P + d.problem] < t_end)) return;
+  unsigned long long top = 0ull;
+  double l = 0.0;
+  for (int64_t i = d.first + threadIdx.x; i < d.first + tile_cells && i < d.hi; i += kBlock64) {
+    l = cell1_pass<kDef>(Q, n, i, e, k, F, lam, S);
+    const unsigned long long lb = is_nan64(l) ? 0ull : (unsigned long long)bits_of(l);
+    top = lb > top ? lb : top;
   }
+  const unsigned long long m = block_max_bits<kBlock64>(of_bits((long long)top));
+  if (threadIdx.x == 0) atomicMax(&slot_base[d.problem], m);
 }
 
 // One tile of kBlock cells per block iteration (tile_cells == kBlock for the FP64
@@ -416,9 +396,11 @@ static int enqueue_batch_step(hyp_batch* b, long long k, double t_end) {
                                        fl, bc, b->st);
     BCK(e);
   } else {
-    batch_f64_cell_kernel<<<b->grid, kBlock, 0, b->stream>>>(b->Q[par], b->total, b->eos, b->F, b->lam, b->tiles,
-                                                             b->ntiles, b->tile_cells, b->b, par, t_end,
-                                                             b->b.slots + (size_t)par * b->P, b->st);
+    const Eos64 k64 = make_eos64(b->eos);
+    auto cell = b->eos.default_exp ? batch_f64_cell_kernel<1> : batch_f64_cell_kernel<0>;
+    cell<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->total, b->eos, k64, b->F, b->lam, b->tiles,
+                                                b->tile_cells, b->b, par, t_end, b->b.slots + (size_t)par * b->P,
+                                                b->st);
     BCK(cudaGetLastError());
     batch_f64_update_kernel<<<b->grid, kBlock, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->F, b->lam,
                                                                b->tiles, b->ntiles, b->tile_cells, b->b, par, t_end,

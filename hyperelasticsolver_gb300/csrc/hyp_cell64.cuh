@@ -1,0 +1,334 @@
+// hyp_cell64.cuh -- one phase of one cell for the FP64 step, in the fewest FP64
+// instructions.
+//
+// What bounds the FP64 kernels on GB300 is one number. Each of an SM's four
+// schedulers issues an FP64 instruction (add, multiply, fused multiply-add, compare,
+// FP32 <-> FP64 conversion) over 64 cycles, whether 1 or 32 lanes are active and
+// whether or not it depends on the one before: measured 64.2 cycles per warp
+// instruction for one dependent chain per scheduler and for eight independent ones, a
+// divide about 9 such slots, a square root about 10. In those 64 cycles the scheduler
+// issues 64 FP32, integer or special-function instructions. So the time of a pass is
+// (FP64 instructions per cell) x 64 cycles, no occupancy or overlap changes it, and
+// everything below trades FP64 instructions for other ones:
+//
+//  - The closed forms use H = G^2 = i1 G - i2 I + p M with M = A A^T = G^-1
+//    (Cayley-Hamilton, p = det G), so G^2 is never formed. With b = b0sq/2 p^(beta/2)
+//    and a = 2/3 b i1, row 1 of the stress is s0 = -2 rho w,
+//      w_j = a G0j + b p M0j + (E3 p - b i2) [j = 0],
+//    and along dA = e_j A[0,:] the derivatives of M's row 1 are dM_0i = [j=0] M_0i +
+//    M_00 [i=j]: the acoustic tensor (n = e1) collapses to Omega = 2 O with
+//      O_ij = f G0i G0j + a G_ij - b p M00 [i=j]   (i, j >= 1),  f = 4/3 b,
+//      O_0j = f G00 G0j + (beta + 2) w_j           (j >= 1),
+//      O_00 = f G00^2 + w_0 + (2 beta + 2)(w_0 - E3 p) + gamma T2 + beta T3
+//             + alpha kE3a Pa (2 Pa - 1),
+//    E3 p = T1 + T2 + T3 its bulk, thermal and shear terms. O is symmetric, so six
+//    entries and the characteristic polynomial of a symmetric matrix do.
+//  - Nothing is scaled that need not be: with R = alpha rho A as stored, N = R R^T and
+//    its cofactors C, one factor each takes them to G and p M, and the flux of rho A
+//    and its non-conservative products need R alone.
+//  - Reciprocals and square roots start from rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64
+//    (special-function instructions, measured error 1e-6) and take one third-order step:
+//    3 slots for a reciprocal, 5 for a (reciprocal) square root, to about an ulp.
+//  - The spectral radius starts from FP32 roots (conversions done on the integer pipe)
+//    and takes two steps with the FP32 slope, enough when the top root stands well
+//    clear; the general eigen-solve is kept for the rest.
+//  - Range and NaN checks compare bit patterns.
+//
+// Per cell 168 FP64 instructions by this count, where the forms of hyp_physics.cuh
+// (which the adjoint and the function-level evaluators use) execute 379; the two agree
+// to a few ulps (tests/test_cell64_host.py).
+#pragma once
+#include <string.h>
+#include "hyp_physics.cuh"
+
+namespace hyp {
+
+HYP_HD long long bits_of(double x) {
+#ifdef __CUDA_ARCH__
+  return __double_as_longlong(x);
+#else
+  long long b;
+  memcpy(&b, &x, sizeof b);
+  return b;
+#endif
+}
+HYP_HD double of_bits(long long b) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double(b);
+#else
+  double x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+HYP_HD unsigned bits_of_f(float x) {
+#ifdef __CUDA_ARCH__
+  return __float_as_uint(x);
+#else
+  unsigned b;
+  memcpy(&b, &x, sizeof b);
+  return b;
+#endif
+}
+HYP_HD float of_bits_f(unsigned b) {
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(b);
+#else
+  float x;
+  memcpy(&x, &b, sizeof x);
+  return x;
+#endif
+}
+
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+HYP_HD bool is_nan64(double x) { return (bits_of(x) & 0x7fffffffffffffffll) > kInfBits; }
+HYP_HD bool is_finite64(double x) { return (bits_of(x) & 0x7fffffffffffffffll) < kInfBits; }
+HYP_HD bool is_positive64(double x) { return bits_of(x) > 0 && bits_of(x) <= kInfBits; }  // x > 0, NaN: no
+// x < t for t < 0, NaN: no: a negative double's bit pattern, unsigned, grows with its size
+HYP_HD bool below_negative64(double x, double t) {
+  return (unsigned long long)bits_of(x) > (unsigned long long)bits_of(t) && !is_nan64(x);
+}
+
+// FP64 -> FP32 (truncated; under- and overflow to 0 and infinity) and FP32 -> FP64
+// (exact for normal values, 0 for subnormal ones) on the integer pipe: a conversion
+// instruction would take a slot of the FP64 pipe.
+HYP_HD float to_f32(double x) {
+  const long long b = bits_of(x);
+  const unsigned s = (unsigned)((unsigned long long)b >> 32) & 0x80000000u;
+  const int ex = (int)((b >> 52) & 0x7ff) - 896;
+  const unsigned m = (unsigned)(b >> 29) & 0x7fffffu;
+  if (ex <= 0) return of_bits_f(s);
+  if (ex >= 255) return of_bits_f(s | (is_nan64(x) ? 0x7fc00000u : 0x7f800000u));
+  return of_bits_f(s | ((unsigned)ex << 23) | m);
+}
+HYP_HD double to_f64(float x) {
+  const unsigned b = bits_of_f(x), ex = (b >> 23) & 0xffu;
+  const unsigned long long s = (unsigned long long)(b & 0x80000000u) << 32;
+  if (ex == 0u) return of_bits((long long)s);
+  if (ex == 255u) return of_bits((long long)(s | (unsigned long long)kInfBits | ((unsigned long long)(b & 0x7fffffu) << 29)));
+  return of_bits((long long)(s | ((unsigned long long)(ex + 896u) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
+}
+
+// 1/x and 1/sqrt(x), sqrt(x): a special-function seed (relative error e0 < 2^-19) and
+// one step of the third-order iterations r (1 + e + e^2), e = 1 - x r (Householder
+// 1970, order 2) and y (1 + e/2 + 3/8 e^2), e = 1 - x y^2: remainders e0^3 and
+// 5/16 (2 e0)^3, below 2^-56. 0, infinities and negative arguments come out as NaN or
+// infinity, never as a finite value.
+HYP_HD double seed_rcp(double x) {
+#ifdef __CUDA_ARCH__
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+#else
+  return (double)(float)(1.0 / x);
+#endif
+}
+HYP_HD double seed_rsqrt(double x) {
+#ifdef __CUDA_ARCH__
+  double r;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  return r;
+#else
+  return (double)(float)(1.0 / sqrt(x));
+#endif
+}
+HYP_HD double rcp64(double x) {
+  const double r = seed_rcp(x);
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+HYP_HD double rsqrt64(double x) {
+  const double y = seed_rsqrt(x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+HYP_HD double sqrt64(double x) {
+  const double y = seed_rsqrt(x), t = x * y;
+  const double e = fma(-t, y, 1.0);
+  return fma(t * e, fma(0.375, e, 0.5), t);
+}
+
+// Constants of one phase's EOS as the forms below use them.
+struct Eos64 {
+  double inv_rho0, inv_rho0sq, rho0sq_icvt;  // 1/rho0, its square, rho0^2 / (cv t0)
+  double hb0sq;                              // b0sq / 2
+  double kU, kE3a, kE3g;                     // as EosT
+  double hbeta, beta2, beta22;               // beta/2, beta + 2, 2 beta + 2
+};
+HYP_HD Eos64 make_eos64(const EosC& e) {
+  Eos64 c;
+  c.inv_rho0 = e.inv_rho0;
+  c.inv_rho0sq = e.inv_rho0 * e.inv_rho0;
+  c.rho0sq_icvt = e.rho0 * e.rho0 * e.inv_cvt0;
+  c.hb0sq = 0.5 * e.b0sq;
+  c.kU = e.kU;
+  c.kE3a = e.kE3a;
+  c.kE3g = e.kE3g;
+  c.hbeta = 0.5 * e.beta;
+  c.beta2 = e.beta + 2.0;
+  c.beta22 = 2.0 * e.beta + 2.0;
+  return c;
+}
+
+// One phase of a cell: primitives, stress row 1 = -2 td w, and what the acoustic
+// tensor takes (unused members cost nothing once inlined).
+struct Cell64 {
+  double td, inv_den;  // rho_true, 1/(alpha rho_true)
+  double u[3], E;
+  double w[3];
+  double G00, G01, G02, G11, G12, G22;
+  double a, b, bM;            // a, b, b p M00
+  double wE;                  // w_0 - E3 p (finite where E3 p is not)
+  double T1, T2, T3, E3p;     // bulk, thermal and shear terms of E3 p, their sum
+  double Pa, Pg, px;          // p^(alpha/2), p^(gamma/2), Pg (x - 1)
+  int st;
+};
+
+// HyperelasticityMPh.jl:106-133 and EquationsOfState.jl:118-190 for one phase: ia =
+// 1/alpha, m = alpha rho u, rE = alpha rho E, R = alpha rho A (column-major). kDef = 1:
+// the default exponents alpha 1, beta 3, gamma 2 at compile time; 0: any.
+template <int kDef>
+HYP_HD Cell64 cell64(const EosC& e, const Eos64& k, double ia, const double* m, double rE, const double* R) {
+  Cell64 o;
+  const double c0 = R[4] * R[8] - R[5] * R[7], c1 = R[1] * R[8] - R[7] * R[2], c2 = R[1] * R[5] - R[4] * R[2];
+  const double d = R[0] * c0 - R[3] * c1 + R[6] * c2;
+  o.st = is_positive64(d) ? HYP_CELL_OK : HYP_CELL_NEG_DET;
+  // rho_true = sqrt(det(R / alpha) / rho0) and its reciprocal from one root
+  const double t = ia * k.inv_rho0;
+  const double x = d * (t * (ia * ia));
+  const double r = rsqrt64(x);
+  o.td = x * r;
+  o.inv_den = r * ia;
+  for (int c = 0; c < 3; ++c) o.u[c] = m[c] * o.inv_den;
+  o.E = rE * o.inv_den;
+  const double e_int = o.E - 0.5 * (o.u[0] * o.u[0] + o.u[1] * o.u[1] + o.u[2] * o.u[2]);
+  // N = R R^T and its cofactors
+  const double n00 = R[0] * R[0] + R[3] * R[3] + R[6] * R[6];
+  const double n11 = R[1] * R[1] + R[4] * R[4] + R[7] * R[7];
+  const double n22 = R[2] * R[2] + R[5] * R[5] + R[8] * R[8];
+  const double n01 = R[0] * R[1] + R[3] * R[4] + R[6] * R[7];
+  const double n02 = R[0] * R[2] + R[3] * R[5] + R[6] * R[8];
+  const double n12 = R[1] * R[2] + R[4] * R[5] + R[7] * R[8];
+  const double k00 = n11 * n22 - n12 * n12, k11 = n00 * n22 - n02 * n02, k22 = n00 * n11 - n01 * n01;
+  const double k01 = n02 * n12 - n01 * n22, k02 = n01 * n12 - n02 * n11, k12 = n01 * n02 - n00 * n12;
+  // M = N inv_den^2, p = (rho_true / rho0)^2, G = adj(M) p: p M = N (ia/rho0)^2 and
+  // G = C (ia inv_den / rho0)^2
+  const double g1 = t * o.inv_den, gs = g1 * g1, ms = t * t;
+  o.G00 = k00 * gs;
+  o.G01 = k01 * gs;
+  o.G02 = k02 * gs;
+  o.G11 = k11 * gs;
+  o.G12 = k12 * gs;
+  o.G22 = k22 * gs;
+  const double i1 = (k00 + k11 + k22) * gs;
+  const double i2 = (n00 + n11 + n22) * ms;  // i2 = p tr M
+  const double s = o.td * k.inv_rho0;        // 1/det A = sqrt(p)
+  const double p = s * s;
+  const double psi = (i1 * (1.0 / 3.0)) * i1 - i2;
+  double Pb, inv_Pg;  // inv_Pg: over cv t0
+  if (kDef == 1) {
+    o.Pa = s;
+    Pb = s * p;
+    o.Pg = p;
+    inv_Pg = (r * r) * k.rho0sq_icvt;
+  } else {
+    const double lp = log(p);
+    o.Pa = exp(0.5 * e.alpha * lp);
+    Pb = exp(0.5 * e.beta * lp);
+    o.Pg = exp(0.5 * e.gamma * lp);
+    inv_Pg = e.inv_cvt0 / o.Pg;
+  }
+  o.b = k.hb0sq * Pb;
+  const double bp = o.b * psi;               // shear energy
+  const double am1 = o.Pa - 1.0, z = k.kU * am1;
+  double xm1 = ((e_int - bp) - z * am1) * inv_Pg;  // x - 1 of the entropy argument (EquationsOfState.jl:150)
+  if (is_nan64(e_int) || is_nan64(xm1) || !is_finite64(p)) o.st |= HYP_CELL_NONFINITE;
+  if (below_negative64(xm1, 1e-6 - 1.0)) xm1 = 1e-6 - 1.0;  // its clamp (:152-154)
+  o.px = o.Pg * xm1;
+  o.T1 = kDef == 1 ? z * s : e.alpha * (z * o.Pa);
+  o.T2 = k.kE3g * o.px;
+  o.T3 = k.hbeta * bp;
+  o.E3p = o.T1 + o.T2 + o.T3;
+  o.a = (2.0 / 3.0) * (o.b * i1);
+  o.bM = o.b * (n00 * ms);
+  o.w[0] = o.a * o.G00 + (o.bM + (o.E3p - o.b * i2));
+  o.wE = o.a * o.G00 + (o.bM - o.b * i2);
+  o.w[1] = o.a * o.G01 + o.b * (n01 * ms);
+  o.w[2] = o.a * o.G02 + o.b * (n02 * ms);
+  return o;
+}
+
+// Spectral radius of 2 O by the general route, for an acoustic tensor whose top root
+// does not stand clear: kept out of line, off the path of every ordinary cell.
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+double radius_general(double o00, double o11, double o22, double o01, double o02, double o12) {
+  const double a[9] = {2.0 * o00, 2.0 * o01, 2.0 * o02, 2.0 * o01, 2.0 * o11, 2.0 * o12, 2.0 * o02, 2.0 * o12, 2.0 * o22};
+  return spectral_radius(a);
+}
+
+// Largest acoustic wave speed sqrt(max |eig Omega|) of one phase (HyperelasticityMPh.jl:258-266).
+template <int kDef>
+HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
+  const double f = (4.0 / 3.0) * c.b;
+  const double f0 = f * c.G00, f1 = f * c.G01, f2 = f * c.G02;
+  double rest;
+  if (kDef == 1)  // -8 E3p + 2 T2 + 3 T3 + kE3a s (2 s - 1), T1 = kE3a s (s - 1)
+    rest = 9.0 * c.w[0] + (-7.0 * c.T1 + (-6.0 * c.T2 + (-5.0 * c.T3 + k.kE3a * c.Pg)));
+  else
+    rest = c.w[0] + k.beta22 * c.wE + e.gamma * c.T2 + e.beta * c.T3 +
+           e.alpha * (k.kE3a * c.Pa * (2.0 * c.Pa - 1.0));
+  const double o00 = f0 * c.G00 + rest;
+  const double o01 = f0 * c.G01 + k.beta2 * c.w[1], o02 = f0 * c.G02 + k.beta2 * c.w[2];
+  const double o11 = f1 * c.G01 + (c.a * c.G11 - c.bM), o22 = f2 * c.G02 + (c.a * c.G22 - c.bM);
+  const double o12 = f1 * c.G02 + c.a * c.G12;
+  // characteristic polynomial mu^3 - c2 mu^2 + c1 mu - c0
+  const double tr = o11 + o22, q = o11 * o22 - o12 * o12;
+  const double c2 = o00 + tr;
+  const double c1 = ((o00 * tr + q) - o01 * o01) - o02 * o02;
+  const double e1 = o01 * o22 - o12 * o02, e2 = o01 * o12 - o11 * o02;
+  const double c0 = (o00 * q - o01 * e1) + o02 * e2;
+  const float C2 = to_f32(c2), C1 = to_f32(c1), C0 = to_f32(c0);
+  const float P = C1 - C2 * C2 * (1.0f / 3.0f);
+  const float Q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
+  if (P < 0.0f && 0.25f * Q * Q + P * P * P * (1.0f / 27.0f) < 0.0f) {  // three real roots
+    const float am = 2.0f * sqrtf(-P * (1.0f / 3.0f));
+    const float cc = fminf(1.0f, fmaxf(-1.0f, 3.0f * Q / (P * am)));
+    const float y = am * cosf(acosf(cc) * (1.0f / 3.0f)) + C2 * (1.0f / 3.0f);  // the largest root
+    const float sm = C2 - y, pr = C0 / y;  // sum and product of the other two
+    const float other = 0.5f * fabsf(sm) + sqrtf(fmaxf(0.25f * sm * sm - pr, 0.0f));
+    const float slope = (3.0f * y - 2.0f * C2) * y + C1;
+    // With the others below 0.35 of it, the seed is within ~1e-6 and the slope within
+    // ~1e-6 of theirs at the root: a step leaves 5e-12, the next 5e-17.
+    if (other < 0.35f * y && slope > 1e-30f && slope < 1e30f) {
+      const double inv = to_f64(1.0f / slope);
+      double rt = to_f64(y);
+      for (int it = 0; it < 2; ++it) rt = rt - (((rt - c2) * rt + c1) * rt - c0) * inv;
+      return sqrt64(rt + rt);
+    }
+  }
+  return sqrt(radius_general(o00, o11, o22, o01, o02, o12));
+}
+
+// Physical x-flux of one phase (HyperelasticityMPh.jl:146-175), the 14 entries after
+// alpha: alpha rho u1 is m1 itself, and the rho A part is u1 R - u (row 1 of R), whose
+// first row is zero.
+HYP_HD void flux64(double alpha, const Cell64& c, const double* m, const double* R, double* f) {
+  const double d2 = 2.0 * (alpha * c.td);  // -alpha s0 = 2 alpha rho w
+  const double S0 = d2 * c.w[0], S1 = d2 * c.w[1], S2 = d2 * c.w[2];
+  f[0] = m[0];
+  f[1] = m[0] * c.u[0] + S0;
+  f[2] = m[0] * c.u[1] + S1;
+  f[3] = m[0] * c.u[2] + S2;
+  f[4] = m[0] * c.E + (c.u[2] * S2 + (c.u[1] * S1 + c.u[0] * S0));
+  for (int b = 0; b < 3; ++b) {
+    f[5 + 3 * b] = 0.0;
+    f[6 + 3 * b] = c.u[0] * R[1 + 3 * b] - c.u[1] * R[3 * b];
+    f[7 + 3 * b] = c.u[0] * R[2 + 3 * b] - c.u[2] * R[3 * b];
+  }
+}
+
+}  // namespace hyp

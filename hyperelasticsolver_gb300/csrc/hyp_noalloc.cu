@@ -25,7 +25,7 @@
 //
 // Errors: a launch error that earlier, unrelated work left pending in the CUDA
 // runtime is cleared on entry (cudaGetLastError) so that it is not reported as
-// this call's; the reset kernel and the first step's two launches are checked one
+// this call's; the reset kernel and each launch of a step are checked one
 // by one, so a launch that fails stops the call before the rest are queued.
 #include <mutex>
 #include "hyp_internal.cuh"
@@ -103,7 +103,6 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   const EosC eos = make_eos(cfg->eos[0].rho0, cfg->eos[0].c0, cfg->eos[0].cv, cfg->eos[0].t0, cfg->eos[0].b0,
                             cfg->eos[0].alpha, cfg->eos[0].beta, cfg->eos[0].gamma);
   const double dx = cfg->x_length / (double)n;
-  const unsigned grid = (unsigned)((n + kBlock - 1) / kBlock);
   // Ping-pong between the caller's output and the scratch state so that the last step writes the output.
   double* cur = (n_steps % 2 == 0) ? d_Q_out : B;
   if (cur != d_Q_in &&
@@ -114,12 +113,11 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   for (int k = 0; k < n_steps; ++k) {
     const int p = k & 1;
     double* nxt = (cur == d_Q_out) ? B : d_Q_out;
-    cell1_f64_kernel<<<grid, kBlock, 0, s>>>(cur, n, eos, F, lam, &st->lam_bits[p], &st->t[p], INFINITY, st);
-    if (k == 0 && cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;
-    update1_f64_kernel<<<grid, kBlock, 0, s>>>(cur, nxt, n, F, lam, &st->lam_bits[p], &st->lam_bits[1 - p],
-                                               &st->t[p], &st->t[1 - p], &st->steps, INFINITY, cfg->cfl, dx,
-                                               cfg->flux, cfg->bc);
-    if (k == 0 && cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;
+    cudaError_t e = launch_cell1(s, cur, n, eos, F, lam, &st->lam_bits[p], &st->t[p], INFINITY, st);
+    if (e != cudaSuccess) return HYP_ERR_CUDA;
+    e = launch_update1(s, cur, nxt, n, F, lam, &st->lam_bits[p], &st->lam_bits[1 - p], &st->t[p], &st->t[1 - p],
+                       &st->steps, INFINITY, cfg->cfl, dx, cfg->flux, cfg->bc);
+    if (e != cudaSuccess) return HYP_ERR_CUDA;
     cur = nxt;
   }
   if (cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;

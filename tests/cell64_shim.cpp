@@ -1,0 +1,36 @@
+// Host build of the FP64 step's compact cell forms (hyp_cell64.cuh) beside the general
+// ones (hyp_physics.cuh), for tests/test_cell64_host.py.
+#include "../hyperelasticsolver_gb300/csrc/hyp_cell64.cuh"
+
+using namespace hyp;
+
+template <int kDef>
+static int compact(const EosC& e, const double* q, double* out) {
+  const Eos64 k = make_eos64(e);
+  const Cell64 c = cell64<kDef>(e, k, rcp64(q[0]), q + 2, q[5], q + 6);
+  flux64(q[0], c, q + 2, q + 6, out);
+  out[14] = c.u[0];
+  out[15] = cmax64<kDef>(e, k, c);
+  return c.st;
+}
+
+extern "C" {
+// q: one phase (15 values); out: flux (14 after alpha), u1, c_max; returns the status bits
+int c64_compact(const double* p, const double* q, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  return e.default_exp ? compact<1>(e, q, out) : compact<0>(e, q, out);
+}
+int c64_general(const double* p, const double* q, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  Prim P;
+  const int st = cons_to_prim(e, q[0], q + 2, q[5], q + 6, P);
+  const StressC c = stress_coeffs(e, P.k, P.w, P.xm1);
+  double s0[3];
+  phase_flux(e, q[0], P, c, out, s0);
+  out[14] = P.u[0];
+  out[15] = phase_cmax(e, P, c);
+  return st;
+}
+float c64_to_f32(double x) { return to_f32(x); }
+double c64_to_f64(float x) { return to_f64(x); }
+}
