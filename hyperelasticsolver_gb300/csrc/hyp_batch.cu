@@ -174,79 +174,73 @@ __global__ void __launch_bounds__(kBlock) batch_join_kernel(const float* __restr
 }
 
 // ---- FP64 ----------------------------------------------------------------------
-// One tile per block: the single problem's cell pass (cell1_pass) and the tile's
-// maximum into its problem's slot.
+// One tile of kCells64 cells per block, as the single problem's kernels (hyp_step1.cu):
+// the cell pass and the tile's maximum into its problem's slot.
 template <int kDef>
 __global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* __restrict__ Q, int64_t n, EosC e,
                                                                   Eos64 k, double* __restrict__ F,
                                                                   double* __restrict__ lam,
-                                                                  const TileDesc* __restrict__ tiles, int tile_cells,
-                                                                  BatchDev b, int par, double t_end,
+                                                                  const TileDesc* __restrict__ tiles, BatchDev b,
+                                                                  int par, double t_end,
                                                                   unsigned long long* slot_base, DevState* S) {
   const TileDesc d = tiles[blockIdx.x];
   if (!(b.t[par * b.P + d.problem] < t_end)) return;
-  unsigned long long top = 0ull;
-  double l = 0.0;
-  for (int64_t i = d.first + threadIdx.x; i < d.first + tile_cells && i < d.hi; i += kBlock64) {
-    l = cell1_pass<kDef>(Q, n, i, e, k, F, lam, S);
-    const unsigned long long lb = is_nan64(l) ? 0ull : (unsigned long long)bits_of(l);
-    top = lb > top ? lb : top;
-  }
-  const unsigned long long m = block_max_bits<kBlock64>(of_bits((long long)top));
+  const int64_t i = d.first + threadIdx.x;
+  const bool own = threadIdx.x < kCells64 && i < d.hi;
+  const double l = own ? cell1_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(&slot_base[d.problem], m);
 }
 
-// One tile of kBlock cells per block iteration (tile_cells == kBlock for the FP64
-// batch); each face of the tile once into shared memory, as update1_f64_kernel.
-__global__ void __launch_bounds__(kBlock) batch_f64_update_kernel(const double* __restrict__ Q, double* __restrict__ Qn,
-                                                                  int64_t n, const double* __restrict__ F,
-                                                                  const double* __restrict__ lam,
-                                                                  const TileDesc* __restrict__ tiles, int ntiles,
-                                                                  int tile_cells, BatchDev b, int par, double t_end,
-                                                                  double cfl, int flux, int bc) {
-  __shared__ double sF[14][kBlock + 1];  // face k of the tile = left face of cell first + k
-  const int P = b.P;
+// Each face of the tile once into shared memory, then the update, as update1_f64_kernel.
+__global__ void __launch_bounds__(kBlock64) batch_f64_update_kernel(const double* __restrict__ Q,
+                                                                    double* __restrict__ Qn, int64_t n,
+                                                                    const double* __restrict__ F,
+                                                                    const double* __restrict__ lam,
+                                                                    const TileDesc* __restrict__ tiles, BatchDev b,
+                                                                    int par, double t_end, double cfl, int flux,
+                                                                    int bc) {
+  __shared__ double sF[14][kBlock64];  // twice the left face of cell first + k
+  __shared__ double s_hdt;
+  const int P = b.P, j = threadIdx.x;
   const bool lxf = flux == HYP_FLUX_LXF;
-  for (int tix = blockIdx.x; tix < ntiles; tix += gridDim.x) {
-    const TileDesc d = tiles[tix];
-    const int p = d.problem;
-    const double tn = b.t[par * P + p];
-    const bool active = tn < t_end;
-    const double lmax = __longlong_as_double((long long)b.slots[par * P + p]);
-    const double dx = b.dx[p];
-    const StepScalars sc = step_scalars(cfl, dx, lmax, lxf);
-    const double dt = sc.dt, lam_lxf = sc.lam_lxf, dtdx = sc.dtdx;
-    if (d.lead && threadIdx.x == 0) {
-      b.t[(1 - par) * P + p] = active ? tn + dt : tn;
-      b.slots[(1 - par) * P + p] = 0ull;
-      if (active) b.steps[p] += 1;
-    }
-    const int64_t i = d.first + threadIdx.x;
-    const bool own = (int)threadIdx.x < tile_cells && i < d.hi;
-    if (!active) {  // a finished problem's cells go to the other buffer unchanged (uniform per tile)
-      if (own)
-        for (int v = 0; v < 14; ++v) Qn[v * n + i] = Q[v * n + i];
-      continue;
-    }
-    if (own) {
-      rusanov_face<kBlock + 1>(Q, F, lam, n, d.lo, d.hi, i, lxf, lam_lxf, sF, threadIdx.x);
-      if ((int)threadIdx.x == tile_cells - 1 || i == d.hi - 1)
-        rusanov_face<kBlock + 1>(Q, F, lam, n, d.lo, d.hi, i + 1, lxf, lam_lxf, sF, threadIdx.x + 1);
-    }
-    __syncthreads();
-    if (own) {
-      const bool frozen = bc == HYP_BC_FROZEN && (i == d.lo || i == d.hi - 1);
+  const TileDesc d = tiles[blockIdx.x];
+  const int p = d.problem;
+  const double tn = b.t[par * P + p];
+  const bool active = tn < t_end;
+  const double lmax = __longlong_as_double((long long)b.slots[par * P + p]);
+  StepScalars sc{0.0, 0.0, 0.0};
+  if (j < 32 || lxf) sc = step_scalars64(cfl, b.dx[p], lmax, lxf);
+  if (j == 0) s_hdt = 0.5 * sc.dtdx;
+  if (d.lead && j == 0) {
+    b.t[(1 - par) * P + p] = active ? tn + sc.dt : tn;
+    b.slots[(1 - par) * P + p] = 0ull;
+    if (active) b.steps[p] += 1;
+  }
+  const int64_t i = d.first + j;
+  const bool own = j < kCells64 && i < d.hi;
+  if (!active) {  // a finished problem's cells go to the other buffer unchanged (uniform per tile)
+    if (own)
+      for (int v = 0; v < 14; ++v) Qn[v * n + i] = Q[v * n + i];
+    return;
+  }
+  double f2[14];
+  if (i <= d.hi) {
+    face_twice(Q, F, lam, n, d.lo, d.hi, i, lxf, sc.lam_lxf, f2);
 #pragma unroll
-      for (int v = 0; v < 14; ++v) {
-        const double qc = Q[v * n + i];
-        Qn[v * n + i] = frozen ? qc : __fma_rn(-dtdx, __dsub_rn(sF[v][threadIdx.x + 1], sF[v][threadIdx.x]), qc);
-      }
-    }
-    __syncthreads();  // the next tile rewrites the face table
+    for (int v = 0; v < 14; ++v) sF[v][j] = f2[v];
+  }
+  __syncthreads();
+  if (!own) return;
+  const bool frozen = bc == HYP_BC_FROZEN && (i == d.lo || i == d.hi - 1);
+  const double hdt = s_hdt;
+#pragma unroll
+  for (int v = 0; v < 14; ++v) {
+    const double qc = Q[v * n + i];
+    Qn[v * n + i] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
   }
 }
 
-// ---- mixed kernel variants (autotuned) -------------------------------------------
 // A variant: block size, resident blocks per SM the registers are budgeted for,
 // and whether the grid is persistent (one wave of blocks striding over the tile
 // table) or one block per tile.
@@ -304,7 +298,6 @@ struct hyp_batch {
   TileDesc* tiles = nullptr;
   TileCtl* ctl = nullptr;  // mixed: per-tile step control
   int ntiles = 0;
-  int tile_cells = 0;
   int variant = 2;
   int grid = 0;
   std::vector<int64_t> offsets;
@@ -342,16 +335,13 @@ static int build_tiles(hyp_batch* b, int cells_per_tile) {
   if (b->mixed) BCK(cudaMalloc(&b->ctl, t.size() * sizeof(TileCtl)));
   BCK(cudaMemcpy(b->tiles, t.data(), t.size() * sizeof(TileDesc), cudaMemcpyHostToDevice));
   b->ntiles = (int)t.size();
-  b->tile_cells = cells_per_tile;
   return HYP_OK;
 }
 
 static int select_variant(hyp_batch* b, int v) {
   if (!b->mixed) {
     b->variant = 0;
-    int rc = build_tiles(b, kBlock);
-    b->grid = b->sms * 8;
-    return rc;
+    return build_tiles(b, kCells64);
   }
   if (v < 0 || v >= kNumVariants) return berr(b, HYP_ERR_INVALID, "no such kernel variant");
   const int res = kVariants[v].minb == 4 ? resident_blocks<256, 4>() : resident_blocks<256, 3>();
@@ -399,12 +389,11 @@ static int enqueue_batch_step(hyp_batch* b, long long k, double t_end) {
     const Eos64 k64 = make_eos64(b->eos);
     auto cell = b->eos.default_exp ? batch_f64_cell_kernel<1> : batch_f64_cell_kernel<0>;
     cell<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->total, b->eos, k64, b->F, b->lam, b->tiles,
-                                                b->tile_cells, b->b, par, t_end, b->b.slots + (size_t)par * b->P,
-                                                b->st);
+                                                b->b, par, t_end, b->b.slots + (size_t)par * b->P, b->st);
     BCK(cudaGetLastError());
-    batch_f64_update_kernel<<<b->grid, kBlock, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->F, b->lam,
-                                                               b->tiles, b->ntiles, b->tile_cells, b->b, par, t_end,
-                                                               b->cfg.cfl, b->cfg.flux, b->cfg.bc);
+    batch_f64_update_kernel<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->F, b->lam,
+                                                                   b->tiles, b->b, par, t_end, b->cfg.cfl,
+                                                                   b->cfg.flux, b->cfg.bc);
     BCK(cudaGetLastError());
   }
   return HYP_OK;

@@ -58,4 +58,59 @@ __device__ __forceinline__ double cell1_pass(const double* __restrict__ Q, int64
   return l;
 }
 
+// Cells a block of the update kernels owns: thread j evaluates the face left of cell
+// first + j, so the last thread's face closes the last owned cell and no thread
+// evaluates two (a second face on one thread is a second pass of its whole warp).
+constexpr int kCells64 = kBlock64 - 1;
+
+// a / b from rb, about 1 / b: a product and one residual correction (Markstein 1990),
+// 3 slots; correctly rounded up to rare last-bit cases.
+__device__ __forceinline__ double quot64(double a, double b, double rb) {
+  const double q = a * rb;
+  return fma(fma(-b, q, a), rb, q);
+}
+
+// step_scalars without FP64 divisions (about 9 slots each): 13 slots for the Rusanov
+// step, 22 for LxF. Arguments too large or small for the special-function seeds, and
+// quotients that are not finite, take the divisions.
+__device__ __forceinline__ StepScalars step_scalars64(double cfl, double dx, double lmax, bool lxf) {
+  auto plain = [](double x) { return x > 1e-250 && x < 1e250; };
+  const double cdx = cfl * dx;
+  if (!plain(lmax) || !plain(dx) || !plain(cdx)) {
+    const double dt = cdx / lmax, lam = dx / dt;
+    return StepScalars{dt, lam, lxf ? 1.0 / lam : dt / dx};
+  }
+  StepScalars s{0.0, 0.0, 0.0};
+  s.dt = quot64(cdx, lmax, rcp64(lmax));
+  if (lxf) {
+    s.lam_lxf = quot64(dx, s.dt, rcp64(s.dt));
+    s.dtdx = quot64(1.0, s.lam_lxf, rcp64(s.lam_lxf));
+  } else {
+    s.dtdx = quot64(s.dt, dx, rcp64(dx));
+  }
+  return s;
+}
+
+// Twice the Rusanov flux of the face between cells f - 1 and f of the problem [lo, hi)
+// (a zero-gradient ghost past either end): (f_a + f_b) - lambda (q_b - q_a), lambda =
+// max(lambda_a, lambda_b) (NumFluxes.jl:25-33, main.jl:45-48) or the LxF one. Doubling is
+// exact, so this is the flux's own rounding with a multiplication less per variable;
+// the rounding sequence is fixed (explicit intrinsics), so the step commutes with x -> -x.
+__device__ __forceinline__ void face_twice(const double* __restrict__ Q, const double* __restrict__ F,
+                                           const double* __restrict__ lam, int64_t n, int64_t lo, int64_t hi,
+                                           int64_t f, bool lxf, double lam_lxf, double* f2) {
+  const int64_t a = f > lo ? f - 1 : lo, b = f < hi ? f : hi - 1;
+  double lf = lam_lxf;
+  if (!lxf) {
+    const double la = lam[a], lb = lam[b];  // la > lb ? la : lb of non-negative values
+    lf = bits_of(la) > bits_of(lb) && !is_nan64(la) ? la : lb;
+  }
+#pragma unroll
+  for (int v = 0; v < 14; ++v) {
+    const int sl = flux_slot1(v);
+    const double dq = __dsub_rn(Q[v * n + b], Q[v * n + a]);
+    f2[v] = sl >= 0 ? __fma_rn(-lf, dq, __dadd_rn(F[sl * n + a], F[sl * n + b])) : __dmul_rn(-lf, dq);
+  }
+}
+
 }  // namespace hyp
