@@ -53,6 +53,8 @@ static int free_ctx(hyp_ctx* c) {
   cudaFree(c->DM);
   cudaFree(c->DP);
   cudaFree(c->FF);
+  cudaFree(c->face_list);
+  cudaFree(c->face_s);
   cudaFree(c->F32);
   cudaFree(c->smin32);
   cudaFree(c->smax32);
@@ -104,6 +106,8 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
   };
   cudaError_t e;
   if ((e = cudaGetDevice(&c->device)) != cudaSuccess) fail(e, "cudaGetDevice");
+  if (rc == HYP_OK && (e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device)) != cudaSuccess)
+    fail(e, "cudaDeviceGetAttribute");
   if (rc == HYP_OK && (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess)
     fail(e, "cudaStreamCreate");
   if (rc == HYP_OK && (e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking)) != cudaSuccess)
@@ -147,6 +151,11 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
     if (rc == HYP_OK && (e = cudaMalloc(&c->smax, (size_t)c->n * sizeof(double))) != cudaSuccess) fail(e, "cudaMalloc(smax)");
     if (rc == HYP_OK && (e = cudaMalloc(&c->DM, nfb)) != cudaSuccess) fail(e, "cudaMalloc(DM)");
     if (rc == HYP_OK && (e = cudaMalloc(&c->DP, nfb)) != cudaSuccess) fail(e, "cudaMalloc(DP)");
+    if (rc == HYP_OK && (e = cudaMalloc(&c->face_list, (size_t)(c->n + 1) * sizeof(int))) != cudaSuccess)
+      fail(e, "cudaMalloc(face list)");
+    if (rc == HYP_OK && cfg->flux == HYP_FLUX_HLL &&
+        (e = cudaMalloc(&c->face_s, (size_t)2 * (c->n + 1) * sizeof(double))) != cudaSuccess)
+      fail(e, "cudaMalloc(face speeds)");
     if (rc == HYP_OK && cfg->flux == HYP_FLUX_LXF && (e = cudaMalloc(&c->FF, nfb)) != cudaSuccess)
       fail(e, "cudaMalloc(face fluxes)");
   } else if (!mixed(c)) {

@@ -27,6 +27,7 @@ struct DevState {
   int err_code;                       // first HYP_CELL_* status raised (0 = none)
   int pad_;
   long long err_cell;                 // cell that raised it
+  int n_listed;                       // two-phase FP64: faces whose path integrals the step still has to do
 };
 
 // Per-cell flux components that are not identically zero for one phase:
@@ -150,6 +151,9 @@ struct hyp_ctx {
   double* smax = nullptr;
   double* DM = nullptr;
   double* DP = nullptr;
+  int* face_list = nullptr;   // two-phase FP64: listed faces [n+1], and (HLL) their s_l, s_r [2][n+1]
+  double* face_s = nullptr;
+  int sms = 0;                // multiprocessors of the device
   hyp::DevState* st = nullptr;
   hyp::DevState* st_host = nullptr;  // pinned mirror
   int cur = 0;             // parity of the buffer that holds the current state

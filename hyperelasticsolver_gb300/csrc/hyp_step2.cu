@@ -2,185 +2,637 @@
 // (main.jl:202-241 with update_cell :43-60 and NumFluxes.hll :70-132) or the
 // path-conservative Lax-Friedrichs flux (update_cell :30-41, NumFluxes.lxf :25-60).
 //
-// Three kernels per step on the context stream:
-//   cell   : per cell, both phases' flux (HyperelasticityMPh.jl:140-175) and
+// Four kernels per step on the context stream:
+//   cell   : per cell and phase, the flux (HyperelasticityMPh.jl:140-175) and
 //            wave-speed bounds (:252-266); lambda_i = max |speed|, block max ->
 //            one atomicMax (main.jl:204-212);
-//   face   : per face, the HLL fluctuations D-, D+ (hll_face2: midpoint speeds,
-//            three 6-point Gauss-Legendre path integrals of B, Q_hll), one
-//            thread per face -- 18 evaluations of B per face instead of the 30
-//            the reference makes, since the integrals repeated in D- and D+ are
-//            the same;
+//   face   : per face and phase, the midpoint's wave speeds and s_l, s_r (HLL), and the
+//            whole face wherever its path integrals vanish; the other faces go to a list;
+//   paths  : the listed faces' 6-point path integrals of B (HLL: three Gauss-Legendre
+//            ones, 18 evaluations of B instead of the 30 the reference makes, since the
+//            integrals repeated in D- and D+ are the same; LxF: one Gauss-Lobatto);
 //   update : dt = cfl dx / max lambda, t += dt, Q_i - dt/dx ((F_r - F_l) + (D-_{i+1/2} + D+_{i-1/2}))
 //            with frozen or transmissive ends; F = 0 for HLL (it folds the conservative
 //            part into D+-), the LxF face flux otherwise.
-// The LxF face kernel takes lambda = dx/dt of this step (main.jl:223) from the
-// max wave speed the cell kernel has just reduced, and integrates B with the
-// 6-point Gauss-Lobatto rule.
+//
+// What bounds them is FP64 issue (hyp_cell64.cuh), so the counts per face matter and
+// nothing else does. B dQ is a column times d(alpha) (HyperelasticityMPh.jl:178-250):
+// where both cells of a face have the same volume fractions every path integral is
+// exactly zero and so is Q_hll's jump in alpha, and the face is the plain HLL (or LxF)
+// formula: about 370 FP64 instructions instead of 10,400 (6,600 with the integrals). That holds on most faces of a run
+// that starts from states of piecewise-constant volume fraction (main.jl:99-106, the
+// smoothed interface away from its 8 cells); where the fractions vary in every cell
+// (main.jl:110-123) all faces are listed.
+#include <algorithm>
 #include "hyp_internal.cuh"
 #include "hyp_physics_mph.cuh"
+#include "hyp_step64.cuh"
 
 namespace hyp {
 
-__device__ __forceinline__ void record_err2(DevState* S, int code, long long cell) {
-  if (atomicCAS(&S->err_code, 0, code) == 0) S->err_cell = cell;
-}
+// The two phases' EOS with the constants of the compact forms.
+struct Eos2x {
+  EosC e[2];
+  Eos64 k[2];
+};
 
-__device__ __forceinline__ double block_max2(double v) {
-  __shared__ double red[kBlock / 32];
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  if (w == 0) {
-    v = l < kBlock / 32 ? red[l] : 0.0;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  }
-  return v;
-}
+// Rows of a phase's 15 whose physical flux is identically zero: alpha and the first row
+// of alpha rho A.
+__device__ __forceinline__ constexpr bool zero_flux_row(int r) { return r == 0 || (r >= 6 && (r - 6) % 3 == 0); }
 
-__global__ void __launch_bounds__(kBlock) cell2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2 E,
-                                                           double* __restrict__ F, double* __restrict__ smin,
-                                                           double* __restrict__ smax, unsigned long long* lam_slot,
-                                                           const double* t_now, double t_end, DevState* S) {
+constexpr int kPairCells = 64;             // cells (faces) of a block: one thread per phase of each
+constexpr int kPair64 = 2 * kPairCells;    // its threads; the phase is uniform over a warp
+
+template <int kDef>
+__global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
+                                                            double* __restrict__ F, double* __restrict__ smin,
+                                                            double* __restrict__ smax, unsigned long long* lam_slot,
+                                                            const double* t_now, double t_end, DevState* S) {
+  __shared__ double s_lo[kPairCells], s_hi[kPairCells];
   if (!(*t_now < t_end)) return;
-  const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
-  double l = 0.0;
+  const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
+  const int64_t i = (int64_t)blockIdx.x * kPairCells + j;
+  double lo = 0.0, hi = 0.0;
   if (i < n) {
-    double q[30], f[30];
-    for (int v = 0; v < 30; ++v) q[v] = Q[v * n + i];
-    int st = flux2(E.e, q, f);
-    double lo = 0.0, hi = 0.0;
-    st |= speeds2(E.e, q, lo, hi);
-    for (int v = 0; v < 30; ++v) F[v * n + i] = f[v];
+    const double* q0 = Q + 15 * ph * n + i;
+    double m[3], R[9];
+    const double alpha = q0[0], rE = q0[5 * n];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) m[v] = q0[(2 + v) * n];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) R[v] = q0[(6 + v) * n];
+    const EosC& e = E.e[ph];
+    const Cell64 c = cell64<kDef>(e, E.k[ph], rcp64(alpha), m, rE, R);
+    double f[14];
+    flux64(alpha, c, m, R, f);
+    double* f0 = F + 15 * ph * n + i;
+#pragma unroll
+    for (int r = 1; r < 15; ++r)
+      if (!zero_flux_row(r)) f0[r * n] = f[r - 1];
+    const double cm = cmax64<kDef>(e, E.k[ph], c);
+    lo = c.u[0] - cm;
+    hi = c.u[0] + cm;
+    if (c.st) record_err64(S, c.st, i);
+    if (ph == 1) {
+      s_lo[j] = lo;
+      s_hi[j] = hi;
+    }
+  }
+  __syncthreads();
+  double l = 0.0;
+  if (ph == 0 && i < n) {
+    if (s_lo[j] < lo) lo = s_lo[j];
+    if (s_hi[j] > hi) hi = s_hi[j];
     smin[i] = lo;
     smax[i] = hi;
     l = fmax(fabs(lo), fabs(hi));
-    if (!(l <= 1.79e308)) st |= HYP_CELL_NONFINITE;
-    if (st) record_err2(S, st, i);
+    if (!is_finite64(l)) record_err64(S, HYP_CELL_NONFINITE, i);
   }
-  const double m = block_max2(l);
-  if (threadIdx.x == 0) atomicMax(lam_slot, (unsigned long long)__double_as_longlong(m));
+  const unsigned long long m = block_max_bits<kPair64>(l);
+  if (threadIdx.x == 0) atomicMax(lam_slot, m);
 }
 
-constexpr int kFaceBlock = 64;
+// ---- faces ---------------------------------------------------------------------
 
-__global__ void __launch_bounds__(kFaceBlock) face2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2 E,
-                                                               Quad6D qd, const double* __restrict__ F,
-                                                               const double* __restrict__ smin,
-                                                               const double* __restrict__ smax, double* __restrict__ DM,
-                                                               double* __restrict__ DP, const double* t_now,
-                                                               double t_end, DevState* S) {
+// Faces whose path integrals are still to be done, and their s_l, s_r (by list
+// position); the count lives in DevState.
+struct FaceList {
+  int* face;
+  double *sl, *sr;
+};
+
+// True if every state within `far` of R (in the Frobenius norm of the change of R =
+// alpha rho A; far2 its square) has det R > 0: ||dR|| ||R^-1|| < 1/3, evaluated in FP32
+// with the cofactor norm. NaN, under- and overflow give false.
+__device__ __forceinline__ bool det_keeps_sign(const float* R, float far2) {
+  const float c00 = R[4] * R[8] - R[5] * R[7], c01 = R[7] * R[2] - R[1] * R[8], c02 = R[1] * R[5] - R[4] * R[2];
+  const float c10 = R[5] * R[6] - R[3] * R[8], c11 = R[0] * R[8] - R[2] * R[6], c12 = R[2] * R[3] - R[0] * R[5];
+  const float c20 = R[3] * R[7] - R[4] * R[6], c21 = R[1] * R[6] - R[0] * R[7], c22 = R[0] * R[4] - R[1] * R[3];
+  const float det = R[0] * c00 + R[3] * c01 + R[6] * c02;
+  const float cc = c00 * c00 + c01 * c01 + c02 * c02 + c10 * c10 + c11 * c11 + c12 * c12 + c20 * c20 + c21 * c21 +
+                   c22 * c22;
+  return det > 0.0f && 9.0f * far2 * cc < det * det;
+}
+
+// HLL faces: s_l, s_r and, where the volume fractions do not jump and no state on the
+// way between the cells (through Q_hll) can be singular, D- and D+ (doubles of the
+// formula of NumFluxes.jl:85-132 with its integrals zero). 186 slots a phase; the others are
+// listed.
+template <int kDef>
+__global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
+                                                            const double* __restrict__ F,
+                                                            const double* __restrict__ smin,
+                                                            const double* __restrict__ smax, double* __restrict__ DM,
+                                                            double* __restrict__ DP, FaceList list,
+                                                            const double* t_now, double t_end, DevState* S) {
+  __shared__ double s_lo[2][kPairCells], s_hi[2][kPairCells];
+  __shared__ int s_flag[2][kPairCells];  // bit 0: both cells equal; bit 1: alpha does not jump
+  __shared__ int s_hard[2][kPairCells];
   if (!(*t_now < t_end)) return;
-  const int64_t f = (int64_t)blockIdx.x * kFaceBlock + threadIdx.x;  // face between cells f-1 and f
-  if (f > n) return;
+  const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
+  const int64_t f = (int64_t)blockIdx.x * kPairCells + j;  // face between cells f-1 and f
   const int64_t nf = n + 1;
+  const bool in = f <= n;
   const int64_t L = f > 0 ? f - 1 : 0, R = f < n ? f : n - 1;
-  double dm[30], dp[30];
-  if (L == R) {  // boundary face with a zero-gradient ghost: no jump, no fluctuation
-    for (int v = 0; v < 30; ++v) dm[v] = dp[v] = 0.0;
-  } else {
-    double QL[30], QR[30], fl[30], fr[30];
-    for (int v = 0; v < 30; ++v) {
-      QL[v] = Q[v * n + L];
-      QR[v] = Q[v * n + R];
-      fl[v] = F[v * n + L];
-      fr[v] = F[v * n + R];
+  const double* ql = Q + 15 * ph * n + (in ? L : 0);
+  const double* qr = Q + 15 * ph * n + (in ? R : 0);
+  double a[15], b[15];
+  bool same = true;
+#pragma unroll
+  for (int r = 0; r < 15; ++r) {
+    a[r] = ql[r * n];
+    b[r] = qr[r * n];
+    same &= bits_of(a[r]) == bits_of(b[r]);
+  }
+  s_flag[ph][j] = (same ? 1 : 0) | (bits_of(a[0]) == bits_of(b[0]) ? 2 : 0);
+  __syncthreads();
+  const int flag = s_flag[0][j] & s_flag[1][j];
+  const bool equal = flag & 1;  // (also the boundary face with its zero-gradient ghost)
+  double* dm = DM + 15 * ph * nf + f;
+  double* dp = DP + 15 * ph * nf + f;
+  // equal cells: no jump, no fluctuation; the midpoint is the cell itself
+  if (in && equal) {
+#pragma unroll
+    for (int r = 0; r < 15; ++r) dm[r * nf] = dp[r * nf] = 0.0;
+  }
+  const bool work = in && !equal;
+  if (work) {  // speeds of the midpoint: the forms are homogeneous, so q_l + q_r serves
+    double m[3], Rm[9];
+#pragma unroll
+    for (int v = 0; v < 3; ++v) m[v] = a[2 + v] + b[2 + v];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) Rm[v] = a[6 + v] + b[6 + v];
+    const Cell64 c = cell64<kDef>(E.e[ph], E.k[ph], rcp64(a[0] + b[0]), m, a[5] + b[5], Rm);
+    const double cm = cmax64<kDef>(E.e[ph], E.k[ph], c);
+    if (c.st) record_err64(S, c.st, R);
+    s_lo[ph][j] = c.u[0] - cm;
+    s_hi[ph][j] = c.u[0] + cm;
+  }
+  __syncthreads();
+  double sl = 0.0, sr = 0.0;
+  bool hard = false;
+  if (work) {
+    const double l0 = s_lo[0][j], l1 = s_lo[1][j], h0 = s_hi[0][j], h1 = s_hi[1][j];
+    const double mmin = l1 < l0 ? l1 : l0, mmax = h1 > h0 ? h1 : h0;
+    if (mmin < sl) sl = mmin;
+    if (smin[L] < sl) sl = smin[L];
+    if (mmax > sr) sr = mmax;
+    if (smax[R] > sr) sr = smax[R];
+    hard = !(flag & 2);
+    if (!hard) {
+      const double idsr = rcp64(sr - sl);
+      const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
+      const double* fl = F + 15 * ph * n + L;
+      const double* fr = F + 15 * ph * n + R;
+      const float g = to_f32(cp), h = to_f32(idsr);
+      float far = 0.0f, farh = 0.0f;  // squared distances of q_r and Q_hll from q_l in R
+      bool finite = true;
+#pragma unroll
+      for (int r = 0; r < 15; ++r) {
+        if (r == 1) {  // alpha rho: updated like the rest, unused by the forms
+          const double df = fr[r * n] - fl[r * n], jump = b[1] - a[1];
+          dm[r * nf] = cm * df + cq * jump;
+          dp[r * nf] = cp * df - cq * jump;
+          continue;
+        }
+        if (r == 0) {
+          dm[0] = dp[0] = 0.0;
+          continue;
+        }
+        const double jump = b[r] - a[r];
+        const double df = zero_flux_row(r) ? 0.0 : fr[r * n] - fl[r * n];
+        finite &= is_finite64(jump) && is_finite64(df);
+        if (r >= 6) {  // Q_hll - q_l = (jump s_r - df) / (s_r - s_l)
+          const float jf = to_f32(jump), hf = jf * g - to_f32(df) * h;
+          far += jf * jf;
+          farh += hf * hf;
+        }
+        const double qj = cq * jump;
+        dm[r * nf] = zero_flux_row(r) ? qj : cm * df + qj;
+        dp[r * nf] = zero_flux_row(r) ? -qj : cp * df - qj;
+      }
+      float Rf[9];
+#pragma unroll
+      for (int v = 0; v < 9; ++v) Rf[v] = to_f32(a[6 + v]);
+      hard = !finite || !det_keeps_sign(Rf, fmaxf(far, farh));
     }
-    int st = hll_face2(E.e, qd, QL, QR, fl, fr, smin[L], smax[R], dm, dp);
-    if (st) record_err2(S, st, R);
   }
-  for (int v = 0; v < 30; ++v) {
-    DM[v * nf + f] = dm[v];
-    DP[v * nf + f] = dp[v];
+  s_hard[ph][j] = hard;
+  __syncthreads();
+  if (ph == 0 && (s_hard[0][j] | s_hard[1][j])) {  // one atomic per warp
+    const unsigned mask = __activemask();
+    const int lead = __ffs(mask) - 1;
+    int at = 0;
+    if ((int)(threadIdx.x & 31) == lead) at = atomicAdd(&S->n_listed, __popc(mask));
+    at = __shfl_sync(mask, at, lead) + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
+    list.face[at] = (int)f;
+    list.sl[at] = sl;
+    list.sr[at] = sr;
   }
 }
 
-__global__ void __launch_bounds__(kFaceBlock) face2_lxf_f64_kernel(
-    const double* __restrict__ Q, int64_t n, Eos2 E, Quad6D lobatto, const double* __restrict__ F,
-    const unsigned long long* lam_now, double cfl, double dx, double* __restrict__ FF, double* __restrict__ DM,
-    double* __restrict__ DP, const double* t_now, double t_end, DevState* S) {
+// LxF faces: twice the conservative flux, (f_l + f_r) - lambda (q_r - q_l), and, where
+// the volume fractions do not jump, the fluctuations' zero; the others are listed.
+__global__ void __launch_bounds__(kPair64) face2_lxf_f64_kernel(const double* __restrict__ Q, int64_t n,
+                                                                const double* __restrict__ F,
+                                                                const unsigned long long* lam_now, double cfl,
+                                                                double dx, double* __restrict__ FF,
+                                                                double* __restrict__ DM, FaceList list,
+                                                                const double* t_now, double t_end, DevState* S) {
+  __shared__ int s_hard[2][kPairCells];
+  __shared__ double s_lam;
   if (!(*t_now < t_end)) return;
-  const double lmax = __longlong_as_double((long long)*lam_now);
-  const double lam = step_scalars(cfl, dx, lmax, true).lam_lxf;  // lambda = dx/dt (main.jl:223)
-  const int64_t f = (int64_t)blockIdx.x * kFaceBlock + threadIdx.x;  // face between cells f-1 and f
-  if (f > n) return;
+  const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
+  const int64_t f = (int64_t)blockIdx.x * kPairCells + j;  // face between cells f-1 and f
   const int64_t nf = n + 1;
+  const bool in = f <= n;
   const int64_t L = f > 0 ? f - 1 : 0, R = f < n ? f : n - 1;
-  double QL[30], QR[30], fl[30], fr[30], ff[30], dm[30], dp[30];
-  for (int v = 0; v < 30; ++v) {
-    QL[v] = Q[v * n + L];
-    QR[v] = Q[v * n + R];
-    fl[v] = F[v * n + L];
-    fr[v] = F[v * n + R];
+  if (threadIdx.x < 32) {  // lambda = dx/dt (main.jl:223)
+    const double lam = step_scalars64(cfl, dx, __longlong_as_double((long long)*lam_now), true).lam_lxf;
+    if (threadIdx.x == 0) s_lam = lam;
   }
-  const int st = lxf_face2(E.e, lobatto, QL, QR, fl, fr, lam, ff, dm, dp);
-  if (st) record_err2(S, st, R);
-  for (int v = 0; v < 30; ++v) {
-    FF[v * nf + f] = ff[v];
-    DM[v * nf + f] = dm[v];
-    DP[v * nf + f] = dp[v];
+  __syncthreads();
+  bool hard = false;
+  if (in) {
+    const double nlam = -s_lam;
+    const double* ql = Q + 15 * ph * n;
+    const double* fc = F + 15 * ph * n;
+    float far = 0.0f, Rf[9];
+    bool finite = true, jumps = false;
+#pragma unroll
+    for (int r = 0; r < 15; ++r) {
+      const double a = ql[r * n + L], b = ql[r * n + R], jump = b - a;
+      const int64_t o = (15 * ph + r) * nf + f;
+      if (zero_flux_row(r)) {
+        FF[o] = nlam * jump;
+      } else {
+        const double fs = fc[r * n + L] + fc[r * n + R];
+        finite &= is_finite64(fs);
+        FF[o] = nlam * jump + fs;
+      }
+      DM[o] = 0.0;
+      finite &= is_finite64(jump);
+      if (r == 0) jumps = bits_of(a) != bits_of(b);
+      if (r >= 6) {
+        const float jf = to_f32(jump);
+        far += jf * jf;
+        Rf[r - 6] = to_f32(a);
+      }
+    }
+    hard = L != R && (jumps || !finite || !det_keeps_sign(Rf, far));
+  }
+  s_hard[ph][j] = hard;
+  __syncthreads();
+  if (ph == 0 && (s_hard[0][j] | s_hard[1][j])) {
+    const unsigned mask = __activemask();
+    const int lead = __ffs(mask) - 1;
+    int at = 0;
+    if ((int)(threadIdx.x & 31) == lead) at = atomicAdd(&S->n_listed, __popc(mask));
+    at = __shfl_sync(mask, at, lead) + __popc(mask & ((1u << (threadIdx.x & 31)) - 1u));
+    list.face[at] = (int)f;
   }
 }
 
-__global__ void __launch_bounds__(kBlock) update2_f64_kernel(const double* __restrict__ Q, double* __restrict__ Qn,
-                                                             int64_t n, const double* __restrict__ FF,
-                                                             const double* __restrict__ DM,
-                                                             const double* __restrict__ DP,
-                                                             const unsigned long long* lam_in,
-                                                             unsigned long long* lam_next, const double* t_in,
-                                                             double* t_out, long long* steps, double t_end,
-                                                             double cfl, double dx, int bc) {
+// ---- path integrals of the listed faces -------------------------------------------
+
+// What the other phase needs of one phase at a node (HyperelasticityMPh.jl:186-217):
+// velocity, stress row 1 (sigma symmetric), temperature dE/dS (:212).
+struct Half64 {
+  double u[3], K[3], T;
+};
+template <int kDef>
+__device__ __forceinline__ int half64(const EosC& e, const Eos64& k, double ia, const double* m, double rE,
+                                      const double* R, Half64& h) {
+  const Cell64 c = cell64<kDef>(e, k, ia, m, rE, R);
+  const double m2 = -2.0 * c.td;
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    h.u[v] = c.u[v];
+    h.K[v] = m2 * c.w[v];
+  }
+  h.T = e.t0 * (c.Pg + c.px);
+  return c.st;
+}
+
+// Interface velocity, stress and its power (HyperelasticityMPh.jl:218-232, omega = 0,
+// k = 1/2): the same for both phases.
+struct Face64 {
+  double u[3], s[3], p;
+};
+__device__ __forceinline__ Face64 interface64(const Half64& a, const Half64& b) {
+  Face64 I;
+  const double inv = rcp64(a.T + b.T), ha = b.T * inv, hb = a.T * inv;
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    I.u[v] = 0.5 * (a.u[v] + b.u[v]);
+    I.s[v] = ha * a.K[v] + hb * b.K[v];
+  }
+  I.p = I.s[0] * I.u[0] + I.s[1] * I.u[1] + I.s[2] * I.u[2];
+  return I;
+}
+
+// acc += wd B(q) e_alpha for one phase's rows (row 1 of B is zero), B's rho A part with
+// alpha rho A / alpha in place of rho A.
+__device__ __forceinline__ void add_b64(double wd, double ia, const double* R, const double* u, const Face64& I,
+                                        double* acc) {
+  acc[0] = fma(wd, I.u[0], acc[0]);
+  acc[2] = fma(wd, I.s[0], acc[2]);
+  acc[3] = fma(wd, I.s[1], acc[3]);
+  acc[4] = fma(wd, I.s[2], acc[4]);
+  acc[5] = fma(wd, I.p, acc[5]);
+  const double wi = wd * ia, d1 = I.u[1] - u[1], d2 = I.u[2] - u[2];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double* r = R + 3 * c;
+    const double w0 = wi * r[0];
+    acc[6 + 3 * c] = fma(wi, r[0] * I.u[0] + r[1] * d1 + r[2] * d2, acc[6 + 3 * c]);
+    acc[7 + 3 * c] = fma(w0, u[1], acc[7 + 3 * c]);
+    acc[8 + 3 * c] = fma(w0, u[2], acc[8 + 3 * c]);
+  }
+}
+
+// One thread per face: acc += the path integral from a to b (30 values each), 6 nodes of
+// both phases, 360 slots a node. Rolled: six copies of the node overflow the
+// instruction cache.
+template <int kDef>
+__device__ __forceinline__ int path_thread(const Eos2x& E, const Quad6D& qd, const double* a, const double* b,
+                                           double* acc) {
+  int st = 0;
+  const double da0 = b[0] - a[0], da1 = b[15] - a[15];
+#pragma unroll 1
+  for (int i = 0; i < 6; ++i) {
+    const double s = qd.x[i];
+    double R[2][9], ia[2];
+    Half64 h[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      double m[3];
+      auto at = [&](int k) { return fma(s, b[15 * p + k] - a[15 * p + k], a[15 * p + k]); };
+#pragma unroll
+      for (int v = 0; v < 3; ++v) m[v] = at(2 + v);
+#pragma unroll
+      for (int v = 0; v < 9; ++v) R[p][v] = at(6 + v);
+      ia[p] = rcp64(at(0));
+      st |= half64<kDef>(E.e[p], E.k[p], ia[p], m, at(5), R[p], h[p]);
+    }
+    const Face64 I = interface64(h[0], h[1]);
+    add_b64(qd.w[i] * da0, ia[0], R[0], h[0].u, I, acc);
+    add_b64(qd.w[i] * da1, ia[1], R[1], h[1].u, I, acc + 15);
+  }
+  return st;
+}
+
+constexpr int kPathBlock = 128;
+constexpr int kGroups = kPathBlock / 16;  // faces a block works on at a time, 16 lanes each
+
+// Per group of 16 lanes: what the nodes add to each row, and the states of the face.
+struct GroupMem {
+  double part[12][15];  // by lane: B's rows times weight and d(alpha)
+  double q[3][30];      // q_l, q_r, Q_hll
+};
+
+// 16 lanes per face, lane r < 12 on node r % 6 of phase r / 6: one integral is one pass
+// of a phase's forms (about 190 slots) and an exchange with the lane of the other phase,
+// against 12 passes on one thread; adds the integral from q[from] to q[to] to the
+// partials.
+template <int kDef>
+__device__ __forceinline__ int path_group(const Eos2x& E, const Quad6D& qd, int lane16, GroupMem& g, int from, int to,
+                                          double* acc) {
+  const int ph = lane16 < 6 ? 0 : 1, node = lane16 < 12 ? lane16 - 6 * ph : 0;
+  const double s = qd.x[node];
+  const double* a = g.q[from] + 15 * ph;
+  const double* b = g.q[to] + 15 * ph;
+  auto at = [&](int k) { return fma(s, b[k] - a[k], a[k]); };
+  double m[3], R[9];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) m[v] = at(2 + v);
+#pragma unroll
+  for (int v = 0; v < 9; ++v) R[v] = at(6 + v);
+  const double ia = rcp64(at(0));
+  Half64 h, o;
+  const EosC& e = E.e[ph];
+  const Eos64 k = ph ? E.k[1] : E.k[0];
+  int st = half64<kDef>(e, k, ia, m, at(5), R, h);
+  const int other = (threadIdx.x & 16) + (ph ? node : node + 6);  // its node's lane of the other phase
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    o.u[v] = __shfl_sync(0xffffffffu, h.u[v], other);
+    o.K[v] = __shfl_sync(0xffffffffu, h.K[v], other);
+  }
+  o.T = __shfl_sync(0xffffffffu, h.T, other);
+  const Face64 I = interface64(h, o);
+  add_b64(qd.w[node] * (b[0] - a[0]), ia, R, h.u, I, acc);
+  return lane16 < 12 ? st : 0;
+}
+
+// The sum over a face's six nodes of row k (30 rows).
+__device__ __forceinline__ double node_sum(const GroupMem& g, int k) {
+  const int ph = k < 15 ? 0 : 1, r = k - 15 * ph;
+  double v = g.part[6 * ph][r];
+#pragma unroll
+  for (int i = 1; i < 6; ++i) v += g.part[6 * ph + i][r];
+  return v;
+}
+
+// Lists of up to kGroupFaces faces per multiprocessor run in groups: a warp spends 620
+// slots on the two faces of its groups, and 6,600 on 32 faces with a thread each, so
+// groups win up to 10.6 x 2 faces on each of an SM's four schedulers. 1000 cells, 50 HLL
+// steps of a Riemann problem (whole run): 22.3 ms before this file's split of the faces,
+// 2.95 ms now; 100,003 cells with all faces listed, 4 steps: 10.3 and 6.6 ms.
+constexpr int kGroupFaces = 80;
+
+// kLxf: one Gauss-Lobatto integral, D- = D+ = half of it (NumFluxes.jl:36-47), stored
+// doubled as the LxF faces are. Otherwise Q_hll and the fluctuations of
+// NumFluxes.jl:85-132.
+template <int kDef, bool kLxf>
+__global__ void __launch_bounds__(kPathBlock, 2)
+    paths2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E, Quad6D qd, const double* __restrict__ F,
+                      double* __restrict__ DM, double* __restrict__ DP, FaceList list, const double* t_now,
+                      double t_end, int sms, DevState* S) {
+  __shared__ GroupMem sg[kGroups];
+  if (!(*t_now < t_end)) return;
+  const int count = S->n_listed;
+  const int64_t nf = n + 1;
+  if (count <= kGroupFaces * sms) {
+    const int blocks = min((int)gridDim.x, 2 * sms);  // a scheduler's second warp covers what is not FP64
+    if ((int)blockIdx.x >= blocks) return;
+    const int lane16 = threadIdx.x & 15;
+    GroupMem& g = sg[threadIdx.x >> 4];
+    // both groups of a warp go round together (the exchanges are warp-wide): an idle one
+    // repeats the list's last face and stores nothing
+    const int first = blockIdx.x * kGroups + (threadIdx.x >> 4), pair = first & ~1;
+    for (int t = first, tp = pair; tp < count; t += blocks * kGroups, tp += blocks * kGroups) {
+      const bool live = t < count;
+      const int at = live ? t : count - 1;
+      const int64_t f = list.face[at], L = f - 1, R = f;
+      for (int k = lane16; k < 30; k += 16) {
+        g.q[0][k] = Q[k * n + L];
+        g.q[1][k] = Q[k * n + R];
+      }
+      __syncwarp();
+      double acc[15];
+#pragma unroll
+      for (int r = 0; r < 15; ++r) acc[r] = 0.0;
+      int st = path_group<kDef>(E, qd, lane16, g, 0, 1, acc);
+      if (lane16 < 12)
+#pragma unroll
+        for (int r = 0; r < 15; ++r) g.part[lane16][r] = acc[r];
+      __syncwarp();
+      if (kLxf) {
+        if (live)
+          for (int k = lane16; k < 30; k += 16) DM[k * nf + f] = node_sum(g, k);
+      } else {
+        const double sl = list.sl[at], sr = list.sr[at], idsr = rcp64(sr - sl);
+        for (int k = lane16; k < 30; k += 16) {
+          const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
+          g.q[2][k] = ((g.q[1][k] * sr - g.q[0][k] * sl) - (node_sum(g, k) + df)) * idsr;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < 15; ++r) acc[r] = 0.0;
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half)
+          st |= path_group<kDef>(E, qd, lane16, g, half ? 2 : 0, half ? 1 : 2, acc);
+        if (lane16 < 12)
+#pragma unroll
+          for (int r = 0; r < 15; ++r) g.part[lane16][r] = acc[r];
+        __syncwarp();
+        const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
+        if (live)
+          for (int k = lane16; k < 30; k += 16) {
+            const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
+            const double inner = df + node_sum(g, k), qj = cq * (g.q[1][k] - g.q[0][k]);
+            DM[k * nf + f] = cm * inner + qj;
+            DP[k * nf + f] = cp * inner - qj;
+          }
+      }
+      if (st && live) record_err64(S, st, R);
+      __syncwarp();
+    }
+    return;
+  }
+  const int t = blockIdx.x * kPathBlock + threadIdx.x;
+  if (t < count) {
+    const int64_t f = list.face[t], L = f - 1, R = f;
+    double a[30], b[30], acc[30];
+    for (int k = 0; k < 30; ++k) {
+      a[k] = Q[k * n + L];
+      b[k] = Q[k * n + R];
+      acc[k] = 0.0;
+    }
+    int st = path_thread<kDef>(E, qd, a, b, acc);
+    if (kLxf) {
+      for (int k = 0; k < 30; ++k) DM[k * nf + f] = acc[k];
+    } else {
+      const double sl = list.sl[t], sr = list.sr[t], idsr = rcp64(sr - sl);
+      double h[30];
+      for (int k = 0; k < 30; ++k) {
+        const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
+        h[k] = ((b[k] * sr - a[k] * sl) - (acc[k] + df)) * idsr;
+        acc[k] = df;
+      }
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) st |= path_thread<kDef>(E, qd, half ? h : a, half ? b : h, acc);
+      const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
+      for (int k = 0; k < 30; ++k) {
+        const double qj = cq * (b[k] - a[k]);
+        DM[k * nf + f] = cm * acc[k] + qj;
+        DP[k * nf + f] = cp * acc[k] - qj;
+      }
+    }
+    if (st) record_err64(S, st, R);
+  }
+}
+
+// FF: twice the LxF face flux (with D- = D+ doubled as well), or null for HLL.
+__global__ void __launch_bounds__(kBlock64) update2_f64_kernel(const double* __restrict__ Q, double* __restrict__ Qn,
+                                                               int64_t n, const double* __restrict__ FF,
+                                                               const double* __restrict__ DM,
+                                                               const double* __restrict__ DP,
+                                                               const unsigned long long* lam_in,
+                                                               unsigned long long* lam_next, const double* t_in,
+                                                               double* t_out, DevState* S, double t_end, double cfl,
+                                                               double dx, int bc) {
+  __shared__ double s_r;
   const double tn = *t_in;
   const bool active = tn < t_end;
-  const double lmax = __longlong_as_double((long long)*lam_in);
-  const StepScalars sc = step_scalars(cfl, dx, lmax, false);
-  const double dt = sc.dt, dtdx = sc.dtdx;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *t_out = active ? tn + dt : tn;
-    *lam_next = 0ull;
-    if (active) *steps += 1;
+  if (threadIdx.x < 32) {
+    const StepScalars sc = step_scalars64(cfl, dx, __longlong_as_double((long long)*lam_in), false);
+    if (threadIdx.x == 0) s_r = FF ? 0.5 * sc.dtdx : sc.dtdx;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      *t_out = active ? tn + sc.dt : tn;
+      *lam_next = 0ull;
+      S->n_listed = 0;
+      if (active) S->steps += 1;
+    }
   }
   if (!active) return;
-  const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+  __syncthreads();
+  const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
   if (i >= n) return;
   const int64_t nf = n + 1;
   if (bc == HYP_BC_FROZEN && (i == 0 || i == n - 1)) {
     for (int v = 0; v < 30; ++v) Qn[v * n + i] = Q[v * n + i];
     return;
   }
+  const double r = s_r;
+#pragma unroll 6
   for (int v = 0; v < 30; ++v) {
     // F_r = F_l = zeros(30) for hll (NumFluxes.jl:82), NF_r = D- of face i+1/2, NF_l = D+ of face i-1/2
-    const double fr = FF ? FF[v * nf + i + 1] : 0.0, fl = FF ? FF[v * nf + i] : 0.0;
-    const double nfr = DM[v * nf + i + 1], nfl = DP[v * nf + i];
-    Qn[v * n + i] = Q[v * n + i] - dtdx * ((fr - fl) + (nfr + nfl));
+    double d = DM[v * nf + i + 1] + DP[v * nf + i];
+    if (FF) d += FF[v * nf + i + 1] - FF[v * nf + i];
+    Qn[v * n + i] = fma(-r, d, Q[v * n + i]);
   }
 }
 
 static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
+static Eos2x eos2x(const hyp_ctx* c) {
+  Eos2x E;
+  for (int p = 0; p < 2; ++p) {
+    E.e[p] = c->eos2.e[p];
+    E.k[p] = make_eos64(E.e[p]);
+  }
+  return E;
+}
+static bool default_exp2(const hyp_ctx* c) { return c->eos2.e[0].default_exp && c->eos2.e[1].default_exp; }
+
 cudaError_t launch_cell2_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end) {
-  cell2_f64_kernel<<<grid_n(c->n, kBlock), kBlock, 0, c->stream>>>(c->Q[p], c->n, c->eos2, c->F, c->smin, c->smax,
-                                                                    lam_slot, t_now, t_end, c->st);
+  auto kern = default_exp2(c) ? cell2_f64_kernel<1> : cell2_f64_kernel<0>;
+  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(c->Q[p], c->n, eos2x(c), c->F, c->smin, c->smax, lam_slot,
+                                                            t_now, t_end, c->st);
   return cudaGetLastError();
 }
 cudaError_t launch_face2_f64(hyp_ctx* c, int p, double t_end) {
-  if (c->cfg.flux == HYP_FLUX_LXF) {
+  const bool lxf = c->cfg.flux == HYP_FLUX_LXF, def = default_exp2(c);
+  const FaceList list{c->face_list, c->face_s, c->face_s ? c->face_s + c->n + 1 : nullptr};
+  const unsigned grid = grid_n(c->n + 1, kPairCells);
+  const Eos2x E = eos2x(c);
+  if (lxf) {
     const double dx = c->cfg.x_length / (double)c->n;
-    face2_lxf_f64_kernel<<<grid_n(c->n + 1, kFaceBlock), kFaceBlock, 0, c->stream>>>(
-        c->Q[p], c->n, c->eos2, c->lobatto, c->F, &c->st->lam_bits[p], c->cfg.cfl, dx, c->FF, c->DM, c->DP,
-        &c->st->t[p], t_end, c->st);
+    face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, c->F, &c->st->lam_bits[p], c->cfg.cfl, dx,
+                                                          c->FF, c->DM, list, &c->st->t[p], t_end, c->st);
   } else {
-    face2_f64_kernel<<<grid_n(c->n + 1, kFaceBlock), kFaceBlock, 0, c->stream>>>(
-        c->Q[p], c->n, c->eos2, c->quad, c->F, c->smin, c->smax, c->DM, c->DP, &c->st->t[p], t_end, c->st);
+    auto kern = def ? face2_f64_kernel<1> : face2_f64_kernel<0>;
+    kern<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, E, c->F, c->smin, c->smax, c->DM, c->DP, list, &c->st->t[p],
+                                          t_end, c->st);
   }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  auto paths = lxf ? (def ? paths2_f64_kernel<1, true> : paths2_f64_kernel<0, true>)
+                   : (def ? paths2_f64_kernel<1, false> : paths2_f64_kernel<0, false>);
+  // a block per 128 faces, were all of them listed; those past the list's end return at once
+  const unsigned pgrid = std::max(grid_n(c->n + 1, kPathBlock), (unsigned)(2 * c->sms));
+  paths<<<pgrid, kPathBlock, 0, c->stream>>>(c->Q[p], c->n, E, lxf ? c->lobatto : c->quad, c->F, c->DM, c->DP, list,
+                                             &c->st->t[p], t_end, c->sms, c->st);
   return cudaGetLastError();
 }
 cudaError_t launch_update2_f64(hyp_ctx* c, int p, double t_end) {
   const double dx = c->cfg.x_length / (double)c->n;
-  update2_f64_kernel<<<grid_n(c->n, kBlock), kBlock, 0, c->stream>>>(
-      c->Q[p], c->Q[1 - p], c->n, c->FF, c->DM, c->DP, &c->st->lam_bits[p], &c->st->lam_bits[1 - p], &c->st->t[p],
-      &c->st->t[1 - p], &c->st->steps, t_end, c->cfg.cfl, dx, c->cfg.bc);
+  const bool lxf = c->cfg.flux == HYP_FLUX_LXF;
+  update2_f64_kernel<<<grid_n(c->n, kBlock64), kBlock64, 0, c->stream>>>(
+      c->Q[p], c->Q[1 - p], c->n, lxf ? c->FF : nullptr, c->DM, lxf ? c->DM : c->DP, &c->st->lam_bits[p],
+      &c->st->lam_bits[1 - p], &c->st->t[p], &c->st->t[1 - p], c->st, t_end, c->cfg.cfl, dx, c->cfg.bc);
   return cudaGetLastError();
 }
 
