@@ -14,7 +14,8 @@
 //  - The closed forms use H = G^2 = i1 G - i2 I + p M with M = A A^T = G^-1
 //    (Cayley-Hamilton, p = det G), so G^2 is never formed. With b = b0sq/2 p^(beta/2)
 //    and a = 2/3 b i1, row 1 of the stress is s0 = -2 rho w,
-//      w_j = a G0j + b p M0j + (E3 p - b i2) [j = 0],
+//      w_j = a G0j + b p M0j + (E3 p - b i2) [j = 0] = b (H_0j - i1/3 G0j) + E3 p [j = 0]
+//    (the first form for j = 1, 2, the second, without cancellation, for j = 0),
 //    and along dA = e_j A[0,:] the derivatives of M's row 1 are dM_0i = [j=0] M_0i +
 //    M_00 [i=j]: the acoustic tensor (n = e1) collapses to Omega = 2 O with
 //      O_ij = f G0i G0j + a G_ij - b p M00 [i=j]   (i, j >= 1),  f = 4/3 b,
@@ -34,7 +35,7 @@
 //    clear; the general eigen-solve is kept for the rest.
 //  - Range and NaN checks compare bit patterns.
 //
-// Per cell 168 FP64 instructions by this count, where the forms of hyp_physics.cuh
+// Per cell 180 FP64 instructions as executed, where the forms of hyp_physics.cuh
 // (which the adjoint and the function-level evaluators use) execute 379; the two agree
 // to a few ulps (tests/test_cell64_host.py).
 #pragma once
@@ -221,10 +222,13 @@ HYP_HD Cell64 cell64(const EosC& e, const Eos64& k, double ia, const double* m, 
   o.G12 = k12 * gs;
   o.G22 = k22 * gs;
   const double i1 = (k00 + k11 + k22) * gs;
-  const double i2 = (n00 + n11 + n22) * ms;  // i2 = p tr M
   const double s = o.td * k.inv_rho0;        // 1/det A = sqrt(p)
   const double p = s * s;
-  const double psi = (i1 * (1.0 / 3.0)) * i1 - i2;
+  // psi = i1^2/3 - i2 = |dev G|^2 / 2, and row 1 of the stress below, from the deviator's
+  // diagonal: small numbers squared instead of large ones subtracted
+  const double th = i1 * (1.0 / 3.0), d0 = o.G00 - th, d1 = o.G11 - th, d2 = o.G22 - th;
+  const double off = o.G01 * o.G01 + o.G02 * o.G02;
+  const double psi = 0.5 * (d0 * d0 + d1 * d1 + d2 * d2) + (o.G12 * o.G12 + off);
   double Pb, inv_Pg;  // inv_Pg: over cv t0
   if (kDef == 1) {
     o.Pa = s;
@@ -251,8 +255,8 @@ HYP_HD Cell64 cell64(const EosC& e, const Eos64& k, double ia, const double* m, 
   o.E3p = o.T1 + o.T2 + o.T3;
   o.a = (2.0 / 3.0) * (o.b * i1);
   o.bM = o.b * (n00 * ms);
-  o.w[0] = o.a * o.G00 + (o.bM + (o.E3p - o.b * i2));
-  o.wE = o.a * o.G00 + (o.bM - o.b * i2);
+  o.wE = o.b * (o.G00 * d0 + off);
+  o.w[0] = o.b * (o.G00 * d0 + off) + o.E3p;
   o.w[1] = o.a * o.G01 + o.b * (n01 * ms);
   o.w[2] = o.a * o.G02 + o.b * (n02 * ms);
   return o;
@@ -294,7 +298,10 @@ HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
   const float C2 = to_f32(c2), C1 = to_f32(c1), C0 = to_f32(c0);
   const float P = C1 - C2 * C2 * (1.0f / 3.0f);
   const float Q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
-  if (P < 0.0f && 0.25f * Q * Q + P * P * P * (1.0f / 27.0f) < 0.0f) {  // three real roots
+  // A symmetric matrix has three real roots; two equal ones (a material at rest or under
+  // isotropic strain has two equal shear speeds) put the cosine at 1 up to rounding,
+  // where the clamp below costs the largest root an error of second order only.
+  if (P < 0.0f) {
     const float am = 2.0f * sqrtf(-P * (1.0f / 3.0f));
     const float cc = fminf(1.0f, fmaxf(-1.0f, 3.0f * Q / (P * am)));
     const float y = am * cosf(acosf(cc) * (1.0f / 3.0f)) + C2 * (1.0f / 3.0f);  // the largest root
