@@ -333,8 +333,7 @@ extern "C" int hyp_adjoint_record(hyp_ctx* c, int n_steps, int ckpt_every, doubl
     if (s % ckpt_every == 0)
       ACK(cudaMemcpyAsync(t->ckpt + (size_t)(s / ckpt_every) * 14 * c->n, c->Q[p], bytes, cudaMemcpyDeviceToDevice,
                           c->stream));
-    ACK(launch_cell1_f64(c, p, &c->st->lam_bits[p], &c->st->t[p], inf));
-    ACK(launch_update1_f64(c, p, inf));
+    ACK(launch_run_step1_f64(c, k, inf, s == 0, s == n_steps - 1));
   }
   ACK(cudaEventRecord(t->ev[1], c->stream));
   if ((rc = ctx_sync_state(c)) != HYP_OK) return rc;
@@ -375,15 +374,30 @@ extern "C" int hyp_adjoint(hyp_ctx* c, const double* dL_dQ_final, double* dL_dQ0
     ACK(cudaEventRecord(t->ev[0], c->stream));
     // rerun the segment from its checkpoint with the step kernels
     ACK(cudaMemcpyAsync(t->seg_Q, t->ckpt + (size_t)s * 14 * n, bytes, cudaMemcpyDeviceToDevice, c->stream));
-    ACK(cudaMemsetAsync(t->seg_lmax, 0, sizeof(unsigned long long), c->stream));
-    for (int k = 0; k < L; ++k) {
-      double* Qk = t->seg_Q + (size_t)k * 14 * n;
-      double* Fk = t->seg_F + (size_t)k * kNFlux1 * n;
-      double* lk = t->seg_lam + (size_t)k * n;
-      ACK(launch_cell1(c->stream, Qk, n, c->eos[0], Fk, lk, &t->seg_lmax[k], &t->seg_t[k], inf, c->st));
-      if (k + 1 < L)
-        ACK(launch_update1(c->stream, Qk, Qk + 14 * n, n, Fk, lk, &t->seg_lmax[k], &t->seg_lmax[k + 1], &t->seg_t[k],
-                           &t->seg_t[k + 1], t->seg_steps, inf, c->cfg.cfl, dx, c->cfg.flux, c->cfg.bc));
+    ACK(cudaMemsetAsync(t->seg_lmax, 0, (size_t)(t->K + 1) * sizeof(unsigned long long), c->stream));
+    ACK(launch_cell1(c->stream, t->seg_Q, n, c->eos[0], t->seg_F, t->seg_lam, t->seg_lmax, t->seg_t, inf, c->st));
+    for (int k = 0; k + 1 < L; ++k) {
+      Step1Args a1;
+      a1.Q = t->seg_Q + (size_t)k * 14 * n;
+      a1.Qn = t->seg_Q + (size_t)(k + 1) * 14 * n;
+      a1.F = t->seg_F + (size_t)k * kNFlux1 * n;
+      a1.Fn = t->seg_F + (size_t)(k + 1) * kNFlux1 * n;
+      a1.lam = t->seg_lam + (size_t)k * n;
+      a1.lamn = t->seg_lam + (size_t)(k + 1) * n;
+      a1.rd = &t->seg_lmax[k];
+      a1.wr = &t->seg_lmax[k + 1];
+      a1.clr[0] = a1.clr[1] = nullptr;
+      a1.t_in = &t->seg_t[k];
+      a1.t_out = &t->seg_t[k + 1];
+      a1.steps = t->seg_steps;
+      a1.t_end = inf;
+      a1.cfl = c->cfg.cfl;
+      a1.dx = dx;
+      a1.n = n;
+      a1.flux = c->cfg.flux;
+      a1.bc = c->cfg.bc;
+      a1.S = c->st;
+      ACK(launch_step1(c->stream, a1, c->eos[0]));
     }
     ACK(cudaEventRecord(t->ev[1], c->stream));
     // adjoint steps a + L - 1 .. a

@@ -46,7 +46,7 @@ struct TileCtl {
 // Per-problem loop control on the device.
 struct BatchDev {
   double* t;                   // [2][P] time before the step of parity p
-  unsigned long long* slots;   // mixed: [3][P] FP32 max-lambda bits; FP64: [2][P] FP64 max-lambda bits
+  unsigned long long* slots;   // [3][P] max-lambda bits, FP32 (mixed) or FP64
   long long* steps;            // [P]
   double* dx;                  // [P]
   int P;
@@ -187,35 +187,43 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* 
   if (!(b.t[par * b.P + d.problem] < t_end)) return;
   const int64_t i = d.first + threadIdx.x;
   const bool own = threadIdx.x < kCells64 && i < d.hi;
-  const double l = own ? cell1_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = own ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(&slot_base[d.problem], m);
 }
 
-// Each face of the tile once into shared memory, then the update, as update1_f64_kernel.
-__global__ void __launch_bounds__(kBlock64) batch_f64_update_kernel(const double* __restrict__ Q,
-                                                                    double* __restrict__ Qn, int64_t n,
-                                                                    const double* __restrict__ F,
-                                                                    const double* __restrict__ lam,
-                                                                    const TileDesc* __restrict__ tiles, BatchDev b,
-                                                                    int par, double t_end, double cfl, int flux,
-                                                                    int bc) {
+// A step of the batch, as step1_f64_kernel: the update and, but for the last step of a
+// call (kCell = false), the cell pass of the new state. The problem's slots: rd holds the
+// max wave speed, its lead tile clears the one a later step writes (a problem past t_end
+// clears all three: whatever steps it next starts with a cell pass).
+template <int kDef, bool kCell>
+__global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
+    const double* __restrict__ Q, double* __restrict__ Qn, int64_t n, EosC e, Eos64 k, const double* __restrict__ F,
+    const double* __restrict__ lam, double* __restrict__ Fn, double* __restrict__ lamn,
+    const TileDesc* __restrict__ tiles, BatchDev b, int par, int rd, int wr, int clr, double t_end, double cfl,
+    int flux, int bc, DevState* S) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell first + k
   __shared__ double s_hdt;
+  __shared__ int s_more;
   const int P = b.P, j = threadIdx.x;
   const bool lxf = flux == HYP_FLUX_LXF;
   const TileDesc d = tiles[blockIdx.x];
   const int p = d.problem;
   const double tn = b.t[par * P + p];
   const bool active = tn < t_end;
-  const double lmax = __longlong_as_double((long long)b.slots[par * P + p]);
+  const double lmax = __longlong_as_double((long long)b.slots[rd * P + p]);
   StepScalars sc{0.0, 0.0, 0.0};
   if (j < 32 || lxf) sc = step_scalars64(cfl, b.dx[p], lmax, lxf);
-  if (j == 0) s_hdt = 0.5 * sc.dtdx;
-  if (d.lead && j == 0) {
-    b.t[(1 - par) * P + p] = active ? tn + sc.dt : tn;
-    b.slots[(1 - par) * P + p] = 0ull;
-    if (active) b.steps[p] += 1;
+  if (j == 0) {
+    s_hdt = 0.5 * sc.dtdx;
+    s_more = kCell && tn + sc.dt < t_end;
+    if (d.lead) {
+      b.t[(1 - par) * P + p] = active ? tn + sc.dt : tn;
+      b.slots[clr * P + p] = 0ull;
+      if (!kCell || !active) b.slots[wr * P + p] = 0ull;
+      if (active) b.steps[p] += 1;
+      else b.slots[rd * P + p] = 0ull;
+    }
   }
   const int64_t i = d.first + j;
   const bool own = j < kCells64 && i < d.hi;
@@ -231,14 +239,21 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_update_kernel(const double
     for (int v = 0; v < 14; ++v) sF[v][j] = f2[v];
   }
   __syncthreads();
-  if (!own) return;
-  const bool frozen = bc == HYP_BC_FROZEN && (i == d.lo || i == d.hi - 1);
-  const double hdt = s_hdt;
+  double q[14];
+  if (own) {
+    const bool frozen = bc == HYP_BC_FROZEN && (i == d.lo || i == d.hi - 1);
+    const double hdt = s_hdt;
 #pragma unroll
-  for (int v = 0; v < 14; ++v) {
-    const double qc = Q[v * n + i];
-    Qn[v * n + i] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+    for (int v = 0; v < 14; ++v) {
+      const double qc = Q[v * n + i];
+      q[v] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+      Qn[v * n + i] = q[v];
+    }
   }
+  if (!kCell || !s_more) return;
+  const double l = own ? cell1_pass<kDef>(q, n, i, e, k, Fn, lamn, S) : 0.0;
+  const unsigned long long m = block_max_bits<kBlock64>(l);
+  if (j == 0) atomicMax(&b.slots[wr * P + p], m);
 }
 
 // A variant: block size, resident blocks per SM the registers are budgeted for,
@@ -289,8 +304,8 @@ struct hyp_batch {
   float* Qh[2] = {nullptr, nullptr};
   // FP64 state
   double* Q[2] = {nullptr, nullptr};
-  double* F = nullptr;
-  double* lam = nullptr;
+  double* F[2] = {nullptr, nullptr};  // of the state of each parity
+  double* lam[2] = {nullptr, nullptr};
   // per-problem control
   BatchDev b{};
   DevState* st = nullptr;
@@ -366,11 +381,12 @@ static MixedArrays batch_arrays(hyp_batch* b, int p) {
   return a;
 }
 
-static int enqueue_batch_step(hyp_batch* b, long long k, double t_end) {
+// (first, last: of the steps of one call)
+static int enqueue_batch_step(hyp_batch* b, long long k, double t_end, bool first, bool last) {
   const int par = (int)(k & 1);
+  const int rd = (int)(k % 3), wr = (int)((k + 1) % 3), clr = (int)((k + 2) % 3);
   if (b->mixed) {
     const MixedArrays a = batch_arrays(b, par);
-    const int rd = (int)(k % 3), wr = (int)((k + 1) % 3), clr = (int)((k + 2) % 3);
     batch_mixed_ctl_kernel<<<(b->ntiles + 255) / 256, 256, 0, b->stream>>>(b->tiles, b->ntiles, b->b, par, rd, wr, clr,
                                                                           t_end, b->cfg.cfl, b->ctl);
     BCK(cudaGetLastError());
@@ -387,13 +403,18 @@ static int enqueue_batch_step(hyp_batch* b, long long k, double t_end) {
     BCK(e);
   } else {
     const Eos64 k64 = make_eos64(b->eos);
-    auto cell = b->eos.default_exp ? batch_f64_cell_kernel<1> : batch_f64_cell_kernel<0>;
-    cell<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->total, b->eos, k64, b->F, b->lam, b->tiles,
-                                                b->b, par, t_end, b->b.slots + (size_t)par * b->P, b->st);
-    BCK(cudaGetLastError());
-    batch_f64_update_kernel<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->F, b->lam,
-                                                                   b->tiles, b->b, par, t_end, b->cfg.cfl,
-                                                                   b->cfg.flux, b->cfg.bc);
+    const bool def = b->eos.default_exp, apart = b->F[1] == b->F[0];
+    if (first || apart) {
+      auto cell = def ? batch_f64_cell_kernel<1> : batch_f64_cell_kernel<0>;
+      cell<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->total, b->eos, k64, b->F[par], b->lam[par], b->tiles,
+                                                  b->b, par, t_end, b->b.slots + (size_t)rd * b->P, b->st);
+      BCK(cudaGetLastError());
+    }
+    auto step = last || apart ? batch_f64_step_kernel<1, false>
+                              : (def ? batch_f64_step_kernel<1, true> : batch_f64_step_kernel<0, true>);
+    step<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->eos, k64, b->F[par],
+                                                b->lam[par], b->F[1 - par], b->lam[1 - par], b->tiles, b->b, par, rd,
+                                                wr, clr, t_end, b->cfg.cfl, b->cfg.flux, b->cfg.bc, b->st);
     BCK(cudaGetLastError());
   }
   return HYP_OK;
@@ -406,8 +427,8 @@ static void free_batch(hyp_batch* b) {
   if (b->graph) cudaGraphExecDestroy(b->graph);
   for (int p = 0; p < 2; ++p) cudaFree(b->Q[p]);
   cudaFree(b->mixed_base);
-  cudaFree(b->F);
-  cudaFree(b->lam);
+  if (b->F[1] != b->F[0]) cudaFree(b->F[1]);
+  cudaFree(b->F[0]);
   cudaFree(b->b.t);
   cudaFree(b->b.slots);
   cudaFree(b->b.steps);
@@ -465,8 +486,13 @@ extern "C" int hyp_batch_create(const hyp_config* cfg, const int64_t* offsets, i
     for (int p = 0; p < 2 && rc == HYP_OK; ++p) ck(cudaMalloc(&b->Q[p], nq * sizeof(double)));
   }
   if (!b->mixed) {
-    ck(cudaMalloc(&b->F, (size_t)kNFlux1 * b->total * sizeof(double)));
-    ck(cudaMalloc(&b->lam, (size_t)b->total * sizeof(double)));
+    const size_t nf = (size_t)(kNFlux1 + 1) * b->total * sizeof(double);  // fluxes, then the wave speeds
+    ck(cudaMalloc(&b->F[0], nf));
+    if (rc == HYP_OK && cudaMalloc(&b->F[1], nf) != cudaSuccess) {
+      (void)cudaGetLastError();  // no room for a second one: the step's kernels run apart
+      b->F[1] = b->F[0];
+    }
+    for (int p = 0; p < 2; ++p) b->lam[p] = b->F[p] + (size_t)kNFlux1 * b->total;
   }
   ck(cudaMalloc(&b->b.t, (size_t)2 * n_problems * sizeof(double)));
   ck(cudaMalloc(&b->b.slots, (size_t)3 * n_problems * sizeof(unsigned long long)));
@@ -565,7 +591,8 @@ extern "C" int hyp_batch_step(hyp_batch* b, int n_steps, double t_end) {
     cudaGraph_t g;
     BCK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     int rc = HYP_OK;
-    for (int s = 0; s < n_steps && rc == HYP_OK; ++s) rc = enqueue_batch_step(b, b->k + s, t_end);
+    for (int s = 0; s < n_steps && rc == HYP_OK; ++s)
+      rc = enqueue_batch_step(b, b->k + s, t_end, s == 0, s == n_steps - 1);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (rc != HYP_OK) return rc;
     BCK(e);

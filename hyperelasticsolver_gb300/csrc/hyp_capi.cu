@@ -47,7 +47,8 @@ static int free_ctx(hyp_ctx* c) {
   for (int p = 0; p < 2; ++p) cudaFree(c->Q[p]);
   cudaFree(c->mixed_base);
   cudaFree(c->F);
-  cudaFree(c->lam);
+  if (c->flux1[1] != c->flux1[0]) cudaFree(c->flux1[1]);
+  cudaFree(c->flux1[0]);
   cudaFree(c->smin);
   cudaFree(c->smax);
   cudaFree(c->DM);
@@ -161,10 +162,13 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
   } else if (!mixed(c)) {
     for (int p = 0; p < 2 && rc == HYP_OK; ++p)
       if ((e = cudaMalloc(&c->Q[p], nq)) != cudaSuccess) fail(e, "cudaMalloc(Q)");
-    if (rc == HYP_OK && (e = cudaMalloc(&c->F, (size_t)kNFlux1 * c->n * sizeof(double))) != cudaSuccess)
-      fail(e, "cudaMalloc(F)");
-    if (rc == HYP_OK && (e = cudaMalloc(&c->lam, (size_t)c->n * sizeof(double))) != cudaSuccess)
-      fail(e, "cudaMalloc(lam)");
+    const size_t nf = (size_t)(kNFlux1 + 1) * c->n * sizeof(double);  // fluxes, then the wave speeds
+    if (rc == HYP_OK && (e = cudaMalloc(&c->flux1[0], nf)) != cudaSuccess) fail(e, "cudaMalloc(F)");
+    if (rc == HYP_OK && cudaMalloc(&c->flux1[1], nf) != cudaSuccess) {
+      (void)cudaGetLastError();  // no room for a second one: the step's kernels run apart
+      c->flux1[1] = c->flux1[0];
+    }
+    for (int p = 0; p < 2; ++p) c->lam1[p] = c->flux1[p] + (size_t)kNFlux1 * c->n;
   } else {
     // per parity one tile-major block of mixed_tiles(n) tiles x 32 rows (hi, lo, lambda,
     // islands: hyp_internal.cuh); a parity's block also stages FP64 uploads and downloads
@@ -326,7 +330,8 @@ static int prof_event(hyp_ctx* c, cudaEvent_t* out) {
 
 // Enqueue step number k (k = steps taken since the upload + steps already
 // enqueued); no host synchronisation.
-static int enqueue_step(hyp_ctx* c, long long k, double t_end, bool prof) {
+// (first, last: of the steps enqueued together, see launch_run_step1_f64)
+static int enqueue_step(hyp_ctx* c, long long k, double t_end, bool prof, bool first, bool last) {
   cudaEvent_t e0 = nullptr, e1 = nullptr, e2 = nullptr;
   int rc;
   if (prof) {
@@ -353,10 +358,15 @@ static int enqueue_step(hyp_ctx* c, long long k, double t_end, bool prof) {
     CK(launch_update2_f64(c, p, t_end));
     if (c->relax) CK(launch_relax2(c, p, t_end));
   } else if (!mixed(c)) {
-    const int p = (int)(k & 1);
-    CK(launch_cell1_f64(c, p, &c->st->lam_bits[p], &c->st->t[p], t_end));
-    if (prof) CK(cudaEventRecord(e1, c->stream));
-    CK(launch_update1_f64(c, p, t_end));
+    if (prof) {
+      const int p = (int)(k & 1);
+      unsigned long long* s = c->st->lam_slots;
+      CK(launch_cell1_f64(c, p, s + k % 3, &c->st->t[p], t_end));
+      CK(cudaEventRecord(e1, c->stream));
+      CK(launch_update1_f64(c, p, s + k % 3, s + (k + 1) % 3, s + (k + 2) % 3, t_end));
+    } else {
+      CK(launch_run_step1_f64(c, k, t_end, first, last));
+    }
   } else {
     CK(launch_step1_mixed(c, k, t_end));
     if (prof) CK(cudaEventRecord(e1, c->stream));
@@ -382,8 +392,9 @@ static int collect_profile(hyp_ctx* c) {
 }
 
 // steps per captured graph: a multiple of the launch pattern's period
-static int graph_period(const hyp_ctx* c) { return mixed1(c) ? 6 : 2; }
-static int graph_steps(const hyp_ctx* c) { return mixed1(c) ? 12 : 16; }
+static bool single(const hyp_ctx* c) { return c->cfg.model == HYP_MODEL_SINGLE; }
+static int graph_period(const hyp_ctx* c) { return single(c) ? 6 : 2; }  // parity x three max-lambda slots
+static int graph_steps(const hyp_ctx* c) { return single(c) ? 12 : 16; }
 
 static int ensure_graph(hyp_ctx* c, long long k0, double t_end) {
   const int key = (int)(k0 % graph_period(c));
@@ -400,7 +411,8 @@ static int ensure_graph(hyp_ctx* c, long long k0, double t_end) {
   cudaGraph_t g;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = HYP_OK;
-  for (int s = 0; s < c->graph_steps && rc == HYP_OK; ++s) rc = enqueue_step(c, k0 + s, t_end, false);
+  for (int s = 0; s < c->graph_steps && rc == HYP_OK; ++s)
+    rc = enqueue_step(c, k0 + s, t_end, false, s == 0, s == c->graph_steps - 1);
   cudaError_t e = cudaStreamEndCapture(c->stream, &g);
   if (rc != HYP_OK) return rc;
   if (e != cudaSuccess) return set_err(c, HYP_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
@@ -451,8 +463,8 @@ extern "C" int hyp_step(hyp_ctx* c, int max_steps, double t_end, int* steps_done
         k += gs;
       }
     }
-    for (; rc == HYP_OK && s < todo; ++s, ++k) {
-      rc = enqueue_step(c, k, t_end, prof);
+    for (long long s0 = s; rc == HYP_OK && s < todo; ++s, ++k) {
+      rc = enqueue_step(c, k, t_end, prof, s == s0, s == todo - 1);
       if (rc == HYP_OK && c->hist_on) {  // t after step k (an inactive step carries t across)
         log_time_kernel<<<1, 1, 0, c->stream>>>(c->st, (int)((k + 1) & 1), c->hist_dev + (k - steps0));
         cudaError_t e = cudaGetLastError();

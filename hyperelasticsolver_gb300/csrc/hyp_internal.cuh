@@ -22,7 +22,8 @@ struct DevState {
   double t[2];                        // time before the step of parity p is t[p]
   unsigned long long lam_bits[2];     // max wave speed of the state of parity p (bits of a double >= 0)
   unsigned long long lam_query;       // hyp_max_wavespeed slot
-  unsigned long long lam_slots[3];    // mixed precision: FP32 max lambda (bits) of states k, k+1 (slot k%3)
+  unsigned long long lam_slots[3];    // single phase: max lambda of states k, k+1 (slot k%3), FP32 bits (mixed)
+                                      // or FP64 bits
   long long steps;                    // steps taken
   int err_code;                       // first HYP_CELL_* status raised (0 = none)
   int pad_;
@@ -121,8 +122,11 @@ struct hyp_ctx {
   cudaEvent_t row_ev[30] = {};         // one per variable row of a pipelined download
   // FP64 state, double-buffered: Q[p] is the state before a step of parity p.
   double* Q[2] = {nullptr, nullptr};
-  double* F = nullptr;     // per-cell fluxes (scratch)
-  double* lam = nullptr;   // per-cell max wave speed (scratch)
+  double* F = nullptr;     // two-phase: per-cell fluxes (scratch)
+  // single-phase: fluxes and wave speeds of the state of each parity; one pair of
+  // buffers for both where a second one does not fit on the device
+  double* flux1[2] = {nullptr, nullptr};
+  double* lam1[2] = {nullptr, nullptr};
   // mixed precision: per parity one block of floats, which also serves as the FP64
   // staging buffer of uploads and downloads. Single-phase: Qh[p] is a tile-major
   // block of the 32 rows (hi, lo, lambda, islands) of mixed_tiles(n) tiles; Ql is not
@@ -213,12 +217,32 @@ void free_snap(hyp_ctx* c);
 // speeds, their maximum into lam_slot), then the update
 cudaError_t launch_cell1(cudaStream_t s, const double* Q, int64_t n, const EosC& e, double* F, double* lam,
                          unsigned long long* lam_slot, const double* t_now, double t_end, DevState* S);
-cudaError_t launch_update1(cudaStream_t s, const double* Q, double* Qn, int64_t n, const double* F, const double* lam,
-                           const unsigned long long* lam_in, unsigned long long* lam_next, const double* t_in,
-                           double* t_out, long long* steps, double t_end, double cfl, double dx, int flux, int bc);
+// One step on plain buffers: the update of Q into Qn from the fluxes F and wave speeds
+// lam of Q, whose maximum is in rd; with Fn, then the cell pass of Qn into Fn, lamn and
+// (maximum) wr if the new time is below t_end. An active step zeroes the clr slots (null:
+// none). Fn and lamn are other buffers than F and lam: neighbouring blocks still read these.
+struct Step1Args {
+  const double* Q;
+  double* Qn;
+  const double *F, *lam;
+  double *Fn, *lamn;
+  const unsigned long long* rd;
+  unsigned long long* wr;
+  unsigned long long* clr[2];
+  const double* t_in;
+  double* t_out;
+  long long* steps;
+  double t_end, cfl, dx;
+  int64_t n;
+  int flux, bc;
+  DevState* S;
+};
+cudaError_t launch_step1(cudaStream_t s, const Step1Args& a, const EosC& e);
 // single-phase FP64 launchers on a context (hyp_step1.cu)
 cudaError_t launch_cell1_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end);
-cudaError_t launch_update1_f64(hyp_ctx* c, int p, double t_end);
+cudaError_t launch_update1_f64(hyp_ctx* c, int p, unsigned long long* rd, unsigned long long* clr0,
+                               unsigned long long* clr1, double t_end);
+cudaError_t launch_run_step1_f64(hyp_ctx* c, long long k, double t_end, bool first, bool last);
 // single-phase mixed-precision launchers (hyp_step1_mixed.cu)
 cudaError_t launch_split(hyp_ctx* c, const double* q, float* hi, float* lo);
 cudaError_t launch_split_n(cudaStream_t s, const double* q, float* hi, float* lo, int rows, int64_t n, int64_t pitch);

@@ -10,7 +10,7 @@
 // caller passes the input and output state, and everything else the step
 // needs (the second state buffer of the ping-pong, per-cell fluxes and wave
 // speeds, loop control) lives in one fixed, file-scope device array of
-// kNoAllocDoubles doubles (65,536 cells at most; 13,631,552 bytes = 13.0 MiB that
+// kNoAllocDoubles doubles (65,536 cells at most; 19,923,040 bytes = 19.0 MiB that
 // every GPU which loads this library keeps until the process exits).
 //
 // Set-up: the first call on a device looks up that array's device address with
@@ -34,10 +34,10 @@ namespace hyp {
 
 constexpr int64_t kNoAllocMaxCells = 65536;
 constexpr size_t kNoAllocState = (size_t)14 * kNoAllocMaxCells;      // second state buffer
-constexpr size_t kNoAllocFlux = (size_t)kNFlux1 * kNoAllocMaxCells;   // per-cell fluxes
-constexpr size_t kNoAllocLam = (size_t)kNoAllocMaxCells;              // per-cell wave speeds
+constexpr size_t kNoAllocFlux = (size_t)kNFlux1 * kNoAllocMaxCells;   // per-cell fluxes (two: a step reads one, writes the other)
+constexpr size_t kNoAllocLam = (size_t)kNoAllocMaxCells;              // per-cell wave speeds (two)
 constexpr size_t kNoAllocCtl = (sizeof(DevState) + sizeof(double) - 1) / sizeof(double);
-constexpr size_t kNoAllocDoubles = kNoAllocState + kNoAllocFlux + kNoAllocLam + kNoAllocCtl;
+constexpr size_t kNoAllocDoubles = kNoAllocState + 2 * kNoAllocFlux + 2 * kNoAllocLam + kNoAllocCtl;
 
 static __device__ __align__(256) double g_noalloc_scratch[kNoAllocDoubles];
 
@@ -49,8 +49,7 @@ double* g_scratch_addr[kMaxDevices] = {};
 __global__ void noalloc_reset_kernel(DevState* st, double t0) {
   st->t[0] = t0;
   st->t[1] = t0;
-  st->lam_bits[0] = 0ull;
-  st->lam_bits[1] = 0ull;
+  for (int s = 0; s < 3; ++s) st->lam_slots[s] = 0ull;
   st->lam_query = 0ull;
   st->steps = 0;
   st->err_code = 0;
@@ -98,8 +97,8 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   const int64_t n = n_cells;
   double* B = base;
   double* F = base + kNoAllocState;
-  double* lam = F + kNoAllocFlux;
-  DevState* st = (DevState*)(lam + kNoAllocLam);
+  double* lam = F + 2 * kNoAllocFlux;
+  DevState* st = (DevState*)(lam + 2 * kNoAllocLam);
   const EosC eos = make_eos(cfg->eos[0].rho0, cfg->eos[0].c0, cfg->eos[0].cv, cfg->eos[0].t0, cfg->eos[0].b0,
                             cfg->eos[0].alpha, cfg->eos[0].beta, cfg->eos[0].gamma);
   const double dx = cfg->x_length / (double)n;
@@ -110,14 +109,35 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
     return HYP_ERR_CUDA;
   noalloc_reset_kernel<<<1, 1, 0, s>>>(st, t0);
   if (cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;
+  if (n_steps > 0 &&
+      launch_cell1(s, cur, n, eos, F, lam, &st->lam_slots[0], &st->t[0], INFINITY, st) != cudaSuccess)
+    return HYP_ERR_CUDA;
   for (int k = 0; k < n_steps; ++k) {
     const int p = k & 1;
+    const bool last = k == n_steps - 1;
     double* nxt = (cur == d_Q_out) ? B : d_Q_out;
-    cudaError_t e = launch_cell1(s, cur, n, eos, F, lam, &st->lam_bits[p], &st->t[p], INFINITY, st);
-    if (e != cudaSuccess) return HYP_ERR_CUDA;
-    e = launch_update1(s, cur, nxt, n, F, lam, &st->lam_bits[p], &st->lam_bits[1 - p], &st->t[p], &st->t[1 - p],
-                       &st->steps, INFINITY, cfg->cfl, dx, cfg->flux, cfg->bc);
-    if (e != cudaSuccess) return HYP_ERR_CUDA;
+    Step1Args a;
+    a.Q = cur;
+    a.Qn = nxt;
+    a.F = F + p * kNoAllocFlux;
+    a.lam = lam + p * kNoAllocLam;
+    a.Fn = last ? nullptr : F + (1 - p) * kNoAllocFlux;
+    a.lamn = last ? nullptr : lam + (1 - p) * kNoAllocLam;
+    a.rd = &st->lam_slots[k % 3];
+    a.wr = &st->lam_slots[(k + 1) % 3];
+    a.clr[0] = &st->lam_slots[(k + 2) % 3];
+    a.clr[1] = nullptr;
+    a.t_in = &st->t[p];
+    a.t_out = &st->t[1 - p];
+    a.steps = &st->steps;
+    a.t_end = INFINITY;
+    a.cfl = cfg->cfl;
+    a.dx = dx;
+    a.n = n;
+    a.flux = cfg->flux;
+    a.bc = cfg->bc;
+    a.S = st;
+    if (launch_step1(s, a, eos) != cudaSuccess) return HYP_ERR_CUDA;
     cur = nxt;
   }
   if (cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;

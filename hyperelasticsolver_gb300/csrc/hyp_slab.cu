@@ -165,7 +165,7 @@ extern "C" int hyp_slab_step(hyp_ctx* c, double lam_max, double* t_out) {
     unsigned long long bits;
     memcpy(&bits, &lam_max, sizeof bits);
     SCK(cudaMemcpyAsync(&c->st->lam_bits[p], &bits, sizeof bits, cudaMemcpyHostToDevice, c->stream));
-    SCK(launch_update1_f64(c, p, INFINITY));
+    SCK(launch_update1_f64(c, p, &c->st->lam_bits[p], &c->st->lam_bits[1 - p], nullptr, INFINITY));
   }
   int rc = ctx_sync_state(c);
   if (rc != HYP_OK) return rc;

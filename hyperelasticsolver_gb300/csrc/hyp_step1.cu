@@ -1,18 +1,18 @@
 // hyp_step1.cu -- single-phase FP64 step: Rusanov / LxF first-order update of
 // main.jl:202-227 with the per-phase model of HyperelasticityMPh.jl at alpha == 1.
 //
-// One step = two kernels on the context stream:
-//   cell   : per cell cons2prim -> stress -> flux (11 non-zero components) and
-//            lambda_i = |u1| + sqrt(max|eig(acoustic)|); block max of lambda by
-//            warp shuffles and one shared-memory pass, one atomicMax per block.
-//            (main.jl:204-211; HyperelasticityMPh.jl:106-175, 252-266)
-//   update : dt = cfl*dx / max lambda, t += dt, and per interior cell
-//            Q - dt/dx (F_{i+1/2} - F_{i-1/2}) with the Rusanov face flux
-//            0.5 (f_L + f_R) - 0.5 max(lambda_L, lambda_R) (Q_R - Q_L)
-//            (NumFluxes.jl:25-33; main.jl:45-48, 43-60); end cells frozen
-//            (main.jl:219-220) or transmissive.
-// The flux/wave-speed work is done once per cell; the update kernel streams
-// state, fluxes and speeds (SoA, coalesced 8-byte loads along the cell index).
+// A run of steps is a cell pass of the first state and one kernel per step after it:
+//   cell : per cell cons2prim -> stress -> flux (11 non-zero components) and
+//          lambda_i = |u1| + sqrt(max|eig(acoustic)|); block max of lambda, one
+//          atomicMax per block (main.jl:204-211; HyperelasticityMPh.jl:106-175, 252-266)
+//   step : dt = cfl*dx / max lambda, t += dt, and per interior cell
+//          Q - dt/dx (F_{i+1/2} - F_{i-1/2}) with the Rusanov face flux
+//          0.5 (f_L + f_R) - 0.5 max(lambda_L, lambda_R) (Q_R - Q_L)
+//          (NumFluxes.jl:25-33; main.jl:45-48, 43-60); end cells frozen
+//          (main.jl:219-220) or transmissive; then, unless it is the run's last step,
+//          the cell pass of the new state from registers.
+// The last step of a run leaves the cell pass out: a state the caller takes home is
+// evaluated (and a bad cell in it reported) only when it is stepped from.
 #include "hyp_internal.cuh"
 #include "hyp_step64.cuh"
 
@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __res
                                                              double t_end, DevState* S) {
   if (!(*t_now < t_end)) return;  // uniform across the grid
   const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
-  const double l = i < n ? cell1_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = i < n ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(lam_slot, m);
 }
@@ -38,47 +38,61 @@ __global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __res
 // exactly. What bounds it: FP64 issue again, 67 slots a cell plus the step's scalars
 // (84 and three divisions per warp with halved faces and a block of 256 whose last
 // thread took two); warp 0 evaluates the scalars while the others wait at the barrier.
-// Whole runs as above: 1000 cells 2.38 -> 1.97 ms, 1,000,003 cells 7.26 -> 6.07 ms.
-__global__ void __launch_bounds__(kBlock64) update1_f64_kernel(const double* __restrict__ Q, double* __restrict__ Qn,
-                                                               int64_t n, const double* __restrict__ F,
-                                                               const double* __restrict__ lam,
-                                                               const unsigned long long* lam_in,
-                                                               unsigned long long* lam_next, const double* t_in,
-                                                               double* t_out, long long* steps, double t_end,
-                                                               double cfl, double dx, int flux, int bc) {
+// With kCell the new state's cell pass follows in the same kernel: its FP64 work is the
+// same, but a small problem saves a launch, the second kernel's ramp and its reload of
+// the state, and the fluxes alternate between two buffers: 1000 cells x 100 steps 1.59 -> 1.40
+// ms, 8192 cells x 4 steps on device buffers 129 -> 110 us, 1,000,003 cells unchanged (6.03 ms).
+template <int kDef, bool kCell>
+__global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e, Eos64 k) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell i0 + k
   __shared__ double s_hdt;             // half dt/dx
+  __shared__ int s_more;               // the state this step makes is stepped from
   const int j = threadIdx.x;
-  const double tn = *t_in;
-  const bool active = tn < t_end;
-  const double lmax = __longlong_as_double((long long)*lam_in);
-  const bool lxf = flux == HYP_FLUX_LXF;
+  const int64_t n = a.n;
+  const double tn = *a.t_in;
+  const bool active = tn < a.t_end;
+  const double lmax = __longlong_as_double((long long)*a.rd);
+  const bool lxf = a.flux == HYP_FLUX_LXF;
   // Rusanov: dt/dx (main.jl:225); LxF: 1/lambda with lambda = dx/dt (main.jl:223, :40)
   StepScalars sc{0.0, 0.0, 0.0};
-  if (j < 32 || lxf) sc = step_scalars64(cfl, dx, lmax, lxf);
-  if (j == 0) s_hdt = 0.5 * sc.dtdx;
-  if (blockIdx.x == 0 && j == 0) {
-    *t_out = active ? tn + sc.dt : tn;
-    *lam_next = 0ull;
-    if (active) *steps += 1;
+  if (j < 32 || lxf) sc = step_scalars64(a.cfl, a.dx, lmax, lxf);
+  if (j == 0) {
+    s_hdt = 0.5 * sc.dtdx;
+    s_more = kCell && tn + sc.dt < a.t_end;
+    if (blockIdx.x == 0) {
+      *a.t_out = active ? tn + sc.dt : tn;
+      if (active) {  // an inactive step leaves the slots of the state it does not step from
+        for (int c = 0; c < 2; ++c)
+          if (a.clr[c]) *a.clr[c] = 0ull;
+        *a.steps += 1;
+      }
+    }
   }
   if (!active) return;  // the same for every block
   const int64_t i = (int64_t)blockIdx.x * kCells64 + j;  // this thread's cell, and the face on its left
   double f2[14];
   if (i <= n) {
-    face_twice(Q, F, lam, n, 0, n, i, lxf, sc.lam_lxf, f2);
+    face_twice(a.Q, a.F, a.lam, n, 0, n, i, lxf, sc.lam_lxf, f2);
 #pragma unroll
     for (int v = 0; v < 14; ++v) sF[v][j] = f2[v];
   }
   __syncthreads();
-  if (j == kCells64 || i >= n) return;
-  const bool frozen = bc_holds(bc, i == 0, i == n - 1);
-  const double hdt = s_hdt;
+  const bool own = j < kCells64 && i < n;
+  double q[14];
+  if (own) {
+    const bool frozen = bc_holds(a.bc, i == 0, i == n - 1);
+    const double hdt = s_hdt;
 #pragma unroll
-  for (int v = 0; v < 14; ++v) {
-    const double qc = Q[v * n + i];
-    Qn[v * n + i] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+    for (int v = 0; v < 14; ++v) {
+      const double qc = a.Q[v * n + i];
+      q[v] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+      a.Qn[v * n + i] = q[v];
+    }
   }
+  if (!kCell || !s_more) return;
+  const double l = own ? cell1_pass<kDef>(q, n, i, e, k, a.Fn, a.lamn, a.S) : 0.0;
+  const unsigned long long m = block_max_bits<kBlock64>(l);
+  if (j == 0) atomicMax(a.wr, m);
 }
 
 cudaError_t launch_cell1(cudaStream_t s, const double* Q, int64_t n, const EosC& e, double* F, double* lam,
@@ -92,23 +106,67 @@ cudaError_t launch_cell1(cudaStream_t s, const double* Q, int64_t n, const EosC&
   return cudaGetLastError();
 }
 
-cudaError_t launch_update1(cudaStream_t s, const double* Q, double* Qn, int64_t n, const double* F, const double* lam,
-                           const unsigned long long* lam_in, unsigned long long* lam_next, const double* t_in,
-                           double* t_out, long long* steps, double t_end, double cfl, double dx, int flux, int bc) {
-  const unsigned grid = (unsigned)((n + kCells64 - 1) / kCells64);
-  update1_f64_kernel<<<grid, kBlock64, 0, s>>>(Q, Qn, n, F, lam, lam_in, lam_next, t_in, t_out, steps, t_end, cfl, dx,
-                                               flux, bc);
+cudaError_t launch_step1(cudaStream_t s, const Step1Args& a, const EosC& e) {
+  const unsigned grid = (unsigned)((a.n + kCells64 - 1) / kCells64);
+  const Eos64 k = make_eos64(e);
+  auto kern = !a.Fn ? step1_f64_kernel<1, false> : (e.default_exp ? step1_f64_kernel<1, true> : step1_f64_kernel<0, true>);
+  kern<<<grid, kBlock64, 0, s>>>(a, e, k);
   return cudaGetLastError();
 }
 
 cudaError_t launch_cell1_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end) {
-  return launch_cell1(c->stream, c->Q[p], c->n, c->eos[0], c->F, c->lam, lam_slot, t_now, t_end, c->st);
+  return launch_cell1(c->stream, c->Q[p], c->n, c->eos[0], c->flux1[p], c->lam1[p], lam_slot, t_now, t_end, c->st);
 }
 
-cudaError_t launch_update1_f64(hyp_ctx* c, int p, double t_end) {
-  return launch_update1(c->stream, c->Q[p], c->Q[1 - p], c->n, c->F, c->lam, &c->st->lam_bits[p],
-                        &c->st->lam_bits[1 - p], &c->st->t[p], &c->st->t[1 - p], &c->st->steps, t_end, c->cfg.cfl,
-                        ctx_dx(c), c->cfg.flux, ctx_bc(c));
+static Step1Args step1_args(hyp_ctx* c, int p, unsigned long long* rd, unsigned long long* wr, unsigned long long* clr0,
+                     unsigned long long* clr1, double t_end) {
+  Step1Args a;
+  a.Q = c->Q[p];
+  a.Qn = c->Q[1 - p];
+  a.F = c->flux1[p];
+  a.lam = c->lam1[p];
+  a.Fn = wr ? c->flux1[1 - p] : nullptr;
+  a.lamn = wr ? c->lam1[1 - p] : nullptr;
+  a.rd = rd;
+  a.wr = wr;
+  a.clr[0] = clr0;
+  a.clr[1] = clr1;
+  a.t_in = &c->st->t[p];
+  a.t_out = &c->st->t[1 - p];
+  a.steps = &c->st->steps;
+  a.t_end = t_end;
+  a.cfl = c->cfg.cfl;
+  a.dx = ctx_dx(c);
+  a.n = c->n;
+  a.flux = c->cfg.flux;
+  a.bc = ctx_bc(c);
+  a.S = c->st;
+  return a;
+}
+
+// The update of the step of parity p, with the max wave speed in `rd`, clearing the
+// `clr` slots.
+cudaError_t launch_update1_f64(hyp_ctx* c, int p, unsigned long long* rd, unsigned long long* clr0,
+                               unsigned long long* clr1, double t_end) {
+  return launch_step1(c->stream, step1_args(c, p, rd, nullptr, clr0, clr1, t_end), c->eos[0]);
+}
+
+// Step k of a run (first / last of it): the max wave speed of the state before step k
+// is in lam_slots[k % 3]. The slots rotate: step k reads k % 3, its cell pass writes
+// (k + 1) % 3 and it clears (k + 2) % 3; a run's last step clears both others, and a step
+// past t_end none, so a run always starts on a cleared slot with the next one cleared.
+// A context without room for the second flux buffer runs the two kernels apart.
+cudaError_t launch_run_step1_f64(hyp_ctx* c, long long k, double t_end, bool first, bool last) {
+  const int p = (int)(k & 1);
+  unsigned long long* s = c->st->lam_slots;
+  unsigned long long *rd = s + k % 3, *nx = s + (k + 1) % 3, *cl = s + (k + 2) % 3;
+  const bool apart = c->flux1[1] == c->flux1[0];
+  if (first || apart) {
+    const cudaError_t e = launch_cell1_f64(c, p, rd, &c->st->t[p], t_end);
+    if (e != cudaSuccess) return e;
+  }
+  if (last || apart) return launch_update1_f64(c, p, rd, nx, cl, t_end);
+  return launch_step1(c->stream, step1_args(c, p, rd, nx, cl, nullptr, t_end), c->eos[0]);
 }
 
 }  // namespace hyp

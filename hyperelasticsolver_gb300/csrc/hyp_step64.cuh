@@ -35,15 +35,12 @@ __device__ __forceinline__ unsigned long long block_max_bits(double l) {
   return m;
 }
 
-// The single-phase cell pass of cell i: its flux (kNFlux1 rows of F) and wave speed,
-// stored and returned; a bad cell is recorded.
+// The single-phase cell pass of cell i in state q: its flux (kNFlux1 rows of F) and wave
+// speed, stored and returned; a bad cell is recorded.
 template <int kDef>
-__device__ __forceinline__ double cell1_pass(const double* __restrict__ Q, int64_t n, int64_t i, const EosC& e,
-                                             const Eos64& k, double* __restrict__ F, double* __restrict__ lam,
-                                             DevState* S) {
-  double q[14], f[14];
-#pragma unroll
-  for (int v = 0; v < 14; ++v) q[v] = Q[v * n + i];
+__device__ __forceinline__ double cell1_pass(const double* q, int64_t n, int64_t i, const EosC& e, const Eos64& k,
+                                             double* __restrict__ F, double* __restrict__ lam, DevState* S) {
+  double f[14];
   const Cell64 c = cell64<kDef>(e, k, 1.0, q + 1, q[4], q + 5);
   flux64(1.0, c, q + 1, q + 5, f);
   const double l = fabs(c.u[0]) + cmax64<kDef>(e, k, c);
@@ -56,6 +53,15 @@ __device__ __forceinline__ double cell1_pass(const double* __restrict__ Q, int64
   const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
   if (st) record_err64(S, st, i);
   return l;
+}
+template <int kDef>
+__device__ __forceinline__ double cell1_load_pass(const double* __restrict__ Q, int64_t n, int64_t i, const EosC& e,
+                                                  const Eos64& k, double* __restrict__ F, double* __restrict__ lam,
+                                                  DevState* S) {
+  double q[14];
+#pragma unroll
+  for (int v = 0; v < 14; ++v) q[v] = Q[v * n + i];
+  return cell1_pass<kDef>(q, n, i, e, k, F, lam, S);
 }
 
 // Cells a block of the update kernels owns: thread j evaluates the face left of cell

@@ -1,0 +1,81 @@
+"""A run of FP64 steps does not depend on how it is cut into calls: steps inside one call
+share kernels (update and next cell pass in one), the first and last of a call do not
+(GPU). Bitwise: the same arithmetic either way."""
+import numpy as np
+import pytest
+
+from hyperelasticsolver_gb300 import _cases as C
+
+pytestmark = pytest.mark.gpu
+
+CUTS = [[1] * 27, [27], [2, 13, 12], [12, 15], [26, 1]]  # 12 steps are one captured graph
+
+
+def state(hyp, n, seed=3):
+    eos = hyp.Barton2009()
+    return eos, C.segment_fill(hyp.Hyperelasticity.prim2cons(eos, C.segment_states(eos, 8, seed=seed)), n)
+
+
+@pytest.mark.parametrize("n", [3, 127, 128, 300])
+@pytest.mark.parametrize("flux,bc", [("rusanov", "frozen"), ("lxf", "transmissive")])
+def test_cuts_agree(hyp, n, flux, bc):
+    eos, Q0 = state(hyp, n)
+    out = []
+    for cut in CUTS:
+        with hyp.Solver(eos, n, flux=flux, bc=bc) as s:
+            s.upload(Q0)
+            for k in cut:
+                assert s.step(max_steps=k)[0] == k
+            out.append((s.download(), s.time()))
+    for Q, t in out[1:]:
+        assert np.array_equal(Q, out[0][0]) and t == out[0][1]
+
+
+def test_stop_at_t_end_and_go_on(hyp):
+    """Steps past t_end leave everything as it is; the run then goes on as if never stopped;
+    profiled, time-logged and recorded runs take the same steps."""
+    eos, Q0 = state(hyp, 200)
+    ref = []
+    with hyp.Solver(eos, 200) as s:
+        s.upload(Q0)
+        for _ in range(31):
+            ref.append((s.step(max_steps=1)[1], s.download()))
+    for stop in (1, 2, 3, 12, 14):
+        with hyp.Solver(eos, 200) as s:
+            s.upload(Q0)
+            t_end = 0.5 * (ref[stop - 2][0] + ref[stop - 1][0]) if stop > 1 else 0.5 * ref[0][0]
+            assert s.step(t_end=t_end) == (stop, ref[stop - 1][0])
+            assert np.array_equal(s.download(), ref[stop - 1][1])
+            assert s.step(max_steps=40, t_end=t_end)[0] == 0
+            s.set_profiling(True)
+            s.step(max_steps=3)
+            s.set_profiling(False)
+            th, _ = s.step_times(5)
+            assert np.array_equal(th, [ref[stop + 3 + k][0] for k in range(5)])
+            s.record(31 - stop - 8, 4)
+            assert s.time()[0] == ref[30][0] and np.array_equal(s.download(), ref[30][1])
+
+
+def test_batch_cuts_agree(hyp):
+    eos = hyp.Barton2009()
+    sizes = [3, 127, 128, 500]
+    Q0 = np.concatenate([state(hyp, n, seed=k)[1] for k, n in enumerate(sizes)], axis=1)
+    out = []
+    for cut in ([1] * 9, [9], [4, 5]):
+        with hyp.Batch(eos, sizes, precision="fp64") as b:
+            b.upload(Q0)
+            for k in cut:
+                b.step(k)
+            mid = b.status()[0][3] + 1e-9  # the largest problem stops at once, coarser ones when they pass it
+            b.step(5, t_end=mid)
+            b.step(3)
+            out.append((b.download(), *b.status()))
+    for o in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(o, out[0]))
+    Q, t, steps = out[0]
+    for p, n in enumerate(sizes):  # each problem as a single run of its own
+        with hyp.Solver(eos, n) as s:
+            lo = sum(sizes[:p])
+            s.upload(np.ascontiguousarray(Q0[:, lo:lo + n]))
+            _, tp = s.step(max_steps=int(steps[p]))
+            assert tp == t[p] and np.array_equal(s.download(), Q[:, lo:lo + n])
