@@ -155,6 +155,7 @@ struct Eos64 {
   double hb0sq;                              // b0sq / 2
   double kU, kE3a, kE3g;                     // as EosT
   double hbeta, beta2, beta22;               // beta/2, beta + 2, 2 beta + 2
+  double h_alphasq;                          // 1 / (2 alpha^2)
 };
 HYP_HD Eos64 make_eos64(const EosC& e) {
   Eos64 c;
@@ -168,6 +169,7 @@ HYP_HD Eos64 make_eos64(const EosC& e) {
   c.hbeta = 0.5 * e.beta;
   c.beta2 = e.beta + 2.0;
   c.beta22 = 2.0 * e.beta + 2.0;
+  c.h_alphasq = 0.5 / (e.alpha * e.alpha);
   return c;
 }
 
@@ -181,7 +183,8 @@ struct Cell64 {
   double a, b, bM;            // a, b, b p M00
   double wE;                  // w_0 - E3 p (finite where E3 p is not)
   double T1, T2, T3, E3p;     // bulk, thermal and shear terms of E3 p, their sum
-  double Pa, Pg, px;          // p^(alpha/2), p^(gamma/2), Pg (x - 1)
+  double Pa, Pb, Pg, px;      // p^(alpha/2), p^(beta/2), p^(gamma/2), Pg (x - 1)
+  bool clamped;               // the entropy argument is at its clamp
   int st;
 };
 
@@ -229,25 +232,26 @@ HYP_HD Cell64 cell64(const EosC& e, const Eos64& k, double ia, const double* m, 
   const double th = i1 * (1.0 / 3.0), d0 = o.G00 - th, d1 = o.G11 - th, d2 = o.G22 - th;
   const double off = o.G01 * o.G01 + o.G02 * o.G02;
   const double psi = 0.5 * (d0 * d0 + d1 * d1 + d2 * d2) + (o.G12 * o.G12 + off);
-  double Pb, inv_Pg;  // inv_Pg: over cv t0
+  double inv_Pg;  // over cv t0
   if (kDef == 1) {
     o.Pa = s;
-    Pb = s * p;
+    o.Pb = s * p;
     o.Pg = p;
     inv_Pg = (r * r) * k.rho0sq_icvt;
   } else {
     const double lp = log(p);
     o.Pa = exp(0.5 * e.alpha * lp);
-    Pb = exp(0.5 * e.beta * lp);
+    o.Pb = exp(0.5 * e.beta * lp);
     o.Pg = exp(0.5 * e.gamma * lp);
     inv_Pg = e.inv_cvt0 / o.Pg;
   }
-  o.b = k.hb0sq * Pb;
+  o.b = k.hb0sq * o.Pb;
   const double bp = o.b * psi;               // shear energy
   const double am1 = o.Pa - 1.0, z = k.kU * am1;
   double xm1 = ((e_int - bp) - z * am1) * inv_Pg;  // x - 1 of the entropy argument (EquationsOfState.jl:150)
   if (is_nan64(e_int) || is_nan64(xm1) || !is_finite64(p)) o.st |= HYP_CELL_NONFINITE;
-  if (below_negative64(xm1, 1e-6 - 1.0)) xm1 = 1e-6 - 1.0;  // its clamp (:152-154)
+  o.clamped = below_negative64(xm1, 1e-6 - 1.0);  // (:152-154)
+  if (o.clamped) xm1 = 1e-6 - 1.0;
   o.px = o.Pg * xm1;
   o.T1 = kDef == 1 ? z * s : e.alpha * (z * o.Pa);
   o.T2 = k.kE3g * o.px;
@@ -274,6 +278,39 @@ double radius_general(double o00, double o11, double o22, double o01, double o02
   return spectral_radius(a);
 }
 
+// The largest eigenvalue of a symmetric O, false where it does not stand clear of the
+// others' moduli: an FP32 root of the characteristic polynomial, then two steps with the
+// FP32 slope.
+HYP_HD bool top_root64(double o00, double o11, double o22, double o01, double o02, double o12, double& root) {
+  // mu^3 - c2 mu^2 + c1 mu - c0
+  const double tr = o11 + o22, q = o11 * o22 - o12 * o12;
+  const double c2 = o00 + tr;
+  const double c1 = ((o00 * tr + q) - o01 * o01) - o02 * o02;
+  const double e1 = o01 * o22 - o12 * o02, e2 = o01 * o12 - o11 * o02;
+  const double c0 = (o00 * q - o01 * e1) + o02 * e2;
+  const float C2 = to_f32(c2), C1 = to_f32(c1), C0 = to_f32(c0);
+  const float P = C1 - C2 * C2 * (1.0f / 3.0f);
+  const float Q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
+  // A symmetric matrix has three real roots; two equal ones (a material at rest or under
+  // isotropic strain has two equal shear speeds) put the cosine at 1 up to rounding,
+  // where the clamp below costs the largest root an error of second order only.
+  if (!(P < 0.0f)) return false;
+  const float am = 2.0f * sqrtf(-P * (1.0f / 3.0f));
+  const float cc = fminf(1.0f, fmaxf(-1.0f, 3.0f * Q / (P * am)));
+  const float y = am * cosf(acosf(cc) * (1.0f / 3.0f)) + C2 * (1.0f / 3.0f);
+  const float sm = C2 - y, pr = C0 / y;  // sum and product of the other two
+  const float other = 0.5f * fabsf(sm) + sqrtf(fmaxf(0.25f * sm * sm - pr, 0.0f));
+  const float slope = (3.0f * y - 2.0f * C2) * y + C1;
+  // With the others below 0.35 of it, the seed is within ~1e-6 and the slope within
+  // ~1e-6 of theirs at the root: a step leaves 5e-12, the next 5e-17.
+  if (!(other < 0.35f * y && slope > 1e-30f && slope < 1e30f)) return false;
+  const double inv = to_f64(1.0f / slope);
+  double rt = to_f64(y);
+  for (int it = 0; it < 2; ++it) rt = rt - (((rt - c2) * rt + c1) * rt - c0) * inv;
+  root = rt;
+  return true;
+}
+
 // Largest acoustic wave speed sqrt(max |eig Omega|) of one phase (HyperelasticityMPh.jl:258-266).
 template <int kDef>
 HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
@@ -289,34 +326,8 @@ HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
   const double o01 = f0 * c.G01 + k.beta2 * c.w[1], o02 = f0 * c.G02 + k.beta2 * c.w[2];
   const double o11 = f1 * c.G01 + (c.a * c.G11 - c.bM), o22 = f2 * c.G02 + (c.a * c.G22 - c.bM);
   const double o12 = f1 * c.G02 + c.a * c.G12;
-  // characteristic polynomial mu^3 - c2 mu^2 + c1 mu - c0
-  const double tr = o11 + o22, q = o11 * o22 - o12 * o12;
-  const double c2 = o00 + tr;
-  const double c1 = ((o00 * tr + q) - o01 * o01) - o02 * o02;
-  const double e1 = o01 * o22 - o12 * o02, e2 = o01 * o12 - o11 * o02;
-  const double c0 = (o00 * q - o01 * e1) + o02 * e2;
-  const float C2 = to_f32(c2), C1 = to_f32(c1), C0 = to_f32(c0);
-  const float P = C1 - C2 * C2 * (1.0f / 3.0f);
-  const float Q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
-  // A symmetric matrix has three real roots; two equal ones (a material at rest or under
-  // isotropic strain has two equal shear speeds) put the cosine at 1 up to rounding,
-  // where the clamp below costs the largest root an error of second order only.
-  if (P < 0.0f) {
-    const float am = 2.0f * sqrtf(-P * (1.0f / 3.0f));
-    const float cc = fminf(1.0f, fmaxf(-1.0f, 3.0f * Q / (P * am)));
-    const float y = am * cosf(acosf(cc) * (1.0f / 3.0f)) + C2 * (1.0f / 3.0f);  // the largest root
-    const float sm = C2 - y, pr = C0 / y;  // sum and product of the other two
-    const float other = 0.5f * fabsf(sm) + sqrtf(fmaxf(0.25f * sm * sm - pr, 0.0f));
-    const float slope = (3.0f * y - 2.0f * C2) * y + C1;
-    // With the others below 0.35 of it, the seed is within ~1e-6 and the slope within
-    // ~1e-6 of theirs at the root: a step leaves 5e-12, the next 5e-17.
-    if (other < 0.35f * y && slope > 1e-30f && slope < 1e30f) {
-      const double inv = to_f64(1.0f / slope);
-      double rt = to_f64(y);
-      for (int it = 0; it < 2; ++it) rt = rt - (((rt - c2) * rt + c1) * rt - c0) * inv;
-      return sqrt64(rt + rt);
-    }
-  }
+  double rt;
+  if (top_root64(o00, o11, o22, o01, o02, o12, rt)) return sqrt64(rt + rt);
   return sqrt(radius_general(o00, o11, o22, o01, o02, o12));
 }
 

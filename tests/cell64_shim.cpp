@@ -1,6 +1,6 @@
 // Host build of the FP64 step's compact cell forms (hyp_cell64.cuh) beside the general
 // ones (hyp_physics.cuh), for tests/test_cell64_host.py.
-#include "../hyperelasticsolver_gb300/csrc/hyp_cell64.cuh"
+#include "../hyperelasticsolver_gb300/csrc/hyp_adjoint64.cuh"
 
 using namespace hyp;
 
@@ -29,6 +29,24 @@ int c64_general(const double* p, const double* q, double* out) {
   phase_flux(e, q[0], P, c, out, s0);
   out[14] = P.u[0];
   out[15] = phase_cmax(e, P, c);
+  return st;
+}
+// out: qb (14), d/db0sq, d/dk0 of one single-phase cell
+int c64_vjp_compact(const double* p, const double* q, const double* fb, double lb, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  const Eos64 k = make_eos64(e);
+  EosBar b{0.0, 0.0};
+  const int st = e.default_exp ? cell_vjp64<1>(e, k, q, fb, lb, out, b) : cell_vjp64<0>(e, k, q, fb, lb, out, b);
+  out[14] = b.b0sq;
+  out[15] = b.k0;
+  return st;
+}
+int c64_vjp_general(const double* p, const double* q, const double* fb, double lb, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  EosBar b{0.0, 0.0};
+  const int st = cell_vjp(e, q, fb, lb, out, b);
+  out[14] = b.b0sq;
+  out[15] = b.k0;
   return st;
 }
 float c64_to_f32(double x) { return to_f32(x); }

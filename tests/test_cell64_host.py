@@ -97,6 +97,31 @@ def test_far_states_and_status(lib, orc, ep):
                 assert np.max(np.abs(g - c)) <= RTOL_FP64 * scale
 
 
+@pytest.mark.parametrize("ep", EOS)
+@pytest.mark.parametrize("strain", [0.0, 0.02, 0.1, 0.4])
+@pytest.mark.parametrize("seeds", ["flux", "speed", "both"])
+def test_vjp_matches_general(lib, orc, ep, strain, seeds):
+    """The compact cell VJP against the general one, over seeds of the flux, the wave speed
+    and both; strain 0.4 includes cells whose wave speeds are close (the general route)
+    and states at the entropy clamp. Each is a sum of products whose factors reach
+    |dF/dq| max|F-bar|: held to the parity tolerance of the largest entry."""
+    rng = np.random.default_rng(9)
+    dp = ctypes.POINTER(ctypes.c_double)
+    e = np.array(ep, dtype=np.float64)
+    for i, s in enumerate(phase_states(orc, ep, rng, 60, (1.0,), strain)):
+        q = np.ascontiguousarray(s[1:])
+        if i % 7 == 3:
+            q[4] -= 3.0 * q[0]  # below the clamp
+        fb = rng.standard_normal(14) if seeds != "speed" else np.zeros(14)
+        lb = ctypes.c_double(rng.standard_normal() if seeds != "flux" else 0.0)
+        out = [np.zeros(16), np.zeros(16)]
+        st = [getattr(lib, n)(e.ctypes.data_as(dp), q.ctypes.data_as(dp), fb.ctypes.data_as(dp), lb, o.ctypes.data_as(dp))
+              for n, o in zip(("c64_vjp_general", "c64_vjp_compact"), out)]
+        assert st[0] == st[1] == 0
+        for part in (slice(0, 14), slice(14, 16)):
+            assert np.max(np.abs(out[0][part] - out[1][part])) <= RTOL_FP64 * np.max(np.abs(out[0]))
+
+
 def test_integer_pipe_conversions(lib):
     rng = np.random.default_rng(5)
     x = np.concatenate([rng.standard_normal(200) * 10.0 ** rng.uniform(-30, 30, 200),
