@@ -101,19 +101,6 @@ struct FaceList {
   double *sl, *sr;
 };
 
-// True if every state within `far` of R (in the Frobenius norm of the change of R =
-// alpha rho A; far2 its square) has det R > 0: ||dR|| ||R^-1|| < 1/3, evaluated in FP32
-// with the cofactor norm. NaN, under- and overflow give false.
-__device__ __forceinline__ bool det_keeps_sign(const float* R, float far2) {
-  const float c00 = R[4] * R[8] - R[5] * R[7], c01 = R[7] * R[2] - R[1] * R[8], c02 = R[1] * R[5] - R[4] * R[2];
-  const float c10 = R[5] * R[6] - R[3] * R[8], c11 = R[0] * R[8] - R[2] * R[6], c12 = R[2] * R[3] - R[0] * R[5];
-  const float c20 = R[3] * R[7] - R[4] * R[6], c21 = R[1] * R[6] - R[0] * R[7], c22 = R[0] * R[4] - R[1] * R[3];
-  const float det = R[0] * c00 + R[3] * c01 + R[6] * c02;
-  const float cc = c00 * c00 + c01 * c01 + c02 * c02 + c10 * c10 + c11 * c11 + c12 * c12 + c20 * c20 + c21 * c21 +
-                   c22 * c22;
-  return det > 0.0f && 9.0f * far2 * cc < det * det;
-}
-
 // HLL faces: s_l, s_r and, where the volume fractions do not jump and no state on the
 // way between the cells (through Q_hll) can be singular, D- and D+ (doubles of the
 // formula of NumFluxes.jl:85-132 with its integrals zero). 186 slots a phase; the others are

@@ -23,17 +23,19 @@ __device__ __forceinline__ void record_err2m(DevState* S, int code, long long ce
   if (atomicCAS(&S->err_code, 0, code) == 0) S->err_cell = cell;
 }
 
-// at most 85 registers: 3 blocks of 256 per SM (0.02-0.03 ms per step better at 2^22
-// cells than 2 blocks at its natural 99)
+constexpr int kCellBlockM = 128;
+
+// at most 85 registers: 6 blocks of 128 per SM (0.02-0.03 ms per step better at 2^22
+// cells than at its natural 99 registers)
 template <int kDef>
-__global__ void __launch_bounds__(kBlock, 3) cell2_mixed_kernel(const float* __restrict__ Qh,
+__global__ void __launch_bounds__(kCellBlockM, 6) cell2_mixed_kernel(const float* __restrict__ Qh,
                                                              const float* __restrict__ Ql, int64_t pitch, int64_t n,
                                                              Eos2M E, float* __restrict__ F, int64_t fpitch,
                                                              float* __restrict__ smin, float* __restrict__ smax,
                                                              unsigned long long* lam_slot, const double* t_now,
                                                              double t_end, DevState* S) {
   if (!(*t_now < t_end)) return;
-  const int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
+  const int64_t i = (int64_t)blockIdx.x * kCellBlockM + threadIdx.x;
   float l = 0.0f;
   if (i < n) {
     float qh[30], ql[30], f[30];
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(kBlock, 3) cell2_mixed_kernel(const float* __r
     if (!(l <= 3.0e38f)) st |= HYP_CELL_NONFINITE;
     if (st) record_err2m(S, st, i);
   }
-  const float m = mixed_block_max<kBlock>(l);
+  const float m = mixed_block_max<kCellBlockM>(l);
   if (threadIdx.x == 0) atomicMax(lam_slot, (unsigned long long)__double_as_longlong((double)m));
 }
 
@@ -359,7 +361,7 @@ static bool default_exps(const hyp_ctx* c) { return c->eos[0].default_exp && c->
 
 cudaError_t launch_cell2_mixed(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end) {
   auto kern = default_exps(c) ? cell2_mixed_kernel<1> : cell2_mixed_kernel<-1>;
-  kern<<<grid_m(c->n, kBlock), kBlock, 0, c->stream>>>(c->Qh[p], c->Ql[p], c->mpitch, c->n, eos2m(c), c->F32, c->n,
+  kern<<<grid_m(c->n, kCellBlockM), kCellBlockM, 0, c->stream>>>(c->Qh[p], c->Ql[p], c->mpitch, c->n, eos2m(c), c->F32, c->n,
                                                         c->smin32, c->smax32, lam_slot, t_now, t_end, c->st);
   return cudaGetLastError();
 }

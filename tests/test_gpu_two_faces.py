@@ -86,7 +86,8 @@ def test_strong_strain_jump_takes_the_integrals(hyp, orc, flux):
 
 
 @pytest.mark.parametrize("flux", ["hll", "lxf"])
-def test_singular_state_on_the_path_is_refused(hyp, orc, flux):
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_singular_state_on_the_path_is_refused(hyp, orc, flux, precision):
     """Two admissible cells of equal volume fractions whose distortions differ by a half
     turn: det of the path's middle is not positive, and the step says so."""
     eos, pb = setup(hyp, orc, 40, flux)
@@ -97,7 +98,7 @@ def test_singular_state_on_the_path_is_refused(hyp, orc, flux):
         A[20:] = np.diag([1.0, -1.0, -1.0])
         P[:, 15 * p + 6:15 * p + 15] = A.reshape(40, 9)
     Q0 = np.ascontiguousarray(orc.prim2cons(pb, P).T)
-    with hyp.Solver(eos, 40, model="multi", flux=flux) as s:
+    with hyp.Solver(eos, 40, model="multi", flux=flux, precision=precision) as s:
         s.upload(Q0)
         with pytest.raises(hyp._lib.NegativeDeterminantError):
             s.step(max_steps=2)
