@@ -4,7 +4,9 @@
 // step. Host arrays in and out (SoA [k][n]).
 #include <cmath>
 #include <vector>
+#include <mutex>
 #include "hyp_internal.cuh"
+#include "hyp_paths64.cuh"
 #include "hyp_hank.cuh"
 #include "hyp_relax.cuh"
 
@@ -19,16 +21,57 @@ struct Buf {
   double* dev = nullptr;
 };
 
+// Device memory of the evaluators: one block per call from a pool of the library's own
+// on each device, which keeps at most kPoolKeep bytes between calls (cudaMalloc and
+// cudaFree of every array are a good part of a small call). The pool is the driver's:
+// safe from several threads, each call's block its own.
+constexpr uint64_t kPoolKeep = (uint64_t)64 << 20;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[256] = {};
+
+cudaMemPool_t eval_pool() {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 256) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps p = {};
+    p.allocType = cudaMemAllocationTypePinned;
+    p.location.type = cudaMemLocationTypeDevice;
+    p.location.id = dev;
+    cudaMemPool_t pool;
+    uint64_t keep = kPoolKeep;
+    if (cudaMemPoolCreate(&pool, &p) != cudaSuccess) return nullptr;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaMemPoolDestroy(pool);
+      return nullptr;
+    }
+    g_pool[dev] = pool;
+  }
+  return g_pool[dev];
+}
+
 int run(int64_t n, std::vector<Buf> bufs, void (*launch)(int64_t, double**, const void*), const void* arg) {
   if (n <= 0) return n == 0 ? HYP_OK : HYP_ERR_INVALID;
   for (auto& b : bufs)
     if (!b.host_in && !b.host_out) return HYP_ERR_INVALID;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return HYP_ERR_NO_DEVICE;
+  const cudaMemPool_t pool = eval_pool();
+  if (!pool) return HYP_ERR_CUDA;
+  size_t rows = 0;
+  for (auto& b : bufs) rows += b.k;
+  double* base = nullptr;
+  // the legacy default stream, as the copies and kernels below
+  if (cudaMallocFromPoolAsync((void**)&base, rows * n * sizeof(double), pool, 0) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return HYP_ERR_CUDA;
+  }
   int rc = HYP_OK;
   std::vector<double*> ptrs;
+  double* at = base;
   for (auto& b : bufs) {
-    if (cudaMalloc(&b.dev, (size_t)b.k * n * sizeof(double)) != cudaSuccess) { rc = HYP_ERR_CUDA; break; }
+    b.dev = at;
+    at += (size_t)b.k * n;
     if (b.host_in && cudaMemcpy(b.dev, b.host_in, (size_t)b.k * n * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
       rc = HYP_ERR_CUDA;
       break;
@@ -37,14 +80,13 @@ int run(int64_t n, std::vector<Buf> bufs, void (*launch)(int64_t, double**, cons
   }
   if (rc == HYP_OK) {
     launch(n, ptrs.data(), arg);
-    if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) rc = HYP_ERR_CUDA;
+    if (cudaGetLastError() != cudaSuccess) rc = HYP_ERR_CUDA;
   }
-  for (auto& b : bufs) {
+  for (auto& b : bufs)
     if (rc == HYP_OK && b.host_out &&
         cudaMemcpy(b.host_out, b.dev, (size_t)b.k * n * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess)
       rc = HYP_ERR_CUDA;
-    if (b.dev) cudaFree(b.dev);
-  }
+  if (cudaFreeAsync(base, 0) != cudaSuccess || cudaStreamSynchronize(0) != cudaSuccess) rc = rc == HYP_OK ? HYP_ERR_CUDA : rc;
   return rc;
 }
 
@@ -401,20 +443,40 @@ extern "C" int hyp_eval_eigvals_dir(const hyp_config* cfg, const double* Q, cons
 }
 namespace {
 struct LxfArg2 {
-  ModelArg m;
+  Eos2x E;
   Quad6D qd;
+  bool def;
 };
-__global__ void k_lxf2(LxfArg2 a, const double* Ql, const double* Qr, const double* lam, double* cons, double* DMo,
-                       double* DPo, int64_t n) {
-  IDX double ql[30], qr[30], fl[30], fr[30], ff[30], dm[30], dp[30];
-  LD(ql, Ql, 30);
-  LD(qr, Qr, 30);
-  flux2(a.m.e, ql, fl);
-  flux2(a.m.e, qr, fr);
-  lxf_face2(a.m.e, a.qd, ql, qr, fl, fr, lam[i], ff, dm, dp);
-  ST(cons, ff, 30);
-  ST(DMo, dm, 30);
-  ST(DPo, dp, 30);
+// The two-phase LxF face (NumFluxes.jl:25-60): conservative part (f_l + f_r)/2 - lambda
+// (Q_r - Q_l)/2, D- = D+ = half the Gauss-Lobatto integral of B, on the step's compact
+// cell forms. A thread per face and 64 to a block, so that a few thousand faces spread
+// over the multiprocessors. 4096 faces, the whole call: 1.43 ms with the general forms and
+// an allocation per array, 0.91 ms.
+constexpr int kFaceBlock64 = 64;
+template <int kDef>
+__global__ void k_lxf2(Eos2x E, Quad6D lobatto, const double* Ql, const double* Qr, const double* lam, double* cons,
+                       double* DMo, double* DPo, int64_t n) {
+  const int64_t i = (int64_t)blockIdx.x * kFaceBlock64 + threadIdx.x;
+  if (i >= n) return;
+  double a[30], b[30], acc[30];
+  LD(a, Ql, 30);
+  LD(b, Qr, 30);
+  const double hl = lam[i] * 0.5;
+  for (int p = 0; p < 2; ++p) {
+    double f[2][14];
+    for (int s = 0; s < 2; ++s) {
+      const double* q = (s ? b : a) + 15 * p;
+      const Cell64 c = cell64<kDef>(E.e[p], E.k[p], rcp64(q[0]), q + 2, q[5], q + 6);
+      flux64(q[0], c, q + 2, q + 6, f[s]);
+    }
+    for (int r = 0; r < 15; ++r) {
+      const double fs = r > 0 ? f[0][r - 1] + f[1][r - 1] : 0.0;
+      cons[(15 * p + r) * n + i] = 0.5 * fs - hl * (b[15 * p + r] - a[15 * p + r]);
+      acc[15 * p + r] = 0.0;
+    }
+  }
+  path_thread<kDef>(E, lobatto, a, b, acc);
+  for (int k = 0; k < 30; ++k) DMo[k * n + i] = DPo[k * n + i] = 0.5 * acc[k];
 }
 }  // namespace
 
@@ -422,12 +484,16 @@ extern "C" int hyp_eval_lxf(const hyp_config* cfg, const double* Ql, const doubl
                             double* cons, double* dm, double* dp, int64_t n) {
   if (!model_ok(cfg)) return HYP_ERR_INVALID;
   if (cfg->model == HYP_MODEL_MULTI) {
-    LxfArg2 a2{model_arg(cfg), gauss_lobatto6()};
+    const ModelArg m2 = model_arg(cfg);
+    LxfArg2 a2{make_eos2x(m2.e), gauss_lobatto6(), m2.e[0].default_exp && m2.e[1].default_exp};
     return run(n,
                {{Ql, nullptr, 30}, {Qr, nullptr, 30}, {lambda, nullptr, 1}, {nullptr, cons, 30}, {nullptr, dm, 30},
                 {nullptr, dp, 30}},
                [](int64_t n, double** d, const void* a) {
-                 k_lxf2<<<grid(n), kBlock>>>(*(const LxfArg2*)a, d[0], d[1], d[2], d[3], d[4], d[5], n);
+                 const LxfArg2& x = *(const LxfArg2*)a;
+                 auto kern = x.def ? k_lxf2<1> : k_lxf2<0>;
+                 kern<<<(unsigned)((n + kFaceBlock64 - 1) / kFaceBlock64), kFaceBlock64>>>(x.E, x.qd, d[0], d[1], d[2],
+                                                                                          d[3], d[4], d[5], n);
                },
                &a2);
   }
