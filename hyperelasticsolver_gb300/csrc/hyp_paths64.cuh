@@ -15,7 +15,7 @@ struct Eos2x {
 
 // Rows of a phase's 15 whose physical flux is identically zero: alpha and the first row
 // of alpha rho A.
-__device__ __forceinline__ constexpr bool zero_flux_row(int r) { return r == 0 || (r >= 6 && (r - 6) % 3 == 0); }
+HYP_HD constexpr bool zero_flux_row(int r) { return r == 0 || (r >= 6 && (r - 6) % 3 == 0); }
 inline Eos2x make_eos2x(const EosC* e) {
   Eos2x E;
   for (int p = 0; p < 2; ++p) {
@@ -31,7 +31,7 @@ struct Half64 {
   double u[3], K[3], T;
 };
 template <int kDef>
-__device__ __forceinline__ int half64(const EosC& e, const Eos64& k, double ia, const double* m, double rE,
+HYP_HD int half64(const EosC& e, const Eos64& k, double ia, const double* m, double rE,
                                       const double* R, Half64& h) {
   const Cell64 c = cell64<kDef>(e, k, ia, m, rE, R);
   const double m2 = -2.0 * c.td;
@@ -49,7 +49,7 @@ __device__ __forceinline__ int half64(const EosC& e, const Eos64& k, double ia, 
 struct Face64 {
   double u[3], s[3], p;
 };
-__device__ __forceinline__ Face64 interface64(const Half64& a, const Half64& b) {
+HYP_HD Face64 interface64(const Half64& a, const Half64& b) {
   Face64 I;
   const double inv = rcp64(a.T + b.T), ha = b.T * inv, hb = a.T * inv;
 #pragma unroll
@@ -63,7 +63,7 @@ __device__ __forceinline__ Face64 interface64(const Half64& a, const Half64& b) 
 
 // acc += wd B(q) e_alpha for one phase's rows (row 1 of B is zero), B's rho A part with
 // alpha rho A / alpha in place of rho A.
-__device__ __forceinline__ void add_b64(double wd, double ia, const double* R, const double* u, const Face64& I,
+HYP_HD void add_b64(double wd, double ia, const double* R, const double* u, const Face64& I,
                                         double* acc) {
   acc[0] = fma(wd, I.u[0], acc[0]);
   acc[2] = fma(wd, I.s[0], acc[2]);
@@ -81,17 +81,96 @@ __device__ __forceinline__ void add_b64(double wd, double ia, const double* R, c
   }
 }
 
-// One thread per face: acc += the path integral from a to b (30 values each), 6 nodes of
-// both phases, 360 slots a node. Rolled: six copies of the node overflow the
-// instruction cache.
+// Nodes a path integral from a to b (30 values) needs to be its 6-point value to FP64
+// rounding: 2, 3 or 6 points of Gauss-Legendre.
+//
+// Along the path B is analytic in s: its singularities are alpha = 0, det R = 0 and a
+// vanishing temperature (the entropy clamp aside). If every one of these quantities
+// changes by at most w (relatively) from a to b, then for |s - s'| <= 1 / (4 w) they stay
+// within a quarter of their values, B within a small factor M of its own, and Cauchy's
+// estimate of its derivatives in the error term of the m-point rule gives
+//   (m!)^4 / ((2m + 1) ((2m)!)^2) (4 w)^(2m) M d(alpha):
+// 5.6e-3 (4w)^4 for m = 2, 3.6e-4 (4w)^6 for m = 3. The rule is taken when this is below
+// 2^-57 alpha M, a sixteenth of the rounding of the flux difference the integral is
+// added to. All estimates in FP32 on generous sides; NaN gives 6.
+HYP_HD int path_nodes(const EosC* e, const double* a, const double* b) {
+  float w = 0.0f, jump = 0.0f;
+  for (int p = 0; p < 2; ++p) {
+    const double *qa = a + 15 * p, *qb = b + 15 * p;
+    const float al = to_f32(qa[0]), be = to_f32(qb[0]), lo = fminf(al, be);
+    if (!(lo > 0.0f)) return 6;
+    const float ra = fabsf(be - al) / lo, ia = 1.0f / al, ib = 1.0f / be;
+    // B depends on the path through q / alpha alone, and q / alpha runs on a straight line
+    float F[9], dF2 = 0.0f, F2 = 0.0f, v2 = 0.0f, dv2 = 0.0f;
+    for (int k = 0; k < 9; ++k) {
+      F[k] = to_f32(qa[6 + k]) * ia;
+      const float d = to_f32(qb[6 + k]) * ib - F[k];
+      dF2 += d * d;
+      F2 += F[k] * F[k];
+    }
+    for (int k = 0; k < 3; ++k) {
+      const float v = to_f32(qa[2 + k]) * ia, d = to_f32(qb[2 + k]) * ib - v;
+      v2 += v * v;
+      dv2 += d * d;
+    }
+    const float rE = to_f32(qa[5]) * ia, drE = fabsf(to_f32(qb[5]) * ib - rE);
+    const float c00 = F[4] * F[8] - F[5] * F[7], c01 = F[7] * F[2] - F[1] * F[8], c02 = F[1] * F[5] - F[4] * F[2];
+    const float c10 = F[5] * F[6] - F[3] * F[8], c11 = F[0] * F[8] - F[2] * F[6], c12 = F[2] * F[3] - F[0] * F[5];
+    const float c20 = F[3] * F[7] - F[4] * F[6], c21 = F[1] * F[6] - F[0] * F[7], c22 = F[0] * F[4] - F[1] * F[3];
+    const float det = F[0] * c00 + F[3] * c01 + F[6] * c02;
+    const float cc = c00 * c00 + c01 * c01 + c02 * c02 + c10 * c10 + c11 * c11 + c12 * c12 + c20 * c20 + c21 * c21 +
+                     c22 * c22;
+    if (!(det > 0.0f)) return 6;
+    // ||dF|| ||F^-1||, with the FP32 rounding of dF
+    const float dF = (sqrtf(dF2) + 2e-7f * sqrtf(F2)) * sqrtf(cc) / det;
+    const float rho = sqrtf(det * (float)e[p].inv_rho0), s = rho * (float)e[p].inv_rho0;
+    if (!(s > 0.25f && s < 4.0f)) return 6;
+    // specific energy minus the elastic part: (x - 1) cv t0 Pg, x the temperature over t0 Pg
+    const float u = sqrtf(v2) / rho, du = (sqrtf(dv2) + 1.5f * sqrtf(v2) * dF) / rho, E = rE / rho;
+    // |G| and its deviator from F: G = rho^2 (F F^T)^-1, tr G = rho^2 cc / det^2
+    const float i1 = rho * rho * cc / (det * det), i2 = s * s * F2 / (rho * rho);  // det G = s^2, tr G^-1 = |F|^2 / rho^2
+    const float psi = fmaxf(i1 * i1 * (1.0f / 3.0f) - i2, 0.0f);
+    const float ga = (float)e[p].gamma, be_ = (float)e[p].beta, aa = (float)e[p].alpha;
+    const float Pa = powf(s, aa), Pb = powf(s, be_), Pg = powf(s, ga);
+    const float cvt0 = (float)e[p].cvt0, kU = (float)e[p].kU, b0sq = (float)e[p].b0sq;
+    const float therm = E - 0.5f * u * u - 0.5f * b0sq * Pb * psi - kU * (Pa - 1.0f) * (Pa - 1.0f);
+    const float x = therm / (cvt0 * Pg) + 1.0f;
+    const float grow = powf(1.25f * fmaxf(s, 1.0f / s), fmaxf(2.0f * fabsf(aa), fmaxf(fabsf(be_), fabsf(ga))));
+    const float dE = drE / rho + 1.5f * fabsf(E) * dF + u * du + du * du +
+                     4.0f * (2.0f * fabsf(kU) * aa * aa + 2.0f * b0sq) * grow * dF;
+    if (!(x > 1e-3f)) return 6;
+    const float wF = 3.0f * dF, wx = dE / (cvt0 * Pg * x) + 2.0f * fabsf(ga) * dF;
+    if (!(ra < 0.125f && wF < 0.125f && wx < 0.125f)) return 6;  // (NaN too)
+    w = fmaxf(w, fmaxf(ra, fmaxf(wF, wx)));
+    jump = fmaxf(jump, ra);
+  }
+  const float d = 4.0f * w, d2 = d * d;
+  if (5.6e-3f * d2 * d2 * jump <= 7e-18f) return 2;
+  if (3.6e-4f * d2 * d2 * d2 * jump <= 7e-18f) return 3;
+  return 6;
+}
+
+// One thread per face: acc += the path integral from a to b (30 values each): the nodes
+// path_nodes asks for, of both phases, 360 slots a node. Rolled: six copies of the node
+// overflow the instruction cache. qd: the 6-point rule.
 template <int kDef>
-__device__ __forceinline__ int path_thread(const Eos2x& E, const Quad6D& qd, const double* a, const double* b,
-                                           double* acc) {
+HYP_HD int path_thread(const Eos2x& E, const Quad6D& qd, const double* a, const double* b, double* acc) {
   int st = 0;
   const double da0 = b[0] - a[0], da1 = b[15] - a[15];
+  const int nodes = path_nodes(E.e, a, b);
 #pragma unroll 1
-  for (int i = 0; i < 6; ++i) {
-    const double s = qd.x[i];
+  for (int i = 0; i < nodes; ++i) {
+    double s, w;
+    if (nodes == 6) {
+      s = qd.x[i];
+      w = qd.w[i];
+    } else if (nodes == 2) {  // 1/2 -+ 1/(2 sqrt 3)
+      s = i ? 0.78867513459481288 : 0.21132486540518712;
+      w = 0.5;
+    } else {  // 1/2, 1/2 -+ sqrt(3/5)/2
+      s = i == 0 ? 0.11270166537925831 : (i == 1 ? 0.5 : 0.88729833462074169);
+      w = i == 1 ? 4.0 / 9.0 : 5.0 / 18.0;
+    }
     double R[2][9], ia[2];
     Half64 h[2];
 #pragma unroll
@@ -106,8 +185,8 @@ __device__ __forceinline__ int path_thread(const Eos2x& E, const Quad6D& qd, con
       st |= half64<kDef>(E.e[p], E.k[p], ia[p], m, at(5), R[p], h[p]);
     }
     const Face64 I = interface64(h[0], h[1]);
-    add_b64(qd.w[i] * da0, ia[0], R[0], h[0].u, I, acc);
-    add_b64(qd.w[i] * da1, ia[1], R[1], h[1].u, I, acc + 15);
+    add_b64(w * da0, ia[0], R[0], h[0].u, I, acc);
+    add_b64(w * da1, ia[1], R[1], h[1].u, I, acc + 15);
   }
   return st;
 }

@@ -325,11 +325,13 @@ __device__ __forceinline__ double node_sum(const GroupMem& g, int k) {
 }
 
 // Lists of up to kGroupFaces faces per multiprocessor run in groups: a warp spends 620
-// slots on the two faces of its groups, and 6,600 on 32 faces with a thread each, so
-// groups win up to 10.6 x 2 faces on each of an SM's four schedulers. 1000 cells, 50 HLL
-// steps of a Riemann problem (whole run): 22.3 ms before this file's split of the faces,
-// 2.95 ms now; 100,003 cells with all faces listed, 4 steps: 10.3 and 6.6 ms.
-constexpr int kGroupFaces = 80;
+// slots on the two faces of its groups, and on 32 faces with a thread each 6,600 (2,300
+// where the states are smooth enough for two nodes, path_nodes): groups win up to 10.6 x
+// 2 (3.7 x 2) faces on each of an SM's four schedulers, 85 (30) a multiprocessor. 1000
+// cells, 50 HLL steps of a Riemann problem (whole run): 22.3 ms before this file's split
+// of the faces, 2.95 ms now; 100,003 cells with all faces listed, 4 steps: 10.3 ms, 6.8 with
+// six nodes a path, 3.3 with the nodes path_nodes asks for.
+constexpr int kGroupFaces = 48;
 
 // kLxf: one Gauss-Lobatto integral, D- = D+ = half of it (NumFluxes.jl:36-47), stored
 // doubled as the LxF faces are. Otherwise Q_hll and the fluctuations of
