@@ -352,10 +352,15 @@ static int enqueue_step(hyp_ctx* c, long long k, double t_end, bool prof, bool f
     if (c->relax) CK(launch_relax2(c, p, t_end));
   } else if (c->cfg.model == HYP_MODEL_MULTI) {
     const int p = (int)(k & 1);
-    CK(launch_cell2_f64(c, p, &c->st->lam_bits[p], &c->st->t[p], t_end));
-    CK(launch_face2_f64(c, p, t_end));
-    if (prof) CK(cudaEventRecord(e1, c->stream));
-    CK(launch_update2_f64(c, p, t_end));
+    if (prof) {
+      unsigned long long* rd = c->st->lam_slots + k % 3;
+      CK(launch_cell2_f64(c, p, rd, &c->st->t[p], t_end));
+      CK(launch_face2_f64(c, p, rd, t_end));
+      CK(cudaEventRecord(e1, c->stream));
+      CK(launch_update2_f64(c, k, t_end));
+    } else {
+      CK(launch_run_step2_f64(c, k, t_end, first, last));
+    }
     if (c->relax) CK(launch_relax2(c, p, t_end));
   } else if (!mixed(c)) {
     if (prof) {
@@ -392,9 +397,10 @@ static int collect_profile(hyp_ctx* c) {
 }
 
 // steps per captured graph: a multiple of the launch pattern's period
-static bool single(const hyp_ctx* c) { return c->cfg.model == HYP_MODEL_SINGLE; }
-static int graph_period(const hyp_ctx* c) { return single(c) ? 6 : 2; }  // parity x three max-lambda slots
-static int graph_steps(const hyp_ctx* c) { return single(c) ? 12 : 16; }
+// (parity x three max-lambda slots; the two-phase mixed step has a slot per parity)
+static bool three_slots(const hyp_ctx* c) { return !mixed(c) || mixed1(c); }
+static int graph_period(const hyp_ctx* c) { return three_slots(c) ? 6 : 2; }
+static int graph_steps(const hyp_ctx* c) { return three_slots(c) ? 12 : 16; }
 
 static int ensure_graph(hyp_ctx* c, long long k0, double t_end) {
   const int key = (int)(k0 % graph_period(c));

@@ -20,10 +20,10 @@ constexpr int kBlock = 256;
 // needs no host round trip (and can be captured in a CUDA graph).
 struct DevState {
   double t[2];                        // time before the step of parity p is t[p]
-  unsigned long long lam_bits[2];     // max wave speed of the state of parity p (bits of a double >= 0)
+  unsigned long long lam_bits[2];     // two-phase mixed, slabs: max wave speed of the state of parity p (bits of a double >= 0)
   unsigned long long lam_query;       // hyp_max_wavespeed slot
-  unsigned long long lam_slots[3];    // single phase: max lambda of states k, k+1 (slot k%3), FP32 bits (mixed)
-                                      // or FP64 bits
+  unsigned long long lam_slots[3];    // max lambda of states k, k+1 (slot k%3): FP64 bits, or the single-phase
+                                      // mixed step's FP32 bits
   long long steps;                    // steps taken
   int err_code;                       // first HYP_CELL_* status raised (0 = none)
   int pad_;
@@ -262,8 +262,9 @@ cudaError_t launch_install1_mixed(hyp_ctx* c, const double* q, unsigned long lon
 cudaError_t launch_step1_mixed(hyp_ctx* c, long long k, double t_end);
 // two-phase FP64 launchers (hyp_step2.cu)
 cudaError_t launch_cell2_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end);
-cudaError_t launch_face2_f64(hyp_ctx* c, int p, double t_end);
-cudaError_t launch_update2_f64(hyp_ctx* c, int p, double t_end);
+cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, double t_end);
+cudaError_t launch_update2_f64(hyp_ctx* c, long long k, double t_end);
+cudaError_t launch_run_step2_f64(hyp_ctx* c, long long k, double t_end, bool first, bool last);
 // two-phase pressure relaxation of the state the step of parity p wrote (hyp_relax.cu)
 cudaError_t launch_relax2(hyp_ctx* c, int p, double t_end);
 Quad6D gauss_legendre6();

@@ -82,10 +82,12 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
   if (own) {
     const bool frozen = bc_holds(a.bc, i == 0, i == n - 1);
     const double hdt = s_hdt;
+    // every load before the first store: the compiler has to keep their order
+#pragma unroll
+    for (int v = 0; v < 14; ++v) q[v] = a.Q[v * n + i];
 #pragma unroll
     for (int v = 0; v < 14; ++v) {
-      const double qc = a.Q[v * n + i];
-      q[v] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+      q[v] = frozen ? q[v] : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), q[v]);
       a.Qn[v * n + i] = q[v];
     }
   }

@@ -2,18 +2,19 @@
 // (main.jl:202-241 with update_cell :43-60 and NumFluxes.hll :70-132) or the
 // path-conservative Lax-Friedrichs flux (update_cell :30-41, NumFluxes.lxf :25-60).
 //
-// Four kernels per step on the context stream:
+// A run of steps is a cell pass of the first state and three kernels per step:
 //   cell   : per cell and phase, the flux (HyperelasticityMPh.jl:140-175) and
 //            wave-speed bounds (:252-266); lambda_i = max |speed|, block max ->
 //            one atomicMax (main.jl:204-212);
 //   face   : per face and phase, the midpoint's wave speeds and s_l, s_r (HLL), and the
 //            whole face wherever its path integrals vanish; the other faces go to a list;
-//   paths  : the listed faces' 6-point path integrals of B (HLL: three Gauss-Legendre
-//            ones, 18 evaluations of B instead of the 30 the reference makes, since the
+//   paths  : the listed faces' path integrals of B (HLL: three Gauss-Legendre ones, up to
+//            18 evaluations of B instead of the 30 the reference makes, since the
 //            integrals repeated in D- and D+ are the same; LxF: one Gauss-Lobatto);
-//   update : dt = cfl dx / max lambda, t += dt, Q_i - dt/dx ((F_r - F_l) + (D-_{i+1/2} + D+_{i-1/2}))
-//            with frozen or transmissive ends; F = 0 for HLL (it folds the conservative
-//            part into D+-), the LxF face flux otherwise.
+//   step   : dt = cfl dx / max lambda, t += dt, Q_i - dt/dx ((F_r - F_l) + (D-_{i+1/2} + D+_{i-1/2}))
+//            with frozen or transmissive ends (F = 0 for HLL, which folds the conservative
+//            part into D+-; the LxF face flux otherwise), then, unless it is the run's
+//            last step, the cell pass of the new state.
 //
 // What bounds them is FP64 issue (hyp_cell64.cuh), so the counts per face matter and
 // nothing else does. B dQ is a column times d(alpha) (HyperelasticityMPh.jl:178-250):
@@ -33,36 +34,34 @@ namespace hyp {
 constexpr int kPairCells = 64;             // cells (faces) of a block: one thread per phase of each
 constexpr int kPair64 = 2 * kPairCells;    // its threads; the phase is uniform over a warp
 
+struct CellOut2 {
+  double *F, *smin, *smax;  // fluxes [30][n], wave-speed bounds
+  int64_t n;
+  DevState* S;
+};
+
+// The cell pass of a block's 64 cells, a thread per phase in state q (15 values; `in`:
+// there is a cell): fluxes, speed bounds, and the block's max |speed| into slot. All
+// threads of the block call it.
 template <int kDef>
-__global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
-                                                            double* __restrict__ F, double* __restrict__ smin,
-                                                            double* __restrict__ smax, unsigned long long* lam_slot,
-                                                            const double* t_now, double t_end, DevState* S) {
+__device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, const Eos2x& E, const CellOut2& o,
+                                           unsigned long long* slot) {
   __shared__ double s_lo[kPairCells], s_hi[kPairCells];
-  if (!(*t_now < t_end)) return;
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
-  const int64_t i = (int64_t)blockIdx.x * kPairCells + j;
   double lo = 0.0, hi = 0.0;
-  if (i < n) {
-    const double* q0 = Q + 15 * ph * n + i;
-    double m[3], R[9];
-    const double alpha = q0[0], rE = q0[5 * n];
-#pragma unroll
-    for (int v = 0; v < 3; ++v) m[v] = q0[(2 + v) * n];
-#pragma unroll
-    for (int v = 0; v < 9; ++v) R[v] = q0[(6 + v) * n];
+  if (in) {
     const EosC& e = E.e[ph];
-    const Cell64 c = cell64<kDef>(e, E.k[ph], rcp64(alpha), m, rE, R);
+    const Cell64 c = cell64<kDef>(e, E.k[ph], rcp64(q[0]), q + 2, q[5], q + 6);
     double f[14];
-    flux64(alpha, c, m, R, f);
-    double* f0 = F + 15 * ph * n + i;
+    flux64(q[0], c, q + 2, q + 6, f);
+    double* f0 = o.F + 15 * ph * o.n + i;
 #pragma unroll
     for (int r = 1; r < 15; ++r)
-      if (!zero_flux_row(r)) f0[r * n] = f[r - 1];
+      if (!zero_flux_row(r)) f0[r * o.n] = f[r - 1];
     const double cm = cmax64<kDef>(e, E.k[ph], c);
     lo = c.u[0] - cm;
     hi = c.u[0] + cm;
-    if (c.st) record_err64(S, c.st, i);
+    if (c.st) record_err64(o.S, c.st, i);
     if (ph == 1) {
       s_lo[j] = lo;
       s_hi[j] = hi;
@@ -70,16 +69,31 @@ __global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __rest
   }
   __syncthreads();
   double l = 0.0;
-  if (ph == 0 && i < n) {
+  if (ph == 0 && in) {
     if (s_lo[j] < lo) lo = s_lo[j];
     if (s_hi[j] > hi) hi = s_hi[j];
-    smin[i] = lo;
-    smax[i] = hi;
+    o.smin[i] = lo;
+    o.smax[i] = hi;
     l = fmax(fabs(lo), fabs(hi));
-    if (!is_finite64(l)) record_err64(S, HYP_CELL_NONFINITE, i);
+    if (!is_finite64(l)) record_err64(o.S, HYP_CELL_NONFINITE, i);
   }
   const unsigned long long m = block_max_bits<kPair64>(l);
-  if (threadIdx.x == 0) atomicMax(lam_slot, m);
+  if (threadIdx.x == 0) atomicMax(slot, m);
+}
+
+template <int kDef>
+__global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __restrict__ Q, Eos2x E, CellOut2 o,
+                                                            unsigned long long* lam_slot, const double* t_now,
+                                                            double t_end) {
+  if (!(*t_now < t_end)) return;
+  const int64_t i = (int64_t)blockIdx.x * kPairCells + threadIdx.x % kPairCells;
+  double q[15];
+  if (i < o.n) {
+    const double* q0 = Q + 15 * (threadIdx.x / kPairCells) * o.n + i;
+#pragma unroll
+    for (int r = 0; r < 15; ++r) q[r] = q0[r * o.n];
+  }
+  cell2_pass<kDef>(q, i < o.n, i, E, o, lam_slot);
 }
 
 // ---- faces ---------------------------------------------------------------------
@@ -350,10 +364,16 @@ __global__ void __launch_bounds__(kPathBlock, 2)
     if ((int)blockIdx.x >= blocks) return;
     const int lane16 = threadIdx.x & 15;
     GroupMem& g = sg[threadIdx.x >> 4];
+    // A list of no more faces than schedulers gives each a warp: both its groups do the
+    // first integral, then each one of the two through Q_hll.
+    const bool wide = !kLxf && count <= 4 * sms;
+    const int grp = (threadIdx.x >> 4) & 1, base = (threadIdx.x >> 4) & ~1;
     // both groups of a warp go round together (the exchanges are warp-wide): an idle one
     // repeats the list's last face and stores nothing
-    const int first = blockIdx.x * kGroups + (threadIdx.x >> 4), pair = first & ~1;
-    for (int t = first, tp = pair; tp < count; t += blocks * kGroups, tp += blocks * kGroups) {
+    const int group = blockIdx.x * kGroups + (threadIdx.x >> 4);
+    const int first = wide ? group >> 1 : group, pair = wide ? first : first & ~1;
+    const int stride = blocks * (wide ? kGroups / 2 : kGroups);
+    for (int t = first, tp = pair; tp < count; t += stride, tp += stride) {
       const bool live = t < count;
       const int at = live ? t : count - 1;
       const int64_t f = list.face[at], L = f - 1, R = f;
@@ -383,17 +403,18 @@ __global__ void __launch_bounds__(kPathBlock, 2)
 #pragma unroll
         for (int r = 0; r < 15; ++r) acc[r] = 0.0;
 #pragma unroll 1
-        for (int half = 0; half < 2; ++half)
-          st |= path_group<kDef>(E, qd, lane16, g, half ? 2 : 0, half ? 1 : 2, acc);
+        for (int h = wide ? grp : 0; h < (wide ? grp + 1 : 2); ++h)
+          st |= path_group<kDef>(E, qd, lane16, g, h ? 2 : 0, h ? 1 : 2, acc);
         if (lane16 < 12)
 #pragma unroll
           for (int r = 0; r < 15; ++r) g.part[lane16][r] = acc[r];
         __syncwarp();
         const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
         if (live)
-          for (int k = lane16; k < 30; k += 16) {
+          for (int k = wide ? threadIdx.x & 31 : lane16; k < 30; k += wide ? 32 : 16) {
             const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
-            const double inner = df + node_sum(g, k), qj = cq * (g.q[1][k] - g.q[0][k]);
+            const double sum = wide ? node_sum(sg[base], k) + node_sum(sg[base + 1], k) : node_sum(g, k);
+            const double inner = df + sum, qj = cq * (g.q[1][k] - g.q[0][k]);
             DM[k * nf + f] = cm * inner + qj;
             DP[k * nf + f] = cp * inner - qj;
           }
@@ -436,45 +457,79 @@ __global__ void __launch_bounds__(kPathBlock, 2)
   }
 }
 
-// FF: twice the LxF face flux (with D- = D+ doubled as well), or null for HLL.
-__global__ void __launch_bounds__(kBlock64) update2_f64_kernel(const double* __restrict__ Q, double* __restrict__ Qn,
-                                                               int64_t n, const double* __restrict__ FF,
-                                                               const double* __restrict__ DM,
-                                                               const double* __restrict__ DP,
-                                                               const unsigned long long* lam_in,
-                                                               unsigned long long* lam_next, const double* t_in,
-                                                               double* t_out, DevState* S, double t_end, double cfl,
-                                                               double dx, int bc) {
+// The update of a step: FF twice the LxF face flux (with D- = D+ doubled as well), or null
+// for HLL. rd: the max wave speed; an active step zeroes the clr slots.
+struct Step2Args {
+  const double* Q;
+  double* Qn;
+  const double *FF, *DM, *DP;
+  const unsigned long long* rd;
+  unsigned long long* wr;
+  unsigned long long* clr[2];
+  const double* t_in;
+  double* t_out;
+  double t_end, cfl, dx;
+  int bc;
+  CellOut2 o;
+};
+
+// A thread per cell and phase; with kCell the new state's cell pass follows in the same
+// kernel (a launch and a reload of the state less per step, which a small problem feels).
+template <int kDef, bool kCell>
+__global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E) {
   __shared__ double s_r;
-  const double tn = *t_in;
-  const bool active = tn < t_end;
+  __shared__ int s_more;
+  const int64_t n = a.o.n, nf = n + 1;
+  const double tn = *a.t_in;
+  const bool active = tn < a.t_end;
   if (threadIdx.x < 32) {
-    const StepScalars sc = step_scalars64(cfl, dx, __longlong_as_double((long long)*lam_in), false);
-    if (threadIdx.x == 0) s_r = FF ? 0.5 * sc.dtdx : sc.dtdx;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      *t_out = active ? tn + sc.dt : tn;
-      *lam_next = 0ull;
-      S->n_listed = 0;
-      if (active) S->steps += 1;
+    const StepScalars sc = step_scalars64(a.cfl, a.dx, __longlong_as_double((long long)*a.rd), false);
+    if (threadIdx.x == 0) {
+      s_r = a.FF ? 0.5 * sc.dtdx : sc.dtdx;
+      s_more = kCell && tn + sc.dt < a.t_end;
+      if (blockIdx.x == 0) {
+        *a.t_out = active ? tn + sc.dt : tn;
+        a.o.S->n_listed = 0;
+        if (active) {
+          for (int c = 0; c < 2; ++c)
+            if (a.clr[c]) *a.clr[c] = 0ull;
+          a.o.S->steps += 1;
+        }
+      }
     }
   }
   if (!active) return;
   __syncthreads();
-  const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
-  if (i >= n) return;
-  const int64_t nf = n + 1;
-  if (bc == HYP_BC_FROZEN && (i == 0 || i == n - 1)) {
-    for (int v = 0; v < 30; ++v) Qn[v * n + i] = Q[v * n + i];
-    return;
+  const int ph = threadIdx.x / kPairCells;
+  const int64_t i = (int64_t)blockIdx.x * kPairCells + threadIdx.x % kPairCells;
+  double q[15];
+  if (i < n) {
+    const bool frozen = a.bc == HYP_BC_FROZEN && (i == 0 || i == n - 1);
+    const double r = s_r;
+    // every load before the first store: the compiler has to keep their order
+    double d[15];
+#pragma unroll
+    for (int v = 0; v < 15; ++v) {
+      const int64_t row = 15 * ph + v;
+      // F_r = F_l = zeros(30) for hll (NumFluxes.jl:82), NF_r = D- of face i+1/2, NF_l = D+ of face i-1/2
+      q[v] = a.Q[row * n + i];
+      d[v] = a.DM[row * nf + i + 1] + a.DP[row * nf + i];
+    }
+    if (a.FF) {
+#pragma unroll
+      for (int v = 0; v < 15; ++v) {
+        const int64_t row = 15 * ph + v;
+        d[v] += a.FF[row * nf + i + 1] - a.FF[row * nf + i];
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 15; ++v) {
+      q[v] = frozen ? q[v] : fma(-r, d[v], q[v]);
+      a.Qn[(15 * ph + v) * n + i] = q[v];
+    }
   }
-  const double r = s_r;
-#pragma unroll 6
-  for (int v = 0; v < 30; ++v) {
-    // F_r = F_l = zeros(30) for hll (NumFluxes.jl:82), NF_r = D- of face i+1/2, NF_l = D+ of face i-1/2
-    double d = DM[v * nf + i + 1] + DP[v * nf + i];
-    if (FF) d += FF[v * nf + i + 1] - FF[v * nf + i];
-    Qn[v * n + i] = fma(-r, d, Q[v * n + i]);
-  }
+  if (!kCell || !s_more) return;
+  cell2_pass<kDef>(q, i < n, i, E, a.o, a.wr);
 }
 
 static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -482,20 +537,21 @@ static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) 
 static Eos2x eos2x(const hyp_ctx* c) { return make_eos2x(c->eos2.e); }
 static bool default_exp2(const hyp_ctx* c) { return c->eos2.e[0].default_exp && c->eos2.e[1].default_exp; }
 
+static CellOut2 cell_out(hyp_ctx* c) { return CellOut2{c->F, c->smin, c->smax, c->n, c->st}; }
+
 cudaError_t launch_cell2_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end) {
   auto kern = default_exp2(c) ? cell2_f64_kernel<1> : cell2_f64_kernel<0>;
-  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(c->Q[p], c->n, eos2x(c), c->F, c->smin, c->smax, lam_slot,
-                                                            t_now, t_end, c->st);
+  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(c->Q[p], eos2x(c), cell_out(c), lam_slot, t_now, t_end);
   return cudaGetLastError();
 }
-cudaError_t launch_face2_f64(hyp_ctx* c, int p, double t_end) {
+cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, double t_end) {
   const bool lxf = c->cfg.flux == HYP_FLUX_LXF, def = default_exp2(c);
   const FaceList list{c->face_list, c->face_s, c->face_s ? c->face_s + c->n + 1 : nullptr};
   const unsigned grid = grid_n(c->n + 1, kPairCells);
   const Eos2x E = eos2x(c);
   if (lxf) {
     const double dx = c->cfg.x_length / (double)c->n;
-    face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, c->F, &c->st->lam_bits[p], c->cfg.cfl, dx,
+    face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, c->F, rd, c->cfg.cfl, dx,
                                                           c->FF, c->DM, list, &c->st->t[p], t_end, c->st);
   } else {
     auto kern = def ? face2_f64_kernel<1> : face2_f64_kernel<0>;
@@ -512,13 +568,44 @@ cudaError_t launch_face2_f64(hyp_ctx* c, int p, double t_end) {
                                              &c->st->t[p], t_end, c->sms, c->st);
   return cudaGetLastError();
 }
-cudaError_t launch_update2_f64(hyp_ctx* c, int p, double t_end) {
-  const double dx = c->cfg.x_length / (double)c->n;
+// The update of step k, and with `cell` the cell pass of the new state.
+static cudaError_t launch_step2(hyp_ctx* c, long long k, double t_end, bool cell) {
+  const int p = (int)(k & 1);
   const bool lxf = c->cfg.flux == HYP_FLUX_LXF;
-  update2_f64_kernel<<<grid_n(c->n, kBlock64), kBlock64, 0, c->stream>>>(
-      c->Q[p], c->Q[1 - p], c->n, lxf ? c->FF : nullptr, c->DM, lxf ? c->DM : c->DP, &c->st->lam_bits[p],
-      &c->st->lam_bits[1 - p], &c->st->t[p], &c->st->t[1 - p], c->st, t_end, c->cfg.cfl, dx, c->cfg.bc);
+  unsigned long long* s = c->st->lam_slots;
+  Step2Args a;
+  a.Q = c->Q[p];
+  a.Qn = c->Q[1 - p];
+  a.FF = lxf ? c->FF : nullptr;
+  a.DM = c->DM;
+  a.DP = lxf ? c->DM : c->DP;
+  a.rd = s + k % 3;
+  a.wr = s + (k + 1) % 3;
+  a.clr[0] = s + (k + 2) % 3;
+  a.clr[1] = cell ? nullptr : a.wr;
+  a.t_in = &c->st->t[p];
+  a.t_out = &c->st->t[1 - p];
+  a.t_end = t_end;
+  a.cfl = c->cfg.cfl;
+  a.dx = c->cfg.x_length / (double)c->n;
+  a.bc = c->cfg.bc;
+  a.o = cell_out(c);
+  auto kern = !cell ? step2_f64_kernel<1, false> : (default_exp2(c) ? step2_f64_kernel<1, true> : step2_f64_kernel<0, true>);
+  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(a, eos2x(c));
   return cudaGetLastError();
+}
+cudaError_t launch_update2_f64(hyp_ctx* c, long long k, double t_end) { return launch_step2(c, k, t_end, false); }
+
+// Step k of a run (first / last of it), the slots as in launch_run_step1_f64. Relaxation
+// changes the new state after the update, so its cell pass waits for the next step.
+cudaError_t launch_run_step2_f64(hyp_ctx* c, long long k, double t_end, bool first, bool last) {
+  const int p = (int)(k & 1);
+  unsigned long long* rd = c->st->lam_slots + k % 3;
+  cudaError_t e = cudaSuccess;
+  if (first || c->relax) e = launch_cell2_f64(c, p, rd, &c->st->t[p], t_end);
+  if (e == cudaSuccess) e = launch_face2_f64(c, p, rd, t_end);
+  if (e == cudaSuccess) e = launch_step2(c, k, t_end, !last && !c->relax);
+  return e;
 }
 
 // Gauss-Legendre 6 on [0,1]: Newton on P6 from Chebyshev-like guesses in long

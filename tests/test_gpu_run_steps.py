@@ -79,3 +79,43 @@ def test_batch_cuts_agree(hyp):
             s.upload(np.ascontiguousarray(Q0[:, lo:lo + n]))
             _, tp = s.step(max_steps=int(steps[p]))
             assert tp == t[p] and np.array_equal(s.download(), Q[:, lo:lo + n])
+
+
+@pytest.mark.parametrize("n", [3, 64, 65, 300])
+@pytest.mark.parametrize("flux", ["hll", "lxf"])
+@pytest.mark.parametrize("relax", [None, "mechanical"])
+def test_two_phase_cuts_agree(hyp, n, flux, relax):
+    from hyperelasticsolver_gb300 import HyperelasticityMPh as HM
+    eos = (hyp.Barton2009(), hyp.Barton2009(_b0=2.1 * 0.1 ** 0.5))
+    Ql, Qr = HM.initial_states(eos, 4)
+    out = []
+    for cut in CUTS:
+        with hyp.Solver(eos, n, model="multi", flux=flux, relax=relax) as s:
+            s.init_tanh(Ql, Qr, 0.2)
+            for k in cut:
+                assert s.step(max_steps=k)[0] == k
+            out.append((s.download(), s.time()))
+    for Q, t in out[1:]:
+        assert np.array_equal(Q, out[0][0]) and t == out[0][1]
+
+
+def test_two_phase_stop_and_profile(hyp):
+    from hyperelasticsolver_gb300 import HyperelasticityMPh as HM
+    eos = (hyp.Barton2009(), hyp.Barton2009(_b0=2.1 * 0.1 ** 0.5))
+    Ql, Qr = HM.initial_states(eos, 6)
+    ref = []
+    with hyp.Solver(eos, 100, model="multi", flux="hll") as s:
+        s.init_riemann(Ql, Qr)
+        for _ in range(20):
+            ref.append((s.step(max_steps=1)[1], s.download()))
+    for stop in (1, 2, 3, 13):
+        with hyp.Solver(eos, 100, model="multi", flux="hll") as s:
+            s.init_riemann(Ql, Qr)
+            t_end = 0.5 * (ref[stop - 2][0] + ref[stop - 1][0]) if stop > 1 else 0.5 * ref[0][0]
+            assert s.step(t_end=t_end) == (stop, ref[stop - 1][0])
+            assert s.step(max_steps=20, t_end=t_end)[0] == 0
+            s.set_profiling(True)
+            s.step(max_steps=2)
+            s.set_profiling(False)
+            assert s.step(max_steps=18 - stop)[1] == ref[19][0]
+            assert np.array_equal(s.download(), ref[19][1])
