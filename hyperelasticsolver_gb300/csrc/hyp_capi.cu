@@ -1,4 +1,5 @@
 // hyp_capi.cu -- context lifecycle, transfers and the step driver of the C ABI.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -109,6 +110,8 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
   if ((e = cudaGetDevice(&c->device)) != cudaSuccess) fail(e, "cudaGetDevice");
   if (rc == HYP_OK && (e = cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->device)) != cudaSuccess)
     fail(e, "cudaDeviceGetAttribute");
+  if (rc == HYP_OK && (e = cudaDeviceGetAttribute(&c->coop, cudaDevAttrCooperativeLaunch, c->device)) != cudaSuccess)
+    fail(e, "cudaDeviceGetAttribute");
   if (rc == HYP_OK && (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess)
     fail(e, "cudaStreamCreate");
   if (rc == HYP_OK && (e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking)) != cudaSuccess)
@@ -162,7 +165,8 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
   } else if (!mixed(c)) {
     for (int p = 0; p < 2 && rc == HYP_OK; ++p)
       if ((e = cudaMalloc(&c->Q[p], nq)) != cudaSuccess) fail(e, "cudaMalloc(Q)");
-    const size_t nf = (size_t)(kNFlux1 + 1) * c->n * sizeof(double);  // fluxes, then the wave speeds
+    // fluxes, then the wave speeds; or the edge cells of a run in one launch
+    const size_t nf = std::max((size_t)(kNFlux1 + 1) * c->n, run1_edge_doubles(c->n)) * sizeof(double);
     if (rc == HYP_OK && (e = cudaMalloc(&c->flux1[0], nf)) != cudaSuccess) fail(e, "cudaMalloc(F)");
     if (rc == HYP_OK && cudaMalloc(&c->flux1[1], nf) != cudaSuccess) {
       (void)cudaGetLastError();  // no room for a second one: the step's kernels run apart
@@ -428,6 +432,9 @@ static int ensure_graph(hyp_ctx* c, long long k0, double t_end) {
   return HYP_OK;
 }
 
+// steps of one run1 launch: a few tens of milliseconds
+constexpr long long kRunSteps = 4096;
+
 // hyp_step_times: the time after a step, copied once the step's kernels are done
 __global__ void log_time_kernel(const DevState* S, int parity, double* out) { *out = S->t[parity]; }
 
@@ -448,11 +455,27 @@ extern "C" int hyp_step(hyp_ctx* c, int max_steps, double t_end, int* steps_done
   // chunks and stop once the device reports t >= t_end.
   const long long chunk = std::isinf(t_end) ? (unlimited ? 0 : max_steps) : 256;
   const int gs = graph_steps(c);
+  // small single-phase FP64 problems: the whole run in one launch (not where each step is
+  // timed or logged)
+  const bool one_launch = !mixed(c) && c->cfg.model == HYP_MODEL_SINGLE && !prof && !c->hist_on && c->coop &&
+                          run1_fits(c->n, c->sms);
   int rc = HYP_OK;
   while (rc == HYP_OK) {
     long long todo = unlimited ? chunk : (max_steps - launched);
     if (!std::isinf(t_end) && todo > chunk) todo = chunk;
     if (todo <= 0) break;
+    if (one_launch) {
+      todo = std::min<long long>(todo, kRunSteps);
+      cudaError_t e = launch_run1_f64(c, steps0 + launched, (int)todo, t_end);
+      if (e != cudaSuccess) rc = set_err(c, HYP_ERR_CUDA, std::string("launch_run1_f64: ") + cudaGetErrorString(e));
+      launched += todo;
+      if (rc != HYP_OK) break;
+      if (std::isinf(t_end) && launched < max_steps) continue;
+      if (std::isinf(t_end)) break;
+      rc = sync_state(c);
+      if (rc != HYP_OK || c->st_host->err_code || !(c->st_host->t[0] < t_end)) break;
+      continue;
+    }
     // Every launched step advances the pattern index. An inactive step (t >= t_end)
     // copies t across and leaves the state and its max-lambda slot alone; active
     // steps always precede inactive ones, so the state index is steps0 + active.

@@ -28,6 +28,7 @@ struct DevState {
   int err_code;                       // first HYP_CELL_* status raised (0 = none)
   int pad_;
   long long err_cell;                 // cell that raised it
+  unsigned run_count, run_done;       // arrivals and exits of a run's blocks (run1_f64_kernel); 0 between launches
   int n_listed;                       // two-phase FP64: faces whose path integrals the step still has to do
 };
 
@@ -158,6 +159,7 @@ struct hyp_ctx {
   int* face_list = nullptr;   // two-phase FP64: listed faces [n+1], and (HLL) their s_l, s_r [2][n+1]
   double* face_s = nullptr;
   int sms = 0;                // multiprocessors of the device
+  int coop = 0;               // it runs cooperative launches
   hyp::DevState* st = nullptr;
   hyp::DevState* st_host = nullptr;  // pinned mirror
   int cur = 0;             // parity of the buffer that holds the current state
@@ -238,6 +240,29 @@ struct Step1Args {
   DevState* S;
 };
 cudaError_t launch_step1(cudaStream_t s, const Step1Args& a, const EosC& e);
+// A run of steps in one launch (run1_f64_kernel), for problems of at most one block per
+// multiprocessor: from Q to out[steps taken & 1] (which may be Q), t_out[0..1] the new
+// time, S->steps advanced. edge: run1_edge_doubles(n) of scratch. S's slots are all zero
+// afterwards (slot0 and the next one before), its run counters before and after.
+struct Run1Args {
+  const double* Q;
+  double* out[2];
+  double* edge;
+  const double* t_in;
+  double* t_out;
+  int max_steps;
+  double t_end, cfl, dx;
+  int64_t n;
+  int flux, bc;
+  int slot0;  // the first step's max-speed slot
+  int tries;  // poll budget of a block's wait
+  DevState* S;
+};
+constexpr int kRunTries = 1 << 24;
+size_t run1_edge_doubles(int64_t n);
+bool run1_fits(int64_t n, int sms);
+cudaError_t launch_run1(cudaStream_t s, Run1Args a, EosC e);
+cudaError_t launch_run1_f64(hyp_ctx* c, long long k, int max_steps, double t_end);
 // single-phase FP64 launchers on a context (hyp_step1.cu)
 cudaError_t launch_cell1_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end);
 cudaError_t launch_update1_f64(hyp_ctx* c, int p, unsigned long long* rd, unsigned long long* clr0,

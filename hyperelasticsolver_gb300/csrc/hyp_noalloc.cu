@@ -10,7 +10,7 @@
 // caller passes the input and output state, and everything else the step
 // needs (the second state buffer of the ping-pong, per-cell fluxes and wave
 // speeds, loop control) lives in one fixed, file-scope device array of
-// kNoAllocDoubles doubles (65,536 cells at most; 19,923,040 bytes = 19.0 MiB that
+// kNoAllocDoubles doubles (65,536 cells at most; 19,923,048 bytes = 19.0 MiB that
 // every GPU which loads this library keeps until the process exits).
 //
 // Set-up: the first call on a device looks up that array's device address with
@@ -45,12 +45,14 @@ namespace {
 constexpr int kMaxDevices = 256;
 std::mutex g_mu;
 double* g_scratch_addr[kMaxDevices] = {};
+int g_run_blocks[kMaxDevices] = {};  // blocks of one cooperative launch of a run (0: none)
 
 __global__ void noalloc_reset_kernel(DevState* st, double t0) {
   st->t[0] = t0;
   st->t[1] = t0;
   for (int s = 0; s < 3; ++s) st->lam_slots[s] = 0ull;
   st->lam_query = 0ull;
+  st->run_count = st->run_done = 0u;
   st->steps = 0;
   st->err_code = 0;
   st->pad_ = 0;
@@ -58,7 +60,7 @@ __global__ void noalloc_reset_kernel(DevState* st, double t0) {
 }
 
 // Device address of the scratch array on the current device (looked up once per device).
-int scratch_base(double** out) {
+int scratch_base(double** out, int* run_blocks) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) return HYP_ERR_NO_DEVICE;
   if (dev < 0 || dev >= kMaxDevices) return HYP_ERR_UNSUPPORTED;
@@ -67,9 +69,15 @@ int scratch_base(double** out) {
     double* p = nullptr;
     cudaError_t e = cudaGetSymbolAddress((void**)&p, g_noalloc_scratch);
     if (e != cudaSuccess || !p) return HYP_ERR_CUDA;
+    int coop = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return HYP_ERR_CUDA;
+    g_run_blocks[dev] = coop ? sms : 0;
     g_scratch_addr[dev] = p;
   }
   *out = g_scratch_addr[dev];
+  *run_blocks = g_run_blocks[dev];
   return HYP_OK;
 }
 }  // namespace
@@ -91,7 +99,8 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
     return HYP_ERR_INVALID;
   (void)cudaGetLastError();  // a pending error from the caller's earlier work is not this call's
   double* base = nullptr;
-  int rc = scratch_base(&base);
+  int run_blocks = 0;
+  int rc = scratch_base(&base, &run_blocks);
   if (rc != HYP_OK) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t n = n_cells;
@@ -102,17 +111,37 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   const EosC eos = make_eos(cfg->eos[0].rho0, cfg->eos[0].c0, cfg->eos[0].cv, cfg->eos[0].t0, cfg->eos[0].b0,
                             cfg->eos[0].alpha, cfg->eos[0].beta, cfg->eos[0].gamma);
   const double dx = cfg->x_length / (double)n;
+  const bool one_launch = n_steps > 0 && t0 < INFINITY && run1_fits(n, run_blocks);
   // Ping-pong between the caller's output and the scratch state so that the last step writes the output.
   double* cur = (n_steps % 2 == 0) ? d_Q_out : B;
-  if (cur != d_Q_in &&
+  if (!one_launch && cur != d_Q_in &&
       cudaMemcpyAsync(cur, d_Q_in, (size_t)14 * n * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
     return HYP_ERR_CUDA;
   noalloc_reset_kernel<<<1, 1, 0, s>>>(st, t0);
   if (cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;
-  if (n_steps > 0 &&
+  if (one_launch) {  // a small problem: every step in one launch, from the input to the output
+    Run1Args a;
+    a.Q = d_Q_in;
+    a.out[0] = a.out[1] = d_Q_out;
+    a.edge = F;
+    a.t_in = st->t;
+    a.t_out = st->t;
+    a.max_steps = n_steps;
+    a.t_end = INFINITY;
+    a.cfl = cfg->cfl;
+    a.dx = dx;
+    a.n = n;
+    a.flux = cfg->flux;
+    a.bc = cfg->bc;
+    a.slot0 = 0;
+    a.tries = kRunTries;
+    a.S = st;
+    if (launch_run1(s, a, eos) != cudaSuccess) return HYP_ERR_CUDA;
+  }
+  if (!one_launch && n_steps > 0 &&
       launch_cell1(s, cur, n, eos, F, lam, &st->lam_slots[0], &st->t[0], INFINITY, st) != cudaSuccess)
     return HYP_ERR_CUDA;
-  for (int k = 0; k < n_steps; ++k) {
+  for (int k = 0; !one_launch && k < n_steps; ++k) {
     const int p = k & 1;
     const bool last = k == n_steps - 1;
     double* nxt = (cur == d_Q_out) ? B : d_Q_out;
@@ -147,6 +176,7 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   if (t_out) *t_out = h.t[n_steps & 1];
   if (h.err_code) {
     if (err_cell) *err_cell = h.err_cell;
+    if (h.err_code & HYP_CELL_TIMEOUT) return HYP_ERR_TIMEOUT;
     return (h.err_code & HYP_CELL_NEG_DET) ? HYP_ERR_NEG_DET : HYP_ERR_NONFINITE;
   }
   return HYP_OK;

@@ -97,6 +97,158 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
   if (j == 0) atomicMax(a.wr, m);
 }
 
+// ---- a whole run in one launch --------------------------------------------------
+
+// Values of a cell its neighbour needs for their face: Q (14), fluxes (11), wave speed.
+constexpr int kEdge = 14 + kNFlux1 + 1;
+
+// Bounded wait of the run's blocks for one another (one arrival per block and step):
+// what the threads of every block wrote before is visible to all after it. False if
+// the wait ran out; the caller leaves the kernel. 8 blocks spend 1.5 us a step here and
+// in the maximum's atomics, 150 blocks 4.2 us; a word per block that every block, or one
+// block for all, reads instead measured no better (1.4 and 5.2 us; 8 blocks 1.2 us more).
+__device__ __forceinline__ bool run_barrier(unsigned* count, unsigned target, int tries) {
+  __shared__ int s_ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
+    int left = tries;
+    unsigned c;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(c) : "l"(count) : "memory");
+    } while (c < target && --left > 0);
+    s_ok = left > 0;
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+// Steps of a problem of at most one block per multiprocessor (127 cells each, 19,304 on
+// 152 of them), all in one cooperative launch. A step of such a problem is one pass of
+// FP64 issue, 240 slots (7.4 us), whatever it does about memory; as kernels of their own,
+// steps spent as long again on the launch, on reloading the state and on the tail. Here
+// a thread keeps its cell's state in registers, a block its cells' fluxes in shared
+// memory, and the blocks meet once a step: before it they publish their edge cells and
+// their part of the maximum wave speed, after it they read their neighbours' edges and
+// the maximum. The arithmetic is that of cell1_pass and step1_f64_kernel, in the same
+// order. 1000 cells x 100
+// steps 1.39 -> 1.26 ms, 8192 cells x 4 steps on device buffers 111 -> 80 us.
+template <int kDef>
+__global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, Eos64 k) {
+  __shared__ double sh[kEdge][kBlock64 + 1];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
+  __shared__ double sF[14][kBlock64];         // twice the left face of cell i0 + j
+  __shared__ double s_hdt, s_t;
+  const int j = threadIdx.x;
+  const int64_t n = a.n, i0 = (int64_t)blockIdx.x * kCells64, i = i0 + j;
+  const int cells = (int)(n - i0 < kCells64 ? n - i0 : kCells64);
+  const bool own = j < cells, lxf = a.flux == HYP_FLUX_LXF;
+  const bool frozen = own && bc_holds(a.bc, i == 0, i == n - 1);
+  double q[14];
+  if (own)
+#pragma unroll
+    for (int v = 0; v < 14; ++v) q[v] = a.Q[v * n + i];
+  double t = *a.t_in;
+  int s = 0;
+  for (; s < a.max_steps && t < a.t_end; ++s) {
+    double* const mine = a.edge + (size_t)((s & 1) * gridDim.x + blockIdx.x) * 2 * kEdge;
+    double l = 0.0, f[14];
+    if (own) {
+      const Cell64 c = cell64<kDef>(e, k, 1.0, q + 1, q[4], q + 5);
+      flux64(1.0, c, q + 1, q + 5, f);
+      l = fabs(c.u[0]) + cmax64<kDef>(e, k, c);
+      const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
+      if (st) record_err64(a.S, st, i);
+#pragma unroll
+      for (int v = 0; v < 14; ++v) {
+        sh[v][j + 1] = q[v];
+        if (flux_slot1(v) >= 0) sh[14 + flux_slot1(v)][j + 1] = f[v];
+      }
+      sh[kEdge - 1][j + 1] = l;
+    }
+    const unsigned long long top = block_max_bits<kBlock64>(l);  // (its barrier publishes sh)
+    if (j < 2 * kEdge) {  // the first and the last cell, for the neighbours
+      const int side = j >= kEdge, r = j - side * kEdge;
+      mine[j] = sh[r][side ? cells : 1];
+    }
+    if (j == 0) atomicMax(&a.S->lam_slots[(a.slot0 + s) % 3], top);
+    if (!run_barrier(&a.S->run_count, (unsigned)(s + 1) * gridDim.x, a.tries)) {
+      if (j == 0) record_err64(a.S, HYP_CELL_TIMEOUT, i0);
+      break;
+    }
+    const double lmax = __longlong_as_double((long long)__ldcg(&a.S->lam_slots[(a.slot0 + s) % 3]));
+    if (blockIdx.x == 0 && j == 0) a.S->lam_slots[(a.slot0 + s + 2) % 3] = 0ull;  // all have read it
+    if (j < 2 * kEdge) {  // the neighbours' cells beside this block's; past an end a zero-gradient ghost
+      const int side = j >= kEdge, r = j - side * kEdge;
+      const int nb = (int)blockIdx.x + (side ? 1 : -1);
+      const double* const theirs = a.edge + (size_t)((s & 1) * gridDim.x + nb) * 2 * kEdge;
+      const bool end = nb < 0 || nb >= (int)gridDim.x;
+      sh[r][side ? cells + 1 : 0] = end ? sh[r][side ? cells : 1] : __ldcg(&theirs[side ? r : kEdge + r]);
+    }
+    StepScalars sc{0.0, 0.0, 0.0};
+    if (j < 32 || lxf) sc = step_scalars64(a.cfl, a.dx, lmax, lxf);
+    if (j == 0) {
+      s_hdt = 0.5 * sc.dtdx;
+      s_t = t + sc.dt;
+    }
+    __syncthreads();
+    double f2[14];
+    if (j <= cells) {  // the face between slots j and j + 1, as face_twice
+      double lf = sc.lam_lxf;
+      if (!lxf) {
+        const double la = sh[kEdge - 1][j], lb = sh[kEdge - 1][j + 1];
+        lf = bits_of(la) > bits_of(lb) && !is_nan64(la) ? la : lb;
+      }
+      if (!own) {  // the right cell of the block's last face
+#pragma unroll
+        for (int v = 0; v < 14; ++v) {
+          q[v] = sh[v][j + 1];
+          if (flux_slot1(v) >= 0) f[v] = sh[14 + flux_slot1(v)][j + 1];
+        }
+      }
+#pragma unroll
+      for (int v = 0; v < 14; ++v) {
+        const int sl = flux_slot1(v);
+        const double dq = __dsub_rn(q[v], sh[v][j]);
+        f2[v] = sl >= 0 ? __fma_rn(-lf, dq, __dadd_rn(sh[14 + sl][j], f[v])) : __dmul_rn(-lf, dq);
+        sF[v][j] = f2[v];
+      }
+    }
+    t = s_t;
+    const double hdt = s_hdt;
+    __syncthreads();
+    if (own && !frozen)
+#pragma unroll
+      for (int v = 0; v < 14; ++v) q[v] = __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), q[v]);
+  }
+  if (own && s > 0) {
+    double* const Qn = a.out[s & 1];
+#pragma unroll
+    for (int v = 0; v < 14; ++v) Qn[v * n + i] = q[v];
+  }
+  if (j == 0) {
+    if (blockIdx.x == 0) {
+      a.t_out[0] = a.t_out[1] = t;
+      a.S->steps += s;
+    }
+    __threadfence();
+    if (atomicAdd(&a.S->run_done, 1u) == gridDim.x - 1) {  // the last block: all others are past the loop
+      a.S->run_count = a.S->run_done = 0u;
+      for (int c = 0; c < 3; ++c) a.S->lam_slots[c] = 0ull;
+    }
+  }
+}
+
+size_t run1_edge_doubles(int64_t n) { return (size_t)((n + kCells64 - 1) / kCells64) * 4 * kEdge; }
+bool run1_fits(int64_t n, int sms) { return (n + kCells64 - 1) / kCells64 <= sms; }
+
+cudaError_t launch_run1(cudaStream_t s, Run1Args a, EosC e) {
+  Eos64 k = make_eos64(e);
+  void* args[] = {&a, &e, &k};
+  const void* kern = e.default_exp ? (const void*)run1_f64_kernel<1> : (const void*)run1_f64_kernel<0>;
+  return cudaLaunchCooperativeKernel(kern, dim3((unsigned)((a.n + kCells64 - 1) / kCells64)), dim3(kBlock64), args, 0,
+                                     s);
+}
+
 cudaError_t launch_cell1(cudaStream_t s, const double* Q, int64_t n, const EosC& e, double* F, double* lam,
                          unsigned long long* lam_slot, const double* t_now, double t_end, DevState* S) {
   const unsigned grid = (unsigned)((n + kBlock64 - 1) / kBlock64);
@@ -151,6 +303,29 @@ static Step1Args step1_args(hyp_ctx* c, int p, unsigned long long* rd, unsigned 
 cudaError_t launch_update1_f64(hyp_ctx* c, int p, unsigned long long* rd, unsigned long long* clr0,
                                unsigned long long* clr1, double t_end) {
   return launch_step1(c->stream, step1_args(c, p, rd, nullptr, clr0, clr1, t_end), c->eos[0]);
+}
+
+// At most max_steps steps from step k on, of a problem that fits run1_fits.
+cudaError_t launch_run1_f64(hyp_ctx* c, long long k, int max_steps, double t_end) {
+  const int p = (int)(k & 1);
+  Run1Args a;
+  a.slot0 = (int)(k % 3);
+  a.Q = c->Q[p];
+  a.out[0] = c->Q[p];
+  a.out[1] = c->Q[1 - p];
+  a.edge = c->flux1[0];
+  a.t_in = &c->st->t[p];
+  a.t_out = c->st->t;
+  a.max_steps = max_steps;
+  a.t_end = t_end;
+  a.cfl = c->cfg.cfl;
+  a.dx = ctx_dx(c);
+  a.n = c->n;
+  a.flux = c->cfg.flux;
+  a.bc = ctx_bc(c);
+  a.tries = kRunTries;
+  a.S = c->st;
+  return launch_run1(c->stream, a, c->eos[0]);
 }
 
 // Step k of a run (first / last of it): the max wave speed of the state before step k

@@ -80,7 +80,10 @@ __device__ __forceinline__ double quot64(double a, double b, double rb) {
 // step, 22 for LxF. Arguments too large or small for the special-function seeds, and
 // quotients that are not finite, take the divisions.
 __device__ __forceinline__ StepScalars step_scalars64(double cfl, double dx, double lmax, bool lxf) {
-  auto plain = [](double x) { return x > 1e-250 && x < 1e250; };
+  auto plain = [](double x) {  // 2^-823 <= x < 2^823, by the exponent: a compare is a slot
+    const long long ex = bits_of(x) >> 52;
+    return ex >= 200 && ex < 1846;
+  };
   const double cdx = cfl * dx;
   if (!plain(lmax) || !plain(dx) || !plain(cdx)) {
     const double dt = cdx / lmax, lam = dx / dt;

@@ -156,7 +156,7 @@ int hyp_last_timing(const hyp_ctx* ctx, double* ms_total, double* ms_cell_kernel
    device SoA states [14][n_cells] (may be the same buffer); cfg must be
    single-phase, FP64, Rusanov or LxF, with cfg->n_cells == n_cells. The step's
    scratch is one fixed static device array sized for at most 65,536 cells
-   (19,923,040 bytes = 19.0 MiB per GPU that loads the library, held until exit);
+   (19,923,048 bytes = 19.0 MiB per GPU that loads the library, held until exit);
    larger n_cells is rejected with HYP_ERR_INVALID. The call synchronises `stream`
    (it reads the step's status back), so it cannot be made inside a stream capture
    or a CUDA graph. Calls share the array, so calls that overlap on the GPU race. Runs
