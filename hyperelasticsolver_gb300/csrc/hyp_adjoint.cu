@@ -159,9 +159,10 @@ __global__ void __launch_bounds__(256) adj_dtdx_kernel(AdjArgs g) {
 // zero tests: 880 -> about 470 FP64 instructions a cell; 65,536 cells, 50 steps with record
 // and recompute 11.4 -> 9.5 ms.
 template <int kDef>
-__global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, Eos64 k64) {
+__global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, Eos64 kc) {
   __shared__ double sh[kAdjBlock / 32];
   __shared__ double s_lamb_max, s_r;
+  const Eos64 k64 = in_registers64(kc);
   const int64_t n = g.n;
   const double lmax = __longlong_as_double((long long)*g.lmax);
   if (threadIdx.x < 32) {  // rb_n: the partial sums in a fixed order
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
     // the partials sum to r rb_n; d r / d lmax = -r / lmax, so dL/d lmax = -(r rb_n) / lmax
     if (threadIdx.x == 0) s_lamb_max = -s / lmax;
   } else if (threadIdx.x < 64) {
-    const double r = step_scalars64(g.cfl, g.dx, lmax, false).dtdx;  // dt/dx of the forward step
+    const double r = step_scalars64(k64, g.cfl, g.dx, lmax, false).dtdx;  // dt/dx of the forward step
     if (threadIdx.x == 32) s_r = r;
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) *g.amax_clr = INT_MAX;

@@ -29,7 +29,7 @@ template <int kDef>
 HYP_HD int cell_vjp64(const EosC& e, const Eos64& k, const double* q, const double* fb, double lb, double* qb,
                       EosBar& eb) {
   const double *m = q + 1, *R = q + 5;
-  const Cell64 c = cell64<kDef>(e, k, 1.0, m, q[4], R);
+  const Cell64 c = cell64<kDef, true>(e, k, 1.0, m, q[4], R);
   const double r = c.inv_den, ms = k.inv_rho0sq;
   const double th = (c.G00 + c.G11 + c.G22) * (1.0 / 3.0);
   const double d0 = c.G00 - th, d1 = c.G11 - th, d2 = c.G22 - th;
@@ -50,13 +50,13 @@ HYP_HD int cell_vjp64(const EosC& e, const Eos64& k, const double* q, const doub
     const double o11 = f1 * c.G01 + (c.a * c.G11 - c.bM), o22 = f2 * c.G02 + (c.a * c.G22 - c.bM);
     const double o12 = f1 * c.G02 + c.a * c.G12;
     double nu;
-    if (!top_root64(o00, o11, o22, o01, o02, o12, nu)) return cell_vjp_general(e, q, fb, lb, qb, eb);
+    if (!top_root64(k, o00, o11, o22, o01, o02, o12, nu)) return cell_vjp_general(e, q, fb, lb, qb, eb);
     u0b = c.u[0] > 0.0 ? lb : (c.u[0] < 0.0 ? -lb : 0.0);
     // d nu / d O = Cof(nu I - O) / its trace; an off-diagonal entry stands for two
     const double b00 = nu - o00, b11 = nu - o11, b22 = nu - o22;
     const double C00 = b11 * b22 - o12 * o12, C11 = b00 * b22 - o02 * o02, C22 = b00 * b11 - o01 * o01;
     const double C01 = o02 * o12 + o01 * b22, C02 = o01 * o12 + o02 * b11, C12 = o01 * o02 + b00 * o12;
-    const double g = lb * rsqrt64(nu + nu) * rcp64(C00 + C11 + C22), g2 = g + g;
+    const double g = lb * rsqrt64(k, nu + nu) * rcp64(k, C00 + C11 + C22), g2 = g + g;
     const double p00 = g * C00, p11 = g * C11, p22 = g * C22, p01 = g2 * C01, p02 = g2 * C02, p12 = g2 * C12;
     // O_ij = f G0i G0j + ...
     const double t0 = 2.0 * p00 * c.G00 + p01 * c.G01 + p02 * c.G02;

@@ -178,13 +178,14 @@ __global__ void __launch_bounds__(kBlock) batch_join_kernel(const float* __restr
 // the cell pass and the tile's maximum into its problem's slot.
 template <int kDef>
 __global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* __restrict__ Q, int64_t n, EosC e,
-                                                                  Eos64 k, double* __restrict__ F,
+                                                                  Eos64 kc, double* __restrict__ F,
                                                                   double* __restrict__ lam,
                                                                   const TileDesc* __restrict__ tiles, BatchDev b,
                                                                   int par, double t_end,
                                                                   unsigned long long* slot_base, DevState* S) {
   const TileDesc d = tiles[blockIdx.x];
   if (!(b.t[par * b.P + d.problem] < t_end)) return;
+  const Eos64 k = in_registers64(kc);
   const int64_t i = d.first + threadIdx.x;
   const bool own = threadIdx.x < kCells64 && i < d.hi;
   const double l = own ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
@@ -198,13 +199,14 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* 
 // clears all three: whatever steps it next starts with a cell pass).
 template <int kDef, bool kCell>
 __global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
-    const double* __restrict__ Q, double* __restrict__ Qn, int64_t n, EosC e, Eos64 k, const double* __restrict__ F,
+    const double* __restrict__ Q, double* __restrict__ Qn, int64_t n, EosC e, Eos64 kc, const double* __restrict__ F,
     const double* __restrict__ lam, double* __restrict__ Fn, double* __restrict__ lamn,
     const TileDesc* __restrict__ tiles, BatchDev b, int par, int rd, int wr, int clr, double t_end, double cfl,
     int flux, int bc, DevState* S) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell first + k
   __shared__ double s_hdt;
   __shared__ int s_more;
+  const Eos64 k = in_registers64(kc);
   const int P = b.P, j = threadIdx.x;
   const bool lxf = flux == HYP_FLUX_LXF;
   const TileDesc d = tiles[blockIdx.x];
@@ -213,7 +215,7 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
   const bool active = tn < t_end;
   const double lmax = __longlong_as_double((long long)b.slots[rd * P + p]);
   StepScalars sc{0.0, 0.0, 0.0};
-  if (j < 32 || lxf) sc = step_scalars64(cfl, b.dx[p], lmax, lxf);
+  if (j < 32 || lxf) sc = step_scalars64(k, cfl, b.dx[p], lmax, lxf);
   if (j == 0) {
     s_hdt = 0.5 * sc.dtdx;
     s_more = kCell && tn + sc.dt < t_end;
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
   }
   double f2[14];
   if (i <= d.hi) {
-    face_twice(Q, F, lam, n, d.lo, d.hi, i, lxf, sc.lam_lxf, f2);
+    face_twice(k, Q, F, lam, n, d.lo, d.hi, i, lxf, sc.lam_lxf, f2);
 #pragma unroll
     for (int v = 0; v < 14; ++v) sF[v][j] = f2[v];
   }
@@ -246,7 +248,7 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
 #pragma unroll
     for (int v = 0; v < 14; ++v) {
       const double qc = Q[v * n + i];
-      q[v] = frozen ? qc : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), qc);
+      q[v] = frozen ? qc : __fma_rn(-hdt, sub64(k, sF[v][j + 1], f2[v]), qc);
       Qn[v * n + i] = q[v];
     }
   }

@@ -466,8 +466,8 @@ __global__ void k_lxf2(Eos2x E, Quad6D lobatto, const double* Ql, const double* 
     double f[2][14];
     for (int s = 0; s < 2; ++s) {
       const double* q = (s ? b : a) + 15 * p;
-      const Cell64 c = cell64<kDef>(E.e[p], E.k[p], rcp64(q[0]), q + 2, q[5], q + 6);
-      flux64(q[0], c, q + 2, q + 6, f[s]);
+      const Cell64 c = cell64<kDef, false>(E.e[p], E.k[p], rcp64(E.k[p], q[0]), q + 2, q[5], q + 6);
+      flux64<false>(E.k[p], q[0], c, q + 2, q + 6, f[s]);
     }
     for (int r = 0; r < 15; ++r) {
       const double fs = r > 0 ? f[0][r - 1] + f[1][r - 1] : 0.0;

@@ -33,14 +33,14 @@ struct Half64 {
 template <int kDef>
 HYP_HD int half64(const EosC& e, const Eos64& k, double ia, const double* m, double rE,
                                       const double* R, Half64& h) {
-  const Cell64 c = cell64<kDef>(e, k, ia, m, rE, R);
-  const double m2 = -2.0 * c.td;
+  const Cell64 c = cell64<kDef, false>(e, k, ia, m, rE, R);
+  const double m2 = -add64(k, c.td, c.td);
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
     h.u[v] = c.u[v];
-    h.K[v] = m2 * c.w[v];
+    h.K[v] = mul64(k, m2, c.w[v]);
   }
-  h.T = e.t0 * (c.Pg + c.px);
+  h.T = e.t0 * add64(k, c.Pg, c.px);
   return c.st;
 }
 
@@ -49,33 +49,33 @@ HYP_HD int half64(const EosC& e, const Eos64& k, double ia, const double* m, dou
 struct Face64 {
   double u[3], s[3], p;
 };
-HYP_HD Face64 interface64(const Half64& a, const Half64& b) {
+HYP_HD Face64 interface64(const Eos64& k, const Half64& a, const Half64& b) {
   Face64 I;
-  const double inv = rcp64(a.T + b.T), ha = b.T * inv, hb = a.T * inv;
+  const double inv = rcp64(k, add64(k, a.T, b.T)), ha = mul64(k, b.T, inv), hb = mul64(k, a.T, inv);
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
-    I.u[v] = 0.5 * (a.u[v] + b.u[v]);
-    I.s[v] = ha * a.K[v] + hb * b.K[v];
+    I.u[v] = mul64(k, k.half, add64(k, a.u[v], b.u[v]));
+    I.s[v] = fma(hb, b.K[v], mul64(k, ha, a.K[v]));
   }
-  I.p = I.s[0] * I.u[0] + I.s[1] * I.u[1] + I.s[2] * I.u[2];
+  I.p = fma(I.s[2], I.u[2], fma(I.s[1], I.u[1], mul64(k, I.s[0], I.u[0])));
   return I;
 }
 
 // acc += wd B(q) e_alpha for one phase's rows (row 1 of B is zero), B's rho A part with
 // alpha rho A / alpha in place of rho A.
-HYP_HD void add_b64(double wd, double ia, const double* R, const double* u, const Face64& I,
-                                        double* acc) {
+HYP_HD void add_b64(const Eos64& k, double wd, double ia, const double* R, const double* u, const Face64& I,
+                    double* acc) {
   acc[0] = fma(wd, I.u[0], acc[0]);
   acc[2] = fma(wd, I.s[0], acc[2]);
   acc[3] = fma(wd, I.s[1], acc[3]);
   acc[4] = fma(wd, I.s[2], acc[4]);
   acc[5] = fma(wd, I.p, acc[5]);
-  const double wi = wd * ia, d1 = I.u[1] - u[1], d2 = I.u[2] - u[2];
+  const double wi = mul64(k, wd, ia), d1 = sub64(k, I.u[1], u[1]), d2 = sub64(k, I.u[2], u[2]);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double* r = R + 3 * c;
-    const double w0 = wi * r[0];
-    acc[6 + 3 * c] = fma(wi, r[0] * I.u[0] + r[1] * d1 + r[2] * d2, acc[6 + 3 * c]);
+    const double w0 = mul64(k, wi, r[0]);
+    acc[6 + 3 * c] = fma(wi, fma(r[2], d2, fma(r[1], d1, mul64(k, r[0], I.u[0]))), acc[6 + 3 * c]);
     acc[7 + 3 * c] = fma(w0, u[1], acc[7 + 3 * c]);
     acc[8 + 3 * c] = fma(w0, u[2], acc[8 + 3 * c]);
   }
@@ -176,17 +176,18 @@ HYP_HD int path_thread(const Eos2x& E, const Quad6D& qd, const double* a, const 
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       double m[3];
-      auto at = [&](int k) { return fma(s, b[15 * p + k] - a[15 * p + k], a[15 * p + k]); };
+      const Eos64& kp = E.k[p];
+      auto at = [&](int r) { return fma(s, sub64(kp, b[15 * p + r], a[15 * p + r]), a[15 * p + r]); };
 #pragma unroll
       for (int v = 0; v < 3; ++v) m[v] = at(2 + v);
 #pragma unroll
       for (int v = 0; v < 9; ++v) R[p][v] = at(6 + v);
-      ia[p] = rcp64(at(0));
-      st |= half64<kDef>(E.e[p], E.k[p], ia[p], m, at(5), R[p], h[p]);
+      ia[p] = rcp64(kp, at(0));
+      st |= half64<kDef>(E.e[p], kp, ia[p], m, at(5), R[p], h[p]);
     }
-    const Face64 I = interface64(h[0], h[1]);
-    add_b64(w * da0, ia[0], R[0], h[0].u, I, acc);
-    add_b64(w * da1, ia[1], R[1], h[1].u, I, acc + 15);
+    const Face64 I = interface64(E.k[0], h[0], h[1]);
+    add_b64(E.k[0], w * da0, ia[0], R[0], h[0].u, I, acc);
+    add_b64(E.k[1], w * da1, ia[1], R[1], h[1].u, I, acc + 15);
   }
   return st;
 }

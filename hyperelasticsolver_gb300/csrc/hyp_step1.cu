@@ -22,11 +22,12 @@ namespace hyp {
 // 10.48 ms with the general forms, 7.26 ms with these; 1000 cells, 100 steps: 4.14 ms at 256
 // threads a block with the general forms, 2.38 ms.
 template <int kDef>
-__global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __restrict__ Q, int64_t n, EosC e, Eos64 k,
+__global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc,
                                                              double* __restrict__ F, double* __restrict__ lam,
                                                              unsigned long long* lam_slot, const double* t_now,
                                                              double t_end, DevState* S) {
   if (!(*t_now < t_end)) return;  // uniform across the grid
+  const Eos64 k = in_registers64(kc);
   const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
   const double l = i < n ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
@@ -43,10 +44,11 @@ __global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __res
 // the state, and the fluxes alternate between two buffers: 1000 cells x 100 steps 1.59 -> 1.40
 // ms, 8192 cells x 4 steps on device buffers 129 -> 110 us, 1,000,003 cells unchanged (6.03 ms).
 template <int kDef, bool kCell>
-__global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e, Eos64 k) {
+__global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e, Eos64 kc) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell i0 + k
   __shared__ double s_hdt;             // half dt/dx
   __shared__ int s_more;               // the state this step makes is stepped from
+  const Eos64 k = in_registers64(kc);
   const int j = threadIdx.x;
   const int64_t n = a.n;
   const double tn = *a.t_in;
@@ -55,7 +57,7 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
   const bool lxf = a.flux == HYP_FLUX_LXF;
   // Rusanov: dt/dx (main.jl:225); LxF: 1/lambda with lambda = dx/dt (main.jl:223, :40)
   StepScalars sc{0.0, 0.0, 0.0};
-  if (j < 32 || lxf) sc = step_scalars64(a.cfl, a.dx, lmax, lxf);
+  if (j < 32 || lxf) sc = step_scalars64(k, a.cfl, a.dx, lmax, lxf);
   if (j == 0) {
     s_hdt = 0.5 * sc.dtdx;
     s_more = kCell && tn + sc.dt < a.t_end;
@@ -72,7 +74,7 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
   const int64_t i = (int64_t)blockIdx.x * kCells64 + j;  // this thread's cell, and the face on its left
   double f2[14];
   if (i <= n) {
-    face_twice(a.Q, a.F, a.lam, n, 0, n, i, lxf, sc.lam_lxf, f2);
+    face_twice(k, a.Q, a.F, a.lam, n, 0, n, i, lxf, sc.lam_lxf, f2);
 #pragma unroll
     for (int v = 0; v < 14; ++v) sF[v][j] = f2[v];
   }
@@ -87,7 +89,7 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
     for (int v = 0; v < 14; ++v) q[v] = a.Q[v * n + i];
 #pragma unroll
     for (int v = 0; v < 14; ++v) {
-      q[v] = frozen ? q[v] : __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), q[v]);
+      q[v] = frozen ? q[v] : __fma_rn(-hdt, sub64(k, sF[v][j + 1], f2[v]), q[v]);
       a.Qn[v * n + i] = q[v];
     }
   }
@@ -132,12 +134,13 @@ __device__ __forceinline__ bool run_barrier(unsigned* count, unsigned target, in
 // their part of the maximum wave speed, after it they read their neighbours' edges and
 // the maximum. The arithmetic is that of cell1_pass and step1_f64_kernel, in the same
 // order. 1000 cells x 100
-// steps 1.39 -> 1.26 ms, 8192 cells x 4 steps on device buffers 111 -> 80 us.
+// steps 1.39 -> 1.26 ms (1.19 since all operators are FMAs), 8192 cells x 4 steps on device buffers 111 -> 80 us.
 template <int kDef>
-__global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, Eos64 k) {
+__global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
   __shared__ double sh[kEdge][kBlock64 + 1];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
   __shared__ double sF[14][kBlock64];         // twice the left face of cell i0 + j
   __shared__ double s_hdt, s_t;
+  const Eos64 k = in_registers64(kc);
   const int j = threadIdx.x;
   const int64_t n = a.n, i0 = (int64_t)blockIdx.x * kCells64, i = i0 + j;
   const int cells = (int)(n - i0 < kCells64 ? n - i0 : kCells64);
@@ -153,9 +156,9 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
     double* const mine = a.edge + (size_t)((s & 1) * gridDim.x + blockIdx.x) * 2 * kEdge;
     double l = 0.0, f[14];
     if (own) {
-      const Cell64 c = cell64<kDef>(e, k, 1.0, q + 1, q[4], q + 5);
-      flux64(1.0, c, q + 1, q + 5, f);
-      l = fabs(c.u[0]) + cmax64<kDef>(e, k, c);
+      const Cell64 c = cell64<kDef, true>(e, k, 1.0, q + 1, q[4], q + 5);
+      flux64<true>(k, 1.0, c, q + 1, q + 5, f);
+      l = add64(k, fabs(c.u[0]), cmax64<kDef>(e, k, c));
       const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
       if (st) record_err64(a.S, st, i);
 #pragma unroll
@@ -185,7 +188,7 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
       sh[r][side ? cells + 1 : 0] = end ? sh[r][side ? cells : 1] : __ldcg(&theirs[side ? r : kEdge + r]);
     }
     StepScalars sc{0.0, 0.0, 0.0};
-    if (j < 32 || lxf) sc = step_scalars64(a.cfl, a.dx, lmax, lxf);
+    if (j < 32 || lxf) sc = step_scalars64(k, a.cfl, a.dx, lmax, lxf);
     if (j == 0) {
       s_hdt = 0.5 * sc.dtdx;
       s_t = t + sc.dt;
@@ -208,8 +211,8 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
 #pragma unroll
       for (int v = 0; v < 14; ++v) {
         const int sl = flux_slot1(v);
-        const double dq = __dsub_rn(q[v], sh[v][j]);
-        f2[v] = sl >= 0 ? __fma_rn(-lf, dq, __dadd_rn(sh[14 + sl][j], f[v])) : __dmul_rn(-lf, dq);
+        const double dq = sub64(k, q[v], sh[v][j]);
+        f2[v] = sl >= 0 ? __fma_rn(-lf, dq, add64(k, sh[14 + sl][j], f[v])) : mul64(k, -lf, dq);
         sF[v][j] = f2[v];
       }
     }
@@ -218,7 +221,7 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
     __syncthreads();
     if (own && !frozen)
 #pragma unroll
-      for (int v = 0; v < 14; ++v) q[v] = __fma_rn(-hdt, __dsub_rn(sF[v][j + 1], f2[v]), q[v]);
+      for (int v = 0; v < 14; ++v) q[v] = __fma_rn(-hdt, sub64(k, sF[v][j + 1], f2[v]), q[v]);
   }
   if (own && s > 0) {
     double* const Qn = a.out[s & 1];

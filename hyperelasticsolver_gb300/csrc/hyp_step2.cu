@@ -44,23 +44,23 @@ struct CellOut2 {
 // there is a cell): fluxes, speed bounds, and the block's max |speed| into slot. All
 // threads of the block call it.
 template <int kDef>
-__device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, const Eos2x& E, const CellOut2& o,
+__device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, const EosC& e, const Eos64& k,
+                                           const CellOut2& o,
                                            unsigned long long* slot) {
   __shared__ double s_lo[kPairCells], s_hi[kPairCells];
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
   double lo = 0.0, hi = 0.0;
   if (in) {
-    const EosC& e = E.e[ph];
-    const Cell64 c = cell64<kDef>(e, E.k[ph], rcp64(q[0]), q + 2, q[5], q + 6);
+    const Cell64 c = cell64<kDef, false>(e, k, rcp64(k, q[0]), q + 2, q[5], q + 6);
     double f[14];
-    flux64(q[0], c, q + 2, q + 6, f);
+    flux64<false>(k, q[0], c, q + 2, q + 6, f);
     double* f0 = o.F + 15 * ph * o.n + i;
 #pragma unroll
     for (int r = 1; r < 15; ++r)
       if (!zero_flux_row(r)) f0[r * o.n] = f[r - 1];
-    const double cm = cmax64<kDef>(e, E.k[ph], c);
-    lo = c.u[0] - cm;
-    hi = c.u[0] + cm;
+    const double cm = cmax64<kDef>(e, k, c);
+    lo = sub64(k, c.u[0], cm);
+    hi = add64(k, c.u[0], cm);
     if (c.st) record_err64(o.S, c.st, i);
     if (ph == 1) {
       s_lo[j] = lo;
@@ -86,14 +86,16 @@ __global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __rest
                                                             unsigned long long* lam_slot, const double* t_now,
                                                             double t_end) {
   if (!(*t_now < t_end)) return;
+  const int ph = threadIdx.x / kPairCells;
+  const Eos64 k = in_registers64(E.k, ph);
   const int64_t i = (int64_t)blockIdx.x * kPairCells + threadIdx.x % kPairCells;
   double q[15];
   if (i < o.n) {
-    const double* q0 = Q + 15 * (threadIdx.x / kPairCells) * o.n + i;
+    const double* q0 = Q + 15 * ph * o.n + i;
 #pragma unroll
     for (int r = 0; r < 15; ++r) q[r] = q0[r * o.n];
   }
-  cell2_pass<kDef>(q, i < o.n, i, E, o, lam_slot);
+  cell2_pass<kDef>(q, i < o.n, i, E.e[ph], k, o, lam_slot);
 }
 
 // ---- faces ---------------------------------------------------------------------
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __rest
   __shared__ int s_hard[2][kPairCells];
   if (!(*t_now < t_end)) return;
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
+  const Eos64 k = in_registers64(E.k, ph);
   const int64_t f = (int64_t)blockIdx.x * kPairCells + j;  // face between cells f-1 and f
   const int64_t nf = n + 1;
   const bool in = f <= n;
@@ -150,14 +153,14 @@ __global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __rest
   if (work) {  // speeds of the midpoint: the forms are homogeneous, so q_l + q_r serves
     double m[3], Rm[9];
 #pragma unroll
-    for (int v = 0; v < 3; ++v) m[v] = a[2 + v] + b[2 + v];
+    for (int v = 0; v < 3; ++v) m[v] = add64(k, a[2 + v], b[2 + v]);
 #pragma unroll
-    for (int v = 0; v < 9; ++v) Rm[v] = a[6 + v] + b[6 + v];
-    const Cell64 c = cell64<kDef>(E.e[ph], E.k[ph], rcp64(a[0] + b[0]), m, a[5] + b[5], Rm);
-    const double cm = cmax64<kDef>(E.e[ph], E.k[ph], c);
+    for (int v = 0; v < 9; ++v) Rm[v] = add64(k, a[6 + v], b[6 + v]);
+    const Cell64 c = cell64<kDef, false>(E.e[ph], k, rcp64(k, add64(k, a[0], b[0])), m, add64(k, a[5], b[5]), Rm);
+    const double cm = cmax64<kDef>(E.e[ph], k, c);
     if (c.st) record_err64(S, c.st, R);
-    s_lo[ph][j] = c.u[0] - cm;
-    s_hi[ph][j] = c.u[0] + cm;
+    s_lo[ph][j] = sub64(k, c.u[0], cm);
+    s_hi[ph][j] = add64(k, c.u[0], cm);
   }
   __syncthreads();
   double sl = 0.0, sr = 0.0;
@@ -171,36 +174,26 @@ __global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __rest
     if (smax[R] > sr) sr = smax[R];
     hard = !(flag & 2);
     if (!hard) {
-      const double idsr = rcp64(sr - sl);
-      const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
+      const double idsr = rcp64(k, sub64(k, sr, sl));
+      const double cm = mul64(k, -sl, idsr), cp = mul64(k, sr, idsr), cq = mul64(k, mul64(k, sl, sr), idsr);
       const double* fl = F + 15 * ph * n + L;
       const double* fr = F + 15 * ph * n + R;
       const float g = to_f32(cp), h = to_f32(idsr);
       float far = 0.0f, farh = 0.0f;  // squared distances of q_r and Q_hll from q_l in R
       bool finite = true;
+      dm[0] = dp[0] = 0.0;
 #pragma unroll
-      for (int r = 0; r < 15; ++r) {
-        if (r == 1) {  // alpha rho: updated like the rest, unused by the forms
-          const double df = fr[r * n] - fl[r * n], jump = b[1] - a[1];
-          dm[r * nf] = cm * df + cq * jump;
-          dp[r * nf] = cp * df - cq * jump;
-          continue;
-        }
-        if (r == 0) {
-          dm[0] = dp[0] = 0.0;
-          continue;
-        }
-        const double jump = b[r] - a[r];
-        const double df = zero_flux_row(r) ? 0.0 : fr[r * n] - fl[r * n];
-        finite &= is_finite64(jump) && is_finite64(df);
+      for (int r = 1; r < 15; ++r) {
+        const double jump = sub64(k, b[r], a[r]), qj = mul64(k, cq, jump);
+        const double df = zero_flux_row(r) ? 0.0 : sub64(k, fr[r * n], fl[r * n]);
+        if (r > 1) finite &= is_finite64(jump) && is_finite64(df);  // (alpha rho is unused by the forms)
         if (r >= 6) {  // Q_hll - q_l = (jump s_r - df) / (s_r - s_l)
           const float jf = to_f32(jump), hf = jf * g - to_f32(df) * h;
           far += jf * jf;
           farh += hf * hf;
         }
-        const double qj = cq * jump;
-        dm[r * nf] = zero_flux_row(r) ? qj : cm * df + qj;
-        dp[r * nf] = zero_flux_row(r) ? -qj : cp * df - qj;
+        dm[r * nf] = zero_flux_row(r) ? qj : fma(cm, df, qj);
+        dp[r * nf] = zero_flux_row(r) ? -qj : fma(cp, df, -qj);
       }
       float Rf[9];
 #pragma unroll
@@ -224,7 +217,7 @@ __global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __rest
 
 // LxF faces: twice the conservative flux, (f_l + f_r) - lambda (q_r - q_l), and, where
 // the volume fractions do not jump, the fluctuations' zero; the others are listed.
-__global__ void __launch_bounds__(kPair64) face2_lxf_f64_kernel(const double* __restrict__ Q, int64_t n,
+__global__ void __launch_bounds__(kPair64) face2_lxf_f64_kernel(const double* __restrict__ Q, int64_t n, Eos64 kc,
                                                                 const double* __restrict__ F,
                                                                 const unsigned long long* lam_now, double cfl,
                                                                 double dx, double* __restrict__ FF,
@@ -233,13 +226,14 @@ __global__ void __launch_bounds__(kPair64) face2_lxf_f64_kernel(const double* __
   __shared__ int s_hard[2][kPairCells];
   __shared__ double s_lam;
   if (!(*t_now < t_end)) return;
+  const Eos64 k = in_registers64(kc);
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
   const int64_t f = (int64_t)blockIdx.x * kPairCells + j;  // face between cells f-1 and f
   const int64_t nf = n + 1;
   const bool in = f <= n;
   const int64_t L = f > 0 ? f - 1 : 0, R = f < n ? f : n - 1;
   if (threadIdx.x < 32) {  // lambda = dx/dt (main.jl:223)
-    const double lam = step_scalars64(cfl, dx, __longlong_as_double((long long)*lam_now), true).lam_lxf;
+    const double lam = step_scalars64(k, cfl, dx, __longlong_as_double((long long)*lam_now), true).lam_lxf;
     if (threadIdx.x == 0) s_lam = lam;
   }
   __syncthreads();
@@ -252,14 +246,14 @@ __global__ void __launch_bounds__(kPair64) face2_lxf_f64_kernel(const double* __
     bool finite = true, jumps = false;
 #pragma unroll
     for (int r = 0; r < 15; ++r) {
-      const double a = ql[r * n + L], b = ql[r * n + R], jump = b - a;
+      const double a = ql[r * n + L], b = ql[r * n + R], jump = sub64(k, b, a);
       const int64_t o = (15 * ph + r) * nf + f;
       if (zero_flux_row(r)) {
-        FF[o] = nlam * jump;
+        FF[o] = mul64(k, nlam, jump);
       } else {
-        const double fs = fc[r * n + L] + fc[r * n + R];
+        const double fs = add64(k, fc[r * n + L], fc[r * n + R]);
         finite &= is_finite64(fs);
-        FF[o] = nlam * jump + fs;
+        FF[o] = fma(nlam, jump, fs);
       }
       DM[o] = 0.0;
       finite &= is_finite64(jump);
@@ -300,23 +294,21 @@ struct GroupMem {
 // against 12 passes on one thread; adds the integral from q[from] to q[to] to the
 // partials.
 template <int kDef>
-__device__ __forceinline__ int path_group(const Eos2x& E, const Quad6D& qd, int lane16, GroupMem& g, int from, int to,
-                                          double* acc) {
+__device__ __forceinline__ int path_group(const Eos2x& E, const Eos64& k, const Quad6D& qd, int lane16, GroupMem& g,
+                                          int from, int to, double* acc) {
   const int ph = lane16 < 6 ? 0 : 1, node = lane16 < 12 ? lane16 - 6 * ph : 0;
   const double s = qd.x[node];
   const double* a = g.q[from] + 15 * ph;
   const double* b = g.q[to] + 15 * ph;
-  auto at = [&](int k) { return fma(s, b[k] - a[k], a[k]); };
+  auto at = [&](int r) { return fma(s, sub64(k, b[r], a[r]), a[r]); };
   double m[3], R[9];
 #pragma unroll
   for (int v = 0; v < 3; ++v) m[v] = at(2 + v);
 #pragma unroll
   for (int v = 0; v < 9; ++v) R[v] = at(6 + v);
-  const double ia = rcp64(at(0));
+  const double ia = rcp64(k, at(0));
   Half64 h, o;
-  const EosC& e = E.e[ph];
-  const Eos64 k = ph ? E.k[1] : E.k[0];
-  int st = half64<kDef>(e, k, ia, m, at(5), R, h);
+  int st = half64<kDef>(E.e[ph], k, ia, m, at(5), R, h);
   const int other = (threadIdx.x & 16) + (ph ? node : node + 6);  // its node's lane of the other phase
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
@@ -324,17 +316,17 @@ __device__ __forceinline__ int path_group(const Eos2x& E, const Quad6D& qd, int 
     o.K[v] = __shfl_sync(0xffffffffu, h.K[v], other);
   }
   o.T = __shfl_sync(0xffffffffu, h.T, other);
-  const Face64 I = interface64(h, o);
-  add_b64(qd.w[node] * (b[0] - a[0]), ia, R, h.u, I, acc);
+  const Face64 I = interface64(k, h, o);
+  add_b64(k, mul64(k, qd.w[node], sub64(k, b[0], a[0])), ia, R, h.u, I, acc);
   return lane16 < 12 ? st : 0;
 }
 
 // The sum over a face's six nodes of row k (30 rows).
-__device__ __forceinline__ double node_sum(const GroupMem& g, int k) {
-  const int ph = k < 15 ? 0 : 1, r = k - 15 * ph;
+__device__ __forceinline__ double node_sum(const Eos64& k, const GroupMem& g, int row) {
+  const int ph = row < 15 ? 0 : 1, r = row - 15 * ph;
   double v = g.part[6 * ph][r];
 #pragma unroll
-  for (int i = 1; i < 6; ++i) v += g.part[6 * ph + i][r];
+  for (int i = 1; i < 6; ++i) v = add64(k, v, g.part[6 * ph + i][r]);
   return v;
 }
 
@@ -363,6 +355,7 @@ __global__ void __launch_bounds__(kPathBlock, 2)
     const int blocks = min((int)gridDim.x, 2 * sms);  // a scheduler's second warp covers what is not FP64
     if ((int)blockIdx.x >= blocks) return;
     const int lane16 = threadIdx.x & 15;
+    const Eos64 k = in_registers64(E.k, lane16 < 6 ? 0 : 1);
     GroupMem& g = sg[threadIdx.x >> 4];
     // A list of no more faces than schedulers gives each a warp: both its groups do the
     // first integral, then each one of the two through Q_hll.
@@ -377,46 +370,47 @@ __global__ void __launch_bounds__(kPathBlock, 2)
       const bool live = t < count;
       const int at = live ? t : count - 1;
       const int64_t f = list.face[at], L = f - 1, R = f;
-      for (int k = lane16; k < 30; k += 16) {
-        g.q[0][k] = Q[k * n + L];
-        g.q[1][k] = Q[k * n + R];
+      for (int r = lane16; r < 30; r += 16) {
+        g.q[0][r] = Q[r * n + L];
+        g.q[1][r] = Q[r * n + R];
       }
       __syncwarp();
       double acc[15];
 #pragma unroll
       for (int r = 0; r < 15; ++r) acc[r] = 0.0;
-      int st = path_group<kDef>(E, qd, lane16, g, 0, 1, acc);
+      int st = path_group<kDef>(E, k, qd, lane16, g, 0, 1, acc);
       if (lane16 < 12)
 #pragma unroll
         for (int r = 0; r < 15; ++r) g.part[lane16][r] = acc[r];
       __syncwarp();
       if (kLxf) {
         if (live)
-          for (int k = lane16; k < 30; k += 16) DM[k * nf + f] = node_sum(g, k);
+          for (int r = lane16; r < 30; r += 16) DM[r * nf + f] = node_sum(k, g, r);
       } else {
-        const double sl = list.sl[at], sr = list.sr[at], idsr = rcp64(sr - sl);
-        for (int k = lane16; k < 30; k += 16) {
-          const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
-          g.q[2][k] = ((g.q[1][k] * sr - g.q[0][k] * sl) - (node_sum(g, k) + df)) * idsr;
+        const double sl = list.sl[at], sr = list.sr[at], idsr = rcp64(k, sub64(k, sr, sl));
+        for (int r = lane16; r < 30; r += 16) {
+          const double df = zero_flux_row(r % 15) ? 0.0 : sub64(k, F[r * n + R], F[r * n + L]);
+          const double qs = fma(g.q[1][r], sr, -mul64(k, g.q[0][r], sl));
+          g.q[2][r] = mul64(k, sub64(k, qs, add64(k, node_sum(k, g, r), df)), idsr);
         }
         __syncwarp();
 #pragma unroll
         for (int r = 0; r < 15; ++r) acc[r] = 0.0;
 #pragma unroll 1
         for (int h = wide ? grp : 0; h < (wide ? grp + 1 : 2); ++h)
-          st |= path_group<kDef>(E, qd, lane16, g, h ? 2 : 0, h ? 1 : 2, acc);
+          st |= path_group<kDef>(E, k, qd, lane16, g, h ? 2 : 0, h ? 1 : 2, acc);
         if (lane16 < 12)
 #pragma unroll
           for (int r = 0; r < 15; ++r) g.part[lane16][r] = acc[r];
         __syncwarp();
-        const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
+        const double cm = mul64(k, -sl, idsr), cp = mul64(k, sr, idsr), cq = mul64(k, mul64(k, sl, sr), idsr);
         if (live)
-          for (int k = wide ? threadIdx.x & 31 : lane16; k < 30; k += wide ? 32 : 16) {
-            const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
-            const double sum = wide ? node_sum(sg[base], k) + node_sum(sg[base + 1], k) : node_sum(g, k);
-            const double inner = df + sum, qj = cq * (g.q[1][k] - g.q[0][k]);
-            DM[k * nf + f] = cm * inner + qj;
-            DP[k * nf + f] = cp * inner - qj;
+          for (int r = wide ? threadIdx.x & 31 : lane16; r < 30; r += wide ? 32 : 16) {
+            const double df = zero_flux_row(r % 15) ? 0.0 : sub64(k, F[r * n + R], F[r * n + L]);
+            const double sum = wide ? add64(k, node_sum(k, sg[base], r), node_sum(k, sg[base + 1], r)) : node_sum(k, g, r);
+            const double inner = add64(k, df, sum), qj = mul64(k, cq, sub64(k, g.q[1][r], g.q[0][r]));
+            DM[r * nf + f] = fma(cm, inner, qj);
+            DP[r * nf + f] = fma(cp, inner, -qj);
           }
       }
       if (st && live) record_err64(S, st, R);
@@ -424,33 +418,40 @@ __global__ void __launch_bounds__(kPathBlock, 2)
     }
     return;
   }
+  Eos2x X;
+  X.e[0] = E.e[0];
+  X.e[1] = E.e[1];
+  X.k[0] = in_registers64(E.k[0]);
+  X.k[1] = in_registers64(E.k[1]);
+  const Eos64& k = X.k[0];
   const int t = blockIdx.x * kPathBlock + threadIdx.x;
   if (t < count) {
     const int64_t f = list.face[t], L = f - 1, R = f;
     double a[30], b[30], acc[30];
-    for (int k = 0; k < 30; ++k) {
-      a[k] = Q[k * n + L];
-      b[k] = Q[k * n + R];
-      acc[k] = 0.0;
+    for (int r = 0; r < 30; ++r) {
+      a[r] = Q[r * n + L];
+      b[r] = Q[r * n + R];
+      acc[r] = 0.0;
     }
-    int st = path_thread<kDef>(E, qd, a, b, acc);
+    int st = path_thread<kDef>(X, qd, a, b, acc);
     if (kLxf) {
-      for (int k = 0; k < 30; ++k) DM[k * nf + f] = acc[k];
+      for (int r = 0; r < 30; ++r) DM[r * nf + f] = acc[r];
     } else {
-      const double sl = list.sl[t], sr = list.sr[t], idsr = rcp64(sr - sl);
+      const double sl = list.sl[t], sr = list.sr[t], idsr = rcp64(k, sub64(k, sr, sl));
       double h[30];
-      for (int k = 0; k < 30; ++k) {
-        const double df = zero_flux_row(k % 15) ? 0.0 : F[k * n + R] - F[k * n + L];
-        h[k] = ((b[k] * sr - a[k] * sl) - (acc[k] + df)) * idsr;
-        acc[k] = df;
+      for (int r = 0; r < 30; ++r) {
+        const double df = zero_flux_row(r % 15) ? 0.0 : sub64(k, F[r * n + R], F[r * n + L]);
+        const double qs = fma(b[r], sr, -mul64(k, a[r], sl));
+        h[r] = mul64(k, sub64(k, qs, add64(k, acc[r], df)), idsr);
+        acc[r] = df;
       }
 #pragma unroll 1
-      for (int half = 0; half < 2; ++half) st |= path_thread<kDef>(E, qd, half ? h : a, half ? b : h, acc);
-      const double cm = (-sl) * idsr, cp = sr * idsr, cq = (sl * sr) * idsr;
-      for (int k = 0; k < 30; ++k) {
-        const double qj = cq * (b[k] - a[k]);
-        DM[k * nf + f] = cm * acc[k] + qj;
-        DP[k * nf + f] = cp * acc[k] - qj;
+      for (int half = 0; half < 2; ++half) st |= path_thread<kDef>(X, qd, half ? h : a, half ? b : h, acc);
+      const double cm = mul64(k, -sl, idsr), cp = mul64(k, sr, idsr), cq = mul64(k, mul64(k, sl, sr), idsr);
+      for (int r = 0; r < 30; ++r) {
+        const double qj = mul64(k, cq, sub64(k, b[r], a[r]));
+        DM[r * nf + f] = fma(cm, acc[r], qj);
+        DP[r * nf + f] = fma(cp, acc[r], -qj);
       }
     }
     if (st) record_err64(S, st, R);
@@ -479,11 +480,13 @@ template <int kDef, bool kCell>
 __global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E) {
   __shared__ double s_r;
   __shared__ int s_more;
+  const int ph = threadIdx.x / kPairCells;
+  const Eos64 k = in_registers64(E.k, ph);
   const int64_t n = a.o.n, nf = n + 1;
   const double tn = *a.t_in;
   const bool active = tn < a.t_end;
   if (threadIdx.x < 32) {
-    const StepScalars sc = step_scalars64(a.cfl, a.dx, __longlong_as_double((long long)*a.rd), false);
+    const StepScalars sc = step_scalars64(k, a.cfl, a.dx, __longlong_as_double((long long)*a.rd), false);
     if (threadIdx.x == 0) {
       s_r = a.FF ? 0.5 * sc.dtdx : sc.dtdx;
       s_more = kCell && tn + sc.dt < a.t_end;
@@ -500,7 +503,6 @@ __global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E
   }
   if (!active) return;
   __syncthreads();
-  const int ph = threadIdx.x / kPairCells;
   const int64_t i = (int64_t)blockIdx.x * kPairCells + threadIdx.x % kPairCells;
   double q[15];
   if (i < n) {
@@ -513,13 +515,13 @@ __global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E
       const int64_t row = 15 * ph + v;
       // F_r = F_l = zeros(30) for hll (NumFluxes.jl:82), NF_r = D- of face i+1/2, NF_l = D+ of face i-1/2
       q[v] = a.Q[row * n + i];
-      d[v] = a.DM[row * nf + i + 1] + a.DP[row * nf + i];
+      d[v] = add64(k, a.DM[row * nf + i + 1], a.DP[row * nf + i]);
     }
     if (a.FF) {
 #pragma unroll
       for (int v = 0; v < 15; ++v) {
         const int64_t row = 15 * ph + v;
-        d[v] += a.FF[row * nf + i + 1] - a.FF[row * nf + i];
+        d[v] = add64(k, d[v], sub64(k, a.FF[row * nf + i + 1], a.FF[row * nf + i]));
       }
     }
 #pragma unroll
@@ -529,7 +531,7 @@ __global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E
     }
   }
   if (!kCell || !s_more) return;
-  cell2_pass<kDef>(q, i < n, i, E, a.o, a.wr);
+  cell2_pass<kDef>(q, i < n, i, E.e[ph], k, a.o, a.wr);
 }
 
 static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -551,7 +553,7 @@ cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, do
   const Eos2x E = eos2x(c);
   if (lxf) {
     const double dx = c->cfg.x_length / (double)c->n;
-    face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, c->F, rd, c->cfg.cfl, dx,
+    face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, E.k[0], c->F, rd, c->cfg.cfl, dx,
                                                           c->FF, c->DM, list, &c->st->t[p], t_end, c->st);
   } else {
     auto kern = def ? face2_f64_kernel<1> : face2_f64_kernel<0>;

@@ -8,9 +8,36 @@ namespace hyp {
 
 // Threads of an FP64 cell block. One block's four warps sit on an SM's four
 // schedulers, so 152 blocks (19,456 cells) already take one pass of the GPU; with 256
-// threads a small problem ran two warps on each scheduler of half as many SMs (1000
-// cells: 33 us per cell pass against 16 with the same code at 128).
+// threads a small problem runs two warps on each scheduler of half as many SMs, twice the
+// time of one.
 constexpr int kBlock64 = 128;
+
+// The constants as register values (hyp_cell64.cuh: an operand from the constant bank or
+// a uniform register slows an FMA by a fifth). Their high words pass through an exclusive
+// or with a zero that only the launch knows (all grids here have gridDim.y = 1) and that a
+// thread's index makes a per-thread value: two integer instructions each, which may be
+// done again where a register is short. Through shared memory instead they took a barrier
+// and 0.9 us more of each kernel.
+__device__ __forceinline__ Eos64 in_registers64(const Eos64& k) {
+  const int zero = (int)(threadIdx.x & (gridDim.y - 1));
+  Eos64 r;
+  const double* from = &k.one;
+  double* to = &r.one;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(Eos64) / sizeof(double)); ++i)
+    to[i] = __hiloint2double(__double2hiint(from[i]) ^ zero, __double2loint(from[i]));
+  return r;
+}
+
+// The caller's phase of two: those of the phase by selection, which leaves registers too.
+__device__ __forceinline__ Eos64 in_registers64(const Eos64* k, int ph) {
+  Eos64 r = in_registers64(k[0]);
+  const double *k0 = &k[0].inv_rho0, *k1 = &k[1].inv_rho0;
+  double* to = &r.inv_rho0;
+#pragma unroll
+  for (int i = 0; i < (int)(&r.h_alphasq - &r.inv_rho0) + 1; ++i) to[i] = ph ? k1[i] : k0[i];
+  return r;
+}
 
 __device__ __forceinline__ void record_err64(DevState* S, int code, long long cell) {
   if (atomicCAS(&S->err_code, 0, code) == 0) S->err_cell = cell;
@@ -41,9 +68,9 @@ template <int kDef>
 __device__ __forceinline__ double cell1_pass(const double* q, int64_t n, int64_t i, const EosC& e, const Eos64& k,
                                              double* __restrict__ F, double* __restrict__ lam, DevState* S) {
   double f[14];
-  const Cell64 c = cell64<kDef>(e, k, 1.0, q + 1, q[4], q + 5);
-  flux64(1.0, c, q + 1, q + 5, f);
-  const double l = fabs(c.u[0]) + cmax64<kDef>(e, k, c);
+  const Cell64 c = cell64<kDef, true>(e, k, 1.0, q + 1, q[4], q + 5);
+  flux64<true>(k, 1.0, c, q + 1, q + 5, f);
+  const double l = add64(k, fabs(c.u[0]), cmax64<kDef>(e, k, c));
 #pragma unroll
   for (int v = 0; v < 14; ++v) {
     const int sl = flux_slot1(v);
@@ -71,15 +98,15 @@ constexpr int kCells64 = kBlock64 - 1;
 
 // a / b from rb, about 1 / b: a product and one residual correction (Markstein 1990),
 // 3 slots; correctly rounded up to rare last-bit cases.
-__device__ __forceinline__ double quot64(double a, double b, double rb) {
-  const double q = a * rb;
+__device__ __forceinline__ double quot64(const Eos64& k, double a, double b, double rb) {
+  const double q = mul64(k, a, rb);
   return fma(fma(-b, q, a), rb, q);
 }
 
 // step_scalars without FP64 divisions (about 9 slots each): 13 slots for the Rusanov
 // step, 22 for LxF. Arguments too large or small for the special-function seeds, and
 // quotients that are not finite, take the divisions.
-__device__ __forceinline__ StepScalars step_scalars64(double cfl, double dx, double lmax, bool lxf) {
+__device__ __forceinline__ StepScalars step_scalars64(const Eos64& k, double cfl, double dx, double lmax, bool lxf) {
   auto plain = [](double x) {  // 2^-823 <= x < 2^823, by the exponent: a compare is a slot
     const long long ex = bits_of(x) >> 52;
     return ex >= 200 && ex < 1846;
@@ -90,12 +117,12 @@ __device__ __forceinline__ StepScalars step_scalars64(double cfl, double dx, dou
     return StepScalars{dt, lam, lxf ? 1.0 / lam : dt / dx};
   }
   StepScalars s{0.0, 0.0, 0.0};
-  s.dt = quot64(cdx, lmax, rcp64(lmax));
+  s.dt = quot64(k, cdx, lmax, rcp64(k, lmax));
   if (lxf) {
-    s.lam_lxf = quot64(dx, s.dt, rcp64(s.dt));
-    s.dtdx = quot64(1.0, s.lam_lxf, rcp64(s.lam_lxf));
+    s.lam_lxf = quot64(k, dx, s.dt, rcp64(k, s.dt));
+    s.dtdx = quot64(k, k.one, s.lam_lxf, rcp64(k, s.lam_lxf));
   } else {
-    s.dtdx = quot64(s.dt, dx, rcp64(dx));
+    s.dtdx = quot64(k, s.dt, dx, rcp64(k, dx));
   }
   return s;
 }
@@ -105,7 +132,7 @@ __device__ __forceinline__ StepScalars step_scalars64(double cfl, double dx, dou
 // max(lambda_a, lambda_b) (NumFluxes.jl:25-33, main.jl:45-48) or the LxF one. Doubling is
 // exact, so this is the flux's own rounding with a multiplication less per variable;
 // the rounding sequence is fixed (explicit intrinsics), so the step commutes with x -> -x.
-__device__ __forceinline__ void face_twice(const double* __restrict__ Q, const double* __restrict__ F,
+__device__ __forceinline__ void face_twice(const Eos64& k, const double* __restrict__ Q, const double* __restrict__ F,
                                            const double* __restrict__ lam, int64_t n, int64_t lo, int64_t hi,
                                            int64_t f, bool lxf, double lam_lxf, double* f2) {
   const int64_t a = f > lo ? f - 1 : lo, b = f < hi ? f : hi - 1;
@@ -117,8 +144,8 @@ __device__ __forceinline__ void face_twice(const double* __restrict__ Q, const d
 #pragma unroll
   for (int v = 0; v < 14; ++v) {
     const int sl = flux_slot1(v);
-    const double dq = __dsub_rn(Q[v * n + b], Q[v * n + a]);
-    f2[v] = sl >= 0 ? __fma_rn(-lf, dq, __dadd_rn(F[sl * n + a], F[sl * n + b])) : __dmul_rn(-lf, dq);
+    const double dq = sub64(k, Q[v * n + b], Q[v * n + a]);
+    f2[v] = sl >= 0 ? __fma_rn(-lf, dq, add64(k, F[sl * n + a], F[sl * n + b])) : mul64(k, -lf, dq);
   }
 }
 

@@ -7,8 +7,8 @@ using namespace hyp;
 template <int kDef>
 static int compact(const EosC& e, const double* q, double* out) {
   const Eos64 k = make_eos64(e);
-  const Cell64 c = cell64<kDef>(e, k, rcp64(q[0]), q + 2, q[5], q + 6);
-  flux64(q[0], c, q + 2, q + 6, out);
+  const Cell64 c = cell64<kDef, false>(e, k, rcp64(k, q[0]), q + 2, q[5], q + 6);
+  flux64<false>(k, q[0], c, q + 2, q + 6, out);
   out[14] = c.u[0];
   out[15] = cmax64<kDef>(e, k, c);
   return c.st;
