@@ -176,19 +176,16 @@ __global__ void __launch_bounds__(kBlock) batch_join_kernel(const float* __restr
 // ---- FP64 ----------------------------------------------------------------------
 // One tile of kCells64 cells per block, as the single problem's kernels (hyp_step1.cu):
 // the cell pass and the tile's maximum into its problem's slot.
-template <int kDef>
-__global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* __restrict__ Q, int64_t n, EosC e,
-                                                                  Eos64 kc, double* __restrict__ F,
-                                                                  double* __restrict__ lam,
-                                                                  const TileDesc* __restrict__ tiles, BatchDev b,
-                                                                  int par, double t_end,
-                                                                  unsigned long long* slot_base, DevState* S) {
+template <int kDef, bool kSoft>
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64_cell_kernel(
+    const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc, double* __restrict__ F, double* __restrict__ lam,
+    const TileDesc* __restrict__ tiles, BatchDev b, int par, double t_end, unsigned long long* slot_base, DevState* S) {
   const TileDesc d = tiles[blockIdx.x];
   if (!(b.t[par * b.P + d.problem] < t_end)) return;
   const Eos64 k = in_registers64(kc);
   const int64_t i = d.first + threadIdx.x;
   const bool own = threadIdx.x < kCells64 && i < d.hi;
-  const double l = own ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = own ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(&slot_base[d.problem], m);
 }
@@ -197,8 +194,8 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_cell_kernel(const double* 
 // call (kCell = false), the cell pass of the new state. The problem's slots: rd holds the
 // max wave speed, its lead tile clears the one a later step writes (a problem past t_end
 // clears all three: whatever steps it next starts with a cell pass).
-template <int kDef, bool kCell>
-__global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
+template <int kDef, bool kCell, bool kSoft>
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64_step_kernel(
     const double* __restrict__ Q, double* __restrict__ Qn, int64_t n, EosC e, Eos64 kc, const double* __restrict__ F,
     const double* __restrict__ lam, double* __restrict__ Fn, double* __restrict__ lamn,
     const TileDesc* __restrict__ tiles, BatchDev b, int par, int rd, int wr, int clr, double t_end, double cfl,
@@ -253,7 +250,7 @@ __global__ void __launch_bounds__(kBlock64) batch_f64_step_kernel(
     }
   }
   if (!kCell || !s_more) return;
-  const double l = own ? cell1_pass<kDef>(q, n, i, e, k, Fn, lamn, S) : 0.0;
+  const double l = own ? cell1_pass<kDef, kSoft>(q, n, i, e, k, Fn, lamn, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (j == 0) atomicMax(&b.slots[wr * P + p], m);
 }
@@ -405,15 +402,17 @@ static int enqueue_batch_step(hyp_batch* b, long long k, double t_end, bool firs
     BCK(e);
   } else {
     const Eos64 k64 = make_eos64(b->eos);
-    const bool def = b->eos.default_exp, apart = b->F[1] == b->F[0];
+    const bool def = b->eos.default_exp, apart = b->F[1] == b->F[0], soft = (unsigned)b->ntiles > kSoftBlocks;
     if (first || apart) {
-      auto cell = def ? batch_f64_cell_kernel<1> : batch_f64_cell_kernel<0>;
+      auto cell = soft ? (def ? batch_f64_cell_kernel<1, true> : batch_f64_cell_kernel<0, true>)
+                       : (def ? batch_f64_cell_kernel<1, false> : batch_f64_cell_kernel<0, false>);
       cell<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->total, b->eos, k64, b->F[par], b->lam[par], b->tiles,
                                                   b->b, par, t_end, b->b.slots + (size_t)rd * b->P, b->st);
       BCK(cudaGetLastError());
     }
-    auto step = last || apart ? batch_f64_step_kernel<1, false>
-                              : (def ? batch_f64_step_kernel<1, true> : batch_f64_step_kernel<0, true>);
+    auto step = last || apart ? batch_f64_step_kernel<1, false, false>
+                : soft        ? (def ? batch_f64_step_kernel<1, true, true> : batch_f64_step_kernel<0, true, true>)
+                              : (def ? batch_f64_step_kernel<1, true, false> : batch_f64_step_kernel<0, true, false>);
     step<<<b->ntiles, kBlock64, 0, b->stream>>>(b->Q[par], b->Q[1 - par], b->total, b->eos, k64, b->F[par],
                                                 b->lam[par], b->F[1 - par], b->lam[1 - par], b->tiles, b->b, par, rd,
                                                 wr, clr, t_end, b->cfg.cfl, b->cfg.flux, b->cfg.bc, b->st);

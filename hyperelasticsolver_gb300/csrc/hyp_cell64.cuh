@@ -47,6 +47,7 @@
 // (which the adjoint and the function-level evaluators use) execute 379; the two agree
 // to a few ulps (tests/test_cell64_host.py).
 #pragma once
+#include <type_traits>
 #include <string.h>
 #include "hyp_physics.cuh"
 
@@ -182,22 +183,83 @@ HYP_HD Eos64 make_eos64(const EosC& e) {
   return c;
 }
 
-// x y, x + y, x - y (k: Eos64 or another struct with one and nz in registers).
-template <class K> HYP_HD double mul64(const K& k, double x, double y) {
+// x y on the integer pipe, rounded to nearest even as the FP64 pipe does: the product of
+// the 53-bit significands from four 32 x 32-bit products, one shift to 53 bits, and the
+// rounding carried into the exponent. worst collects the largest distance of a product's
+// exponent sum from the low end of what this holds for (operands with a zero exponent
+// count as zeros); beyond kSoftWide some product overflowed, underflowed, or had an
+// infinity or NaN for a factor, and the caller takes the hardware's products instead.
+// About 50 instructions and 62 cycles of a scheduler's issue, but none of its FP64 pipe:
+// 16 register FMAs take a warp 1029 cycles, 8 and 8 of these together 545 (4 warps a
+// scheduler) or 732 (a single warp).
+constexpr unsigned kSoftLow = 0x40300000u, kSoftWide = 0x60000000u;
+HYP_HD double soft_mul64(double x, double y, unsigned& worst) {
+  typedef unsigned long long u64;
+  const u64 bx = (u64)bits_of(x), by = (u64)bits_of(y);
+  const unsigned xh = (unsigned)(bx >> 32), xl = (unsigned)bx, yh = (unsigned)(by >> 32), yl = (unsigned)by;
+  const unsigned ex = xh & 0x7ff00000u, ey = yh & 0x7ff00000u, sum = ex + ey;
+  // significands: x's shifted to bit 63, y's as it is; their product's high 64 bits have
+  // 52 or 53 bits
+  const unsigned ah = (xh << 11 | xl >> 21) | 0x80000000u, al = xl << 11, bh = (yh & 0xfffffu) | 0x100000u;
+  const u64 ll = (u64)al * yl, t = (u64)ah * yl + (ll >> 32), u = (u64)al * bh + (unsigned)t;
+  const u64 P = (u64)ah * bh + (t >> 32) + (u >> 32);
+  const unsigned ph = (unsigned)(P >> 32), pl = (unsigned)P, lh = (unsigned)u, l0 = (unsigned)ll;
+  const unsigned full = ph >> 20, up = 1u - full;  // 53 bits already, or one to shift
+  unsigned mh = up ? ph << 1 | pl >> 31 : ph, ml = up ? pl << 1 | lh >> 31 : pl;
+  const unsigned rest = lh << up, base = sum - 0x40000000u + (full << 20);
+#ifdef __CUDA_ARCH__
+  mh = __funnelshift_l(pl, ph, up);
+  ml = __funnelshift_l(lh, pl, up);
+  unsigned none;  // a carry out of rest.l0 + (one half less a bit) + (ml odd) rounds up
+  asm("add.cc.u32 %2, %3, 0xffffffff;\n\t"
+      "addc.cc.u32 %2, %4, 0xffffffff;\n\t"
+      "addc.cc.u32 %2, %5, 0x7fffffff;\n\t"
+      "addc.cc.u32 %0, %0, 0;\n\t"
+      "addc.u32 %1, %1, %6;"
+      : "+r"(ml), "+r"(mh), "=&r"(none)
+      : "r"(ml & 1u), "r"(l0), "r"(rest), "r"(base));
+  (void)none;
+#else
+  const u64 r = (u64)rest << 32 | l0, half = 1ull << 63;
+  const u64 m = ((u64)(mh + base) << 32 | ml) + (r > half || (r == half && (ml & 1u)) ? 1u : 0u);
+  mh = (unsigned)(m >> 32);
+  ml = (unsigned)m;
+#endif
+  const bool zero = (ex < ey ? ex : ey) == 0u;
+  const unsigned off = (zero ? 0x7fe00000u : sum) - kSoftLow;
+  worst = off > worst ? off : worst;
+  const unsigned sign = (xh ^ yh) & 0x80000000u;
+  return of_bits((long long)((u64)((zero ? 0u : mh) | sign) << 32 | (zero ? 0u : ml)));
+}
+
+// The constants for forms whose lone products run on the FP64 pipe, and on the integer pipe.
+struct Plain64 : Eos64 {
+  HYP_HD explicit Plain64(const Eos64& k) : Eos64(k) {}
+  HYP_HD bool out_of_range() const { return false; }
+};
+struct Soft64 : Eos64 {
+  mutable unsigned worst;
+  HYP_HD explicit Soft64(const Eos64& k) : Eos64(k), worst(0u) {}
+  HYP_HD bool out_of_range() const { return worst > kSoftWide; }
+};
+
+// x y, x + y, x - y: on the FP64 pipe, products by a Soft64 on the integer pipe.
+HYP_HD double mul64(const Soft64& k, double x, double y) { return soft_mul64(x, y, k.worst); }
+HYP_HD double mul64(const Eos64& k, double x, double y) {
 #ifdef __CUDA_ARCH__
   return __fma_rn(x, y, k.nz);
 #else
   return x * y;
 #endif
 }
-template <class K> HYP_HD double add64(const K& k, double x, double y) {
+HYP_HD double add64(const Eos64& k, double x, double y) {
 #ifdef __CUDA_ARCH__
   return __fma_rn(x, k.one, y);
 #else
   return x + y;
 #endif
 }
-template <class K> HYP_HD double sub64(const K& k, double x, double y) { return add64(k, x, -y); }
+HYP_HD double sub64(const Eos64& k, double x, double y) { return add64(k, x, -y); }
 
 HYP_HD double rcp64(const Eos64& k, double x) {
   const double r = seed_rcp(x);
@@ -234,8 +296,8 @@ struct Cell64 {
 // 1/alpha (kUnit: alpha is 1, ia not read), m = alpha rho u, rE = alpha rho E, R = alpha
 // rho A (column-major). kDef = 1: the default exponents alpha 1, beta 3, gamma 2 at
 // compile time; 0: any.
-template <int kDef, bool kUnit>
-HYP_HD Cell64 cell64(const EosC& e, const Eos64& k, double ia, const double* m, double rE, const double* R) {
+template <int kDef, bool kUnit, class K>
+HYP_HD Cell64 cell64(const EosC& e, const K& k, double ia, const double* m, double rE, const double* R) {
   Cell64 o;
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
   auto A = [&k](double x, double y) { return add64(k, x, y); };
@@ -326,7 +388,8 @@ double radius_general(double o00, double o11, double o22, double o01, double o02
 // The largest eigenvalue of a symmetric O, false where it does not stand clear of the
 // others' moduli: an FP32 root of the characteristic polynomial, then two steps with the
 // FP32 slope.
-HYP_HD bool top_root64(const Eos64& k, double o00, double o11, double o22, double o01, double o02, double o12,
+template <class K>
+HYP_HD bool top_root64(const K& k, double o00, double o11, double o22, double o01, double o02, double o12,
                        double& root) {
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
   auto A = [&k](double x, double y) { return add64(k, x, y); };
@@ -360,8 +423,8 @@ HYP_HD bool top_root64(const Eos64& k, double o00, double o11, double o22, doubl
 }
 
 // Largest acoustic wave speed sqrt(max |eig Omega|) of one phase (HyperelasticityMPh.jl:258-266).
-template <int kDef>
-HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
+template <int kDef, class K>
+HYP_HD double cmax64(const EosC& e, const K& k, const Cell64& c) {
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
   const double f = M(k.four3, c.b);
   const double f0 = M(f, c.G00), f1 = M(f, c.G01), f2 = M(f, c.G02);
@@ -383,8 +446,8 @@ HYP_HD double cmax64(const EosC& e, const Eos64& k, const Cell64& c) {
 // Physical x-flux of one phase (HyperelasticityMPh.jl:146-175), the 14 entries after
 // alpha: alpha rho u1 is m1 itself, and the rho A part is u1 R - u (row 1 of R), whose
 // first row is zero.
-template <bool kUnit>
-HYP_HD void flux64(const Eos64& k, double alpha, const Cell64& c, const double* m, const double* R, double* f) {
+template <bool kUnit, class K>
+HYP_HD void flux64(const K& k, double alpha, const Cell64& c, const double* m, const double* R, double* f) {
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
   const double den = kUnit ? c.td : M(alpha, c.td), d2 = add64(k, den, den);  // -alpha s0 = 2 alpha rho w
   const double S0 = M(d2, c.w[0]), S1 = M(d2, c.w[1]), S2 = M(d2, c.w[2]);
@@ -398,6 +461,46 @@ HYP_HD void flux64(const Eos64& k, double alpha, const Cell64& c, const double* 
     f[6 + 3 * b] = fma(c.u[0], R[1 + 3 * b], -M(c.u[1], R[3 * b]));
     f[7 + 3 * b] = fma(c.u[0], R[2 + 3 * b], -M(c.u[2], R[3 * b]));
   }
+}
+
+// All of a cell's forms with the hardware's products, out of line: for cells whose products
+// leave soft_mul64's range, which have to come out as the FP64 pipe makes them. q: m, rE,
+// R; out: flux (14), u1, c_max.
+template <int kDef, bool kUnit>
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+int cell_plain64(const EosC& e, const Eos64& k, double alpha, const double* q, double* out) {
+  const Cell64 c = cell64<kDef, kUnit>(e, k, kUnit ? 1.0 : rcp64(k, alpha), q, q[3], q + 4);
+  flux64<kUnit>(k, alpha, c, q, q + 4, out);
+  out[14] = c.u[0];
+  out[15] = cmax64<kDef>(e, k, c);
+  return c.st;
+}
+
+// One phase of a cell: status, u1, c_max and with kFlux the flux; kSoft: lone products on
+// the integer pipe, the same values bit for bit.
+template <int kDef, bool kUnit, bool kFlux, bool kSoft>
+HYP_HD int cell_speed64(const EosC& e, const Eos64& k, double alpha, const double* m, double rE, const double* R,
+                        double* f, double& u1, double& cm) {
+  const typename std::conditional<kSoft, Soft64, Plain64>::type s(k);
+  const Cell64 c = cell64<kDef, kUnit>(e, s, kUnit ? 1.0 : rcp64(k, alpha), m, rE, R);
+  if (kFlux) flux64<kUnit>(s, alpha, c, m, R, f);
+  u1 = c.u[0];
+  cm = cmax64<kDef>(e, s, c);
+  if (!kSoft || !s.out_of_range()) return c.st;
+  double q[13], out[16];
+  for (int v = 0; v < 3; ++v) q[v] = m[v];
+  q[3] = rE;
+  for (int v = 0; v < 9; ++v) q[4 + v] = R[v];
+  const int st = cell_plain64<kDef, kUnit>(e, k, alpha, q, out);
+  if (kFlux)
+    for (int v = 0; v < 14; ++v) f[v] = out[v];
+  u1 = out[14];
+  cm = out[15];
+  return st;
 }
 
 }  // namespace hyp

@@ -21,15 +21,15 @@ namespace hyp {
 // What bounds it: FP64 issue (hyp_cell64.cuh). 1,000,003 cells, whole 10-step run with its copies:
 // 10.48 ms with the general forms, 7.26 ms with these; 1000 cells, 100 steps: 4.14 ms at 256
 // threads a block with the general forms, 2.38 ms.
-template <int kDef>
-__global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc,
+template <int kDef, bool kSoft>
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) cell1_f64_kernel(const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc,
                                                              double* __restrict__ F, double* __restrict__ lam,
                                                              unsigned long long* lam_slot, const double* t_now,
                                                              double t_end, DevState* S) {
   if (!(*t_now < t_end)) return;  // uniform across the grid
   const Eos64 k = in_registers64(kc);
   const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
-  const double l = i < n ? cell1_load_pass<kDef>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = i < n ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(lam_slot, m);
 }
@@ -43,8 +43,8 @@ __global__ void __launch_bounds__(kBlock64) cell1_f64_kernel(const double* __res
 // same, but a small problem saves a launch, the second kernel's ramp and its reload of
 // the state, and the fluxes alternate between two buffers: 1000 cells x 100 steps 1.59 -> 1.40
 // ms, 8192 cells x 4 steps on device buffers 129 -> 110 us, 1,000,003 cells unchanged (6.03 ms).
-template <int kDef, bool kCell>
-__global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e, Eos64 kc) {
+template <int kDef, bool kCell, bool kSoft>
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) step1_f64_kernel(Step1Args a, EosC e, Eos64 kc) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell i0 + k
   __shared__ double s_hdt;             // half dt/dx
   __shared__ int s_more;               // the state this step makes is stepped from
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kBlock64) step1_f64_kernel(Step1Args a, EosC e
     }
   }
   if (!kCell || !s_more) return;
-  const double l = own ? cell1_pass<kDef>(q, n, i, e, k, a.Fn, a.lamn, a.S) : 0.0;
+  const double l = own ? cell1_pass<kDef, kSoft>(q, n, i, e, k, a.Fn, a.lamn, a.S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (j == 0) atomicMax(a.wr, m);
 }
@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
     double* const mine = a.edge + (size_t)((s & 1) * gridDim.x + blockIdx.x) * 2 * kEdge;
     double l = 0.0, f[14];
     if (own) {
-      const Cell64 c = cell64<kDef, true>(e, k, 1.0, q + 1, q[4], q + 5);
-      flux64<true>(k, 1.0, c, q + 1, q + 5, f);
-      l = add64(k, fabs(c.u[0]), cmax64<kDef>(e, k, c));
-      const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
+      double u1, cm;
+      int st = cell_speed64<kDef, true, true, false>(e, k, 1.0, q + 1, q[4], q + 5, f, u1, cm);
+      l = add64(k, fabs(u1), cm);
+      st |= is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE;
       if (st) record_err64(a.S, st, i);
 #pragma unroll
       for (int v = 0; v < 14; ++v) {
@@ -256,17 +256,19 @@ cudaError_t launch_cell1(cudaStream_t s, const double* Q, int64_t n, const EosC&
                          unsigned long long* lam_slot, const double* t_now, double t_end, DevState* S) {
   const unsigned grid = (unsigned)((n + kBlock64 - 1) / kBlock64);
   const Eos64 k = make_eos64(e);
-  if (e.default_exp)
-    cell1_f64_kernel<1><<<grid, kBlock64, 0, s>>>(Q, n, e, k, F, lam, lam_slot, t_now, t_end, S);
-  else
-    cell1_f64_kernel<0><<<grid, kBlock64, 0, s>>>(Q, n, e, k, F, lam, lam_slot, t_now, t_end, S);
+  auto kern = grid > kSoftBlocks ? (e.default_exp ? cell1_f64_kernel<1, true> : cell1_f64_kernel<0, true>)
+                                 : (e.default_exp ? cell1_f64_kernel<1, false> : cell1_f64_kernel<0, false>);
+  kern<<<grid, kBlock64, 0, s>>>(Q, n, e, k, F, lam, lam_slot, t_now, t_end, S);
   return cudaGetLastError();
 }
 
 cudaError_t launch_step1(cudaStream_t s, const Step1Args& a, const EosC& e) {
   const unsigned grid = (unsigned)((a.n + kCells64 - 1) / kCells64);
   const Eos64 k = make_eos64(e);
-  auto kern = !a.Fn ? step1_f64_kernel<1, false> : (e.default_exp ? step1_f64_kernel<1, true> : step1_f64_kernel<0, true>);
+  auto kern = !a.Fn ? step1_f64_kernel<1, false, false>
+              : grid > kSoftBlocks
+                  ? (e.default_exp ? step1_f64_kernel<1, true, true> : step1_f64_kernel<0, true, true>)
+                  : (e.default_exp ? step1_f64_kernel<1, true, false> : step1_f64_kernel<0, true, false>);
   kern<<<grid, kBlock64, 0, s>>>(a, e, k);
   return cudaGetLastError();
 }

@@ -43,7 +43,7 @@ struct CellOut2 {
 // The cell pass of a block's 64 cells, a thread per phase in state q (15 values; `in`:
 // there is a cell): fluxes, speed bounds, and the block's max |speed| into slot. All
 // threads of the block call it.
-template <int kDef>
+template <int kDef, bool kSoft>
 __device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, const EosC& e, const Eos64& k,
                                            const CellOut2& o,
                                            unsigned long long* slot) {
@@ -51,17 +51,15 @@ __device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, 
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
   double lo = 0.0, hi = 0.0;
   if (in) {
-    const Cell64 c = cell64<kDef, false>(e, k, rcp64(k, q[0]), q + 2, q[5], q + 6);
-    double f[14];
-    flux64<false>(k, q[0], c, q + 2, q + 6, f);
+    double f[14], u1, cm;
+    const int st = cell_speed64<kDef, false, true, kSoft>(e, k, q[0], q + 2, q[5], q + 6, f, u1, cm);
     double* f0 = o.F + 15 * ph * o.n + i;
 #pragma unroll
     for (int r = 1; r < 15; ++r)
       if (!zero_flux_row(r)) f0[r * o.n] = f[r - 1];
-    const double cm = cmax64<kDef>(e, k, c);
-    lo = sub64(k, c.u[0], cm);
-    hi = add64(k, c.u[0], cm);
-    if (c.st) record_err64(o.S, c.st, i);
+    lo = sub64(k, u1, cm);
+    hi = add64(k, u1, cm);
+    if (st) record_err64(o.S, st, i);
     if (ph == 1) {
       s_lo[j] = lo;
       s_hi[j] = hi;
@@ -81,8 +79,8 @@ __device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, 
   if (threadIdx.x == 0) atomicMax(slot, m);
 }
 
-template <int kDef>
-__global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __restrict__ Q, Eos2x E, CellOut2 o,
+template <int kDef, bool kSoft>
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) cell2_f64_kernel(const double* __restrict__ Q, Eos2x E, CellOut2 o,
                                                             unsigned long long* lam_slot, const double* t_now,
                                                             double t_end) {
   if (!(*t_now < t_end)) return;
@@ -95,7 +93,7 @@ __global__ void __launch_bounds__(kPair64) cell2_f64_kernel(const double* __rest
 #pragma unroll
     for (int r = 0; r < 15; ++r) q[r] = q0[r * o.n];
   }
-  cell2_pass<kDef>(q, i < o.n, i, E.e[ph], k, o, lam_slot);
+  cell2_pass<kDef, kSoft>(q, i < o.n, i, E.e[ph], k, o, lam_slot);
 }
 
 // ---- faces ---------------------------------------------------------------------
@@ -111,8 +109,8 @@ struct FaceList {
 // way between the cells (through Q_hll) can be singular, D- and D+ (doubles of the
 // formula of NumFluxes.jl:85-132 with its integrals zero). 186 slots a phase; the others are
 // listed.
-template <int kDef>
-__global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
+template <int kDef, bool kSoft>
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) face2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
                                                             const double* __restrict__ F,
                                                             const double* __restrict__ smin,
                                                             const double* __restrict__ smax, double* __restrict__ DM,
@@ -156,11 +154,12 @@ __global__ void __launch_bounds__(kPair64) face2_f64_kernel(const double* __rest
     for (int v = 0; v < 3; ++v) m[v] = add64(k, a[2 + v], b[2 + v]);
 #pragma unroll
     for (int v = 0; v < 9; ++v) Rm[v] = add64(k, a[6 + v], b[6 + v]);
-    const Cell64 c = cell64<kDef, false>(E.e[ph], k, rcp64(k, add64(k, a[0], b[0])), m, add64(k, a[5], b[5]), Rm);
-    const double cm = cmax64<kDef>(E.e[ph], k, c);
-    if (c.st) record_err64(S, c.st, R);
-    s_lo[ph][j] = sub64(k, c.u[0], cm);
-    s_hi[ph][j] = add64(k, c.u[0], cm);
+    double u1, cm;
+    const int st = cell_speed64<kDef, false, false, kSoft>(E.e[ph], k, add64(k, a[0], b[0]), m, add64(k, a[5], b[5]), Rm, nullptr,
+                                                    u1, cm);
+    if (st) record_err64(S, st, R);
+    s_lo[ph][j] = sub64(k, u1, cm);
+    s_hi[ph][j] = add64(k, u1, cm);
   }
   __syncthreads();
   double sl = 0.0, sr = 0.0;
@@ -476,8 +475,8 @@ struct Step2Args {
 
 // A thread per cell and phase; with kCell the new state's cell pass follows in the same
 // kernel (a launch and a reload of the state less per step, which a small problem feels).
-template <int kDef, bool kCell>
-__global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E) {
+template <int kDef, bool kCell, bool kSoft>
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) step2_f64_kernel(Step2Args a, Eos2x E) {
   __shared__ double s_r;
   __shared__ int s_more;
   const int ph = threadIdx.x / kPairCells;
@@ -531,7 +530,7 @@ __global__ void __launch_bounds__(kPair64) step2_f64_kernel(Step2Args a, Eos2x E
     }
   }
   if (!kCell || !s_more) return;
-  cell2_pass<kDef>(q, i < n, i, E.e[ph], k, a.o, a.wr);
+  cell2_pass<kDef, kSoft>(q, i < n, i, E.e[ph], k, a.o, a.wr);
 }
 
 static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
@@ -542,8 +541,11 @@ static bool default_exp2(const hyp_ctx* c) { return c->eos2.e[0].default_exp && 
 static CellOut2 cell_out(hyp_ctx* c) { return CellOut2{c->F, c->smin, c->smax, c->n, c->st}; }
 
 cudaError_t launch_cell2_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end) {
-  auto kern = default_exp2(c) ? cell2_f64_kernel<1> : cell2_f64_kernel<0>;
-  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(c->Q[p], eos2x(c), cell_out(c), lam_slot, t_now, t_end);
+  const unsigned grid = grid_n(c->n, kPairCells);
+  const bool def = default_exp2(c);
+  auto kern = grid > kSoftBlocks ? (def ? cell2_f64_kernel<1, true> : cell2_f64_kernel<0, true>)
+                                 : (def ? cell2_f64_kernel<1, false> : cell2_f64_kernel<0, false>);
+  kern<<<grid, kPair64, 0, c->stream>>>(c->Q[p], eos2x(c), cell_out(c), lam_slot, t_now, t_end);
   return cudaGetLastError();
 }
 cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, double t_end) {
@@ -556,7 +558,8 @@ cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, do
     face2_lxf_f64_kernel<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, E.k[0], c->F, rd, c->cfg.cfl, dx,
                                                           c->FF, c->DM, list, &c->st->t[p], t_end, c->st);
   } else {
-    auto kern = def ? face2_f64_kernel<1> : face2_f64_kernel<0>;
+    auto kern = grid > kSoftBlocks ? (def ? face2_f64_kernel<1, true> : face2_f64_kernel<0, true>)
+                                   : (def ? face2_f64_kernel<1, false> : face2_f64_kernel<0, false>);
     kern<<<grid, kPair64, 0, c->stream>>>(c->Q[p], c->n, E, c->F, c->smin, c->smax, c->DM, c->DP, list, &c->st->t[p],
                                           t_end, c->st);
   }
@@ -592,8 +595,12 @@ static cudaError_t launch_step2(hyp_ctx* c, long long k, double t_end, bool cell
   a.dx = c->cfg.x_length / (double)c->n;
   a.bc = c->cfg.bc;
   a.o = cell_out(c);
-  auto kern = !cell ? step2_f64_kernel<1, false> : (default_exp2(c) ? step2_f64_kernel<1, true> : step2_f64_kernel<0, true>);
-  kern<<<grid_n(c->n, kPairCells), kPair64, 0, c->stream>>>(a, eos2x(c));
+  const unsigned grid = grid_n(c->n, kPairCells);
+  const bool def = default_exp2(c);
+  auto kern = !cell ? step2_f64_kernel<1, false, false>
+              : grid > kSoftBlocks ? (def ? step2_f64_kernel<1, true, true> : step2_f64_kernel<0, true, true>)
+                                   : (def ? step2_f64_kernel<1, true, false> : step2_f64_kernel<0, true, false>);
+  kern<<<grid, kPair64, 0, c->stream>>>(a, eos2x(c));
   return cudaGetLastError();
 }
 cudaError_t launch_update2_f64(hyp_ctx* c, long long k, double t_end) { return launch_step2(c, k, t_end, false); }

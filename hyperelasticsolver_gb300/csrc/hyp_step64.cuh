@@ -12,6 +12,17 @@ namespace hyp {
 // time of one.
 constexpr int kBlock64 = 128;
 
+// Grids of more blocks than this, one a multiprocessor, take the lone products of a cell
+// pass on the integer pipe (hyp_cell64.cuh): the two pipes overlap where a scheduler has
+// warps to choose from, so those kernels keep to 128 registers and four blocks resident
+// (1,000,003 cells x 10 steps: 4.53 ms, with two, three, five 5.19, 4.71, 4.68, and 5.48
+// with all products on the FP64 pipe). 50 steps of 20,000 cells (158 blocks) 1.05 -> 1.01 ms, of
+// 38,000 1.18 -> 1.13, of 70,000 1.99 -> 1.64; two phases (64 cells a block), 20 HLL steps of
+// 9,700 cells (152 blocks) 1.02 -> 1.10 ms, of 14,000 1.15 on either pipe, of 38,000 1.57 ->
+// 1.51, and 20 LxF steps 0.78 -> 0.83, 0.92 -> 0.88, 1.42 -> 1.26.
+constexpr unsigned kSoftBlocks = 152;
+constexpr int kSoftResident = 4;
+
 // The constants as register values (hyp_cell64.cuh: an operand from the constant bank or
 // a uniform register slows an FMA by a fifth). Their high words pass through an exclusive
 // or with a zero that only the launch knows (all grids here have gridDim.y = 1) and that a
@@ -64,31 +75,31 @@ __device__ __forceinline__ unsigned long long block_max_bits(double l) {
 
 // The single-phase cell pass of cell i in state q: its flux (kNFlux1 rows of F) and wave
 // speed, stored and returned; a bad cell is recorded.
-template <int kDef>
+template <int kDef, bool kSoft>
 __device__ __forceinline__ double cell1_pass(const double* q, int64_t n, int64_t i, const EosC& e, const Eos64& k,
                                              double* __restrict__ F, double* __restrict__ lam, DevState* S) {
   double f[14];
-  const Cell64 c = cell64<kDef, true>(e, k, 1.0, q + 1, q[4], q + 5);
-  flux64<true>(k, 1.0, c, q + 1, q + 5, f);
-  const double l = add64(k, fabs(c.u[0]), cmax64<kDef>(e, k, c));
+  double u1, cm;
+  int st = cell_speed64<kDef, true, true, kSoft>(e, k, 1.0, q + 1, q[4], q + 5, f, u1, cm);
+  const double l = add64(k, fabs(u1), cm);
 #pragma unroll
   for (int v = 0; v < 14; ++v) {
     const int sl = flux_slot1(v);
     if (sl >= 0) F[sl * n + i] = f[v];
   }
   lam[i] = l;
-  const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
+  st |= is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE;
   if (st) record_err64(S, st, i);
   return l;
 }
-template <int kDef>
+template <int kDef, bool kSoft>
 __device__ __forceinline__ double cell1_load_pass(const double* __restrict__ Q, int64_t n, int64_t i, const EosC& e,
                                                   const Eos64& k, double* __restrict__ F, double* __restrict__ lam,
                                                   DevState* S) {
   double q[14];
 #pragma unroll
   for (int v = 0; v < 14; ++v) q[v] = Q[v * n + i];
-  return cell1_pass<kDef>(q, n, i, e, k, F, lam, S);
+  return cell1_pass<kDef, kSoft>(q, n, i, e, k, F, lam, S);
 }
 
 // Cells a block of the update kernels owns: thread j evaluates the face left of cell

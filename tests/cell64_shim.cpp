@@ -7,11 +7,7 @@ using namespace hyp;
 template <int kDef>
 static int compact(const EosC& e, const double* q, double* out) {
   const Eos64 k = make_eos64(e);
-  const Cell64 c = cell64<kDef, false>(e, k, rcp64(k, q[0]), q + 2, q[5], q + 6);
-  flux64<false>(k, q[0], c, q + 2, q + 6, out);
-  out[14] = c.u[0];
-  out[15] = cmax64<kDef>(e, k, c);
-  return c.st;
+  return cell_speed64<kDef, false, true, true>(e, k, q[0], q + 2, q[5], q + 6, out, out[14], out[15]);
 }
 
 extern "C" {
@@ -48,6 +44,18 @@ int c64_vjp_general(const double* p, const double* q, const double* fb, double l
   out[14] = b.b0sq;
   out[15] = b.k0;
   return st;
+}
+// the forms with the hardware's products (cell_plain64)
+int c64_plain(const double* p, const double* q, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  const Eos64 k = make_eos64(e);
+  return e.default_exp ? cell_plain64<1, false>(e, k, q[0], q + 2, out) : cell_plain64<0, false>(e, k, q[0], q + 2, out);
+}
+double c64_soft_mul(double x, double y, int* in_range) {
+  unsigned worst = 0u;
+  const double r = soft_mul64(x, y, worst);
+  *in_range = worst <= kSoftWide;
+  return r;
 }
 float c64_to_f32(double x) { return to_f32(x); }
 double c64_to_f64(float x) { return to_f64(x); }

@@ -135,3 +135,41 @@ def test_integer_pipe_conversions(lib):
         if abs(f) > 1.2e-38 or f == 0.0:
             assert lib.c64_to_f64(f) == f
     assert np.isnan(lib.c64_to_f32(np.nan)) and np.isnan(lib.c64_to_f64(np.nan))
+
+
+def test_integer_products_are_the_hardware_s(lib):
+    """soft_mul64 against the FP64 product, bit for bit: random significands, short ones
+    (ties), zeros of both signs and exponents over the range; beyond it the products are
+    flagged, and infinities and NaN too."""
+    lib.c64_soft_mul.restype = ctypes.c_double
+    lib.c64_soft_mul.argtypes = [ctypes.c_double, ctypes.c_double, ctypes.POINTER(ctypes.c_int)]
+    rng = np.random.default_rng(11)
+    x, y = rng.uniform(-2, 2, 40000), rng.uniform(-2, 2, 40000)
+    x[::5] = rng.integers(-(1 << 27), 1 << 27, x[::5].size) * 2.0 ** -20
+    y[::5] = rng.integers(-(1 << 27), 1 << 27, x[::5].size) * 2.0 ** -25
+    x[1::5] *= 2.0 ** rng.integers(-400, 400, x[1::5].size)
+    y[1::5] *= 2.0 ** rng.integers(-80, 80, x[1::5].size)
+    x[2::50], y[3::50], x[4::50] = 0.0, -0.0, 1.0
+    ok = ctypes.c_int()
+    for a, b in zip(x.tolist(), y.tolist()):
+        r = lib.c64_soft_mul(a, b, ctypes.byref(ok))
+        assert ok.value and np.float64(r).tobytes() == np.float64(a * b).tobytes(), (a, b, r)
+    for a, b in ((1e-200, 1e-200), (1e200, 1e200), (np.inf, 2.0), (3.0, np.nan), (-np.inf, -np.inf), (np.nan, np.nan)):
+        lib.c64_soft_mul(a, b, ctypes.byref(ok))
+        assert not ok.value, (a, b)
+
+
+@pytest.mark.parametrize("ep", EOS)
+def test_integer_products_leave_the_forms_as_they_are(lib, orc, ep):
+    """Flux, speed and status bit for bit those of the hardware's products, in ordinary
+    states and where products leave the range (tiny and large momenta, NaN, infinities)."""
+    rng = np.random.default_rng(5)
+    for q in phase_states(orc, ep, rng, 40, (1.0, 0.3, 1e-6), 0.1):
+        for v, x in ((None, 0), (3, 0.0), (3, 1e-170), (4, 1e-300), (2, 1e160), (5, np.inf), (7, np.nan), (10, -np.inf),
+                     (6, -q[6]), (4, np.nan)):
+            p = q.copy()
+            if v is not None:
+                p[v] = x
+            s0, a = ev(lib, "c64_plain", ep, p)
+            s1, b = ev(lib, "c64_compact", ep, p)
+            assert s0 == s1 and a.tobytes() == b.tobytes(), (v, x)
