@@ -267,7 +267,7 @@ int ctx_finish_install(hyp_ctx* c, double t0) { return ctx_finish_install_from(c
 
 // Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister), or
 // null for memory the device does not map (pageable, or not host memory).
-static const double* mapped_host(const void* p) {
+const double* mapped_host(const void* p) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError();
