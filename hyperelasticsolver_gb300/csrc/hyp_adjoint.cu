@@ -156,9 +156,12 @@ __global__ void __launch_bounds__(256) adj_dtdx_kernel(AdjArgs g) {
 
 // What bounds it: FP64 issue (hyp_cell64.cuh). The VJP on the compact forms, masked
 // differences shared between the face terms, dt/dx on one warp of a block and integer
-// zero tests: 880 -> about 470 FP64 instructions a cell; 65,536 cells, 50 steps with record
-// and recompute 11.4 -> 9.5 ms.
-template <int kDef>
+// zero tests: 880 -> about 560 FP64 instructions a cell; 65,536 cells, 50 steps with record
+// and recompute 11.4 -> 9.5 ms. With every operator an FMA on registers and the wave
+// speeds' terms only in warps that have one 8.09 -> 7.64 ms; with lone products on the integer
+// pipe (kSoft) 7.37 to 7.6 at the two blocks a multiprocessor that its registers allow, held
+// to three and four blocks 8.26 and 7.49 for the spills.
+template <int kDef, bool kSoft>
 __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, Eos64 kc) {
   __shared__ double sh[kAdjBlock / 32];
   __shared__ double s_lamb_max, s_r;
@@ -179,6 +182,7 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
   __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
   EosBar eb{0.0, 0.0};
+  const unsigned lanes = __ballot_sync(0xffffffffu, i < n);
   if (i < n) {
     const double r = s_r;
     const int64_t il = i > 0 ? i - 1 : 0, ir = i < n - 1 ? i + 1 : n - 1;
@@ -187,6 +191,8 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
     const double li = g.lam[i], ll = g.lam[il], lr = g.lam[ir];
     const bool takeL = !(ll > li);  // the left face took lambda_i
     const bool takeR = li > lr;     // the right face took lambda_i
+    // where the wave speed is monotone one of the two holds for a whole warp
+    const bool anyL = __any_sync(lanes, il != i && takeL), anyR = __any_sync(lanes, ir != i && takeR);
     // face adjoints Fb = r (Qb1_R - Qb1_L): half goes to each cell's flux (all of it to
     // the cell beside a ghost, whose face is its flux), -+ lambda/2 to the state
     const double cL = il != i ? 0.5 * r : r, cR = ir != i ? 0.5 * r : r;
@@ -201,13 +207,13 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
       const double qc = g.Q[v * n + i];
       q[v] = qc;
       const double bc = g.Qb1[v * n + i], bi = ui ? bc : 0.0;
-      const double gL = bi - (ul ? g.Qb1[v * n + il] : 0.0);
-      const double gR = (ur ? g.Qb1[v * n + ir] : 0.0) - bi;
+      const double gL = sub64(k64, bi, ul ? g.Qb1[v * n + il] : 0.0);
+      const double gR = sub64(k64, ur ? g.Qb1[v * n + ir] : 0.0, bi);
       qb[v] = fma(hR, gR, fma(hL, gL, bc));
-      dL = fma(gL, qc - g.Q[v * n + il], dL);
-      dR = fma(gR, g.Q[v * n + ir] - qc, dR);
+      if (anyL) dL = fma(gL, sub64(k64, qc, g.Q[v * n + il]), dL);
+      if (anyR) dR = fma(gR, sub64(k64, g.Q[v * n + ir], qc), dR);
       if (flux_slot1(v) >= 0) {
-        fb[v] = fma(cR, gR, cL * gL);
+        fb[v] = fma(cR, gR, mul64(k64, cL, gL));
         any |= (unsigned long long)bits_of(fb[v]) << 1;
       } else {
         fb[v] = 0.0;
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
     any |= (unsigned long long)bits_of(lamb) << 1;
     // where the face adjoints vanish (a region where the adjoint field is constant) the
     // VJP adds exact zeros: skip it
-    if (any) cell_vjp64<kDef>(e, k64, q, fb, lamb, qb, eb);
+    if (any) cell_vjp64<kDef, kSoft>(e, k64, q, fb, lamb, qb, eb);
 #pragma unroll
     for (int v = 0; v < 14; ++v) g.Qb0[v * n + i] = qb[v];
   }
@@ -430,7 +436,9 @@ extern "C" int hyp_adjoint(hyp_ctx* c, const double* dL_dQ_final, double* dL_dQ0
       g.part_grid = t->part_grid;
       adj_dtdx_kernel<<<t->part_grid, 256, 0, c->stream>>>(g);
       ACK(cudaGetLastError());
-      auto cell = c->eos[0].default_exp ? adj_cell_kernel<1> : adj_cell_kernel<0>;
+      const bool def = c->eos[0].default_exp;
+      auto cell = (unsigned)t->cell_grid > kSoftBlocks ? (def ? adj_cell_kernel<1, true> : adj_cell_kernel<0, true>)
+                                                       : (def ? adj_cell_kernel<1, false> : adj_cell_kernel<0, false>);
       cell<<<t->cell_grid, kAdjBlock, 0, c->stream>>>(g, c->eos[0], make_eos64(c->eos[0]));
       ACK(cudaGetLastError());
       cur = 1 - cur;

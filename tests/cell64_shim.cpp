@@ -32,7 +32,16 @@ int c64_vjp_compact(const double* p, const double* q, const double* fb, double l
   const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
   const Eos64 k = make_eos64(e);
   EosBar b{0.0, 0.0};
-  const int st = e.default_exp ? cell_vjp64<1>(e, k, q, fb, lb, out, b) : cell_vjp64<0>(e, k, q, fb, lb, out, b);
+  const int st = e.default_exp ? cell_vjp64<1, true>(e, k, q, fb, lb, out, b) : cell_vjp64<0, true>(e, k, q, fb, lb, out, b);
+  out[14] = b.b0sq;
+  out[15] = b.k0;
+  return st;
+}
+int c64_vjp_plain(const double* p, const double* q, const double* fb, double lb, double* out) {
+  const EosC e = make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]);
+  const Eos64 k = make_eos64(e);
+  EosBar b{0.0, 0.0};
+  const int st = e.default_exp ? cell_vjp64<1, false>(e, k, q, fb, lb, out, b) : cell_vjp64<0, false>(e, k, q, fb, lb, out, b);
   out[14] = b.b0sq;
   out[15] = b.k0;
   return st;

@@ -173,3 +173,23 @@ def test_integer_products_leave_the_forms_as_they_are(lib, orc, ep):
             s0, a = ev(lib, "c64_plain", ep, p)
             s1, b = ev(lib, "c64_compact", ep, p)
             assert s0 == s1 and a.tobytes() == b.tobytes(), (v, x)
+
+
+@pytest.mark.parametrize("ep", EOS)
+def test_integer_products_leave_the_vjp_as_it_is(lib, orc, ep):
+    """As above for the adjoint's cell."""
+    dp = ctypes.POINTER(ctypes.c_double)
+    rng = np.random.default_rng(6)
+    e = np.array(ep, dtype=np.float64)
+    for s in phase_states(orc, ep, rng, 30, (1.0,), 0.1):
+        fb, lb = rng.standard_normal(14), rng.standard_normal()
+        for v, x in ((None, 0), (2, 0.0), (3, 1e-170), (1, 1e160), (4, np.inf), (6, np.nan)):
+            q, out = s[1:].copy(), [np.zeros(16), np.zeros(16)]
+            if v is not None:
+                q[v] = x
+            st = []
+            for n, o in zip(("c64_vjp_plain", "c64_vjp_compact"), out):
+                o[:14] = fb
+                st.append(getattr(lib, n)(e.ctypes.data_as(dp), q.ctypes.data_as(dp), fb.ctypes.data_as(dp),
+                                          ctypes.c_double(lb), o.ctypes.data_as(dp)))
+            assert st[0] == st[1] and out[0].tobytes() == out[1].tobytes(), (v, x)
