@@ -294,13 +294,12 @@ struct Cell64 {
 
 // HyperelasticityMPh.jl:106-133 and EquationsOfState.jl:118-190 for one phase: ia =
 // 1/alpha (kUnit: alpha is 1, ia not read), m = alpha rho u, rE = alpha rho E, R = alpha
-// rho A (column-major). kDef = 1: the default exponents alpha 1, beta 3, gamma 2 at
-// compile time; 0: any.
-template <int kDef, bool kUnit, class K>
-HYP_HD Cell64 cell64(const EosC& e, const K& k, double ia, const double* m, double rE, const double* R) {
-  Cell64 o;
+// rho A (column-major). In three parts, the first two independent of each other: density,
+// velocity and energies; N = R R^T and its cofactors; the rest. kDef = 1: the default
+// exponents alpha 1, beta 3, gamma 2 at compile time; 0: any.
+template <bool kUnit, class K>
+HYP_HD double cell_density64(const K& k, double ia, const double* m, double rE, const double* R, Cell64& o) {
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
-  auto A = [&k](double x, double y) { return add64(k, x, y); };
   const double c0 = fma(R[4], R[8], -M(R[5], R[7])), c1 = fma(R[1], R[8], -M(R[7], R[2]));
   const double c2 = fma(R[1], R[5], -M(R[4], R[2]));
   const double d = fma(R[6], c2, fma(-R[3], c1, M(R[0], c0)));
@@ -313,26 +312,47 @@ HYP_HD Cell64 cell64(const EosC& e, const K& k, double ia, const double* m, doub
   o.inv_den = kUnit ? r : M(r, ia);
   for (int c = 0; c < 3; ++c) o.u[c] = M(m[c], o.inv_den);
   o.E = M(rE, o.inv_den);
-  const double e_int = fma(-k.half, fma(o.u[2], o.u[2], fma(o.u[1], o.u[1], M(o.u[0], o.u[0]))), o.E);
-  // N = R R^T and its cofactors
-  const double n00 = fma(R[6], R[6], fma(R[3], R[3], M(R[0], R[0])));
+  return fma(-k.half, fma(o.u[2], o.u[2], fma(o.u[1], o.u[1], M(o.u[0], o.u[0]))), o.E);  // e_int
+}
+
+struct Gram64 {
+  double n00, n01, n02;                 // of N
+  double k00, k01, k02, k11, k12, k22;  // its cofactors
+};
+template <class K>
+HYP_HD Gram64 gram64(const K& k, const double* R) {
+  auto M = [&k](double x, double y) { return mul64(k, x, y); };
+  Gram64 g;
+  g.n00 = fma(R[6], R[6], fma(R[3], R[3], M(R[0], R[0])));
+  g.n01 = fma(R[6], R[7], fma(R[3], R[4], M(R[0], R[1])));
+  g.n02 = fma(R[6], R[8], fma(R[3], R[5], M(R[0], R[2])));
   const double n11 = fma(R[7], R[7], fma(R[4], R[4], M(R[1], R[1])));
   const double n22 = fma(R[8], R[8], fma(R[5], R[5], M(R[2], R[2])));
-  const double n01 = fma(R[6], R[7], fma(R[3], R[4], M(R[0], R[1])));
-  const double n02 = fma(R[6], R[8], fma(R[3], R[5], M(R[0], R[2])));
   const double n12 = fma(R[7], R[8], fma(R[4], R[5], M(R[1], R[2])));
-  const double k00 = fma(n11, n22, -M(n12, n12)), k11 = fma(n00, n22, -M(n02, n02)), k22 = fma(n00, n11, -M(n01, n01));
-  const double k01 = fma(n02, n12, -M(n01, n22)), k02 = fma(n01, n12, -M(n02, n11)), k12 = fma(n01, n02, -M(n00, n12));
+  g.k00 = fma(n11, n22, -M(n12, n12));
+  g.k11 = fma(g.n00, n22, -M(g.n02, g.n02));
+  g.k22 = fma(g.n00, n11, -M(g.n01, g.n01));
+  g.k01 = fma(g.n02, n12, -M(g.n01, n22));
+  g.k02 = fma(g.n01, n12, -M(g.n02, n11));
+  g.k12 = fma(g.n01, g.n02, -M(g.n00, n12));
+  return g;
+}
+
+template <int kDef, bool kUnit, class K>
+HYP_HD void cell_stress64(const EosC& e, const K& k, double ia, double e_int, const Gram64& g, Cell64& o) {
+  auto M = [&k](double x, double y) { return mul64(k, x, y); };
+  auto A = [&k](double x, double y) { return add64(k, x, y); };
+  const double t = kUnit ? k.inv_rho0 : M(ia, k.inv_rho0);
   // M = N inv_den^2, p = (rho_true / rho0)^2, G = adj(M) p: p M = N (ia/rho0)^2 and
   // G = C (ia inv_den / rho0)^2
   const double g1 = M(t, o.inv_den), gs = M(g1, g1), ms = kUnit ? k.inv_rho0sq : M(t, t);
-  o.G00 = M(k00, gs);
-  o.G01 = M(k01, gs);
-  o.G02 = M(k02, gs);
-  o.G11 = M(k11, gs);
-  o.G12 = M(k12, gs);
-  o.G22 = M(k22, gs);
-  const double i1 = M(A(A(k00, k11), k22), gs);
+  o.G00 = M(g.k00, gs);
+  o.G01 = M(g.k01, gs);
+  o.G02 = M(g.k02, gs);
+  o.G11 = M(g.k11, gs);
+  o.G12 = M(g.k12, gs);
+  o.G22 = M(g.k22, gs);
+  const double i1 = M(A(A(g.k00, g.k11), g.k22), gs);
   const double s = M(o.td, k.inv_rho0);  // 1/det A = sqrt(p)
   const double p = M(s, s);
   // psi = i1^2/3 - i2 = |dev G|^2 / 2, and row 1 of the stress below, from the deviator's
@@ -364,12 +384,19 @@ HYP_HD Cell64 cell64(const EosC& e, const K& k, double ia, const double* m, doub
   o.T3 = M(k.hbeta, bp);
   o.E3p = A(A(o.T1, o.T2), o.T3);
   o.a = M(k.two3, M(o.b, i1));
-  o.bM = M(o.b, M(n00, ms));
+  o.bM = M(o.b, M(g.n00, ms));
   const double h = fma(o.G00, d0, off);
   o.wE = M(o.b, h);
   o.w[0] = fma(o.b, h, o.E3p);
-  o.w[1] = fma(o.a, o.G01, M(o.b, M(n01, ms)));
-  o.w[2] = fma(o.a, o.G02, M(o.b, M(n02, ms)));
+  o.w[1] = fma(o.a, o.G01, M(o.b, M(g.n01, ms)));
+  o.w[2] = fma(o.a, o.G02, M(o.b, M(g.n02, ms)));
+}
+
+template <int kDef, bool kUnit, class K>
+HYP_HD Cell64 cell64(const EosC& e, const K& k, double ia, const double* m, double rE, const double* R) {
+  Cell64 o;
+  const double e_int = cell_density64<kUnit>(k, ia, m, rE, R, o);
+  cell_stress64<kDef, kUnit>(e, k, ia, e_int, gram64(k, R), o);
   return o;
 }
 

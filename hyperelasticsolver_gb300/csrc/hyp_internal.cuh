@@ -257,6 +257,7 @@ struct Run1Args {
   int flux, bc;
   int slot0;  // the first step's max-speed slot
   int tries;  // poll budget of a block's wait
+  int sms;    // multiprocessors of the device
   DevState* S;
 };
 constexpr int kRunTries = 1 << 24;

@@ -136,6 +136,7 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
     a.slot0 = 0;
     a.tries = kRunTries;
     a.S = st;
+    a.sms = run_blocks;
     if (launch_run1(s, a, eos) != cudaSuccess) return HYP_ERR_CUDA;
   }
   if (!one_launch && n_steps > 0 &&

@@ -125,6 +125,22 @@ __device__ __forceinline__ bool run_barrier(unsigned* count, unsigned target, in
   return s_ok != 0;
 }
 
+// The end of a run at time t after s steps: the device struct, with its slots and counters
+// at zero again.
+__device__ __forceinline__ void run1_finish(const Run1Args& a, double t, int s) {
+  if (threadIdx.x == 0) {
+    if (blockIdx.x == 0) {
+      a.t_out[0] = a.t_out[1] = t;
+      a.S->steps += s;
+    }
+    __threadfence();
+    if (atomicAdd(&a.S->run_done, 1u) == gridDim.x - 1) {  // the last block: all others are past the loop
+      a.S->run_count = a.S->run_done = 0u;
+      for (int c = 0; c < 3; ++c) a.S->lam_slots[c] = 0ull;
+    }
+  }
+}
+
 // Steps of a problem of at most one block per multiprocessor (127 cells each, 19,304 on
 // 152 of them), all in one cooperative launch. A step of such a problem is one pass of
 // FP64 issue, 240 slots (7.4 us), whatever it does about memory; as kernels of their own,
@@ -134,7 +150,7 @@ __device__ __forceinline__ bool run_barrier(unsigned* count, unsigned target, in
 // their part of the maximum wave speed, after it they read their neighbours' edges and
 // the maximum. The arithmetic is that of cell1_pass and step1_f64_kernel, in the same
 // order. 1000 cells x 100
-// steps 1.39 -> 1.26 ms (1.19 since all operators are FMAs), 8192 cells x 4 steps on device buffers 111 -> 80 us.
+// steps 1.39 -> 1.26 ms (1.19 since all operators are FMAs; now run1_split_f64_kernel's size), 8192 cells x 4 steps on device buffers 111 -> 80 us.
 template <int kDef>
 __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
   __shared__ double sh[kEdge][kBlock64 + 1];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
@@ -228,25 +244,169 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
 #pragma unroll
     for (int v = 0; v < 14; ++v) Qn[v * n + i] = q[v];
   }
-  if (j == 0) {
-    if (blockIdx.x == 0) {
-      a.t_out[0] = a.t_out[1] = t;
-      a.S->steps += s;
-    }
-    __threadfence();
-    if (atomicAdd(&a.S->run_done, 1u) == gridDim.x - 1) {  // the last block: all others are past the loop
-      a.S->run_count = a.S->run_done = 0u;
-      for (int c = 0; c < 3; ++c) a.S->lam_slots[c] = 0ull;
-    }
-  }
+  run1_finish(a, t, s);
 }
 
-size_t run1_edge_doubles(int64_t n) { return (size_t)((n + kCells64 - 1) / kCells64) * 4 * kEdge; }
+// The same for problems of at most 63 cells per multiprocessor (9576 on 152), two threads a
+// cell, on different schedulers: FP64 issue is what a step of run1_f64_kernel waits for, and
+// most schedulers have no warp of it. The second thread (half 1) forms N and its cofactors
+// beside the first one's density and energies, the flux beside its wave speed, and half of
+// the variables' faces and updates: about 160 FP64 instructions in sequence instead of 255.
+// The state lives in shared memory. The arithmetic is the same, instruction by instruction.
+// Whole runs, one thread a cell and two: 1000 cells x 100 steps 1.22 -> 0.99 ms, 8192 cells x 4
+// steps on device buffers 81 -> 73 us, 50 steps of 64 to 9576 cells 0.61 to 0.77 -> 0.51 to
+// 0.65 ms.
+constexpr int kSplitSlots = 64, kSplitCells = kSplitSlots - 1;
+constexpr int kGram = sizeof(Gram64) / sizeof(double), kCellShared = 8;
+
+template <int kDef>
+__global__ void __launch_bounds__(2 * kSplitSlots) run1_split_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
+  __shared__ double sh[kEdge][kSplitSlots + 2];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
+  __shared__ double sF[14][kSplitSlots];         // twice the left face of cell i0 + j
+  __shared__ double sG[kGram][kSplitSlots], sC[kCellShared][kSplitSlots];
+  __shared__ double s_hdt, s_t;
+  const Eos64 k = in_registers64(kc);
+  const int half = threadIdx.x / kSplitSlots, j = threadIdx.x % kSplitSlots;
+  const int64_t n = a.n, i0 = (int64_t)blockIdx.x * kSplitCells, i = i0 + j;
+  const int cells = (int)(n - i0 < kSplitCells ? n - i0 : kSplitCells);
+  const bool own = j < cells, lxf = a.flux == HYP_FLUX_LXF;
+  const bool frozen = own && bc_holds(a.bc, i == 0, i == n - 1);
+  if (own)
+#pragma unroll
+    for (int u = 0; u < 7; ++u) sh[u + 7 * half][j + 1] = a.Q[(u + 7 * half) * n + i];
+  double t = *a.t_in;
+  int s = 0;
+  for (; s < a.max_steps && t < a.t_end; ++s) {
+    double* const mine = a.edge + (size_t)((s & 1) * gridDim.x + blockIdx.x) * 2 * kEdge;
+    __syncthreads();  // the state, by both halves
+    double q[14], l = 0.0, e_int = 0.0;
+    Cell64 c;
+    if (own) {
+#pragma unroll
+      for (int v = 0; v < 14; ++v) q[v] = sh[v][j + 1];
+      if (half) {
+        const Gram64 g = gram64(k, q + 5);
+        const double* p = &g.n00;
+#pragma unroll
+        for (int v = 0; v < kGram; ++v) sG[v][j] = p[v];
+      } else {
+        e_int = cell_density64<true>(k, 1.0, q + 1, q[4], q + 5, c);
+      }
+    }
+    __syncthreads();
+    if (own && !half) {
+      Gram64 g;
+      double* p = &g.n00;
+#pragma unroll
+      for (int v = 0; v < kGram; ++v) p[v] = sG[v][j];
+      cell_stress64<kDef, true>(e, k, 1.0, e_int, g, c);
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        sC[v][j] = c.u[v];
+        sC[3 + v][j] = c.w[v];
+      }
+      sC[6][j] = c.E;
+      sC[7][j] = c.td;
+    }
+    __syncthreads();
+    if (own) {
+      if (half) {
+#pragma unroll
+        for (int v = 0; v < 3; ++v) {
+          c.u[v] = sC[v][j];
+          c.w[v] = sC[3 + v][j];
+        }
+        c.E = sC[6][j];
+        c.td = sC[7][j];
+        double f[14];
+        flux64<true>(k, 1.0, c, q + 1, q + 5, f);
+#pragma unroll
+        for (int v = 0; v < 14; ++v)
+          if (flux_slot1(v) >= 0) sh[14 + flux_slot1(v)][j + 1] = f[v];
+      } else {
+        l = add64(k, fabs(c.u[0]), cmax64<kDef>(e, k, c));
+        const int st = c.st | (is_finite64(l) ? HYP_CELL_OK : HYP_CELL_NONFINITE);
+        if (st) record_err64(a.S, st, i);
+        sh[kEdge - 1][j + 1] = l;
+      }
+    }
+    const unsigned long long top = block_max_bits<2 * kSplitSlots>(l);  // (its barrier publishes sh)
+    if ((int)threadIdx.x < 2 * kEdge) {  // the first and the last cell, for the neighbours
+      const int side = threadIdx.x >= kEdge, r = threadIdx.x - side * kEdge;
+      mine[threadIdx.x] = sh[r][side ? cells : 1];
+    }
+    if (threadIdx.x == 0) atomicMax(&a.S->lam_slots[(a.slot0 + s) % 3], top);
+    if (!run_barrier(&a.S->run_count, (unsigned)(s + 1) * gridDim.x, a.tries)) {
+      if (threadIdx.x == 0) record_err64(a.S, HYP_CELL_TIMEOUT, i0);
+      break;
+    }
+    const double lmax = __longlong_as_double((long long)__ldcg(&a.S->lam_slots[(a.slot0 + s) % 3]));
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.S->lam_slots[(a.slot0 + s + 2) % 3] = 0ull;  // all have read it
+    if ((int)threadIdx.x < 2 * kEdge) {  // the neighbours' cells beside this block's, as run1_f64_kernel
+      const int side = threadIdx.x >= kEdge, r = threadIdx.x - side * kEdge;
+      const int nb = (int)blockIdx.x + (side ? 1 : -1);
+      const double* const theirs = a.edge + (size_t)((s & 1) * gridDim.x + nb) * 2 * kEdge;
+      const bool end = nb < 0 || nb >= (int)gridDim.x;
+      sh[r][side ? cells + 1 : 0] = end ? sh[r][side ? cells : 1] : __ldcg(&theirs[side ? r : kEdge + r]);
+    }
+    StepScalars sc{0.0, 0.0, 0.0};
+    if (threadIdx.x >= 96 || lxf) sc = step_scalars64(k, a.cfl, a.dx, lmax, lxf);  // (a warp that loads no halo)
+    if (threadIdx.x == 96) {
+      s_hdt = 0.5 * sc.dtdx;
+      s_t = t + sc.dt;
+    }
+    __syncthreads();
+    double f2[7];
+    auto faces = [&](auto first) {  // the face between slots j and j + 1, as face_twice
+      double lf = sc.lam_lxf;
+      if (!lxf) {
+        const double la = sh[kEdge - 1][j], lb = sh[kEdge - 1][j + 1];
+        lf = bits_of(la) > bits_of(lb) && !is_nan64(la) ? la : lb;
+      }
+#pragma unroll
+      for (int u = 0; u < 7; ++u) {
+        const int v = decltype(first)::value + u, sl = flux_slot1(v);
+        const double dq = sub64(k, sh[v][j + 1], sh[v][j]);
+        f2[u] = sl >= 0 ? __fma_rn(-lf, dq, add64(k, sh[14 + sl][j], sh[14 + sl][j + 1])) : mul64(k, -lf, dq);
+        sF[v][j] = f2[u];
+      }
+    };
+    if (j <= cells) {
+      if (half)
+        faces(std::integral_constant<int, 7>{});
+      else
+        faces(std::integral_constant<int, 0>{});
+    }
+    t = s_t;
+    const double hdt = s_hdt;
+    __syncthreads();
+    if (own && !frozen)
+#pragma unroll
+      for (int u = 0; u < 7; ++u) {
+        const int v = u + 7 * half;
+        sh[v][j + 1] = __fma_rn(-hdt, sub64(k, sF[v][j + 1], f2[u]), sh[v][j + 1]);
+      }
+  }
+  if (own && s > 0) {  // (each thread its own variables)
+    double* const Qn = a.out[s & 1];
+#pragma unroll
+    for (int u = 0; u < 7; ++u) Qn[(u + 7 * half) * n + i] = sh[u + 7 * half][j + 1];
+  }
+  run1_finish(a, t, s);
+}
+
+// (the split kernel's blocks are the smaller ones)
+size_t run1_edge_doubles(int64_t n) { return (size_t)((n + kSplitCells - 1) / kSplitCells) * 4 * kEdge; }
 bool run1_fits(int64_t n, int sms) { return (n + kCells64 - 1) / kCells64 <= sms; }
 
 cudaError_t launch_run1(cudaStream_t s, Run1Args a, EosC e) {
   Eos64 k = make_eos64(e);
   void* args[] = {&a, &e, &k};
+  const unsigned split = (unsigned)((a.n + kSplitCells - 1) / kSplitCells);
+  if (split <= (unsigned)a.sms) {
+    const void* kern = e.default_exp ? (const void*)run1_split_f64_kernel<1> : (const void*)run1_split_f64_kernel<0>;
+    return cudaLaunchCooperativeKernel(kern, dim3(split), dim3(2 * kSplitSlots), args, 0, s);
+  }
   const void* kern = e.default_exp ? (const void*)run1_f64_kernel<1> : (const void*)run1_f64_kernel<0>;
   return cudaLaunchCooperativeKernel(kern, dim3((unsigned)((a.n + kCells64 - 1) / kCells64)), dim3(kBlock64), args, 0,
                                      s);
@@ -329,6 +489,7 @@ cudaError_t launch_run1_f64(hyp_ctx* c, long long k, int max_steps, double t_end
   a.flux = c->cfg.flux;
   a.bc = ctx_bc(c);
   a.tries = kRunTries;
+  a.sms = c->sms;
   a.S = c->st;
   return launch_run1(c->stream, a, c->eos[0]);
 }

@@ -16,7 +16,7 @@ def state(hyp, n, seed=3):
     return eos, C.segment_fill(hyp.Hyperelasticity.prim2cons(eos, C.segment_states(eos, 8, seed=seed)), n)
 
 
-@pytest.mark.parametrize("n", [3, 127, 128, 300, 19304, 19305])  # 19304: the last of one launch on 152 SMs
+@pytest.mark.parametrize("n", [3, 63, 64, 127, 128, 300, 9576, 9577, 19304, 19305])  # 9576, 19304: the last of each form of one launch on 152 SMs
 @pytest.mark.parametrize("flux,bc", [("rusanov", "frozen"), ("lxf", "transmissive")])
 def test_cuts_agree(hyp, n, flux, bc):
     eos, Q0 = state(hyp, n)
