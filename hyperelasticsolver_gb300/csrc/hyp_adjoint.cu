@@ -158,9 +158,9 @@ __global__ void __launch_bounds__(256) adj_dtdx_kernel(AdjArgs g) {
 // differences shared between the face terms, dt/dx on one warp of a block and integer
 // zero tests: 880 -> about 560 FP64 instructions a cell; 65,536 cells, 50 steps with record
 // and recompute 11.4 -> 9.5 ms. With every operator an FMA on registers and the wave
-// speeds' terms only in warps that have one 8.09 -> 7.64 ms; with lone products on the integer
-// pipe (kSoft) 7.37 to 7.6 at the two blocks a multiprocessor that its registers allow, held
-// to three and four blocks 8.26 and 7.49 for the spills.
+// speeds' terms only in warps that have one 8.09 -> 7.61 ms; with lone products on the integer
+// pipe (kSoft) 7.44 at the two blocks a multiprocessor that its registers allow, held to
+// three and four blocks 8.18 and 7.53 for the spills.
 template <int kDef, bool kSoft>
 __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, Eos64 kc) {
   __shared__ double sh[kAdjBlock / 32];

@@ -209,22 +209,13 @@ HYP_HD int cell_vjp64(const EosC& e, const Eos64& k, const double* q, const doub
                       EosBar& eb) {
   const typename std::conditional<kSoft, Soft64, Plain64>::type s(k);
   if (!kSoft) return cell_vjp_of64<kDef>(e, s, q, fb, lb, qb, eb);
-  double qs[14], qa[14], fs[14];
+  double qs[14];
   for (int v = 0; v < 14; ++v) qs[v] = qb[v];
   EosBar es = eb;
   const int st = cell_vjp_of64<kDef>(e, s, q, fb, lb, qs, es);
   if (s.out_of_range()) {
-    double qo[14];
-    for (int v = 0; v < 14; ++v) {
-      qa[v] = q[v];
-      fs[v] = fb[v];
-      qo[v] = qb[v];
-    }
-    EosBar eo = eb;
-    const int plain = cell_vjp_plain64<kDef>(e, k, qa, fs, lb, qo, eo);
-    for (int v = 0; v < 14; ++v) qb[v] = qo[v];
-    eb = eo;
-    return plain;
+    const Eos64 kc = k;  // (the constants' registers have no address)
+    return cell_vjp_plain64<kDef>(e, kc, q, fb, lb, qb, eb);
   }
   for (int v = 0; v < 14; ++v) qb[v] = qs[v];
   eb = es;
