@@ -155,7 +155,7 @@ extern "C" int hyp_create(const hyp_config* cfg, hyp_ctx** out) {
     if (rc == HYP_OK && (e = cudaMalloc(&c->smax, (size_t)c->n * sizeof(double))) != cudaSuccess) fail(e, "cudaMalloc(smax)");
     if (rc == HYP_OK && (e = cudaMalloc(&c->DM, nfb)) != cudaSuccess) fail(e, "cudaMalloc(DM)");
     if (rc == HYP_OK && (e = cudaMalloc(&c->DP, nfb)) != cudaSuccess) fail(e, "cudaMalloc(DP)");
-    if (rc == HYP_OK && (e = cudaMalloc(&c->face_list, (size_t)(c->n + 1) * sizeof(int))) != cudaSuccess)
+    if (rc == HYP_OK && (e = cudaMalloc(&c->face_list, (size_t)face_list_ints(c->n) * sizeof(int))) != cudaSuccess)
       fail(e, "cudaMalloc(face list)");
     if (rc == HYP_OK && cfg->flux == HYP_FLUX_HLL &&
         (e = cudaMalloc(&c->face_s, (size_t)2 * (c->n + 1) * sizeof(double))) != cudaSuccess)

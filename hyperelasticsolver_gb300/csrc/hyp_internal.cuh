@@ -156,7 +156,8 @@ struct hyp_ctx {
   double* smax = nullptr;
   double* DM = nullptr;
   double* DP = nullptr;
-  int* face_list = nullptr;   // two-phase FP64: listed faces [n+1], and (HLL) their s_l, s_r [2][n+1]
+  // two-phase FP64: listed faces [n+1] and a mark per face block, and (HLL) s_l, s_r [2][n+1]
+  int* face_list = nullptr;
   double* face_s = nullptr;
   int sms = 0;                // multiprocessors of the device
   int coop = 0;               // it runs cooperative launches
@@ -291,6 +292,7 @@ cudaError_t launch_step1_mixed(hyp_ctx* c, long long k, double t_end);
 cudaError_t launch_cell2_f64(hyp_ctx* c, int p, unsigned long long* lam_slot, const double* t_now, double t_end);
 cudaError_t launch_face2_f64(hyp_ctx* c, int p, const unsigned long long* rd, double t_end);
 cudaError_t launch_update2_f64(hyp_ctx* c, long long k, double t_end);
+int64_t face_list_ints(int64_t n);  // of hyp_ctx::face_list
 cudaError_t launch_run_step2_f64(hyp_ctx* c, long long k, double t_end, bool first, bool last);
 // two-phase pressure relaxation of the state the step of parity p wrote (hyp_relax.cu)
 cudaError_t launch_relax2(hyp_ctx* c, int p, double t_end);
