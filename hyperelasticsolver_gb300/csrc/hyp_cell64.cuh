@@ -43,7 +43,8 @@
 //    65536 cells x 10 steps 7.10 -> 6.51 ms, two phases of 1000 cells x 50 steps 2.25 -> 2.17
 //    ms, 65536 cells x 50 steps forward and back 9.55 -> 8.69 ms.
 //
-// Per cell 180 FP64 instructions as executed, where the forms of hyp_physics.cuh
+// Per cell 183 FP64 instructions as executed (106 with the lone products on the integer
+// pipe, soft_mul64), where the forms of hyp_physics.cuh
 // (which the adjoint and the function-level evaluators use) execute 379; the two agree
 // to a few ulps (tests/test_cell64_host.py).
 #pragma once
