@@ -154,15 +154,94 @@ __global__ void __launch_bounds__(256) adj_dtdx_kernel(AdjArgs g) {
   }
 }
 
+// Cell i of an adjoint step: Qb0 of it and what it adds to eb; r and lamb_max: dt/dx and the
+// adjoint of the max wave speed; lanes: the warp's lanes that call it together (0: the lane is
+// on its own); form: the compact forms with the hardware's products or lone ones on the integer
+// pipe, or the general form. Returns what is left to do (hyp_adjoint64.cuh).
+enum { kFormPlain, kFormSoft, kFormGeneral };
+template <int kDef, int kForm>
+__device__ __forceinline__ int adj_cell(const AdjArgs& g, const EosC& e, const Eos64& k64, int64_t i, double r,
+                                        double lamb_max, unsigned lanes, EosBar& eb) {
+  const int64_t n = g.n;
+  const int64_t il = i > 0 ? i - 1 : 0, ir = i < n - 1 ? i + 1 : n - 1;
+  const bool ui = updated(i, n, g.trans);
+  const bool ul = il != i && updated(il, n, g.trans), ur = ir != i && updated(ir, n, g.trans);
+  const double li = g.lam[i], ll = g.lam[il], lr = g.lam[ir];
+  const bool takeL = !(ll > li);  // the left face took lambda_i
+  const bool takeR = li > lr;     // the right face took lambda_i
+  // where the wave speed is monotone one of the two holds for a whole warp
+  const bool hasL = il != i && takeL, hasR = ir != i && takeR;
+  const bool anyL = lanes ? __any_sync(lanes, hasL) : hasL, anyR = lanes ? __any_sync(lanes, hasR) : hasR;
+  // face adjoints Fb = r (Qb1_R - Qb1_L): half goes to each cell's flux (all of it to
+  // the cell beside a ghost, whose face is its flux), -+ lambda/2 to the state
+  const double cL = il != i ? 0.5 * r : r, cR = ir != i ? 0.5 * r : r;
+  const double hL = il != i ? -(0.5 * r) * face_lambda(ll, li) : 0.0;
+  const double hR = ir != i ? (0.5 * r) * face_lambda(li, lr) : 0.0;
+  double q[14], qb[14], fb[14];
+  double lamb = (int)i == *g.amax_rd ? lamb_max : 0.0;
+  double dL = 0.0, dR = 0.0;
+  unsigned long long any = 0ull;
+#pragma unroll
+  for (int v = 0; v < 14; ++v) {
+    const double qc = g.Q[v * n + i];
+    q[v] = qc;
+    const double bc = g.Qb1[v * n + i], bi = ui ? bc : 0.0;
+    const double gL = sub64(k64, bi, ul ? g.Qb1[v * n + il] : 0.0);
+    const double gR = sub64(k64, ur ? g.Qb1[v * n + ir] : 0.0, bi);
+    qb[v] = fma(hR, gR, fma(hL, gL, bc));
+    if (anyL) dL = fma(gL, sub64(k64, qc, g.Q[v * n + il]), dL);
+    if (anyR) dR = fma(gR, sub64(k64, g.Q[v * n + ir], qc), dR);
+    if (flux_slot1(v) >= 0) {
+      fb[v] = fma(cR, gR, mul64(k64, cL, gL));
+      any |= (unsigned long long)bits_of(fb[v]) << 1;
+    } else {
+      fb[v] = 0.0;
+    }
+  }
+  if (hasL) lamb -= (0.5 * r) * dL;
+  if (hasR) lamb -= (0.5 * r) * dR;
+  any |= (unsigned long long)bits_of(lamb) << 1;
+  // where the face adjoints vanish (a region where the adjoint field is constant) the
+  // VJP adds exact zeros: skip it
+  int left = kVjpDone, st;
+  if (any) {
+    if (kForm == kFormGeneral)
+      cell_vjp(e, q, fb, lamb, qb, eb);
+    else
+      left = cell_vjp_try64<kDef, kForm == kFormSoft>(e, k64, q, fb, lamb, qb, eb, st);
+  }
+#pragma unroll
+  for (int v = 0; v < 14; ++v) g.Qb0[v * n + i] = qb[v];
+  return left;
+}
+
+// What a cell left to do, out of line.
+template <int kDef>
+static __device__ __noinline__ EosBar adj_cell_again(const AdjArgs& g, const EosC& e, const Eos64& kc, int64_t i, double r,
+                                                     double lamb_max, int left) {
+  const Eos64 k = in_registers64(kc);
+  EosBar eb{0.0, 0.0};
+  if (left == kVjpPlain) left = adj_cell<kDef, kFormPlain>(g, e, k, i, r, lamb_max, 0u, eb);
+  if (left == kVjpGeneral) {
+    eb = EosBar{0.0, 0.0};
+    adj_cell<kDef, kFormGeneral>(g, e, k, i, r, lamb_max, 0u, eb);
+  }
+  return eb;
+}
+
 // What bounds it: FP64 issue (hyp_cell64.cuh). The VJP on the compact forms, masked
 // differences shared between the face terms, dt/dx on one warp of a block and integer
 // zero tests: 880 -> about 560 FP64 instructions a cell; 65,536 cells, 50 steps with record
 // and recompute 11.4 -> 9.5 ms. With every operator an FMA on registers and the wave
 // speeds' terms only in warps that have one 8.09 -> 7.61 ms; with lone products on the integer
 // pipe (kSoft) 7.44 at the two blocks a multiprocessor that its registers allow, held to
-// three and four blocks 8.18 and 7.53 for the spills.
+// three and four blocks 8.18 and 7.53 for the spills. A step of 65,536 cells with a dense
+// adjoint 79 us in a short run and 154 after 1000 steps, when the tails' cells went through
+// the forms three times; 78 and 78 since they are told by their state and evaluated once.
 template <int kDef, bool kSoft>
-__global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, Eos64 kc) {
+__global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(const __grid_constant__ AdjArgs g,
+                                                             const __grid_constant__ EosC e,
+                                                             const __grid_constant__ Eos64 kc) {
   __shared__ double sh[kAdjBlock / 32];
   __shared__ double s_lamb_max, s_r;
   const Eos64 k64 = in_registers64(kc);
@@ -184,49 +263,8 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(AdjArgs g, EosC e, 
   EosBar eb{0.0, 0.0};
   const unsigned lanes = __ballot_sync(0xffffffffu, i < n);
   if (i < n) {
-    const double r = s_r;
-    const int64_t il = i > 0 ? i - 1 : 0, ir = i < n - 1 ? i + 1 : n - 1;
-    const bool ui = updated(i, n, g.trans);
-    const bool ul = il != i && updated(il, n, g.trans), ur = ir != i && updated(ir, n, g.trans);
-    const double li = g.lam[i], ll = g.lam[il], lr = g.lam[ir];
-    const bool takeL = !(ll > li);  // the left face took lambda_i
-    const bool takeR = li > lr;     // the right face took lambda_i
-    // where the wave speed is monotone one of the two holds for a whole warp
-    const bool anyL = __any_sync(lanes, il != i && takeL), anyR = __any_sync(lanes, ir != i && takeR);
-    // face adjoints Fb = r (Qb1_R - Qb1_L): half goes to each cell's flux (all of it to
-    // the cell beside a ghost, whose face is its flux), -+ lambda/2 to the state
-    const double cL = il != i ? 0.5 * r : r, cR = ir != i ? 0.5 * r : r;
-    const double hL = il != i ? -(0.5 * r) * face_lambda(ll, li) : 0.0;
-    const double hR = ir != i ? (0.5 * r) * face_lambda(li, lr) : 0.0;
-    double q[14], qb[14], fb[14];
-    double lamb = (int)i == *g.amax_rd ? s_lamb_max : 0.0;
-    double dL = 0.0, dR = 0.0;
-    unsigned long long any = 0ull;
-#pragma unroll
-    for (int v = 0; v < 14; ++v) {
-      const double qc = g.Q[v * n + i];
-      q[v] = qc;
-      const double bc = g.Qb1[v * n + i], bi = ui ? bc : 0.0;
-      const double gL = sub64(k64, bi, ul ? g.Qb1[v * n + il] : 0.0);
-      const double gR = sub64(k64, ur ? g.Qb1[v * n + ir] : 0.0, bi);
-      qb[v] = fma(hR, gR, fma(hL, gL, bc));
-      if (anyL) dL = fma(gL, sub64(k64, qc, g.Q[v * n + il]), dL);
-      if (anyR) dR = fma(gR, sub64(k64, g.Q[v * n + ir], qc), dR);
-      if (flux_slot1(v) >= 0) {
-        fb[v] = fma(cR, gR, mul64(k64, cL, gL));
-        any |= (unsigned long long)bits_of(fb[v]) << 1;
-      } else {
-        fb[v] = 0.0;
-      }
-    }
-    if (il != i && takeL) lamb -= (0.5 * r) * dL;
-    if (ir != i && takeR) lamb -= (0.5 * r) * dR;
-    any |= (unsigned long long)bits_of(lamb) << 1;
-    // where the face adjoints vanish (a region where the adjoint field is constant) the
-    // VJP adds exact zeros: skip it
-    if (any) cell_vjp64<kDef, kSoft>(e, k64, q, fb, lamb, qb, eb);
-#pragma unroll
-    for (int v = 0; v < 14; ++v) g.Qb0[v * n + i] = qb[v];
+    const int left = adj_cell<kDef, kSoft ? kFormSoft : kFormPlain>(g, e, k64, i, s_r, s_lamb_max, lanes, eb);
+    if (left) eb = adj_cell_again<kDef>(g, e, kc, i, s_r, s_lamb_max, left);
   }
   const double b0 = block_sum<kAdjBlock>(eb.b0sq, sh);
   const double k0 = block_sum<kAdjBlock>(eb.k0, sh);

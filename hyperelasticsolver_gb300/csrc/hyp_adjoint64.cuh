@@ -16,19 +16,15 @@
 
 namespace hyp {
 
-// Out of line: cells whose top eigenvalue does not stand clear.
-#ifdef __CUDACC__
-static __host__ __device__ __noinline__
-#else
-inline
-#endif
-int cell_vjp_general(const EosC& e, const double* q, const double* fb, double lb, double* qb, EosBar& eb) {
-  return cell_vjp(e, q, fb, lb, qb, eb);
-}
+// What an evaluation on the compact forms leaves to do: nothing; the same with the hardware's
+// products (cell_try64); the general form (cell_vjp), for a top eigenvalue that does not stand
+// clear. In the last two cases qb and eb mean nothing. A kernel does either out of line with
+// its inputs loaded again: called from here they would lie in local memory in every cell.
+enum { kVjpDone = 0, kVjpPlain = 1, kVjpGeneral = 2 };
 
 template <int kDef, class K>
 HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const double* fb, double lb, double* qb,
-                         EosBar& eb) {
+                         EosBar& eb, int& st) {
   auto M = [&k](double x, double y) { return mul64(k, x, y); };
   auto A = [&k](double x, double y) { return add64(k, x, y); };
   auto S = [&k](double x, double y) { return sub64(k, x, y); };
@@ -38,6 +34,7 @@ HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const doubl
   };
   const double *m = q + 1, *R = q + 5;
   const Cell64 c = cell64<kDef, true>(e, k, 1.0, m, q[4], R);
+  st = c.st;
   const double r = c.inv_den, ms = k.inv_rho0sq;
   const double i1 = A(A(c.G00, c.G11), c.G22), th = M(k.third, i1);
   const double d0 = S(c.G00, th), d1 = S(c.G11, th), d2 = S(c.G22, th);
@@ -59,7 +56,7 @@ HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const doubl
     const double o11 = fma(f1, c.G01, fma(c.a, c.G11, -c.bM)), o22 = fma(f2, c.G02, fma(c.a, c.G22, -c.bM));
     const double o12 = fma(f1, c.G02, M(c.a, c.G12));
     double nu;
-    if (!top_root64(k, o00, o11, o22, o01, o02, o12, nu)) return cell_vjp_general(e, q, fb, lb, qb, eb);
+    if (!top_root64(k, o00, o11, o22, o01, o02, o12, nu)) return out_of_range(k) ? kVjpPlain : kVjpGeneral;
     u0b = c.u[0] > 0.0 ? lb : (c.u[0] < 0.0 ? -lb : 0.0);
     // d nu / d O = Cof(nu I - O) / its trace; an off-diagonal entry stands for two
     const double b00 = S(nu, o00), b11 = S(nu, o11), b22 = S(nu, o22);
@@ -188,37 +185,37 @@ HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const doubl
     qb[6 + 3 * b] = A(qb[6 + 3 * b], fma(db, fma(x[2], y[0], -M(x[0], y[2])), fma(N12, r2, fma(N11, r1, fma(N01, r0, Rb[3 * b + 1])))));
     qb[7 + 3 * b] = A(qb[7 + 3 * b], fma(db, fma(x[0], y[1], -M(x[1], y[0])), fma(N22, r2, fma(N12, r1, fma(N02, r0, Rb[3 * b + 2])))));
   }
-  return c.st;
-}
-
-// With the hardware's products, out of line (cell_plain64).
-template <int kDef>
-#ifdef __CUDACC__
-static __host__ __device__ __noinline__
-#else
-inline
-#endif
-int cell_vjp_plain64(const EosC& e, const Eos64& k, const double* q, const double* fb, double lb, double* qb,
-                     EosBar& eb) {
-  return cell_vjp_of64<kDef>(e, k, q, fb, lb, qb, eb);
+  return out_of_range(k) || (std::is_same<K, Soft64>::value && st) ? kVjpPlain : kVjpDone;
 }
 
 // kSoft: lone products on the integer pipe (hyp_cell64.cuh), the same values bit for bit.
 template <int kDef, bool kSoft>
+HYP_HD int cell_vjp_try64(const EosC& e, const Eos64& k, const double* q, const double* fb, double lb, double* qb,
+                          EosBar& eb, int& st) {
+  if (kSoft && !(soft_inputs64(q + 1, 13) & soft_inputs64(fb, 14) & soft_inputs64(&lb, 1))) return kVjpPlain;
+  return cell_vjp_of64<kDef>(e, typename std::conditional<kSoft, Soft64, Plain64>::type(k), q, fb, lb, qb, eb, st);
+}
+
+// All of it; returns the status.
+template <int kDef, bool kSoft>
 HYP_HD int cell_vjp64(const EosC& e, const Eos64& k, const double* q, const double* fb, double lb, double* qb,
                       EosBar& eb) {
-  const typename std::conditional<kSoft, Soft64, Plain64>::type s(k);
-  if (!kSoft) return cell_vjp_of64<kDef>(e, s, q, fb, lb, qb, eb);
   double qs[14];
   for (int v = 0; v < 14; ++v) qs[v] = qb[v];
-  EosBar es = eb;
-  const int st = cell_vjp_of64<kDef>(e, s, q, fb, lb, qs, es);
-  if (s.out_of_range()) {
-    const Eos64 kc = k;  // (the constants' registers have no address)
-    return cell_vjp_plain64<kDef>(e, kc, q, fb, lb, qb, eb);
+  const EosBar es = eb;
+  auto restore = [&] {
+    for (int v = 0; v < 14; ++v) qb[v] = qs[v];
+    eb = es;
+  };
+  int st, left = cell_vjp_try64<kDef, kSoft>(e, k, q, fb, lb, qb, eb, st);
+  if (left == kVjpPlain) {
+    restore();
+    left = cell_vjp_try64<kDef, false>(e, k, q, fb, lb, qb, eb, st);
   }
-  for (int v = 0; v < 14; ++v) qb[v] = qs[v];
-  eb = es;
+  if (left == kVjpGeneral) {
+    restore();
+    st = cell_vjp(e, q, fb, lb, qb, eb);
+  }
   return st;
 }
 

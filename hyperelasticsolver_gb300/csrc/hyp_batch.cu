@@ -180,14 +180,15 @@ __global__ void __launch_bounds__(kBlock) batch_join_kernel(const float* __restr
 // the cell pass and the tile's maximum into its problem's slot.
 template <int kDef, bool kSoft>
 __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64_cell_kernel(
-    const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc, double* __restrict__ F, double* __restrict__ lam,
+    const double* __restrict__ Q, int64_t n, const __grid_constant__ EosC e, const __grid_constant__ Eos64 kc,
+    double* __restrict__ F, double* __restrict__ lam,
     const TileDesc* __restrict__ tiles, BatchDev b, int par, double t_end, unsigned long long* slot_base, DevState* S) {
   const TileDesc d = tiles[blockIdx.x];
   if (!(b.t[par * b.P + d.problem] < t_end)) return;
   const Eos64 k = in_registers64(kc);
   const int64_t i = d.first + threadIdx.x;
   const bool own = threadIdx.x < kCells64 && i < d.hi;
-  const double l = own ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = own ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, kc, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(&slot_base[d.problem], m);
 }
@@ -198,8 +199,8 @@ __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64
 // clears all three: whatever steps it next starts with a cell pass).
 template <int kDef, bool kCell, bool kSoft>
 __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64_step_kernel(
-    const double* __restrict__ Q, double* __restrict__ Qn, int64_t n, EosC e, Eos64 kc, const double* __restrict__ F,
-    const double* __restrict__ lam, double* __restrict__ Fn, double* __restrict__ lamn,
+    const double* __restrict__ Q, double* Qn, int64_t n, const __grid_constant__ EosC e,
+    const __grid_constant__ Eos64 kc, const double* __restrict__ F, const double* __restrict__ lam, double* __restrict__ Fn, double* __restrict__ lamn,
     const TileDesc* __restrict__ tiles, BatchDev b, int par, int rd, int wr, int clr, double t_end, double cfl,
     int flux, int bc, DevState* S) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell first + k
@@ -252,7 +253,7 @@ __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) batch_f64
     }
   }
   if (!kCell || !s_more) return;
-  const double l = own ? cell1_pass<kDef, kSoft>(q, n, i, e, k, Fn, lamn, S) : 0.0;
+  const double l = own ? cell1_pass<kDef, kSoft>(q, Qn, n, i, e, kc, k, Fn, lamn, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (j == 0) atomicMax(&b.slots[wr * P + p], m);
 }

@@ -187,9 +187,10 @@ HYP_HD Eos64 make_eos64(const EosC& e) {
 // x y on the integer pipe, rounded to nearest even as the FP64 pipe does: the product of
 // the 53-bit significands from four 32 x 32-bit products, one shift to 53 bits, and the
 // rounding carried into the exponent. worst collects the largest distance of a product's
-// exponent sum from the low end of what this holds for (operands with a zero exponent
-// count as zeros); beyond kSoftWide some product overflowed, underflowed, or had an
-// infinity or NaN for a factor, and the caller takes the hardware's products instead.
+// exponent sum from the low end of what this holds for; beyond kSoftWide some product
+// overflowed or underflowed. Factors of a zero exponent count as zeros, of the largest one
+// as numbers: subnormal, infinite and NaN ones are what soft_inputs64 and the callers' check
+// of status and result are for (cell_try64).
 // About 50 instructions and 62 cycles of a scheduler's issue, but none of its FP64 pipe:
 // 16 register FMAs take a warp 1029 cycles, 8 and 8 of these together 545 (4 warps a
 // scheduler) or 732 (a single warp).
@@ -236,13 +237,32 @@ HYP_HD double soft_mul64(double x, double y, unsigned& worst) {
 // The constants for forms whose lone products run on the FP64 pipe, and on the integer pipe.
 struct Plain64 : Eos64 {
   HYP_HD explicit Plain64(const Eos64& k) : Eos64(k) {}
-  HYP_HD bool out_of_range() const { return false; }
 };
 struct Soft64 : Eos64 {
   mutable unsigned worst;
   HYP_HD explicit Soft64(const Eos64& k) : Eos64(k), worst(0u) {}
-  HYP_HD bool out_of_range() const { return worst > kSoftWide; }
 };
+HYP_HD bool out_of_range(const Eos64&) { return false; }
+HYP_HD bool out_of_range(const Soft64& k) { return k.worst > kSoftWide; }
+
+// Whether n values are what the forms may take on the integer pipe: zeros, or 2^-250 to 2^251
+// in size. The tail of a wave has others: its components shrink by a factor a cell, down to
+// zero, and squares of them leave the range of a double. A tail's cells are told here, by
+// their state, before anything is evaluated: after 200 to 1000 steps of a run they had taken
+// the integer products, a general form on their results and then the hardware's products
+// (two phases, 40,000 cells, 500 steps 89 -> 74 us a step; the adjoint of 65,536 cells
+// 154 -> 78). Each product that fails by itself on the FP64 pipe, where it is met, was no
+// way: its 79 branches keep the compiler from mixing the two pipes' instructions (1,000,003
+// cells 332 -> 437 us a step).
+HYP_HD bool soft_inputs64(const double* x, int n) {
+  constexpr unsigned lo = (1023u - 250u) << 21, wide = 501u << 21;
+  bool in = true;
+  for (int v = 0; v < n; ++v) {
+    const unsigned long long b = (unsigned long long)bits_of(x[v]) << 1;
+    in &= (unsigned)(b >> 32) - lo < wide || b == 0ull;
+  }
+  return in;
+}
 
 // x y, x + y, x - y: on the FP64 pipe, products by a Soft64 on the integer pipe.
 HYP_HD double mul64(const Soft64& k, double x, double y) { return soft_mul64(x, y, k.worst); }
@@ -468,6 +488,7 @@ HYP_HD double cmax64(const EosC& e, const K& k, const Cell64& c) {
   const double o12 = fma(f1, c.G02, M(c.a, c.G12));
   double rt;
   if (top_root64(k, o00, o11, o22, o01, o02, o12, rt)) return sqrt64(k, add64(k, rt, rt));
+  if (out_of_range(k)) return 0.0;  // O means nothing; the cell is evaluated again
   return sqrt(radius_general(o00, o11, o22, o01, o02, o12));
 }
 
@@ -491,44 +512,38 @@ HYP_HD void flux64(const K& k, double alpha, const Cell64& c, const double* m, c
   }
 }
 
-// All of a cell's forms with the hardware's products, out of line: for cells whose products
-// leave soft_mul64's range, which have to come out as the FP64 pipe makes them. q: m, rE,
-// R; out: flux (14), u1, c_max.
-template <int kDef, bool kUnit>
-#ifdef __CUDACC__
-static __host__ __device__ __noinline__
-#else
-inline
-#endif
-int cell_plain64(const EosC& e, const Eos64& k, double alpha, const double* q, double* out) {
-  const Cell64 c = cell64<kDef, kUnit>(e, k, kUnit ? 1.0 : rcp64(k, alpha), q, q[3], q + 4);
-  flux64<kUnit>(k, alpha, c, q, q + 4, out);
-  out[14] = c.u[0];
-  out[15] = cmax64<kDef>(e, k, c);
-  return c.st;
-}
-
 // One phase of a cell: status, u1, c_max and with kFlux the flux; kSoft: lone products on
-// the integer pipe, the same values bit for bit.
+// the integer pipe, the same values bit for bit. False where those are not held for: a state
+// or product out of their range, or a bad cell; the results then mean nothing, and the caller
+// evaluates the cell with the hardware's products. A kernel does so out of line with the
+// state loaded again, so that nothing of the ordinary path is kept for it.
 template <int kDef, bool kUnit, bool kFlux, bool kSoft>
-HYP_HD int cell_speed64(const EosC& e, const Eos64& k, double alpha, const double* m, double rE, const double* R,
-                        double* f, double& u1, double& cm) {
+HYP_HD bool cell_try64(const EosC& e, const Eos64& k, double alpha, const double* m, double rE, const double* R,
+                       double* f, double& u1, double& cm, int& st) {
+  if (kSoft && !(soft_inputs64(m, 3) & soft_inputs64(&rE, 1) & soft_inputs64(R, 9) & (kUnit || soft_inputs64(&alpha, 1))))
+    return false;
   const typename std::conditional<kSoft, Soft64, Plain64>::type s(k);
   const Cell64 c = cell64<kDef, kUnit>(e, s, kUnit ? 1.0 : rcp64(k, alpha), m, rE, R);
   if (kFlux) flux64<kUnit>(s, alpha, c, m, R, f);
   u1 = c.u[0];
   cm = cmax64<kDef>(e, s, c);
-  if (!kSoft || !s.out_of_range()) return c.st;
-  double q[13], out[16];
-  for (int v = 0; v < 3; ++v) q[v] = m[v];
-  q[3] = rE;
-  for (int v = 0; v < 9; ++v) q[4 + v] = R[v];
-  const int st = cell_plain64<kDef, kUnit>(e, k, alpha, q, out);
-  if (kFlux)
-    for (int v = 0; v < 14; ++v) f[v] = out[v];
-  u1 = out[14];
-  cm = out[15];
+  st = c.st;
+  return !kSoft || (!out_of_range(s) && !st && is_finite64(cm));
+}
+
+// The same with the second evaluation in it. cell_plain64: with the hardware's products, q
+// m, rE, R and out flux (14), u1, c_max.
+template <int kDef, bool kUnit, bool kFlux, bool kSoft>
+HYP_HD int cell_speed64(const EosC& e, const Eos64& k, double alpha, const double* m, double rE, const double* R,
+                        double* f, double& u1, double& cm) {
+  int st;
+  if (!cell_try64<kDef, kUnit, kFlux, kSoft>(e, k, alpha, m, rE, R, f, u1, cm, st))
+    cell_try64<kDef, kUnit, kFlux, false>(e, k, alpha, m, rE, R, f, u1, cm, st);
   return st;
+}
+template <int kDef, bool kUnit>
+HYP_HD int cell_plain64(const EosC& e, const Eos64& k, double alpha, const double* q, double* out) {
+  return cell_speed64<kDef, kUnit, true, false>(e, k, alpha, q, q[3], q + 4, out, out[14], out[15]);
 }
 
 }  // namespace hyp

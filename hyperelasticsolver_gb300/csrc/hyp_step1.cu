@@ -22,14 +22,16 @@ namespace hyp {
 // 10.48 ms with the general forms, 7.26 ms with these; 1000 cells, 100 steps: 4.14 ms at 256
 // threads a block with the general forms, 2.38 ms.
 template <int kDef, bool kSoft>
-__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) cell1_f64_kernel(const double* __restrict__ Q, int64_t n, EosC e, Eos64 kc,
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) cell1_f64_kernel(const double* __restrict__ Q, int64_t n,
+                                                             const __grid_constant__ EosC e,
+                                                             const __grid_constant__ Eos64 kc,
                                                              double* __restrict__ F, double* __restrict__ lam,
                                                              unsigned long long* lam_slot, const double* t_now,
                                                              double t_end, DevState* S) {
   if (!(*t_now < t_end)) return;  // uniform across the grid
   const Eos64 k = in_registers64(kc);
   const int64_t i = (int64_t)blockIdx.x * kBlock64 + threadIdx.x;
-  const double l = i < n ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, k, F, lam, S) : 0.0;
+  const double l = i < n ? cell1_load_pass<kDef, kSoft>(Q, n, i, e, kc, k, F, lam, S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (threadIdx.x == 0) atomicMax(lam_slot, m);
 }
@@ -44,7 +46,8 @@ __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) cell1_f64
 // the state, and the fluxes alternate between two buffers: 1000 cells x 100 steps 1.59 -> 1.40
 // ms, 8192 cells x 4 steps on device buffers 129 -> 110 us, 1,000,003 cells unchanged (6.03 ms).
 template <int kDef, bool kCell, bool kSoft>
-__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) step1_f64_kernel(Step1Args a, EosC e, Eos64 kc) {
+__global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) step1_f64_kernel(Step1Args a, const __grid_constant__ EosC e,
+                                                                                    const __grid_constant__ Eos64 kc) {
   __shared__ double sF[14][kBlock64];  // twice the left face of cell i0 + k
   __shared__ double s_hdt;             // half dt/dx
   __shared__ int s_more;               // the state this step makes is stepped from
@@ -94,7 +97,7 @@ __global__ void __launch_bounds__(kBlock64, kSoft ? kSoftResident : 0) step1_f64
     }
   }
   if (!kCell || !s_more) return;
-  const double l = own ? cell1_pass<kDef, kSoft>(q, n, i, e, k, a.Fn, a.lamn, a.S) : 0.0;
+  const double l = own ? cell1_pass<kDef, kSoft>(q, a.Qn, n, i, e, kc, k, a.Fn, a.lamn, a.S) : 0.0;
   const unsigned long long m = block_max_bits<kBlock64>(l);
   if (j == 0) atomicMax(a.wr, m);
 }

@@ -40,26 +40,49 @@ struct CellOut2 {
   DevState* S;
 };
 
-// The cell pass of a block's 64 cells, a thread per phase in state q (15 values; `in`:
-// there is a cell): fluxes, speed bounds, and the block's max |speed| into slot. All
+// A phase's rows of F, u1 and c_max (returned) of cell i in state q (at Q too), with a bad
+// cell recorded; E: the kernel's parameter, k: its constants of the phase in registers.
+template <int kDef>
+static __device__ __noinline__ double2 cell2_again(const double* Q, int64_t i, int ph, const Eos2x& E, const CellOut2& o);
+template <int kDef, bool kSoft>
+__device__ __forceinline__ double2 cell2_phase(const double* q, const double* Q, int64_t i, int ph, const Eos2x& E,
+                                               const Eos64& k, const CellOut2& o) {
+  double f[14], u1, cm;
+  int st;
+  if (!cell_try64<kDef, false, true, kSoft>(E.e[ph], k, q[0], q + 2, q[5], q + 6, f, u1, cm, st) && kSoft)
+    return cell2_again<kDef>(Q, i, ph, E, o);
+  double* f0 = o.F + 15 * ph * o.n + i;
+#pragma unroll
+  for (int r = 1; r < 15; ++r)
+    if (!zero_flux_row(r)) f0[r * o.n] = f[r - 1];
+  if (st) record_err64(o.S, st, i);
+  return make_double2(u1, cm);
+}
+__device__ __forceinline__ void load_phase(const double* Q, int64_t n, int64_t i, int ph, double* q) {
+  const double* q0 = Q + 15 * ph * n + i;
+#pragma unroll
+  for (int r = 0; r < 15; ++r) q[r] = q0[r * n];
+}
+template <int kDef>
+static __device__ __noinline__ double2 cell2_again(const double* Q, int64_t i, int ph, const Eos2x& E, const CellOut2& o) {
+  double q[15];
+  load_phase(Q, o.n, i, ph, q);
+  return cell2_phase<kDef, false>(q, Q, i, ph, E, in_registers64(E.k, ph), o);
+}
+
+// The cell pass of a block's 64 cells, a thread per phase in state q (15 values, at Q too;
+// `in`: there is a cell): fluxes, speed bounds, and the block's max |speed| into slot. All
 // threads of the block call it.
 template <int kDef, bool kSoft>
-__device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, const EosC& e, const Eos64& k,
-                                           const CellOut2& o,
-                                           unsigned long long* slot) {
+__device__ __forceinline__ void cell2_pass(const double* q, const double* Q, bool in, int64_t i, const Eos2x& E,
+                                           const Eos64& k, const CellOut2& o, unsigned long long* slot) {
   __shared__ double s_lo[kPairCells], s_hi[kPairCells];
   const int ph = threadIdx.x / kPairCells, j = threadIdx.x % kPairCells;
   double lo = 0.0, hi = 0.0;
   if (in) {
-    double f[14], u1, cm;
-    const int st = cell_speed64<kDef, false, true, kSoft>(e, k, q[0], q + 2, q[5], q + 6, f, u1, cm);
-    double* f0 = o.F + 15 * ph * o.n + i;
-#pragma unroll
-    for (int r = 1; r < 15; ++r)
-      if (!zero_flux_row(r)) f0[r * o.n] = f[r - 1];
-    lo = sub64(k, u1, cm);
-    hi = add64(k, u1, cm);
-    if (st) record_err64(o.S, st, i);
+    const double2 s = cell2_phase<kDef, kSoft>(q, Q, i, ph, E, k, o);
+    lo = sub64(k, s.x, s.y);
+    hi = add64(k, s.x, s.y);
     if (ph == 1) {
       s_lo[j] = lo;
       s_hi[j] = hi;
@@ -80,7 +103,8 @@ __device__ __forceinline__ void cell2_pass(const double* q, bool in, int64_t i, 
 }
 
 template <int kDef, bool kSoft>
-__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) cell2_f64_kernel(const double* __restrict__ Q, Eos2x E, CellOut2 o,
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) cell2_f64_kernel(const double* __restrict__ Q, const __grid_constant__ Eos2x E,
+                                                            const __grid_constant__ CellOut2 o,
                                                             unsigned long long* lam_slot, const double* t_now,
                                                             double t_end) {
   if (!(*t_now < t_end)) return;
@@ -88,12 +112,8 @@ __global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) cell2_f64_
   const Eos64 k = in_registers64(E.k, ph);
   const int64_t i = (int64_t)blockIdx.x * kPairCells + threadIdx.x % kPairCells;
   double q[15];
-  if (i < o.n) {
-    const double* q0 = Q + 15 * ph * o.n + i;
-#pragma unroll
-    for (int r = 0; r < 15; ++r) q[r] = q0[r * o.n];
-  }
-  cell2_pass<kDef, kSoft>(q, i < o.n, i, E.e[ph], k, o, lam_slot);
+  if (i < o.n) load_phase(Q, o.n, i, ph, q);
+  cell2_pass<kDef, kSoft>(q, Q, i < o.n, i, E, k, o, lam_slot);
 }
 
 // ---- faces ---------------------------------------------------------------------
@@ -106,12 +126,43 @@ struct FaceList {
   double *sl, *sr;
 };
 
+// u1 and c_max of a phase at the midpoint of q_l = a and q_r = b (the forms are homogeneous, so
+// q_l + q_r serves), a bad state recorded with the right cell.
+template <int kDef>
+static __device__ __noinline__ double2 mid2_again(const double* Q, int64_t n, int64_t L, int64_t R, int ph, const Eos2x& E,
+                                                  DevState* S);
+template <int kDef, bool kSoft>
+__device__ __forceinline__ double2 mid2(const double* a, const double* b, const double* Q, int64_t n, int64_t L, int64_t R,
+                                        int ph, const Eos2x& E, const Eos64& k, DevState* S) {
+  double m[3], Rm[9];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) m[v] = add64(k, a[2 + v], b[2 + v]);
+#pragma unroll
+  for (int v = 0; v < 9; ++v) Rm[v] = add64(k, a[6 + v], b[6 + v]);
+  double u1, cm;
+  int st;
+  if (!cell_try64<kDef, false, false, kSoft>(E.e[ph], k, add64(k, a[0], b[0]), m, add64(k, a[5], b[5]), Rm, nullptr, u1,
+                                             cm, st) && kSoft)
+    return mid2_again<kDef>(Q, n, L, R, ph, E, S);
+  if (st) record_err64(S, st, R);
+  return make_double2(u1, cm);
+}
+template <int kDef>
+static __device__ __noinline__ double2 mid2_again(const double* Q, int64_t n, int64_t L, int64_t R, int ph, const Eos2x& E,
+                                                  DevState* S) {
+  double a[15], b[15];
+  load_phase(Q, n, L, ph, a);
+  load_phase(Q, n, R, ph, b);
+  return mid2<kDef, false>(a, b, Q, n, L, R, ph, E, in_registers64(E.k, ph), S);
+}
+
 // HLL faces: s_l, s_r and, where the volume fractions do not jump and no state on the
 // way between the cells (through Q_hll) can be singular, D- and D+ (doubles of the
 // formula of NumFluxes.jl:85-132 with its integrals zero). 186 slots a phase; the others are
 // listed.
 template <int kDef, bool kSoft>
-__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) face2_f64_kernel(const double* __restrict__ Q, int64_t n, Eos2x E,
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) face2_f64_kernel(const double* __restrict__ Q, int64_t n,
+                                                            const __grid_constant__ Eos2x E,
                                                             const double* __restrict__ F,
                                                             const double* __restrict__ smin,
                                                             const double* __restrict__ smax, double* __restrict__ DM,
@@ -149,18 +200,10 @@ __global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) face2_f64_
     for (int r = 0; r < 15; ++r) dm[r * nf] = dp[r * nf] = 0.0;
   }
   const bool work = in && !equal;
-  if (work) {  // speeds of the midpoint: the forms are homogeneous, so q_l + q_r serves
-    double m[3], Rm[9];
-#pragma unroll
-    for (int v = 0; v < 3; ++v) m[v] = add64(k, a[2 + v], b[2 + v]);
-#pragma unroll
-    for (int v = 0; v < 9; ++v) Rm[v] = add64(k, a[6 + v], b[6 + v]);
-    double u1, cm;
-    const int st = cell_speed64<kDef, false, false, kSoft>(E.e[ph], k, add64(k, a[0], b[0]), m, add64(k, a[5], b[5]), Rm, nullptr,
-                                                    u1, cm);
-    if (st) record_err64(S, st, R);
-    s_lo[ph][j] = sub64(k, u1, cm);
-    s_hi[ph][j] = add64(k, u1, cm);
+  if (work) {
+    const double2 s = mid2<kDef, kSoft>(a, b, Q, n, L, R, ph, E, k, S);
+    s_lo[ph][j] = sub64(k, s.x, s.y);
+    s_hi[ph][j] = add64(k, s.x, s.y);
   }
   __syncthreads();
   double sl = 0.0, sr = 0.0;
@@ -489,7 +532,8 @@ struct Step2Args {
 // A thread per cell and phase; with kCell the new state's cell pass follows in the same
 // kernel (a launch and a reload of the state less per step, which a small problem feels).
 template <int kDef, bool kCell, bool kSoft, bool kLxf>
-__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) step2_f64_kernel(Step2Args a, Eos2x E) {
+__global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) step2_f64_kernel(const __grid_constant__ Step2Args a,
+                                                                                    const __grid_constant__ Eos2x E) {
   __shared__ double s_r;
   __shared__ int s_more;
   const int ph = threadIdx.x / kPairCells;
@@ -557,7 +601,7 @@ __global__ void __launch_bounds__(kPair64, kSoft ? kSoftResident : 0) step2_f64_
     }
   }
   if (!kCell || !s_more) return;
-  cell2_pass<kDef, kSoft>(q, i < n, i, E.e[ph], k, a.o, a.wr);
+  cell2_pass<kDef, kSoft>(q, a.Qn, i < n, i, E, k, a.o, a.wr);
 }
 
 static inline unsigned grid_n(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }

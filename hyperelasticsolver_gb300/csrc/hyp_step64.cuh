@@ -73,14 +73,21 @@ __device__ __forceinline__ unsigned long long block_max_bits(double l) {
   return m;
 }
 
-// The single-phase cell pass of cell i in state q: its flux (kNFlux1 rows of F) and wave
-// speed, stored and returned; a bad cell is recorded.
+// The single-phase cell pass of cell i in state q, which is at Q too: its flux (kNFlux1 rows
+// of F) and wave speed, stored and returned; a bad cell is recorded. e and kc are the
+// kernel's own parameters (__grid_constant__: they have an address), k is kc in registers.
+template <int kDef>
+static __device__ __noinline__ double cell1_again(const double* Q, int64_t n, int64_t i, const EosC& e, const Eos64& kc,
+                                                  double* F, double* lam, DevState* S);
 template <int kDef, bool kSoft>
-__device__ __forceinline__ double cell1_pass(const double* q, int64_t n, int64_t i, const EosC& e, const Eos64& k,
-                                             double* __restrict__ F, double* __restrict__ lam, DevState* S) {
+__device__ __forceinline__ double cell1_pass(const double* q, const double* Q, int64_t n, int64_t i, const EosC& e,
+                                             const Eos64& kc, const Eos64& k, double* __restrict__ F,
+                                             double* __restrict__ lam, DevState* S) {
   double f[14];
   double u1, cm;
-  int st = cell_speed64<kDef, true, true, kSoft>(e, k, 1.0, q + 1, q[4], q + 5, f, u1, cm);
+  int st;
+  if (!cell_try64<kDef, true, true, kSoft>(e, k, 1.0, q + 1, q[4], q + 5, f, u1, cm, st) && kSoft)
+    return cell1_again<kDef>(Q, n, i, e, kc, F, lam, S);
   const double l = add64(k, fabs(u1), cm);
 #pragma unroll
   for (int v = 0; v < 14; ++v) {
@@ -93,13 +100,18 @@ __device__ __forceinline__ double cell1_pass(const double* q, int64_t n, int64_t
   return l;
 }
 template <int kDef, bool kSoft>
-__device__ __forceinline__ double cell1_load_pass(const double* __restrict__ Q, int64_t n, int64_t i, const EosC& e,
-                                                  const Eos64& k, double* __restrict__ F, double* __restrict__ lam,
-                                                  DevState* S) {
+__device__ __forceinline__ double cell1_load_pass(const double* Q, int64_t n, int64_t i, const EosC& e,
+                                                  const Eos64& kc, const Eos64& k, double* __restrict__ F,
+                                                  double* __restrict__ lam, DevState* S) {
   double q[14];
 #pragma unroll
   for (int v = 0; v < 14; ++v) q[v] = Q[v * n + i];
-  return cell1_pass<kDef, kSoft>(q, n, i, e, k, F, lam, S);
+  return cell1_pass<kDef, kSoft>(q, Q, n, i, e, kc, k, F, lam, S);
+}
+template <int kDef>
+static __device__ __noinline__ double cell1_again(const double* Q, int64_t n, int64_t i, const EosC& e, const Eos64& kc,
+                                                  double* F, double* lam, DevState* S) {
+  return cell1_load_pass<kDef, false>(Q, n, i, e, kc, in_registers64(kc), F, lam, S);
 }
 
 // Cells a block of the update kernels owns: thread j evaluates the face left of cell
