@@ -337,7 +337,7 @@ HYP_HD void acoustic_omega_dir(const EosT<R>& e, const KinT<R>& k, const PowsT<R
 template <class R> struct CubicTop {
   R c2, c1, c0;
   R r;          // Newton-refined real root of largest seed modulus
-  float other;  // single-precision estimate of the larger other modulus (-1: unknown)
+  R other;      // single-precision estimate of the larger other modulus (-1: unknown)
 };
 
 // FP32 reciprocal of a Newton step's slope: the step's own error is then ~1e-7 of
@@ -354,10 +354,36 @@ template <class R> HYP_HD R newton_recip(R fp) {
 
 template <class R> HYP_HD CubicTop<R> cubic_top(const R* a) {
   CubicTop<R> t;
-  const R c2 = a[0] + a[4] + a[8];
-  const R c1 = (a[0] * a[4] - a[3] * a[1]) + (a[0] * a[8] - a[6] * a[2]) + (a[4] * a[8] - a[7] * a[5]);
-  const R c0 = det3(a);
+  R c2 = a[0] + a[4] + a[8];
+  R c1 = (a[0] * a[4] - a[3] * a[1]) + (a[0] * a[8] - a[6] * a[2]) + (a[4] * a[8] - a[7] * a[5]);
+  R c0 = det3(a);
+  t.c2 = c2;
+  t.c1 = c1;
+  t.c0 = c0;
   float C2 = (float)c2, C1 = (float)c1, C0 = (float)c0;
+  // The seeds take up to the sixth power of the roots' size. Where that is no FP32 number
+  // (speeds of a kilometre a second in metres, say) the polynomial is that of the matrix times
+  // a power of two.
+  const float m2 = fabsf(C2), m1 = fabsf(C1), m0 = fabsf(C0);
+  R unit = R(1);  // one over that
+  bool scaled = false;
+  if (!(m2 < 0x1p20f && m1 < 0x1p40f && m0 < 0x1p60f && (m2 > 0x1p-18f || m1 > 0x1p-36f || m0 > 0x1p-54f))) {
+    R m = R(0), s = R(1);
+    for (int k = 0; k < 9; ++k) m = fmax(m, fabs(a[k]));
+    scaled = m > R(0) && m < R(1e300);
+    if (scaled) {
+      const R dn = R(1.0 / 65536.0), up = R(65536);
+      for (; m > R(256); m = m * dn) s = s * dn;
+      for (; m < R(1.0 / 256.0); m = m * up) s = s * up;
+      c2 = c2 * s;
+      c1 = c1 * s * s;
+      c0 = c0 * s * s * s;
+      C2 = (float)c2;
+      C1 = (float)c1;
+      C0 = (float)c0;
+      unit = R(1) / s;
+    }
+  }
   float p = C1 - C2 * C2 * (1.0f / 3.0f);
   float q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
   float disc = 0.25f * q * q + p * p * p * (1.0f / 27.0f);
@@ -385,11 +411,12 @@ template <class R> HYP_HD CubicTop<R> cubic_top(const R* a) {
     R fp = (R(3) * r - R(2) * c2) * r + c1;
     r = (fp != R(0)) ? r - f * newton_recip(fp) : r;
   }
-  t.c2 = c2;
-  t.c1 = c1;
-  t.c0 = c0;
   t.r = r;
-  t.other = (other == other && seed == seed) ? other : -1.0f;
+  t.other = (other == other && seed == seed) ? (R)other : R(-1);
+  if (scaled) {
+    t.r = r * unit;
+    if (t.other > R(0)) t.other = t.other * unit;
+  }
   return t;
 }
 
@@ -480,7 +507,7 @@ template <class R> HYP_HD void eig_core(const R* a, R* mods) {
 template <class R> HYP_HD R spectral_radius(const R* a) {
   const CubicTop<R> t = cubic_top(a);
   const R top = fabs(t.r);
-  if (t.other >= 0.0f && R(t.other) < R(0.9) * top) return top;
+  if (t.other >= R(0) && t.other < R(0.9) * top) return top;
   R m1, m2;
   if (symmetric_to_rounding(a)) {
     R d[3];
