@@ -100,24 +100,24 @@ HYP_HD bool below_negative64(double x, double t) {
   return (unsigned long long)bits_of(x) > (unsigned long long)bits_of(t) && !is_nan64(x);
 }
 
-// FP64 -> FP32 (truncated; under- and overflow to 0 and infinity) and FP32 -> FP64
-// (exact for normal values, 0 for subnormal ones) on the integer pipe: a conversion
-// instruction would take a slot of the FP64 pipe.
-HYP_HD float to_f32(double x) {
+// FP64 -> FP32 of x 2^-s (truncated; under- and overflow to 0 and infinity) and FP32 ->
+// FP64 of x 2^s (exact for normal values and results, 0 for subnormal x) on the integer pipe:
+// a conversion instruction would take a slot of the FP64 pipe.
+HYP_HD float to_f32(double x, int s = 0) {
   const long long b = bits_of(x);
-  const unsigned s = (unsigned)((unsigned long long)b >> 32) & 0x80000000u;
-  const int ex = (int)((b >> 52) & 0x7ff) - 896;
+  const unsigned sg = (unsigned)((unsigned long long)b >> 32) & 0x80000000u;
+  const int ex = (int)((b >> 52) & 0x7ff) - 896 - s;
   const unsigned m = (unsigned)(b >> 29) & 0x7fffffu;
-  if (ex <= 0) return of_bits_f(s);
-  if (ex >= 255) return of_bits_f(s | (is_nan64(x) ? 0x7fc00000u : 0x7f800000u));
-  return of_bits_f(s | ((unsigned)ex << 23) | m);
+  if (ex <= 0) return of_bits_f(sg);
+  if (ex >= 255) return of_bits_f(sg | (is_nan64(x) ? 0x7fc00000u : 0x7f800000u));
+  return of_bits_f(sg | ((unsigned)ex << 23) | m);
 }
-HYP_HD double to_f64(float x) {
+HYP_HD double to_f64(float x, int s = 0) {
   const unsigned b = bits_of_f(x), ex = (b >> 23) & 0xffu;
-  const unsigned long long s = (unsigned long long)(b & 0x80000000u) << 32;
-  if (ex == 0u) return of_bits((long long)s);
-  if (ex == 255u) return of_bits((long long)(s | (unsigned long long)kInfBits | ((unsigned long long)(b & 0x7fffffu) << 29)));
-  return of_bits((long long)(s | ((unsigned long long)(ex + 896u) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
+  const unsigned long long sg = (unsigned long long)(b & 0x80000000u) << 32;
+  if (ex == 0u) return of_bits((long long)sg);
+  if (ex == 255u) return of_bits((long long)(sg | (unsigned long long)kInfBits | ((unsigned long long)(b & 0x7fffffu) << 29)));
+  return of_bits((long long)(sg | ((unsigned long long)(ex + 896u + (unsigned)s) << 52) | ((unsigned long long)(b & 0x7fffffu) << 29)));
 }
 
 // 1/x and 1/sqrt(x), sqrt(x): a special-function seed (relative error e0 < 2^-19) and
@@ -435,7 +435,9 @@ double radius_general(double o00, double o11, double o22, double o01, double o02
 
 // The largest eigenvalue of a symmetric O, false where it does not stand clear of the
 // others' moduli: an FP32 root of the characteristic polynomial, then two steps with the
-// FP32 slope.
+// FP32 slope. FP32 has the polynomial with the power of two of the trace taken out: its last
+// coefficient is the sixth power of a speed, which in centimetres per picosecond or
+// millimetres per second is not an FP32 number.
 template <class K>
 HYP_HD bool top_root64(const K& k, double o00, double o11, double o22, double o01, double o02, double o12,
                        double& root) {
@@ -447,7 +449,9 @@ HYP_HD bool top_root64(const K& k, double o00, double o11, double o22, double o0
   const double c1 = fma(-o02, o02, fma(-o01, o01, fma(o00, tr, q)));
   const double e1 = fma(o01, o22, -M(o12, o02)), e2 = fma(o01, o12, -M(o11, o02));
   const double c0 = fma(o02, e2, fma(-o01, e1, M(o00, q)));
-  const float C2 = to_f32(c2), C1 = to_f32(c1), C0 = to_f32(c0);
+  const int sh = (int)(bits_of(c2) >> 52) - 1023;  // of c2 > 0
+  if (!(sh > -300 && sh < 300)) return false;
+  const float C2 = to_f32(c2, sh), C1 = to_f32(c1, 2 * sh), C0 = to_f32(c0, 3 * sh);
   const float P = C1 - C2 * C2 * (1.0f / 3.0f);
   const float Q = -2.0f / 27.0f * C2 * C2 * C2 + C2 * C1 * (1.0f / 3.0f) - C0;
   // A symmetric matrix has three real roots; two equal ones (a material at rest or under
@@ -462,9 +466,9 @@ HYP_HD bool top_root64(const K& k, double o00, double o11, double o22, double o0
   const float slope = (3.0f * y - 2.0f * C2) * y + C1;
   // With the others below 0.35 of it, the seed is within ~1e-6 and the slope within
   // ~1e-6 of theirs at the root: a step leaves 5e-12, the next 5e-17.
-  if (!(other < 0.35f * y && slope > 1e-30f && slope < 1e30f)) return false;
-  const double inv = to_f64(1.0f / slope);
-  double rt = to_f64(y);
+  if (!(other < 0.35f * y && slope > 1e-30f)) return false;
+  const double inv = to_f64(1.0f / slope, -2 * sh);
+  double rt = to_f64(y, sh);
   for (int it = 0; it < 2; ++it) rt = fma(-inv, fma(fma(A(rt, -c2), rt, c1), rt, -c0), rt);
   root = rt;
   return true;

@@ -42,3 +42,17 @@ def test_general_forms(lib, orc, ep, strain):  # noqa: F811
             for kr in (-40, 0, 10):
                 s, out = ev(lib, "c64_general", *in_units(ep, q, ku, kr))
                 assert s == 0 and np.array_equal(out, out_units(ref, ku, kr)), (ku, kr)
+
+
+@pytest.mark.parametrize("ep", EOS)
+@pytest.mark.parametrize("strain", [0.0, 0.02, 0.1, 0.3])
+@pytest.mark.parametrize("form", ["c64_compact", "c64_plain"])
+def test_compact_forms(lib, orc, ep, strain, form):  # noqa: F811
+    rng = np.random.default_rng(12)
+    for q in phase_states(orc, ep, rng, 20, (1.0, 0.25), strain):
+        st, ref = ev(lib, form, ep, q)
+        assert st == 0
+        for ku in SPEEDS:
+            for kr in (-40, 0, 10):
+                s, out = ev(lib, form, *in_units(ep, q, ku, kr))
+                assert s == 0 and np.array_equal(out, out_units(ref, ku, kr)), (ku, kr)
