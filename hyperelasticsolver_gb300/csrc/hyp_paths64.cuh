@@ -99,7 +99,10 @@ HYP_HD int path_nodes(const EosC* e, const double* a, const double* b) {
     const double *qa = a + 15 * p, *qb = b + 15 * p;
     const float al = to_f32(qa[0]), be = to_f32(qb[0]), lo = fminf(al, be);
     if (!(lo > 0.0f)) return 6;
-    const float ra = fabsf(be - al) / lo, ia = 1.0f / al, ib = 1.0f / be;
+    // the jump itself, subtracted in FP64 (of FP32 fractions it would be 0 below 1e-7 of them,
+    // and the bound with it) and rounded up
+    const float da = 1.0001f * fabsf(to_f32(qb[0] - qa[0]));
+    const float ra = da / lo, ia = 1.0f / al, ib = 1.0f / be;
     // B depends on the path through q / alpha alone, and q / alpha runs on a straight line
     float F[9], dF2 = 0.0f, F2 = 0.0f, v2 = 0.0f, dv2 = 0.0f;
     for (int k = 0; k < 9; ++k) {
