@@ -475,7 +475,7 @@ __global__ void k_lxf2(Eos2x E, Quad6D lobatto, const double* Ql, const double* 
       acc[15 * p + r] = 0.0;
     }
   }
-  path_thread<kDef>(E, lobatto, a, b, acc);
+  path_thread<kDef, true>(E, lobatto, a, b, acc);
   for (int k = 0; k < 30; ++k) DMo[k * n + i] = DPo[k * n + i] = 0.5 * acc[k];
 }
 }  // namespace

@@ -155,12 +155,14 @@ HYP_HD int path_nodes(const EosC* e, const double* a, const double* b) {
 
 // One thread per face: acc += the path integral from a to b (30 values each): the nodes
 // path_nodes asks for, of both phases, 360 slots a node. Rolled: six copies of the node
-// overflow the instruction cache. qd: the 6-point rule.
-template <int kDef>
+// overflow the instruction cache. qd: the 6-point rule; kSix: always that, for who gets the
+// integral by itself (path_nodes keeps its error small beside a flux difference, not beside
+// the integral, which is as small as the volume fractions' jump).
+template <int kDef, bool kSix = false>
 HYP_HD int path_thread(const Eos2x& E, const Quad6D& qd, const double* a, const double* b, double* acc) {
   int st = 0;
   const double da0 = b[0] - a[0], da1 = b[15] - a[15];
-  const int nodes = path_nodes(E.e, a, b);
+  const int nodes = kSix ? 6 : path_nodes(E.e, a, b);
 #pragma unroll 1
   for (int i = 0; i < nodes; ++i) {
     double s, w;
