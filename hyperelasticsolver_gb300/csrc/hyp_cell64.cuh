@@ -131,7 +131,7 @@ HYP_HD double seed_rcp(double x) {
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   return r;
 #else
-  return (double)(float)(1.0 / x);
+  return of_bits(bits_of(1.0 / x) & ~0xffffffffll);
 #endif
 }
 HYP_HD double seed_rsqrt(double x) {
@@ -140,7 +140,7 @@ HYP_HD double seed_rsqrt(double x) {
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
   return r;
 #else
-  return (double)(float)(1.0 / sqrt(x));
+  return of_bits(bits_of(1.0 / sqrt(x)) & ~0xffffffffll);
 #endif
 }
 // Constants of one phase's EOS and of the forms below. A kernel takes them through
@@ -296,6 +296,42 @@ HYP_HD double sqrt64(const Eos64& k, double x) {
   const double y = seed_rsqrt(x), t = mul64(k, x, y);
   const double e = fma(-t, y, k.one);
   return fma(mul64(k, t, e), fma(k.c375, e, k.half), t);
+}
+
+// a / b from rb, about 1 / b: a product and one residual correction (Markstein 1990),
+// 3 slots; correctly rounded up to rare last-bit cases.
+HYP_HD double quot64(const Eos64& k, double a, double b, double rb) {
+  const double q = mul64(k, a, rb);
+  return fma(fma(-b, q, a), rb, q);
+}
+
+// A step's dt = cfl dx / max lambda, the LxF lambda = dx / dt and dt/dx (main.jl:223-225;
+// for LxF the update's dt/dx is 1 / lambda, main.jl:40) without FP64 divisions (about 9 slots
+// each): 13 slots for the Rusanov step, 22 for LxF. Where an argument or a quotient is too
+// large or small for the special-function seeds and the correction, or not finite, the
+// divisions.
+struct StepScalars {
+  double dt, lam_lxf, dtdx;
+};
+HYP_HD StepScalars step_scalars64(const Eos64& k, double cfl, double dx, double lmax, bool lxf) {
+  auto plain = [](double x) {  // 2^-823 <= x < 2^823, by the exponent: a compare is a slot
+    const long long ex = bits_of(x) >> 52;
+    return ex >= 200 && ex < 1846;
+  };
+  const double cdx = cfl * dx;
+  StepScalars s{0.0, 0.0, 0.0};
+  s.dt = quot64(k, cdx, lmax, rcp64(k, lmax));
+  bool in = plain(lmax) && plain(dx) && plain(cdx) && plain(s.dt);
+  if (lxf) {
+    s.lam_lxf = quot64(k, dx, s.dt, rcp64(k, s.dt));
+    s.dtdx = quot64(k, k.one, s.lam_lxf, rcp64(k, s.lam_lxf));
+    in = in && plain(s.lam_lxf);
+  } else {
+    s.dtdx = quot64(k, s.dt, dx, rcp64(k, dx));
+  }
+  if (in && plain(s.dtdx)) return s;
+  const double dt = cdx / lmax, lam = dx / dt;
+  return StepScalars{dt, lam, lxf ? 1.0 / lam : dt / dx};
 }
 
 // One phase of a cell: primitives, stress row 1 = -2 td w, and what the acoustic

@@ -119,37 +119,6 @@ static __device__ __noinline__ double cell1_again(const double* Q, int64_t n, in
 // evaluates two (a second face on one thread is a second pass of its whole warp).
 constexpr int kCells64 = kBlock64 - 1;
 
-// a / b from rb, about 1 / b: a product and one residual correction (Markstein 1990),
-// 3 slots; correctly rounded up to rare last-bit cases.
-__device__ __forceinline__ double quot64(const Eos64& k, double a, double b, double rb) {
-  const double q = mul64(k, a, rb);
-  return fma(fma(-b, q, a), rb, q);
-}
-
-// step_scalars without FP64 divisions (about 9 slots each): 13 slots for the Rusanov
-// step, 22 for LxF. Arguments too large or small for the special-function seeds, and
-// quotients that are not finite, take the divisions.
-__device__ __forceinline__ StepScalars step_scalars64(const Eos64& k, double cfl, double dx, double lmax, bool lxf) {
-  auto plain = [](double x) {  // 2^-823 <= x < 2^823, by the exponent: a compare is a slot
-    const long long ex = bits_of(x) >> 52;
-    return ex >= 200 && ex < 1846;
-  };
-  const double cdx = cfl * dx;
-  if (!plain(lmax) || !plain(dx) || !plain(cdx)) {
-    const double dt = cdx / lmax, lam = dx / dt;
-    return StepScalars{dt, lam, lxf ? 1.0 / lam : dt / dx};
-  }
-  StepScalars s{0.0, 0.0, 0.0};
-  s.dt = quot64(k, cdx, lmax, rcp64(k, lmax));
-  if (lxf) {
-    s.lam_lxf = quot64(k, dx, s.dt, rcp64(k, s.dt));
-    s.dtdx = quot64(k, k.one, s.lam_lxf, rcp64(k, s.lam_lxf));
-  } else {
-    s.dtdx = quot64(k, s.dt, dx, rcp64(k, dx));
-  }
-  return s;
-}
-
 // Twice the Rusanov flux of the face between cells f - 1 and f of the problem [lo, hi)
 // (a zero-gradient ghost past either end): (f_a + f_b) - lambda (q_b - q_a), lambda =
 // max(lambda_a, lambda_b) (NumFluxes.jl:25-33, main.jl:45-48) or the LxF one. Doubling is

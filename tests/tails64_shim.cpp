@@ -6,6 +6,8 @@ using namespace hyp;
 
 static EosC eos(const double* p) { return make_eos(p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7]); }
 
+static const double EP0[8] = {8.93, 4.6, 3.9e-4, 300.0, 2.1, 1.0, 3.0, 2.0};
+
 extern "C" {
 // q: one phase (15 values); out, plain: flux (14), u1, c_max by integer and by the hardware's
 // products, st their statuses; returns whether the integer products are held for
@@ -31,5 +33,10 @@ void t64_vjp(const double* p, const double* q, const double* fb, double lb, doub
   int st;
   left[0] = cell_vjp_try64<1, true>(e, k, q, fb, lb, qb, c, st);
   left[1] = cell_vjp_try64<1, false>(e, k, q, fb, lb, qb, d, st);
+}
+// dt, the LxF lambda and dt/dx of a step
+void t64_scalars(double cfl, double dx, double lmax, int lxf, double* out) {
+  const StepScalars s = step_scalars64(make_eos64(eos(EP0)), cfl, dx, lmax, lxf != 0);
+  out[0] = s.dt, out[1] = s.lam_lxf, out[2] = s.dtdx;
 }
 }

@@ -90,3 +90,30 @@ def test_values_past_the_range(lib, x):
                 for f in (fb, np.where(np.arange(14) % 3, fb, 0.0), np.where(np.arange(14) == 4, x, fb)):
                     left, a, b = vjp(lib, q[1:], f, 0.3)
                     assert a.tobytes() == b.tobytes(), v
+
+
+@pytest.mark.parametrize("lxf", [False, True])
+def test_step_scalars(lib, lxf):
+    """dt = cfl dx / max speed, lambda and dt/dx against divisions: 2 ulps a quotient where all
+    of them are ordinary, and the divisions themselves (infinities and zeros included) where
+    an argument or a quotient leaves the range of the reciprocals."""
+    rng = np.random.default_rng(6)
+    cases = [(0.5, 10.0 ** a, 10.0 ** b) for a, b in rng.uniform(-8, 8, (200, 2))]
+    cases += [(0.5, 10.0 ** a, 10.0 ** b) for a, b in rng.uniform(-320, 308, (2000, 2))]
+    cases += [(0.5, x, y) for x in (1e-240, 1e-3, 1e240) for y in (0.0, 5e-324, 1e-247, 1e-100, 1.0, 1e100, 1e246, 1e300, np.inf)]
+    fast = 0
+    for cfl, dx, lmax in cases:
+        out = np.zeros(3)
+        lib.t64_scalars(ctypes.c_double(cfl), ctypes.c_double(dx), ctypes.c_double(lmax), int(lxf), out.ctypes.data_as(DP))
+        with np.errstate(all="ignore"):
+            dt = np.float64(cfl) * dx / np.float64(lmax)
+            lam = dx / dt
+            ref = np.array([dt, lam, np.float64(1.0) / lam if lxf else dt / dx])
+        if not lxf:
+            out[1] = ref[1]  # not a Rusanov step's
+        assert np.array_equal(np.isnan(out), np.isnan(ref)), (dx, lmax, out, ref)
+        fin = np.isfinite(ref) & (np.abs(ref) > 1e-290)
+        assert np.all(np.abs(out[fin] - ref[fin]) <= 6 * 2.0 ** -53 * ref[fin]), (dx, lmax, out, ref)
+        assert np.array_equal(out[~fin], ref[~fin], equal_nan=True), (dx, lmax, out, ref)
+        fast += bool(fin.all())
+    assert fast > 300
