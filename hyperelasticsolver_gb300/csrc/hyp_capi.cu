@@ -218,7 +218,7 @@ static int check_cell_error(hyp_ctx* c) {
   c->err_cell = c->st_host->err_cell;
   char buf[160];
   if (code & HYP_CELL_TIMEOUT) {
-    snprintf(buf, sizeof buf, "a device wait for a tile load timed out (tile starting at cell %lld)", (long long)c->err_cell);
+    snprintf(buf, sizeof buf, "a device wait timed out (of the tile or block starting at cell %lld)", (long long)c->err_cell);
     return set_err(c, HYP_ERR_TIMEOUT, buf);
   }
   if (code & HYP_CELL_RELAX) {
@@ -592,7 +592,7 @@ extern "C" int hyp_set_eos(hyp_ctx* c, int phase, const hyp_barton2009* eos) {
 
 extern "C" int hyp_set_wait_limit(hyp_ctx* c, int tries) {
   if (!c || tries < 0) return HYP_ERR_INVALID;
-  c->wait_tries = tries;
+  c->wait_tries = c->run_tries = tries;
   for (auto& g : c->graph)  // graphs hold the previous kernel arguments
     if (g) {
       cudaGraphExecDestroy(g);

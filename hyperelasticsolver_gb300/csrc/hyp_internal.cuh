@@ -70,6 +70,7 @@ struct StepTiming {
 namespace hyp {
 struct AdjTape;
 struct SnapBuf;
+constexpr int kRunTries = 1 << 24;  // default poll budget of a run's block (run1_f64_kernel)
 // Mixed-precision state of one parity: kMixedRows rows per cell, rows 0-13 hi
 // parts, 14-27 lo parts, 28 the cell's wave speed, 29-31 its island outputs.
 // Row-major blocks (the batch solver, the two-phase step's 60 rows): row r of cell
@@ -116,7 +117,8 @@ struct hyp_ctx {
   float* mixed_base = nullptr;          // one allocation holding both parities' blocks
   int64_t mpitch = 0;                   // two-phase: row pitch (floats, a multiple of 4)
   int mixed_kind = HYP_MIXED_TILE;      // kernel family (hyp_set_mixed_kernel)
-  int wait_tries = hyp::kWaitTries;     // poll budget of the TMA kernel's barrier waits
+  int wait_tries = hyp::kWaitTries;     // poll budget of the TMA kernel's barrier waits (hyp_set_wait_limit)
+  int run_tries = hyp::kRunTries;       // and of the waits of a run's blocks for one another
   int tma_grid = 0;
   hyp::EosMixed eos_mixed;
   // two-phase (FP64): cell fluxes F [30][n], wave-speed bounds, face fluctuations [30][n+1]
@@ -240,7 +242,6 @@ struct Run1Args {
   int sms;    // multiprocessors of the device
   DevState* S;
 };
-constexpr int kRunTries = 1 << 24;
 size_t run1_edge_doubles(int64_t n);
 bool run1_fits(int64_t n, int sms);
 cudaError_t launch_run1(cudaStream_t s, Run1Args a, EosC e);

@@ -491,7 +491,7 @@ cudaError_t launch_run1_f64(hyp_ctx* c, long long k, int max_steps, double t_end
   a.n = c->n;
   a.flux = c->cfg.flux;
   a.bc = ctx_bc(c);
-  a.tries = kRunTries;
+  a.tries = c->run_tries;
   a.sms = c->sms;
   a.S = c->st;
   return launch_run1(c->stream, a, c->eos[0]);

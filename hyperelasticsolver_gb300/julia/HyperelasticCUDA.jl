@@ -288,7 +288,7 @@ function set_mixed_kernel!(s::Solver, kind::Symbol)
   k = Dict(:tile => 0, :tma => 1, :pair => 2)[kind]
   check(ccall((:hyp_set_mixed_kernel, libhyp), Cint, (Ptr{Cvoid}, Cint), s.h, k), "hyp_set_mixed_kernel", s.h)
 end
-"set_wait_limit!(s, tries): poll budget of the persistent kernel's device waits (0: every wait times out)"
+"set_wait_limit!(s, tries): poll budget of the device waits: the persistent kernel's, and those of a small FP64 run's blocks (0: every wait times out)"
 set_wait_limit!(s::Solver, tries::Integer) =
   check(ccall((:hyp_set_wait_limit, libhyp), Cint, (Ptr{Cvoid}, Cint), s.h, tries), "hyp_set_wait_limit", s.h)
 "snapshot(s): cons2prim of the current state, one row per cell ([alpha, rho, u, S, A] per phase)"

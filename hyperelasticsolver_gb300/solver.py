@@ -123,7 +123,8 @@ class Solver:
         L.check(L.load().hyp_set_mixed_kernel(self._h, self.MIXED_KERNELS[kernel]), self._h, "hyp_set_mixed_kernel")
 
     def set_wait_limit(self, tries):
-        """Poll budget of the TMA kernel's device waits; 0 makes each wait time out at once."""
+        """Poll budget of the device waits (the TMA kernel's; those of the blocks of a small
+        single-phase FP64 run for one another); 0 makes each wait time out at once."""
         L.check(L.load().hyp_set_wait_limit(self._h, int(tries)), self._h, "hyp_set_wait_limit")
 
     def set_profiling(self, on):

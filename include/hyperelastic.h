@@ -186,11 +186,12 @@ int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in, double* d_
 enum { HYP_MIXED_TILE = 0, HYP_MIXED_TMA = 1, HYP_MIXED_PAIR = 2 };
 int hyp_set_mixed_kernel(hyp_ctx* ctx, int kind);
 
-/* Poll budget of the TMA kernel's device-side barrier waits (default 2^20). A wait
-   that runs out records HYP_CELL_TIMEOUT, lets its in-flight copy land and ends the
-   block, and the step returns HYP_ERR_TIMEOUT; the context stays usable (upload a
-   state again). A budget of 0 makes every wait run out at once: the timeout path
-   exercised without a fault. */
+/* Poll budget of the device-side waits: of the TMA kernel's barriers (default 2^20) and,
+   where a small single-phase FP64 problem runs in one launch, of its blocks for one
+   another once a step (default 2^24). A wait that runs out records HYP_CELL_TIMEOUT, lets
+   its in-flight copy land and ends the block, and the step returns HYP_ERR_TIMEOUT; the
+   context stays usable (upload a state again). A budget of 0 makes every wait run out at
+   once: the timeout path exercised without a fault. */
 int hyp_set_wait_limit(hyp_ctx* ctx, int tries);
 
 /* ---- domain decomposition: a context as one slab of a longer 1D domain ------ */
