@@ -457,7 +457,7 @@ extern "C" int hyp_step(hyp_ctx* c, int max_steps, double t_end, int* steps_done
   const int gs = graph_steps(c);
   // small single-phase FP64 problems: the whole run in one launch (not where each step is
   // timed or logged)
-  const bool one_launch = !mixed(c) && c->cfg.model == HYP_MODEL_SINGLE && !prof && !c->hist_on && c->coop &&
+  bool one_launch = !mixed(c) && c->cfg.model == HYP_MODEL_SINGLE && !prof && !c->hist_on && c->coop &&
                           run1_fits(c->n, c->sms);
   int rc = HYP_OK;
   while (rc == HYP_OK) {
@@ -467,6 +467,11 @@ extern "C" int hyp_step(hyp_ctx* c, int max_steps, double t_end, int* steps_done
     if (one_launch) {
       todo = std::min<long long>(todo, kRunSteps);
       cudaError_t e = launch_run1_f64(c, steps0 + launched, (int)todo, t_end);
+      if (launch_refused(e)) {
+        (void)cudaGetLastError();
+        one_launch = false;
+        continue;
+      }
       if (e != cudaSuccess) rc = set_err(c, HYP_ERR_CUDA, std::string("launch_run1_f64: ") + cudaGetErrorString(e));
       launched += todo;
       if (rc != HYP_OK) break;

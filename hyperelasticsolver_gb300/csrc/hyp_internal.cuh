@@ -244,6 +244,12 @@ struct Run1Args {
 };
 size_t run1_edge_doubles(int64_t n);
 bool run1_fits(int64_t n, int sms);
+// Whether a cooperative launch failed because the process may not have all its blocks at once
+// (it was given a part of the multiprocessors, which their number does not tell): nothing has
+// run, and the steps' own kernels do.
+inline bool launch_refused(cudaError_t e) {
+  return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported;
+}
 cudaError_t launch_run1(cudaStream_t s, Run1Args a, EosC e);
 cudaError_t launch_run1_f64(hyp_ctx* c, long long k, int max_steps, double t_end);
 // single-phase FP64 launchers on a context (hyp_step1.cu)

@@ -111,12 +111,7 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
   const EosC eos = make_eos(cfg->eos[0].rho0, cfg->eos[0].c0, cfg->eos[0].cv, cfg->eos[0].t0, cfg->eos[0].b0,
                             cfg->eos[0].alpha, cfg->eos[0].beta, cfg->eos[0].gamma);
   const double dx = cfg->x_length / (double)n;
-  const bool one_launch = n_steps > 0 && t0 < INFINITY && run1_fits(n, run_blocks);
-  // Ping-pong between the caller's output and the scratch state so that the last step writes the output.
-  double* cur = (n_steps % 2 == 0) ? d_Q_out : B;
-  if (!one_launch && cur != d_Q_in &&
-      cudaMemcpyAsync(cur, d_Q_in, (size_t)14 * n * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
-    return HYP_ERR_CUDA;
+  bool one_launch = n_steps > 0 && t0 < INFINITY && run1_fits(n, run_blocks);
   noalloc_reset_kernel<<<1, 1, 0, s>>>(st, t0);
   if (cudaGetLastError() != cudaSuccess) return HYP_ERR_CUDA;
   if (one_launch) {  // a small problem: every step in one launch, from the input to the output
@@ -137,8 +132,19 @@ extern "C" int hyp_step_noalloc_f64(const hyp_config* cfg, const double* d_Q_in,
     a.tries = kRunTries;
     a.S = st;
     a.sms = run_blocks;
-    if (launch_run1(s, a, eos) != cudaSuccess) return HYP_ERR_CUDA;
+    const cudaError_t e = launch_run1(s, a, eos);
+    if (launch_refused(e)) {
+      (void)cudaGetLastError();
+      one_launch = false;
+    } else if (e != cudaSuccess) {
+      return HYP_ERR_CUDA;
+    }
   }
+  // Ping-pong between the caller's output and the scratch state so that the last step writes the output.
+  double* cur = (n_steps % 2 == 0) ? d_Q_out : B;
+  if (!one_launch && cur != d_Q_in &&
+      cudaMemcpyAsync(cur, d_Q_in, (size_t)14 * n * sizeof(double), cudaMemcpyDeviceToDevice, s) != cudaSuccess)
+    return HYP_ERR_CUDA;
   if (!one_launch && n_steps > 0 &&
       launch_cell1(s, cur, n, eos, F, lam, &st->lam_slots[0], &st->t[0], INFINITY, st) != cudaSuccess)
     return HYP_ERR_CUDA;
