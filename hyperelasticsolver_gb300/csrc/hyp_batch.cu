@@ -329,6 +329,7 @@ struct hyp_batch {
 };
 
 static int berr(hyp_batch* b, int code, const std::string& m) {
+  if (code == HYP_ERR_CUDA) (void)cudaGetLastError();  // reported here, not by the next call's launches too
   if (b) b->err = m;
   return code;
 }
@@ -555,7 +556,7 @@ extern "C" int hyp_batch_upload(hyp_batch* b, const double* Q, double t0) {
   if (b->mixed) {
     // A page-locked array is read in place: one pass at the host link's rate (676.9 MB of
     // 512 problems: 3.46 ms) instead of a copy and a pass over it (3.89 ms).
-    const double* stage = mapped_host(Q);
+    const double* stage = mapped_host(Q, bytes);
     if (!stage) {
       BCK(cudaMemcpyAsync(b->Qh[1], Q, bytes, cudaMemcpyHostToDevice, b->stream));
       stage = (const double*)b->Qh[1];
@@ -581,7 +582,7 @@ extern "C" int hyp_batch_download(hyp_batch* b, double* Q) {
     // 4.38 with 14 copies, so that takes one). Joining in place, as the upload splits, took
     // 4.46 ms, for the tiles' short stores.
     double* stage = (double*)b->Qh[1 - b->cur];
-    const int rows = bytes >= ((size_t)64 << 20) && mapped_host(Q) ? 1 : 14;
+    const int rows = bytes >= ((size_t)64 << 20) && mapped_host(Q, bytes) ? 1 : 14;
     for (int v = 0; v < 14; v += rows) {
       batch_join_kernel<<<b->sms * 8, kBlock, 0, b->stream>>>(b->Qh[b->cur], b->total, stage, b->tiles, b->ntiles, v,
                                                               v + rows);

@@ -1,4 +1,5 @@
 // hyp_capi.cu -- context lifecycle, transfers and the step driver of the C ABI.
+#include <cuda.h>
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -16,6 +17,7 @@ using namespace hyp;
   } while (0)
 
 static int set_err(hyp_ctx* c, int code, const std::string& msg) {
+  if (code == HYP_ERR_CUDA) (void)cudaGetLastError();  // reported here, not by the next call's launches too
   if (c) c->err = msg;
   return code;
 }
@@ -265,15 +267,31 @@ int ctx_finish_install_from(hyp_ctx* c, const double* src, double t0) {
 
 int ctx_finish_install(hyp_ctx* c, double t0) { return ctx_finish_install_from(c, nullptr, t0); }
 
-// Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister), or
-// null for memory the device does not map (pageable, or not host memory).
-const double* mapped_host(const void* p) {
+// Device address of page-locked host memory (cudaHostAlloc / cudaHostRegister), or null for
+// memory of which the device does not map all `bytes` (pageable, registered in part, or not
+// host memory). Only the driver knows how far a registration reaches.
+const double* mapped_host(const void* p, size_t bytes) {
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return nullptr;
   }
-  return a.type == cudaMemoryTypeHost ? (const double*)a.devicePointer : nullptr;
+  if (a.type != cudaMemoryTypeHost) return nullptr;
+  void* entry = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &entry, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+      found != cudaDriverEntryPointSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  const auto get = (CUresult(*)(void*, CUpointer_attribute, CUdeviceptr))entry;
+  CUdeviceptr start = 0;
+  size_t size = 0;
+  if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, (CUdeviceptr)p) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, (CUdeviceptr)p) != CUDA_SUCCESS)
+    return nullptr;
+  const size_t at = (size_t)((CUdeviceptr)p - start);
+  return (CUdeviceptr)p >= start && at <= size && bytes <= size - at ? (const double*)a.devicePointer : nullptr;
 }
 
 extern "C" int hyp_upload(hyp_ctx* c, const double* Q, int64_t n_cells, int n_vars, double t0) {
@@ -283,9 +301,9 @@ extern "C" int hyp_upload(hyp_ctx* c, const double* Q, int64_t n_cells, int n_va
   // Mixed precision from page-locked memory: the install kernel reads the host array
   // in place (one pass over the host link, split and wave speeds included) instead of
   // a copy into the staging block followed by a pass over it.
-  const double* mapped = mixed(c) ? mapped_host(Q) : nullptr;
-  if (mapped) return ctx_finish_install_from(c, mapped, t0);
   const size_t bytes = (size_t)n_vars * n_cells * sizeof(double);
+  const double* mapped = mixed(c) ? mapped_host(Q, bytes) : nullptr;
+  if (mapped) return ctx_finish_install_from(c, mapped, t0);
   CK(cudaMemcpyAsync(ctx_install_target(c), Q, bytes, cudaMemcpyHostToDevice, c->stream));
   return ctx_finish_install(c, t0);
 }

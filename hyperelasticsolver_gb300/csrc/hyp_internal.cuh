@@ -183,7 +183,7 @@ int ctx_check_cell_error(hyp_ctx* c);
 // Installing a state generated on the device (hyp_capi.cu): write it, FP64 [nvar][n],
 // to ctx_install_target(c), then call ctx_finish_install(c, t0).
 double* ctx_install_target(hyp_ctx* c);
-const double* mapped_host(const void* p);
+const double* mapped_host(const void* p, size_t bytes);
 int ctx_finish_install(hyp_ctx* c, double t0);
 // The same from an FP64 state [nvar][n] at src: device memory, or host memory the
 // device maps (mixed contexts read it in place, so the host link is the only transfer).
