@@ -156,12 +156,11 @@ __global__ void __launch_bounds__(256) adj_dtdx_kernel(AdjArgs g) {
 
 // Cell i of an adjoint step: Qb0 of it and what it adds to eb; r and lamb_max: dt/dx and the
 // adjoint of the max wave speed; lanes: the warp's lanes that call it together (0: the lane is
-// on its own); form: the compact forms with the hardware's products or lone ones on the integer
-// pipe, or the general form. Returns what is left to do (hyp_adjoint64.cuh).
-enum { kFormPlain, kFormSoft, kFormGeneral };
-template <int kDef, int kForm>
-__device__ __forceinline__ int adj_cell(const AdjArgs& g, const EosC& e, const Eos64& k64, int64_t i, double r,
-                                        double lamb_max, unsigned lanes, EosBar& eb) {
+// on its own). False, with results that mean nothing, where kSoft's integer products are not
+// held for (hyp_adjoint64.cuh).
+template <int kDef, bool kSoft>
+__device__ __forceinline__ bool adj_cell(const AdjArgs& g, const EosC& e, const Eos64& k64, int64_t i, double r,
+                                         double lamb_max, unsigned lanes, EosBar& eb) {
   const int64_t n = g.n;
   const int64_t il = i > 0 ? i - 1 : 0, ir = i < n - 1 ? i + 1 : n - 1;
   const bool ui = updated(i, n, g.trans);
@@ -203,29 +202,19 @@ __device__ __forceinline__ int adj_cell(const AdjArgs& g, const EosC& e, const E
   any |= (unsigned long long)bits_of(lamb) << 1;
   // where the face adjoints vanish (a region where the adjoint field is constant) the
   // VJP adds exact zeros: skip it
-  int left = kVjpDone, st;
-  if (any) {
-    if (kForm == kFormGeneral)
-      cell_vjp(e, q, fb, lamb, qb, eb);
-    else
-      left = cell_vjp_try64<kDef, kForm == kFormSoft>(e, k64, q, fb, lamb, qb, eb, st);
-  }
+  int end = kVjpDone, st;
+  if (any) end = cell_vjp_try64<kDef, kSoft>(e, k64, q, fb, lamb, qb, eb, st);
 #pragma unroll
   for (int v = 0; v < 14; ++v) g.Qb0[v * n + i] = qb[v];
-  return left;
+  return end != kVjpPlain;
 }
 
-// What a cell left to do, out of line.
+// With the hardware's products, out of line.
 template <int kDef>
 static __device__ __noinline__ EosBar adj_cell_again(const AdjArgs& g, const EosC& e, const Eos64& kc, int64_t i, double r,
-                                                     double lamb_max, int left) {
-  const Eos64 k = in_registers64(kc);
+                                                     double lamb_max) {
   EosBar eb{0.0, 0.0};
-  if (left == kVjpPlain) left = adj_cell<kDef, kFormPlain>(g, e, k, i, r, lamb_max, 0u, eb);
-  if (left == kVjpGeneral) {
-    eb = EosBar{0.0, 0.0};
-    adj_cell<kDef, kFormGeneral>(g, e, k, i, r, lamb_max, 0u, eb);
-  }
+  adj_cell<kDef, false>(g, e, in_registers64(kc), i, r, lamb_max, 0u, eb);
   return eb;
 }
 
@@ -237,7 +226,7 @@ static __device__ __noinline__ EosBar adj_cell_again(const AdjArgs& g, const Eos
 // pipe (kSoft) 7.44 at the two blocks a multiprocessor that its registers allow, held to
 // three and four blocks 8.18 and 7.53 for the spills. A step of 65,536 cells with a dense
 // adjoint 79 us in a short run and 154 after 1000 steps, when the tails' cells went through
-// the forms three times; 78 and 78 since they are told by their state and evaluated once.
+// the forms three times; 79 and 79 since they are told by their state and evaluated once.
 template <int kDef, bool kSoft>
 __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(const __grid_constant__ AdjArgs g,
                                                              const __grid_constant__ EosC e,
@@ -262,10 +251,8 @@ __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(const __grid_consta
   const int64_t i = (int64_t)blockIdx.x * kAdjBlock + threadIdx.x;
   EosBar eb{0.0, 0.0};
   const unsigned lanes = __ballot_sync(0xffffffffu, i < n);
-  if (i < n) {
-    const int left = adj_cell<kDef, kSoft ? kFormSoft : kFormPlain>(g, e, k64, i, s_r, s_lamb_max, lanes, eb);
-    if (left) eb = adj_cell_again<kDef>(g, e, kc, i, s_r, s_lamb_max, left);
-  }
+  if (i < n && !adj_cell<kDef, kSoft>(g, e, k64, i, s_r, s_lamb_max, lanes, eb) && kSoft)
+    eb = adj_cell_again<kDef>(g, e, kc, i, s_r, s_lamb_max);
   const double b0 = block_sum<kAdjBlock>(eb.b0sq, sh);
   const double k0 = block_sum<kAdjBlock>(eb.k0, sh);
   if (threadIdx.x == 0) {

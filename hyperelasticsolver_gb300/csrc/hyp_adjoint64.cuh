@@ -16,11 +16,20 @@
 
 namespace hyp {
 
-// What an evaluation on the compact forms leaves to do: nothing; the same with the hardware's
-// products (cell_try64); the general form (cell_vjp), for a top eigenvalue that does not stand
-// clear. In the last two cases qb and eb mean nothing. A kernel does either out of line with
-// its inputs loaded again: called from here they would lie in local memory in every cell.
+// How an evaluation ended: on the compact forms; not at all, with qb and eb that mean nothing
+// and the same to be done with the hardware's products (cell_try64); by the general form, for a
+// top eigenvalue that does not stand clear.
 enum { kVjpDone = 0, kVjpPlain = 1, kVjpGeneral = 2 };
+
+// The general form, out of line.
+#ifdef __CUDACC__
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+int cell_vjp_general(const EosC& e, const double* q, const double* fb, double lb, double* qb, EosBar* eb) {
+  return cell_vjp(e, q, fb, lb, qb, *eb);
+}
 
 template <int kDef, class K>
 HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const double* fb, double lb, double* qb,
@@ -56,7 +65,24 @@ HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const doubl
     const double o11 = fma(f1, c.G01, fma(c.a, c.G11, -c.bM)), o22 = fma(f2, c.G02, fma(c.a, c.G22, -c.bM));
     const double o12 = fma(f1, c.G02, M(c.a, c.G12));
     double nu;
-    if (!top_root64(k, o00, o11, o22, o01, o02, o12, nu)) return out_of_range(k) ? kVjpPlain : kVjpGeneral;
+    if (!top_root64(k, o00, o11, o22, o01, o02, o12, nu)) {
+      if (out_of_range(k)) return kVjpPlain;
+      // on copies: the arrays themselves, had they an address, would lie in local memory in
+      // every cell
+      double qs[14], fs[14], bs[14];
+      EosBar es = eb;
+#pragma unroll
+      for (int v = 0; v < 14; ++v) {
+        qs[v] = q[v];
+        fs[v] = fb[v];
+        bs[v] = qb[v];
+      }
+      st = cell_vjp_general(e, qs, fs, lb, bs, &es);
+#pragma unroll
+      for (int v = 0; v < 14; ++v) qb[v] = bs[v];
+      eb = es;
+      return kVjpGeneral;
+    }
     u0b = c.u[0] > 0.0 ? lb : (c.u[0] < 0.0 ? -lb : 0.0);
     // d nu / d O = Cof(nu I - O) / its trace; an off-diagonal entry stands for two
     const double b00 = S(nu, o00), b11 = S(nu, o11), b22 = S(nu, o22);
@@ -203,18 +229,11 @@ HYP_HD int cell_vjp64(const EosC& e, const Eos64& k, const double* q, const doub
   double qs[14];
   for (int v = 0; v < 14; ++v) qs[v] = qb[v];
   const EosBar es = eb;
-  auto restore = [&] {
+  int st;
+  if (cell_vjp_try64<kDef, kSoft>(e, k, q, fb, lb, qb, eb, st) == kVjpPlain) {
     for (int v = 0; v < 14; ++v) qb[v] = qs[v];
     eb = es;
-  };
-  int st, left = cell_vjp_try64<kDef, kSoft>(e, k, q, fb, lb, qb, eb, st);
-  if (left == kVjpPlain) {
-    restore();
-    left = cell_vjp_try64<kDef, false>(e, k, q, fb, lb, qb, eb, st);
-  }
-  if (left == kVjpGeneral) {
-    restore();
-    st = cell_vjp(e, q, fb, lb, qb, eb);
+    cell_vjp_try64<kDef, false>(e, k, q, fb, lb, qb, eb, st);
   }
   return st;
 }
