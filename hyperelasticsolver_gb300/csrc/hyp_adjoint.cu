@@ -226,7 +226,7 @@ static __device__ __noinline__ EosBar adj_cell_again(const AdjArgs& g, const Eos
 // pipe (kSoft) 7.44 at the two blocks a multiprocessor that its registers allow, held to
 // three and four blocks 8.18 and 7.53 for the spills. A step of 65,536 cells with a dense
 // adjoint 79 us in a short run and 154 after 1000 steps, when the tails' cells went through
-// the forms three times; 79 and 79 since they are told by their state and evaluated once.
+// the forms three times; 78 and 78 since they are told by their state and evaluated once.
 template <int kDef, bool kSoft>
 __global__ void __launch_bounds__(kAdjBlock) adj_cell_kernel(const __grid_constant__ AdjArgs g,
                                                              const __grid_constant__ EosC e,

@@ -218,7 +218,9 @@ HYP_HD int cell_vjp_of64(const EosC& e, const K& k, const double* q, const doubl
 template <int kDef, bool kSoft>
 HYP_HD int cell_vjp_try64(const EosC& e, const Eos64& k, const double* q, const double* fb, double lb, double* qb,
                           EosBar& eb, int& st) {
-  if (kSoft && !(soft_inputs64(q + 1, 13) & soft_inputs64(fb, 14) & soft_inputs64(&lb, 1))) return kVjpPlain;
+  // (the adjoints, which have tails of their own, enter linearly)
+  if (kSoft && !warp_holds(soft_inputs64(q + 1, 13) & soft_inputs64(fb, 14, 500u) & soft_inputs64(&lb, 1, 500u)))
+    return kVjpPlain;
   return cell_vjp_of64<kDef>(e, typename std::conditional<kSoft, Soft64, Plain64>::type(k), q, fb, lb, qb, eb, st);
 }
 

@@ -245,23 +245,35 @@ struct Soft64 : Eos64 {
 HYP_HD bool out_of_range(const Eos64&) { return false; }
 HYP_HD bool out_of_range(const Soft64& k) { return k.worst > kSoftWide; }
 
-// Whether n values are what the forms may take on the integer pipe: zeros, or 2^-250 to 2^251
-// in size. The tail of a wave has others: its components shrink by a factor a cell, down to
-// zero, and squares of them leave the range of a double. A tail's cells are told here, by
-// their state, before anything is evaluated: after 200 to 1000 steps of a run they had taken
-// the integer products, a general form on their results and then the hardware's products
-// (two phases, 40,000 cells, 500 steps 89 -> 74 us a step; the adjoint of 65,536 cells
-// 154 -> 78). Each product that fails by itself on the FP64 pipe, where it is met, was no
+// Whether n values are what the forms may take on the integer pipe: zeros, or 2^-lo (250 for a
+// state, of which they form fourth powers) to 2^251 in size. The tail of a wave has others: its
+// components shrink by a factor a cell, down to zero, and squares of them leave the range of a
+// double. A tail's cells are told here, by their state, before anything is evaluated: after 200
+// to 1000 steps of a run they had taken the integer products, a general form on their results
+// and then the hardware's products (two phases, 40,000 cells, 500 steps 89 -> 70 us a step; an
+// adjoint step of 65,536 cells after 1000 steps 154 -> 78 with a dense seed, 140 -> 55 with a
+// density misfit's). Each product that fails by itself on the FP64 pipe, where it is met, was no
 // way: its 79 branches keep the compiler from mixing the two pipes' instructions (1,000,003
 // cells 332 -> 437 us a step).
-HYP_HD bool soft_inputs64(const double* x, int n) {
-  constexpr unsigned lo = (1023u - 250u) << 21, wide = 501u << 21;
+HYP_HD bool soft_inputs64(const double* x, int n, unsigned lo = 250u) {
+  const unsigned least = (1023u - lo) << 21, wide = (lo + 251u) << 21;
   bool in = true;
   for (int v = 0; v < n; ++v) {
     const unsigned long long b = (unsigned long long)bits_of(x[v]) << 1;
-    in &= (unsigned)(b >> 32) - lo < wide || b == 0ull;
+    in &= (unsigned)(b >> 32) - least < wide || b == 0ull;
   }
   return in;
+}
+
+// Whether all of the warp's cells at hand are held for: one that is not has the whole warp
+// take the hardware's products, which costs what they cost for that one alone, instead of one
+// pass after the other (the runs above: 74 -> 70 us and, with the misfit's seed, 73 -> 55).
+HYP_HD bool warp_holds(bool in) {
+#ifdef __CUDA_ARCH__
+  return !__any_sync(__activemask(), !in);
+#else
+  return in;
+#endif
 }
 
 // x y, x + y, x - y: on the FP64 pipe, products by a Soft64 on the integer pipe.
@@ -562,7 +574,8 @@ HYP_HD void flux64(const K& k, double alpha, const Cell64& c, const double* m, c
 template <int kDef, bool kUnit, bool kFlux, bool kSoft>
 HYP_HD bool cell_try64(const EosC& e, const Eos64& k, double alpha, const double* m, double rE, const double* R,
                        double* f, double& u1, double& cm, int& st) {
-  if (kSoft && !(soft_inputs64(m, 3) & soft_inputs64(&rE, 1) & soft_inputs64(R, 9) & (kUnit || soft_inputs64(&alpha, 1))))
+  if (kSoft && !warp_holds(soft_inputs64(m, 3) & soft_inputs64(&rE, 1) & soft_inputs64(R, 9) &
+                           (kUnit || soft_inputs64(&alpha, 1))))
     return false;
   const typename std::conditional<kSoft, Soft64, Plain64>::type s(k);
   const Cell64 c = cell64<kDef, kUnit>(e, s, kUnit ? 1.0 : rcp64(k, alpha), m, rE, R);
