@@ -43,10 +43,10 @@
 //    65536 cells x 10 steps 7.10 -> 6.51 ms, two phases of 1000 cells x 50 steps 2.25 -> 2.17
 //    ms, 65536 cells x 50 steps forward and back 9.55 -> 8.69 ms.
 //
-// Per cell 183 FP64 instructions as executed (106 with the lone products on the integer
-// pipe, soft_mul64), where the forms of hyp_physics.cuh
-// (which the adjoint and the function-level evaluators use) execute 379; the two agree
-// to a few ulps (tests/test_cell64_host.py).
+// Per cell 183 FP64 instructions as executed (106 to 110 with the lone products on the
+// integer pipe, soft_mul64), where the forms of hyp_physics.cuh (which the function-level
+// evaluators use, and these forms where wave speeds are close) execute 379; the two agree to
+// a few ulps (tests/test_cell64_host.py).
 #pragma once
 #include <type_traits>
 #include <string.h>

@@ -15,7 +15,7 @@ constexpr int kBlock64 = 128;
 // Grids of more blocks than this, one a multiprocessor, take the lone products of a cell
 // pass on the integer pipe (hyp_cell64.cuh): the two pipes overlap where a scheduler has
 // warps to choose from, so those kernels keep to 128 registers and four blocks resident
-// (1,000,003 cells x 10 steps: 4.53 ms, with two, three, five 5.19, 4.71, 4.68, and 5.48
+// (1,000,003 cells x 10 steps: 4.53 ms, 4.49 now; with two, three, five 5.19, 4.71, 4.68, and 5.48
 // with all products on the FP64 pipe). 50 steps of 20,000 cells (158 blocks) 1.05 -> 1.01 ms, of
 // 38,000 1.18 -> 1.13, of 70,000 1.99 -> 1.64; two phases (64 cells a block), 20 HLL steps of
 // 9,700 cells (152 blocks) 1.02 -> 1.10 ms, of 14,000 1.15 on either pipe, of 38,000 1.57 ->
