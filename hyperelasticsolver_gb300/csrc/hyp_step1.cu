@@ -154,8 +154,10 @@ __device__ __forceinline__ void run1_finish(const Run1Args& a, double t, int s) 
 // the maximum. The arithmetic is that of cell1_pass and step1_f64_kernel, in the same
 // order. 1000 cells x 100
 // steps 1.39 -> 1.26 ms (1.19 since all operators are FMAs; now run1_split_f64_kernel's size), 8192 cells x 4 steps on device buffers 111 -> 80 us.
+// One block a multiprocessor may have all its registers (201; held to 168 it spills: 15,000
+// cells x 50 steps 608 -> 596 us).
 template <int kDef>
-__global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
+__global__ void __launch_bounds__(kBlock64, 1) run1_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
   __shared__ double sh[kEdge][kBlock64 + 1];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
   __shared__ double sF[14][kBlock64];         // twice the left face of cell i0 + j
   __shared__ double s_hdt, s_t;
@@ -258,12 +260,13 @@ __global__ void __launch_bounds__(kBlock64) run1_f64_kernel(Run1Args a, EosC e, 
 // The state lives in shared memory. The arithmetic is the same, instruction by instruction.
 // Whole runs, one thread a cell and two: 1000 cells x 100 steps 1.22 -> 0.99 ms, 8192 cells x 4
 // steps on device buffers 81 -> 73 us, 50 steps of 64 to 9576 cells 0.61 to 0.77 -> 0.51 to
-// 0.65 ms.
+// 0.65 ms. With 211 registers instead of 168 (one block a multiprocessor) 1000 cells x 100 steps
+// 941 -> 920 us.
 constexpr int kSplitSlots = 64, kSplitCells = kSplitSlots - 1;
 constexpr int kGram = sizeof(Gram64) / sizeof(double), kCellShared = 8;
 
 template <int kDef>
-__global__ void __launch_bounds__(2 * kSplitSlots) run1_split_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
+__global__ void __launch_bounds__(2 * kSplitSlots, 1) run1_split_f64_kernel(Run1Args a, EosC e, Eos64 kc) {
   __shared__ double sh[kEdge][kSplitSlots + 2];  // slot j + 1: cell i0 + j; slot 0 and the last: the halo
   __shared__ double sF[14][kSplitSlots];         // twice the left face of cell i0 + j
   __shared__ double sG[kGram][kSplitSlots], sC[kCellShared][kSplitSlots];
